@@ -1,33 +1,30 @@
 // Weight-streaming frozen-linear forward for few tokens (decode shapes).
 //
-//   y[m, out] = x[m, in] . W_deq[out, in]^T      m <= 16, x bf16, y fp32/bf16/fp16
+//   y[m, out] = x[m, in] . W_deq[out, in]^T  (+ residual)     m <= 16, x bf16, y fp32/bf16/fp16
 //
 // The call is bound by reading the packed codes once from HBM
 // (CAIF_DeviceFrozenLinear::ForwardImpl, src/caif_device_frozen_linear.cpp:381-524,
 // does the same product after writing and re-reading an fp32 copy of the whole
 // weight, :319-334).  Design:
-//   * one persistent CTA per SM owns a contiguous range of rows of the
-//     [out, in] code matrix, i.e. one contiguous slab of HBM, cut into items of
-//     16 rows (the M of the tensor-core instruction);
-//   * the slab streams through a shared-memory ring of three items with bulk
-//     async copies (cp.async.bulk + mbarrier transaction counts), started before
-//     the kernel waits for the previous kernel in the stream (programmatic
-//     dependent launch): the frozen codes never depend on earlier work;
-//   * 16 warps split the reduction dimension; each lane pulls 16 bytes of codes
-//     of rows g and g+8 from the ring, turns nibbles/bytes into exact bf16
-//     integers with logic ops (no int->float converts), and feeds them as the A
-//     operand of bf16 tensor-core MMAs against token fragments (B operand) that
-//     stay in registers for the whole kernel;
-//   * int4 group scales multiply the fp32 partial sum once per 128-element
-//     chunk; the int8 per-tensor scale multiplies the final sum;
-//   * the warps never synchronise with each other in the main loop: each parks
-//     its partial sums of every item (live tokens only) in shared memory, and
-//     one pass at the end adds the 16 partials of each output in a fixed order
-//     and stores four rows (or, for 9 to 16 tokens, one row of four tokens) per
-//     thread.
-// After the previous kernel has completed the launch is bound by the logic ops
-// of the dequantization (two cycles per warp instruction on this GPU, seven of
-// them per eight int4 weights), not by HBM: see the design notes of the package.
+//   * one CTA per SM owns a contiguous range of rows of the [out, in] code matrix,
+//     cut into tiles of 16 rows (the M of the tensor-core instruction).  Copies of
+//     the frozen codes and scales never depend on earlier work and start before the
+//     kernel waits for the previous one in the stream (programmatic dependent launch);
+//   * the warps split the reduction dimension; a warp copies its own pieces of a
+//     tile into its own ring (cp.async, 16 bytes a lane) and every lane reads back
+//     exactly what it copied, so the main loop has no barrier and no shared
+//     address arithmetic;
+//   * a lane turns nibbles/bytes of rows g and g+8 into exact bf16 integers with
+//     logic ops (no int->float converts), and feeds them as the A operand of bf16
+//     tensor-core MMAs against token fragments (B operand) in registers.  Rows too
+//     long for the registers are taken in segments of the reduction dimension,
+//     one after the other over all tiles of the CTA;
+//   * int4 group scales (copied to shared memory ahead of the previous kernel's
+//     end) multiply the fp32 partial sum once per 128-element chunk; the int8
+//     per-tensor scale multiplies the final sum;
+//   * each warp parks its partial sums of every tile (live tokens only) in shared
+//     memory, and one pass at the end adds the warps' partials of each output in a
+//     fixed order; consecutive lanes store consecutive rows of a token.
 // Codes and activations are exact in bf16 and products accumulate in fp32, so
 // the result matches an fp32 GEMM on the dequantized weight up to summation
 // order.  The summation order of an output does not depend on which CTA owns
@@ -62,13 +59,10 @@ int take_decode_timeout_flag()
 namespace
 {
 
-constexpr int kItemRows = 16;                    // weight rows per work item (the MMA's M)
+constexpr int kTileRows = 16;                    // weight rows per tile (the MMA's M)
 constexpr int kRowQuantum = 8;                   // CTA row ranges start on multiples of this
-constexpr int kMaxStages = 8;
-constexpr int kWarps = 16;                       // 4 per scheduler: the 128-register budget holds
-constexpr int kThreads = kWarps * 32;
-constexpr int kRingDepth = 3;                    // items in flight per SM
-constexpr uint32_t kSmemBudget = 220u * 1024u;   // dynamic shared memory of the one CTA per SM
+constexpr uint32_t kSmemFull = 220u * 1024u;     // dynamic shared memory of a CTA that takes the SM alone
+constexpr uint32_t kSmemHalf = 112u * 1024u;     // ... of one that leaves room for the next launch's CTA
 constexpr uint32_t kSpinLimit = 1u << 22;        // polls of one wait before it gives up (tens of ms)
 constexpr uint32_t kSpinLimitTest = 1u << 12;    // the same for the self-test of the give-up path
 
@@ -88,11 +82,6 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes)
                : "memory");
 }
 
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
-{
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
 __device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity)
 {
   uint32_t done;
@@ -106,31 +95,19 @@ __device__ __forceinline__ bool mbar_try(uint32_t addr, uint32_t parity)
   return done != 0;
 }
 
-// Bounded wait, called by all lanes of a warp.  Gives up after `limit` polls, or as soon as
-// another warp of the CTA has given up, and says so: a copy that never lands turns into a
-// flag and missing outputs instead of a hung GPU.  The answer is the same in every lane.
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32_t limit, volatile uint32_t *abort_word)
+// Bounded wait: a copy that never lands turns into a flag and missing outputs instead of a hung GPU.
+__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, uint32_t limit)
 {
   const uint32_t addr = smem_u32(bar);
-  bool done = mbar_try(addr, parity);
-  if (!done)
+  for (uint32_t spin = 0; spin < limit; ++spin)
   {
-    for (uint32_t spin = 0; spin < limit && !done; ++spin)
+    if (mbar_try(addr, parity))
     {
-      done = mbar_try(addr, parity);
-      if (!done && (spin & 255u) == 255u && *abort_word != 0u)
-      {
-        break;
-      }
+      return true;
     }
   }
-  done = __all_sync(0xFFFFFFFFu, done);
-  if (!done)
-  {
-    *abort_word = 1u;
-    atomicExch(&g_decode_timeout_flag, 1u);
-  }
-  return done;
+  atomicExch(&g_decode_timeout_flag, 1u);
+  return false;
 }
 
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint64_t *bar)
@@ -140,15 +117,42 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t
                : "memory");
 }
 
-// D(16x8, fp32) += A(16x16, bf16, row) * B(16x8, bf16, col).  Not volatile: a
-// pure function of its operands, so the compiler may interleave independent
-// accumulation chains.
-__device__ __forceinline__ void mma_bf16_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
-                                               uint32_t b0, uint32_t b1)
+// D(16x8, fp32) = A(16x16, bf16, row) * B(16x8, bf16, col) + C.  Not volatile: a pure function of its operands, so
+// the compiler may interleave independent accumulation chains.  C apart from D: a chain starts from values that
+// are kept (or from zero) without copying them first.
+__device__ __forceinline__ void mma_bf16_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3,
+                                               uint32_t b0, uint32_t b1, const float *c)
 {
-  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
+}
+
+// 16 bytes of global memory into shared memory
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void *src)
+{
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+
+template <int N>
+__device__ __forceinline__ void cp_async_wait()
+{
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+// activations are the previous kernel's output: never moved ahead of the wait on that kernel; zeros where not `live`
+__device__ __forceinline__ void ldg128(const void *p, bool live, uint32_t &a, uint32_t &b, uint32_t &c, uint32_t &d)
+{
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.u32 q, %5, 0;\n\t"
+      "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
+      "@q ld.global.v4.u32 {%0,%1,%2,%3}, [%4];\n\t}"
+      : "=&r"(a), "=&r"(b), "=&r"(c), "=&r"(d)
+      : "l"(p), "r"(live ? 1u : 0u)
+      : "memory");
 }
 
 __device__ __forceinline__ uint32_t sub_bf16x2(uint32_t a, uint32_t b)
@@ -173,7 +177,7 @@ __device__ __forceinline__ uint32_t lop3_and_xor(uint32_t a, uint32_t b, uint32_
 }
 
 // Explicit shared-space accesses with 32-bit addresses.  Volatile keeps them in
-// program order after the (volatile) barrier wait that guards the data.
+// program order after the (volatile) wait that guards the data.
 __device__ __forceinline__ uint4 lds128(uint32_t addr)
 {
   uint4 v;
@@ -188,10 +192,10 @@ __device__ __forceinline__ float lds_half(uint32_t addr)
   return __half2float(__ushort_as_half(h));
 }
 
-__device__ __forceinline__ float lds_f32(uint32_t addr)
+__device__ __forceinline__ float2 lds_f32x2(uint32_t addr)
 {
-  float v;
-  asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  float2 v;
+  asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
   return v;
 }
 
@@ -217,45 +221,66 @@ struct DecodeParams
   int64_t y_ld;           // row pitch of the result, in elements
   int64_t y_col0;         // first column this launch writes
   int y_dtype;
+  int accumulate;         // y = round_y(round_y(product) + y)
   int m;
   int in_dim;
   int out_dim;
   int groups_per_row;     // int4: in_dim / group_size
   int chunks_per_group;   // int4: group_size / 128
+  int num_chunks;         // 64-byte pieces of a row
+  int num_ksegs;          // passes over the CTA's rows, NCH pieces a warp each
   int num_quanta;         // ceil(out / 8)
-  int stages;
-  int vec4;               // fp32 results may be stored four rows at a time (16-byte aligned on every buffer)
   int tokp;               // tokens per parked row: m rounded up to 2, 4, 8 or 16
-  int park_items;         // items whose partial sums fit the parking area: the CTA reduces and stores that often
-  uint32_t partial_offset; // byte offset of the parked partial sums in dynamic shared memory
-  uint32_t row_bytes;      // packed bytes per weight row
-  uint32_t row_stride;     // row pitch in the ring
-  uint32_t stage_bytes;    // ring stage pitch
-  uint32_t spin_limit;     // polls of one wait before it gives up
-  uint32_t stall_bytes;    // self-test only: bytes the first item announces but never receives
+  int round_tiles;        // tiles whose partial sums fit the parking area: the CTA reduces and stores that often
+  uint32_t scale_offset;  // byte offset of the scales in dynamic shared memory
+  uint32_t scale_bytes;   // int4: one buffer of them (round_tiles tiles); two buffers when there are several rounds
+  uint32_t park_offset;   // byte offset of the parked partial sums
+  uint32_t row_bytes;     // packed bytes per weight row
+  uint32_t spin_limit;    // polls of one wait before it gives up
+  uint32_t stall_bytes;   // self-test only: bytes the first wait announces but never receives
 };
 
 // int4 codes are turned into the bf16 integers 136 + q (q in [-8,7]): the
 // nibble, flipped to offset binary, is dropped into the mantissa of 128.0.  The
 // constant is taken out again by starting each accumulator at -136 * (sum of x
 // over the same 128 elements), so no subtract runs per weight.
-constexpr float kInt4Offset = 136.0f;
+constexpr uint32_t kMinus136x2 = 0xC308C308u;
 
-// BITS: 4 or 8.  MT: token tiles of 8 (1 -> m <= 8, 2 -> m <= 16).
-// NCH: chunks (64 bytes of one row: a quad of lanes x 16 bytes) per warp.
-template <int BITS, int MT, int NCH>
-__global__ void __launch_bounds__(kThreads, 1) linear_decode_kernel(const __grid_constant__ DecodeParams p)
+// WARPS: 8 or 16.  BITS: 4 or 8.  MT: token tiles of 8 (1 -> m <= 8, 2 -> m <= 16).
+// NCH: chunks (64 bytes of one row: a quad of lanes x 16 bytes) per warp and pass; PCH of them per ring slot.
+// Shared memory per CTA: the rings (8 KB a warp; 6 with two token tiles, whose parked sums take more), the
+// scales, the parked sums.
+template <int WARPS, int BITS, int MT, int NCH, int PCH>
+struct DecodeCfg
 {
+  static constexpr int THREADS = WARPS * 32;
+  static constexpr int CTAS_PER_SM = WARPS == 8 ? 2 : 1;
+  // a multiple of the slots of a tile
+  static constexpr int DEPTH = (MT == 2 && NCH / PCH == 1) ? 6 / PCH : 8 / PCH;
+  static constexpr uint32_t SLOT_BYTES = PCH * 2u * 512u;
+  static constexpr uint32_t WARP_RING = DEPTH * SLOT_BYTES;
+};
+
+// parked sums of one warp and tile: [16 rows][tokp], groups of four tokens of a row swapped so that the 16-byte
+// reads of the reduction, eight rows at a time, fall into different banks
+__device__ __forceinline__ uint32_t park_swizzle(int row, int tokp)
+{
+  return tokp == 16 ? static_cast<uint32_t>((row >> 1) & 3) : (tokp == 8 ? static_cast<uint32_t>((row >> 2) & 1) : 0u);
+}
+
+template <int WARPS, int BITS, int MT, int NCH, int PCH>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_kernel(const __grid_constant__ DecodeParams p)
+{
+  typedef DecodeCfg<WARPS, BITS, MT, NCH, PCH> Cfg;
   constexpr int ELEMS = 128 / BITS;      // codes per 16-byte load: 32 or 16
   constexpr int CHUNK_K = 4 * ELEMS;     // k covered by a quad of lanes: 128 or 64
   constexpr int XR = ELEMS / 2;          // bf16x2 registers of x per chunk and token tile: 16 or 8
-  constexpr int WARPS = kWarps;
+  constexpr int NSLAB = NCH / PCH;       // ring slots per tile and pass
   constexpr int CHAINS = (MT == 1) ? 2 : 1;   // accumulation chains per token tile
+  static_assert(NCH % PCH == 0, "whole slots");
 
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ uint64_t full_bar[kMaxStages];   // a stage's copies have landed
-  __shared__ uint64_t empty_bar[kMaxStages];  // all warps are done reading a stage
-  __shared__ uint32_t cta_abort;              // a wait of this CTA has run out
+  __shared__ uint64_t scale_bar[2];   // a round's scales have landed
 
   const int tid = threadIdx.x;
   const int warp = tid >> 5;
@@ -267,476 +292,487 @@ __global__ void __launch_bounds__(kThreads, 1) linear_decode_kernel(const __grid
   const int q_end = static_cast<int>((static_cast<int64_t>(blockIdx.x + 1) * p.num_quanta) / gridDim.x);
   const int row_begin = q_begin * kRowQuantum;
   const int row_end = min(q_end * kRowQuantum, p.out_dim);
-  const int my_items = (row_end - row_begin + kItemRows - 1) / kItemRows;
-  const int num_chunks = p.in_dim / CHUNK_K;
-  const int stages = p.stages;
+  const int my_tiles = (row_end - row_begin + kTileRows - 1) / kTileRows;
   const uint32_t smem_base = smem_u32(smem);
-  const uint32_t part_base = smem_base + p.partial_offset;
-  volatile uint32_t *abort_word = &cta_abort;
+  const uint32_t ring = smem_base + static_cast<uint32_t>(warp) * Cfg::WARP_RING + static_cast<uint32_t>(lane) * 16u;
 
-  // One thread starts the copies of an item: its rows are contiguous in memory, so one bulk copy
-  // brings the codes and a second one the scales.
-  auto issue = [&](int item, int s)
+  // The copies run DEPTH slots ahead of the compute loop, in its order: rounds, passes over k, tiles, slots.  Rows past
+  // the CTA's last one are read as that one (their sums are never stored), pieces past the row's end not at all
+  // (their activations are zero).
+  int f_round = 0;   // first tile of the round being fetched
+  int f_tile = 0;
+  int f_kseg = 0;
+  const uint8_t *f_lo;   // this lane's first piece of row g, and of row g + 8, of the tile
+  const uint8_t *f_hi;
+  auto row_ptr = [&](int row)
   {
-    const int row0 = row_begin + item * kItemRows;
-    const int rows = min(kItemRows, row_end - row0);
-    const uint32_t stage = smem_base + static_cast<uint32_t>(s) * p.stage_bytes;
-    const uint32_t code_bytes = static_cast<uint32_t>(rows) * p.row_bytes;
-    const uint32_t scale_bytes = (BITS == 4) ? static_cast<uint32_t>(rows * p.groups_per_row * 2) : 0u;
-    mbar_expect_tx(&full_bar[s], code_bytes + scale_bytes + (item == 0 ? p.stall_bytes : 0u));
-    if (p.num_seg == 1)
-    {
-      bulk_g2s(stage, p.codes[0] + static_cast<size_t>(row0) * p.row_bytes, code_bytes, &full_bar[s]);
-      if (BITS == 4)
-      {
-        const uint8_t *src = static_cast<const uint8_t *>(p.scales[0]) + static_cast<size_t>(row0) * p.groups_per_row * 2;
-        bulk_g2s(stage + static_cast<uint32_t>(kItemRows) * p.row_stride, src, scale_bytes, &full_bar[s]);
-      }
-      return;
-    }
-    // an item that straddles two code matrices takes one pair of copies from each
-    int row = row0;
-    while (row < row0 + rows)
+    row = min(row, row_end - 1);
+    const uint8_t *base = p.codes[0];
+    if (p.num_seg > 1)
     {
       int sg = 0;
       while (sg + 1 < p.num_seg && row >= p.seg_row0[sg + 1])
       {
         ++sg;
       }
-      const int n = min(row0 + rows, p.seg_row0[sg + 1]) - row;
-      const size_t local = static_cast<size_t>(row - p.seg_row0[sg]);
-      const uint32_t done_rows = static_cast<uint32_t>(row - row0);
-      bulk_g2s(stage + done_rows * p.row_bytes, p.codes[sg] + local * p.row_bytes, static_cast<uint32_t>(n) * p.row_bytes,
-               &full_bar[s]);
-      if (BITS == 4)
+      base = p.codes[sg];
+      row -= p.seg_row0[sg];
+    }
+    return base + static_cast<size_t>(row) * p.row_bytes + static_cast<uint32_t>((f_kseg * NCH * WARPS + warp) * 64 + t * 16);
+  };
+  auto fetch_rows = [&]()
+  {
+    const int row = row_begin + f_tile * kTileRows + g;
+    f_lo = row_ptr(row);
+    f_hi = row_ptr(row + 8);
+  };
+  auto fetch = [&](int slab, uint32_t dst)
+  {
+    if (f_round < my_tiles)
+    {
+      const int pieces = p.num_chunks - f_kseg * (NCH * WARPS) - warp;
+#pragma unroll
+      for (int j = 0; j < PCH; ++j)
       {
-        const uint32_t per_row = static_cast<uint32_t>(p.groups_per_row) * 2u;
-        const uint8_t *src = static_cast<const uint8_t *>(p.scales[sg]) + local * per_row;
-        bulk_g2s(stage + static_cast<uint32_t>(kItemRows) * p.row_stride + done_rows * per_row, src,
-                 static_cast<uint32_t>(n) * per_row, &full_bar[s]);
+        const int off = (slab * PCH + j) * WARPS;
+        if (off < pieces)
+        {
+          cp_async16(dst + j * 1024u, f_lo + off * 64);
+          cp_async16(dst + j * 1024u + 512u, f_hi + off * 64);
+        }
       }
-      row += n;
+      if (slab == NSLAB - 1)
+      {
+        if (++f_tile == min(f_round + p.round_tiles, my_tiles))
+        {
+          if (++f_kseg == p.num_ksegs)
+          {
+            f_kseg = 0;
+            f_round = f_tile;
+          }
+          f_tile = f_round;
+        }
+        fetch_rows();
+      }
+    }
+    cp_async_commit();
+  };
+  // One thread copies a round's scales: contiguous in memory, one copy per code matrix the rows touch.
+  auto fetch_scales = [&](int round, int first_tile)
+  {
+    uint64_t *bar = &scale_bar[round & 1];
+    const int row0 = row_begin + first_tile * kTileRows;
+    const int row1 = min(row_end, row0 + p.round_tiles * kTileRows);
+    const uint32_t per_row = (BITS == 4) ? static_cast<uint32_t>(p.groups_per_row) * 2u : 0u;
+    mbar_expect_tx(bar, static_cast<uint32_t>(row1 - row0) * per_row + (round == 0 ? p.stall_bytes : 0u));
+    if (BITS == 4)
+    {
+      uint32_t dst = smem_base + p.scale_offset + static_cast<uint32_t>(round & 1) * p.scale_bytes;
+      for (int row = row0; row < row1;)
+      {
+        int sg = 0;
+        while (sg + 1 < p.num_seg && row >= p.seg_row0[sg + 1])
+        {
+          ++sg;
+        }
+        const int n = min(row1, p.seg_row0[sg + 1]) - row;
+        const uint8_t *src = static_cast<const uint8_t *>(p.scales[sg]) + static_cast<size_t>(row - p.seg_row0[sg]) * per_row;
+        bulk_g2s(dst, src, static_cast<uint32_t>(n) * per_row, bar);
+        dst += static_cast<uint32_t>(n) * per_row;
+        row += n;
+      }
     }
   };
 
+  // The frozen codes and scales never depend on earlier work in the stream: their copies start before the wait on
+  // the previous kernel.  The next kernel in the stream may place its CTAs as soon as this grid's CTAs have all
+  // come this far (programmatic dependent launch).
+  fetch_rows();
+#pragma unroll
+  for (int i = 0; i < Cfg::DEPTH; ++i)
+  {
+    fetch(i % NSLAB, ring + static_cast<uint32_t>(i) * Cfg::SLOT_BYTES);
+  }
   if (tid == 0)
   {
-    cta_abort = 0u;
-    for (int s = 0; s < stages; ++s)
-    {
-      mbar_init(&full_bar[s], 1);
-      mbar_init(&empty_bar[s], WARPS);
-    }
+    mbar_init(&scale_bar[0], 1);
+    mbar_init(&scale_bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  // The frozen codes and scales never depend on earlier work in the stream: the ring starts before
-  // the wait on the previous kernel.  The next kernel in the stream may place its CTAs as soon as
-  // this grid's CTAs have all come this far (programmatic dependent launch).
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // Warp 0 is the only producer; it knows how many items it has started (needed if it gives up).
-  int issued_items = min(stages, my_items);
-  if (tid == 0)
-  {
-    for (int i = 0; i < issued_items; ++i)
+    fetch_scales(0, 0);
+    if (p.round_tiles < my_tiles)
     {
-      issue(i, i);
+      fetch_scales(1, p.round_tiles);
     }
   }
-
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // Activations and the output are touched only after the previous kernel has completed.
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
-  // Token fragments (B operand), resident for the whole kernel.  For the 16
-  // bytes of codes a lane reads at k-offset kb, the register order pairs the
-  // elements the way the logic-op dequantization emits them:
+  // Token fragments (B operand) of one pass over k.  For the 16 bytes of codes a lane reads, the register order
+  // pairs the elements the way the logic-op dequantization emits them:
   //   int4, word wi: (8wi+0, 8wi+4) (8wi+2, 8wi+6) (8wi+1, 8wi+5) (8wi+3, 8wi+7)
   //   int8, word wi: (4wi+0, 4wi+2) (4wi+1, 4wi+3)
   uint32_t xf[NCH][MT][XR];
-  float sx[NCH][MT][2];     // int4: -136 * (sum of x over the chunk's 128 elements), tokens 2t and 2t+1 of tile mt
-  uint32_t code_off[NCH];   // byte offset of this lane's 16 bytes of row g inside a stage
-  uint32_t scale_off[NCH];  // byte offset of row g's scale for the chunk inside a stage
-#pragma unroll
-  for (int ch = 0; ch < NCH; ++ch)
+  float sx[NCH][MT][4];     // int4: -136 * (sum of x over the chunk's 128 elements) as an accumulator fragment
+  uint32_t scale_off[NCH];  // byte offset of row g's scale for the chunk inside a tile's scales
+  auto load_x = [&](int kseg)
   {
-    const int cidx = warp + ch * WARPS;
-    code_off[ch] = static_cast<uint32_t>(g) * p.row_stride + static_cast<uint32_t>(cidx) * 64u + static_cast<uint32_t>(t) * 16u;
-    scale_off[ch] = static_cast<uint32_t>(kItemRows) * p.row_stride +
-                    static_cast<uint32_t>(g * p.groups_per_row + cidx / p.chunks_per_group) * 2u;
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-    {
-      const int token = g + 8 * mt;
-      const bool live = (cidx < num_chunks) && (token < p.m);
-      uint32_t raw[XR];
-      if (live)
-      {
-        const uint4 *src =
-            reinterpret_cast<const uint4 *>(p.x + static_cast<size_t>(token) * p.in_dim + cidx * CHUNK_K + t * ELEMS);
-#pragma unroll
-        for (int i = 0; i < XR / 4; ++i)
-        {
-          const uint4 v = __ldg(src + i);
-          raw[4 * i + 0] = v.x;
-          raw[4 * i + 1] = v.y;
-          raw[4 * i + 2] = v.z;
-          raw[4 * i + 3] = v.w;
-        }
-      }
-      else
-      {
-#pragma unroll
-        for (int i = 0; i < XR; ++i)
-        {
-          raw[i] = 0u;
-        }
-      }
-      if (BITS == 4)
-      {
-#pragma unroll
-        for (int wi = 0; wi < 4; ++wi)
-        {
-          xf[ch][mt][4 * wi + 0] = __byte_perm(raw[4 * wi + 0], raw[4 * wi + 2], 0x5410);
-          xf[ch][mt][4 * wi + 1] = __byte_perm(raw[4 * wi + 1], raw[4 * wi + 3], 0x5410);
-          xf[ch][mt][4 * wi + 2] = __byte_perm(raw[4 * wi + 0], raw[4 * wi + 2], 0x7632);
-          xf[ch][mt][4 * wi + 3] = __byte_perm(raw[4 * wi + 1], raw[4 * wi + 3], 0x7632);
-        }
-        {
-          float lane_sum = 0.0f;
-#pragma unroll
-          for (int i = 0; i < XR; ++i)
-          {
-            lane_sum += __uint_as_float(raw[i] << 16) + __uint_as_float(raw[i] & 0xFFFF0000u);
-          }
-          lane_sum += __shfl_xor_sync(0xFFFFFFFFu, lane_sum, 1);
-          lane_sum += __shfl_xor_sync(0xFFFFFFFFu, lane_sum, 2);
-          sx[ch][mt][0] = -kInt4Offset * __shfl_sync(0xFFFFFFFFu, lane_sum, (2 * t) * 4);
-          sx[ch][mt][1] = -kInt4Offset * __shfl_sync(0xFFFFFFFFu, lane_sum, (2 * t + 1) * 4);
-        }
-      }
-      else
-      {
-        sx[ch][mt][0] = 0.0f;
-        sx[ch][mt][1] = 0.0f;
-#pragma unroll
-        for (int wi = 0; wi < 4; ++wi)
-        {
-          xf[ch][mt][2 * wi + 0] = __byte_perm(raw[2 * wi + 0], raw[2 * wi + 1], 0x5410);
-          xf[ch][mt][2 * wi + 1] = __byte_perm(raw[2 * wi + 0], raw[2 * wi + 1], 0x7632);
-        }
-      }
-    }
-  }
-  const uint32_t row8_off = 8u * p.row_stride;
-  const uint32_t scale8_off = static_cast<uint32_t>(8 * p.groups_per_row) * 2u;
-  // parked partial sums: [item][warp][row][token], tokens fastest and only the live ones (tokp of
-  // them): a lane's two tokens of a row are one 8-byte store.  With 16 tokens the groups of four
-  // tokens of a row are stored in an order that depends on the row (quad ^ ((row >> 1) & 3)), so that
-  // the 16-byte reads of the final reduction, eight rows at a time, fall into different banks.
-  const uint32_t part_warp_bytes = static_cast<uint32_t>(kItemRows * p.tokp) * 4u;
-  const uint32_t part_item_bytes = WARPS * part_warp_bytes;
-  uint32_t part_write_off[MT];
-#pragma unroll
-  for (int mt = 0; mt < MT; ++mt)
-  {
-    if (MT == 2)
-    {
-      const int quad = ((t >> 1) + 2 * mt) ^ ((g >> 1) & 3);
-      part_write_off[mt] = static_cast<uint32_t>(warp) * part_warp_bytes +
-                           static_cast<uint32_t>(g * 16 + 4 * quad + 2 * (t & 1)) * 4u;
-    }
-    else
-    {
-      part_write_off[mt] =
-          static_cast<uint32_t>(warp) * part_warp_bytes + static_cast<uint32_t>(g * p.tokp + 2 * t) * 4u;
-    }
-  }
-  // int8: the per-tensor scale of every segment; an output row takes the one of its segment
-  float seg_scale[kMaxSegments];
-#pragma unroll
-  for (int sg = 0; sg < kMaxSegments; ++sg)
-  {
-    seg_scale[sg] = 1.0f;
-    if (BITS == 8 && sg < p.num_seg && p.scales[sg] != nullptr)
-    {
-      seg_scale[sg] = static_cast<const float *>(p.scales[sg])[0];
-    }
-  }
-  auto tensor_scale_of = [&](int row)
-  {
-    float v = seg_scale[0];
-#pragma unroll
-    for (int sg = 1; sg < kMaxSegments; ++sg)
-    {
-      if (sg < p.num_seg && row >= p.seg_row0[sg])
-      {
-        v = seg_scale[sg];
-      }
-    }
-    return v;
-  };
-  int s = 0;             // ring stage of the current item
-  uint32_t s_par = 0;    // its phase parity
-  bool ok = true;
-  // Rounds: the parking area holds the partial sums of park_items items (all of a CTA's items for the
-  // usual layer sizes, so one round); after each round the CTA adds them up and stores the outputs.
-  for (int round_begin = 0; round_begin < my_items; round_begin += p.park_items)
-  {
-  const int round_end = min(round_begin + p.park_items, my_items);
-  for (int it = round_begin; it < round_end; ++it)
-  {
-    ok = mbar_wait(&full_bar[s], s_par, p.spin_limit, abort_word);
-    if (!ok)
-    {
-      break;
-    }
-    const uint32_t stage_addr = smem_base + static_cast<uint32_t>(s) * p.stage_bytes;
-    // yacc[mt][0..1]: row g, tokens 2t, 2t+1 of tile mt;  [2..3]: row g+8
-    float yacc[MT][4];
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-    {
-      yacc[mt][0] = yacc[mt][1] = yacc[mt][2] = yacc[mt][3] = 0.0f;
-    }
-
-    // all shared-memory reads of the item first, so the stage can be released early and the
-    // MMAs of different chunks overlap
-    uint32_t wlo_all[NCH][4];
-    uint32_t whi_all[NCH][4];
-    float s_lo_all[NCH];
-    float s_hi_all[NCH];
+    // all loads first: one round trip
 #pragma unroll
     for (int ch = 0; ch < NCH; ++ch)
     {
-      s_lo_all[ch] = 0.0f;
-      s_hi_all[ch] = 0.0f;
-      if (warp + ch * WARPS < num_chunks)
-      {
-        const uint4 lo = lds128(stage_addr + code_off[ch]);
-        const uint4 hi = lds128(stage_addr + code_off[ch] + row8_off);
-        wlo_all[ch][0] = lo.x;
-        wlo_all[ch][1] = lo.y;
-        wlo_all[ch][2] = lo.z;
-        wlo_all[ch][3] = lo.w;
-        whi_all[ch][0] = hi.x;
-        whi_all[ch][1] = hi.y;
-        whi_all[ch][2] = hi.z;
-        whi_all[ch][3] = hi.w;
-        if (BITS == 4)
-        {
-          s_lo_all[ch] = lds_half(stage_addr + scale_off[ch]);
-          s_hi_all[ch] = lds_half(stage_addr + scale_off[ch] + scale8_off);
-        }
-      }
-    }
-    // every read of the stage has been issued: count this warp out
-    __syncwarp();
-    if (lane == 0)
-    {
-      mbar_arrive(&empty_bar[s]);
-    }
-#pragma unroll
-    for (int ch = 0; ch < NCH; ++ch)
-    {
-      const uint32_t(&wlo)[4] = wlo_all[ch];
-      const uint32_t(&whi)[4] = whi_all[ch];
-      const float s_lo = s_lo_all[ch];
-      const float s_hi = s_hi_all[ch];
-      if (warp + ch * WARPS < num_chunks)
-      {
-        float c[CHAINS][MT][4];
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-        {
-          c[0][mt][0] = c[0][mt][2] = (BITS == 4) ? sx[ch][mt][0] : 0.0f;  // -136 * sum(x): ends as sum(x * q)
-          c[0][mt][1] = c[0][mt][3] = (BITS == 4) ? sx[ch][mt][1] : 0.0f;
-          if (CHAINS == 2)
-          {
-            c[CHAINS - 1][mt][0] = c[CHAINS - 1][mt][1] = c[CHAINS - 1][mt][2] = c[CHAINS - 1][mt][3] = 0.0f;
-          }
-        }
-#pragma unroll
-        for (int wi = 0; wi < 4; ++wi)
-        {
-          if (BITS == 4)
-          {
-            uint32_t a_lo[4];
-            uint32_t a_hi[4];
-            {
-              const uint32_t ev = lop3_and_xor(wlo[wi], 0x0F0F0F0Fu, 0x08080808u);
-              const uint32_t od = lop3_and_xor(wlo[wi] >> 4, 0x0F0F0F0Fu, 0x08080808u);
-              a_lo[0] = __byte_perm(ev, 0x43434343u, 0x4240);
-              a_lo[1] = __byte_perm(ev, 0x43434343u, 0x4341);
-              a_lo[2] = __byte_perm(od, 0x43434343u, 0x4240);
-              a_lo[3] = __byte_perm(od, 0x43434343u, 0x4341);
-            }
-            {
-              const uint32_t ev = lop3_and_xor(whi[wi], 0x0F0F0F0Fu, 0x08080808u);
-              const uint32_t od = lop3_and_xor(whi[wi] >> 4, 0x0F0F0F0Fu, 0x08080808u);
-              a_hi[0] = __byte_perm(ev, 0x43434343u, 0x4240);
-              a_hi[1] = __byte_perm(ev, 0x43434343u, 0x4341);
-              a_hi[2] = __byte_perm(od, 0x43434343u, 0x4240);
-              a_hi[3] = __byte_perm(od, 0x43434343u, 0x4341);
-            }
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-            {
-              const int j = 2 * wi + h;  // k-step: pairs 2j, 2j+1
-#pragma unroll
-              for (int mt = 0; mt < MT; ++mt)
-              {
-                mma_bf16_16816(c[h % CHAINS][mt], a_lo[2 * h], a_hi[2 * h], a_lo[2 * h + 1], a_hi[2 * h + 1],
-                               xf[ch][mt][2 * j], xf[ch][mt][2 * j + 1]);
-              }
-            }
-          }
-          else
-          {
-            uint32_t a_lo[2];
-            uint32_t a_hi[2];
-#pragma unroll
-            for (int sh = 0; sh < 2; ++sh)
-            {
-              const uint32_t sel = sh ? 0x4341u : 0x4240u;
-              const uint32_t pl = __byte_perm(wlo[wi], 0u, sel);
-              const uint32_t ph = __byte_perm(whi[wi], 0u, sel);
-              a_lo[sh] = sub_bf16x2(lop3_and_or(pl, 0x007F007Fu, 0x43004300u), lop3_and_or(pl, 0x00800080u, 0x43004300u));
-              a_hi[sh] = sub_bf16x2(lop3_and_or(ph, 0x007F007Fu, 0x43004300u), lop3_and_or(ph, 0x00800080u, 0x43004300u));
-            }
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
-            {
-              mma_bf16_16816(c[wi % CHAINS][mt], a_lo[0], a_hi[0], a_lo[1], a_hi[1], xf[ch][mt][2 * wi],
-                             xf[ch][mt][2 * wi + 1]);
-            }
-          }
-        }
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-        {
-          float sum[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-          {
-            sum[i] = (CHAINS == 2) ? (c[0][mt][i] + c[CHAINS - 1][mt][i]) : c[0][mt][i];
-          }
-          if (BITS == 4)
-          {
-            // the chunk lies inside one scale group of rows g and g+8; scaling per
-            // 128-element chunk equals scaling per group up to rounding order
-            yacc[mt][0] = fmaf(s_lo, sum[0], yacc[mt][0]);
-            yacc[mt][1] = fmaf(s_lo, sum[1], yacc[mt][1]);
-            yacc[mt][2] = fmaf(s_hi, sum[2], yacc[mt][2]);
-            yacc[mt][3] = fmaf(s_hi, sum[3], yacc[mt][3]);
-          }
-          else
-          {
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-            {
-              yacc[mt][i] += sum[i];
-            }
-          }
-        }
-      }
-    }
-    // park this warp's partial sums of the item; nobody reads them before the end of the kernel
-    {
-      const uint32_t d0 = part_base + static_cast<uint32_t>(it - round_begin) * part_item_bytes;
+      const int c = (kseg * NCH + ch) * WARPS + warp;
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt)
       {
-        if (MT == 2 || 2 * t < p.tokp)
-        {
-          const uint32_t d = d0 + part_write_off[mt];
-          sts_f32x2(d, yacc[mt][0], yacc[mt][1]);                                        // row g,   tokens 2t, 2t+1
-          sts_f32x2(d + static_cast<uint32_t>(8 * p.tokp) * 4u, yacc[mt][2], yacc[mt][3]);  // row g+8
-        }
-      }
-    }
-    // warp 0 refills this item's stage once all warps have read it (they read it at the top of the
-    // iteration, so by now this rarely waits)
-    if (warp == 0 && it + stages < my_items)
-    {
-      ok = mbar_wait(&empty_bar[s], s_par, p.spin_limit, abort_word);
-      if (!ok)
-      {
-        break;
-      }
-      if (lane == 0)
-      {
-        issue(it + stages, s);
-      }
-      issued_items = it + stages + 1;
-    }
-
-    if (++s == stages)
-    {
-      s = 0;
-      s_par ^= 1u;
-    }
-  }
-  __syncthreads();
-  if (*abort_word != 0u)
-  {
-    // A wait ran out somewhere in the CTA; the outputs stay unwritten and the host sees the flag.
-    // Before the CTA gives its shared memory back, every copy that was started into the ring must
-    // have landed (a copy must not arrive in memory that already belongs to another CTA).  Warp 0
-    // started them all and waits for them; these waits are bounded too.
-    if (warp == 0)
-    {
-      for (int st = 0; st < stages && st < issued_items; ++st)
-      {
-        // the last item started into this stage; once it has landed the earlier ones have too
-        const int j = issued_items - 1 - ((issued_items - 1 - st) % stages);
-        const uint32_t addr = smem_u32(&full_bar[st]);
-        const uint32_t parity = static_cast<uint32_t>(j / stages) & 1u;
-        bool done = false;
-        for (uint32_t spin = 0; spin < p.spin_limit && !done; ++spin)
-        {
-          done = mbar_try(addr, parity);
-        }
-      }
-    }
-    return;
-  }
-
-  // Cross-warp reduction: an output is the sum of its WARPS partial sums in warp order.
-  if (MT == 2)
-  {
-    // a thread takes four tokens of one row; consecutive lanes take consecutive rows, so the stores
-    // of a token are contiguous across the warp
-    const int n = (round_end - round_begin) * 64;
-    for (int o = tid; o < n; o += WARPS * 32)
-    {
-      const int r16 = o & 15;
-      const int tq = (o >> 4) & 3;
-      const int item = o >> 6;
-      const int quad = tq ^ ((r16 >> 1) & 3);
-      const uint32_t src = part_base + static_cast<uint32_t>(item) * part_item_bytes +
-                           static_cast<uint32_t>(r16 * 16 + 4 * quad) * 4u;
-      float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        const int token = g + 8 * mt;
+        const bool live = c < p.num_chunks && token < p.m;
+        const __nv_bfloat16 *src = p.x + static_cast<size_t>(token) * p.in_dim + c * CHUNK_K + t * ELEMS;
 #pragma unroll
-      for (int w = 0; w < WARPS; ++w)
-      {
-        const uint4 v = lds128(src + static_cast<uint32_t>(w) * part_warp_bytes);
-        acc[0] += __uint_as_float(v.x);
-        acc[1] += __uint_as_float(v.y);
-        acc[2] += __uint_as_float(v.z);
-        acc[3] += __uint_as_float(v.w);
+        for (int i = 0; i < XR / 4; ++i)
+        {
+          ldg128(src + 8 * i, live, xf[ch][mt][4 * i], xf[ch][mt][4 * i + 1], xf[ch][mt][4 * i + 2], xf[ch][mt][4 * i + 3]);
+        }
       }
-      const int row = row_begin + (round_begin + item) * kItemRows + r16;
-      if (row < row_end)
+    }
+#pragma unroll
+    for (int ch = 0; ch < NCH; ++ch)
+    {
+      const int c = (kseg * NCH + ch) * WARPS + warp;
+      scale_off[ch] = (BITS == 4 && c < p.num_chunks)
+                          ? static_cast<uint32_t>(g * p.groups_per_row + c / p.chunks_per_group) * 2u
+                          : 0u;
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
       {
-        const float tensor_scale = (BITS == 8) ? tensor_scale_of(row) : 1.0f;
+        uint32_t(&f)[XR] = xf[ch][mt];
+#pragma unroll
+        for (int wi = 0; wi < 4; ++wi)
+        {
+          if (BITS == 4)
+          {
+            const uint32_t r0 = f[(4 * wi + 0) % XR], r1 = f[(4 * wi + 1) % XR], r2 = f[(4 * wi + 2) % XR],
+                           r3 = f[(4 * wi + 3) % XR];
+            f[(4 * wi + 0) % XR] = __byte_perm(r0, r2, 0x5410);
+            f[(4 * wi + 1) % XR] = __byte_perm(r1, r3, 0x5410);
+            f[(4 * wi + 2) % XR] = __byte_perm(r0, r2, 0x7632);
+            f[(4 * wi + 3) % XR] = __byte_perm(r1, r3, 0x7632);
+          }
+          else
+          {
+            const uint32_t r0 = f[2 * wi], r1 = f[2 * wi + 1];
+            f[2 * wi] = __byte_perm(r0, r1, 0x5410);
+            f[2 * wi + 1] = __byte_perm(r0, r1, 0x7632);
+          }
+        }
+        // the sums come from the tensor core too: the accumulators of weight rows whose codes are all -136
+        float c0[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (BITS == 4)
+        {
+          float c1[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+          for (int j = 0; j < XR / 2; j += 2)
+          {
+            mma_bf16_16816(c0, kMinus136x2, kMinus136x2, kMinus136x2, kMinus136x2, f[2 * j], f[2 * j + 1], c0);
+            mma_bf16_16816(c1, kMinus136x2, kMinus136x2, kMinus136x2, kMinus136x2, f[2 * j + 2], f[2 * j + 3], c1);
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+          {
+            c0[i] += c1[i];
+          }
+        }
 #pragma unroll
         for (int i = 0; i < 4; ++i)
         {
-          const int token = 4 * tq + i;
-          if (token < p.m)
+          sx[ch][mt][i] = c0[i];
+        }
+      }
+    }
+  };
+
+  const uint32_t scale8_off = static_cast<uint32_t>(8 * p.groups_per_row) * 2u;
+  const uint32_t tile_scale_bytes = 2u * scale8_off;
+  const uint32_t park_warp_bytes = static_cast<uint32_t>(kTileRows * p.tokp) * 4u;
+  const uint32_t park_tile_bytes = WARPS * park_warp_bytes;
+  const uint32_t park_base = smem_base + p.park_offset;
+  // a lane's two tokens of a row are one 8-byte store (row g + 8 has the swizzle of row g)
+  uint32_t park_off[MT];
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt)
+  {
+    const uint32_t quad = static_cast<uint32_t>((t >> 1) + 2 * mt) ^ park_swizzle(g, p.tokp);
+    park_off[mt] = static_cast<uint32_t>(warp) * park_warp_bytes +
+                   (static_cast<uint32_t>(g * p.tokp) + 4u * quad + 2u * static_cast<uint32_t>(t & 1)) * 4u;
+  }
+  // int8: an output row takes the per-tensor scale of its segment
+  auto tensor_scale_of = [&](int row)
+  {
+    int sg = 0;
+    while (sg + 1 < p.num_seg && row >= p.seg_row0[sg + 1])
+    {
+      ++sg;
+    }
+    return p.scales[sg] != nullptr ? __ldg(static_cast<const float *>(p.scales[sg])) : 1.0f;
+  };
+
+  const float zero4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  uint32_t slot = 0;   // byte offset in the ring
+  int round = 0;
+  for (int round_begin = 0; round_begin < my_tiles; round_begin += p.round_tiles, ++round)
+  {
+    const int round_end = min(round_begin + p.round_tiles, my_tiles);
+    const uint32_t scale_base = smem_base + p.scale_offset + static_cast<uint32_t>(round & 1) * p.scale_bytes;
+    for (int kseg = 0; kseg < p.num_ksegs; ++kseg)
+    {
+      if (round == 0 || p.num_ksegs > 1)
+      {
+        load_x(kseg);
+      }
+      if (kseg == 0)
+      {
+        if (round == 0)
+        {
+          __syncthreads();   // the barriers are initialised
+        }
+        const bool landed = mbar_wait(&scale_bar[round & 1], static_cast<uint32_t>(round >> 1) & 1u, p.spin_limit);
+        if (__syncthreads_or(landed ? 0 : 1))
+        {
+          // A wait ran out; the outputs stay unwritten and the host sees the flag.  Copies that were started must
+          // land before the shared memory belongs to another CTA.
+          cp_async_wait<0>();
+          for (int i = 0; i < 64; ++i)
           {
-            const float v = (BITS == 8) ? acc[i] * tensor_scale : acc[i];
-            const int64_t idx = static_cast<int64_t>(token) * p.y_ld + p.y_col0 + row;
+            __nanosleep(2000);
+          }
+          return;
+        }
+      }
+      for (int tile = round_begin; tile < round_end; ++tile)
+      {
+        const uint32_t tile_scales = scale_base + static_cast<uint32_t>(tile - round_begin) * tile_scale_bytes;
+        // yacc[mt][0..1]: row g, tokens 2t, 2t+1 of tile mt;  [2..3]: row g+8
+        float yacc[MT][4];
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+        {
+          yacc[mt][0] = yacc[mt][1] = yacc[mt][2] = yacc[mt][3] = 0.0f;
+        }
+#pragma unroll
+        for (int slab = 0; slab < NSLAB; ++slab)
+        {
+          cp_async_wait<Cfg::DEPTH - 1>();
+          const uint32_t src = ring + slot;
+#pragma unroll
+          for (int j = 0; j < PCH; ++j)
+          {
+            const int ch = slab * PCH + j;
+            {
+              const uint4 lo = lds128(src + j * 1024u);
+              const uint4 hi = lds128(src + j * 1024u + 512u);
+              const uint32_t wlo[4] = {lo.x, lo.y, lo.z, lo.w};
+              const uint32_t whi[4] = {hi.x, hi.y, hi.z, hi.w};
+              float s_lo = 0.0f;
+              float s_hi = 0.0f;
+              if (BITS == 4)
+              {
+                s_lo = lds_half(tile_scales + scale_off[ch]);
+                s_hi = lds_half(tile_scales + scale_off[ch] + scale8_off);
+              }
+              float c[CHAINS][MT][4];
+#pragma unroll
+              for (int wi = 0; wi < 4; ++wi)
+              {
+                if (BITS == 4)
+                {
+                  uint32_t a_lo[4];
+                  uint32_t a_hi[4];
+                  {
+                    const uint32_t ev = lop3_and_xor(wlo[wi], 0x0F0F0F0Fu, 0x08080808u);
+                    const uint32_t od = lop3_and_xor(wlo[wi] >> 4, 0x0F0F0F0Fu, 0x08080808u);
+                    a_lo[0] = __byte_perm(ev, 0x43434343u, 0x4240);
+                    a_lo[1] = __byte_perm(ev, 0x43434343u, 0x4341);
+                    a_lo[2] = __byte_perm(od, 0x43434343u, 0x4240);
+                    a_lo[3] = __byte_perm(od, 0x43434343u, 0x4341);
+                  }
+                  {
+                    const uint32_t ev = lop3_and_xor(whi[wi], 0x0F0F0F0Fu, 0x08080808u);
+                    const uint32_t od = lop3_and_xor(whi[wi] >> 4, 0x0F0F0F0Fu, 0x08080808u);
+                    a_hi[0] = __byte_perm(ev, 0x43434343u, 0x4240);
+                    a_hi[1] = __byte_perm(ev, 0x43434343u, 0x4341);
+                    a_hi[2] = __byte_perm(od, 0x43434343u, 0x4240);
+                    a_hi[3] = __byte_perm(od, 0x43434343u, 0x4341);
+                  }
+#pragma unroll
+                  for (int h = 0; h < 2; ++h)
+                  {
+                    const int jj = 2 * wi + h;  // k-step: pairs 2jj, 2jj+1
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt)
+                    {
+                      mma_bf16_16816(c[h % CHAINS][mt], a_lo[2 * h], a_hi[2 * h], a_lo[2 * h + 1], a_hi[2 * h + 1],
+                                     xf[ch][mt][2 * jj], xf[ch][mt][2 * jj + 1],
+                                     jj == 0 ? sx[ch][mt] : (jj < CHAINS ? zero4 : c[h % CHAINS][mt]));
+                    }
+                  }
+                }
+                else
+                {
+                  uint32_t a_lo[2];
+                  uint32_t a_hi[2];
+#pragma unroll
+                  for (int sh = 0; sh < 2; ++sh)
+                  {
+                    const uint32_t sel = sh ? 0x4341u : 0x4240u;
+                    const uint32_t pl = __byte_perm(wlo[wi], 0u, sel);
+                    const uint32_t ph = __byte_perm(whi[wi], 0u, sel);
+                    a_lo[sh] =
+                        sub_bf16x2(lop3_and_or(pl, 0x007F007Fu, 0x43004300u), lop3_and_or(pl, 0x00800080u, 0x43004300u));
+                    a_hi[sh] =
+                        sub_bf16x2(lop3_and_or(ph, 0x007F007Fu, 0x43004300u), lop3_and_or(ph, 0x00800080u, 0x43004300u));
+                  }
+#pragma unroll
+                  for (int mt = 0; mt < MT; ++mt)
+                  {
+                    mma_bf16_16816(c[wi % CHAINS][mt], a_lo[0], a_hi[0], a_lo[1], a_hi[1], xf[ch][mt][2 * wi],
+                                   xf[ch][mt][2 * wi + 1], wi < CHAINS ? zero4 : c[wi % CHAINS][mt]);
+                  }
+                }
+              }
+#pragma unroll
+              for (int mt = 0; mt < MT; ++mt)
+              {
+                float sum[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                {
+                  sum[i] = (CHAINS == 2) ? (c[0][mt][i] + c[CHAINS - 1][mt][i]) : c[0][mt][i];
+                }
+                if (BITS == 4)
+                {
+                  // the chunk lies inside one scale group of rows g and g+8; scaling per
+                  // 128-element chunk equals scaling per group up to rounding order
+                  yacc[mt][0] = fmaf(s_lo, sum[0], yacc[mt][0]);
+                  yacc[mt][1] = fmaf(s_lo, sum[1], yacc[mt][1]);
+                  yacc[mt][2] = fmaf(s_hi, sum[2], yacc[mt][2]);
+                  yacc[mt][3] = fmaf(s_hi, sum[3], yacc[mt][3]);
+                }
+                else
+                {
+#pragma unroll
+                  for (int i = 0; i < 4; ++i)
+                  {
+                    yacc[mt][i] += sum[i];
+                  }
+                }
+              }
+            }
+          }
+          // the slot's contents are in registers (the MMAs above consumed them): refill it
+          fetch(slab, src);
+          slot = (slot + Cfg::SLOT_BYTES == Cfg::WARP_RING) ? 0u : slot + Cfg::SLOT_BYTES;
+        }
+        // park this warp's partial sums of the tile; nobody else reads them before the end of the round
+        const uint32_t d0 = park_base + static_cast<uint32_t>(tile - round_begin) * park_tile_bytes;
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+        {
+          if (MT == 2 || 2 * t < p.tokp)
+          {
+            const uint32_t d = d0 + park_off[mt];
+            const uint32_t d8 = d + static_cast<uint32_t>(8 * p.tokp) * 4u;
+            if (kseg > 0)
+            {
+              const float2 o = lds_f32x2(d);
+              const float2 o8 = lds_f32x2(d8);
+              yacc[mt][0] += o.x;
+              yacc[mt][1] += o.y;
+              yacc[mt][2] += o8.x;
+              yacc[mt][3] += o8.y;
+            }
+            sts_f32x2(d, yacc[mt][0], yacc[mt][1]);    // row g,   tokens 2t, 2t+1
+            sts_f32x2(d8, yacc[mt][2], yacc[mt][3]);   // row g+8
+          }
+        }
+      }
+    }
+    __syncthreads();
+    if (tid == 0 && round_end + p.round_tiles < my_tiles)
+    {
+      fetch_scales(round + 2, round_end + p.round_tiles);
+    }
+
+    // Cross-warp reduction: an output is the sum of its warps' partial sums in warp order.  A thread takes up to
+    // four tokens of one row; consecutive lanes take consecutive rows, so a token's stores are contiguous across
+    // the warp.  With peers the plain stores travel over NVLink and are complete when the kernel is.
+    const int rows = (round_end - round_begin) * kTileRows;
+    const int live_rows = min(rows, row_end - row_begin - round_begin * kTileRows);
+    const int quads = (p.m + 3) >> 2;
+    for (int tq = tid >> 7; tq < quads; tq += (WARPS * 32) / 128)
+    {
+      for (int local = tid & 127; local < live_rows; local += 128)
+      {
+        const int r16 = local & 15;
+        const uint32_t src = park_base + static_cast<uint32_t>(local >> 4) * park_tile_bytes +
+                             (static_cast<uint32_t>(r16 * p.tokp) +
+                              4u * (static_cast<uint32_t>(tq) ^ park_swizzle(r16, p.tokp))) * 4u;
+        float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+        if (p.tokp > 2)
+        {
+#pragma unroll
+          for (int w = 0; w < WARPS; ++w)
+          {
+            const uint4 v = lds128(src + static_cast<uint32_t>(w) * park_warp_bytes);
+            acc[0] += __uint_as_float(v.x);
+            acc[1] += __uint_as_float(v.y);
+            acc[2] += __uint_as_float(v.z);
+            acc[3] += __uint_as_float(v.w);
+          }
+        }
+        else
+        {
+#pragma unroll
+          for (int w = 0; w < WARPS; ++w)
+          {
+            const float2 v = lds_f32x2(src + static_cast<uint32_t>(w) * park_warp_bytes);
+            acc[0] += v.x;
+            acc[1] += v.y;
+          }
+        }
+        const int row = row_begin + round_begin * kTileRows + local;
+        if (BITS == 8)
+        {
+          const float tensor_scale = tensor_scale_of(row);
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+          {
+            acc[i] *= tensor_scale;
+          }
+        }
+        const int live = min(4, p.m - 4 * tq);
+        int64_t idx = static_cast<int64_t>(4 * tq) * p.y_ld + p.y_col0 + row;
+        if (p.y_dtype == CAIFQ_F32 && !p.accumulate && p.num_y == 1)
+        {
+          float *dst = static_cast<float *>(p.y[0]) + idx;
+#pragma unroll
+          for (int i = 0; i < 4; ++i, dst += p.y_ld)
+          {
+            if (i < live)
+            {
+              *dst = acc[i];
+            }
+          }
+        }
+        else
+        {
+#pragma unroll 1
+          for (int i = 0; i < live; ++i, idx += p.y_ld)
+          {
+            float v = i == 0 ? acc[0] : (i == 1 ? acc[1] : (i == 2 ? acc[2] : acc[3]));
+            if (p.accumulate)
+            {
+              v = round_through_rt(v, p.y_dtype) + load_as_float(p.y[0], idx, p.y_dtype);
+            }
             for (int r = 0; r < p.num_y; ++r)
             {
               store_from_float(p.y[r], idx, p.y_dtype, v);
@@ -745,69 +781,10 @@ __global__ void __launch_bounds__(kThreads, 1) linear_decode_kernel(const __grid
         }
       }
     }
-  }
-  else
-  {
-    // a thread takes four consecutive rows of one live token
-    const int quads = (round_end - round_begin) * 4 * p.m;
-    for (int o = tid; o < quads; o += WARPS * 32)
+    if (round_end < my_tiles)
     {
-      const int rq = o & 3;
-      const int token = (o >> 2) % p.m;
-      const int item = (o >> 2) / p.m;
-      const uint32_t src = part_base + static_cast<uint32_t>(item) * part_item_bytes +
-                           static_cast<uint32_t>((4 * rq) * p.tokp + token) * 4u;
-      float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll
-      for (int w = 0; w < WARPS; ++w)
-      {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-        {
-          acc[i] += lds_f32(src + static_cast<uint32_t>(w) * part_warp_bytes + static_cast<uint32_t>(i * p.tokp) * 4u);
-        }
-      }
-      const int row = row_begin + (round_begin + item) * kItemRows + 4 * rq;
-      if (BITS == 8)
-      {
-        // (four rows that start on a multiple of four lie in one segment: segments start on multiples of 8)
-        const float tensor_scale = tensor_scale_of(row);
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-        {
-          acc[i] *= tensor_scale;
-        }
-      }
-      // plain stores; with peers they travel over NVLink and are complete when the kernel is
-      const int64_t idx = static_cast<int64_t>(token) * p.y_ld + p.y_col0 + row;
-      if (p.vec4 && row + 3 < row_end)
-      {
-        const float4 v = make_float4(acc[0], acc[1], acc[2], acc[3]);
-        for (int r = 0; r < p.num_y; ++r)
-        {
-          *reinterpret_cast<float4 *>(static_cast<float *>(p.y[r]) + idx) = v;
-        }
-      }
-      else
-      {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-        {
-          if (row + i < row_end)
-          {
-            for (int r = 0; r < p.num_y; ++r)
-            {
-              store_from_float(p.y[r], idx + i, p.y_dtype, acc[i]);
-            }
-          }
-        }
-      }
+      __syncthreads();   // the parking area is free for the next round
     }
-  }
-  if (round_end < my_items)
-  {
-    __syncthreads();   // the parking area is free for the next round
-  }
   }  // rounds
 }
 
@@ -859,10 +836,10 @@ void decode_stall_next_launch() { t_stall_next = true; }
 namespace
 {
 
-template <int BITS, int MT, int NCH>
+template <int WARPS, int BITS, int MT, int NCH, int PCH>
 int launch_decode_inst(const DecodeParams &p, uint32_t smem, cudaStream_t s)
 {
-  auto kernel = linear_decode_kernel<BITS, MT, NCH>;
+  auto kernel = linear_decode_kernel<WARPS, BITS, MT, NCH, PCH>;
   static std::atomic<bool> configured[kMaxDevices];
   int dev = 0;
   CAIFQ_CHECK_CUDA(cudaGetDevice(&dev));
@@ -874,7 +851,7 @@ int launch_decode_inst(const DecodeParams &p, uint32_t smem, cudaStream_t s)
   if (!configured[dev].load(std::memory_order_acquire))
   {
     CAIFQ_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          static_cast<int>(kSmemBudget)));
+                                          static_cast<int>(kSmemFull)));
     configured[dev].store(true, std::memory_order_release);
   }
   int grid = sm_count();
@@ -888,7 +865,7 @@ int launch_decode_inst(const DecodeParams &p, uint32_t smem, cudaStream_t s)
   }();
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
-  cfg.blockDim = dim3(kThreads);
+  cfg.blockDim = dim3(WARPS * 32);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[1];
@@ -903,32 +880,42 @@ int launch_decode_inst(const DecodeParams &p, uint32_t smem, cudaStream_t s)
   return CAIFQ_OK;
 }
 
-int chunks_per_warp(const caifq_weight &w)
-{
-  const int chunk_k = (w.storage == CAIFQ_I4) ? 128 : 64;
-  const int chunks = w.in_dim / chunk_k;
-  return (chunks + kWarps - 1) / kWarps;
-}
-
 int tokp_for(int64_t m) { return m <= 2 ? 2 : (m <= 4 ? 4 : (m <= 8 ? 8 : 16)); }
 
 struct Layout
 {
-  uint32_t stage_bytes;
-  uint32_t partial_bytes;
-  int stages;
-  int park_items;
+  int warps;
+  int nch;
+  uint32_t scale_offset;
+  uint32_t scale_bytes;
+  uint32_t park_offset;
+  uint32_t smem_bytes;   // 0: a tile does not fit
+  int round_tiles;
 };
 
 Layout layout_for(const caifq_weight &w, int64_t m)
 {
   Layout l{};
   const bool i4 = (w.storage == CAIFQ_I4);
-  const uint32_t row_bytes = i4 ? static_cast<uint32_t>(w.in_dim / 2) : static_cast<uint32_t>(w.in_dim);
-  const uint32_t scale_bytes = i4 ? static_cast<uint32_t>(kItemRows * (w.in_dim / w.group_size) * 2) : 0u;
-  l.stage_bytes = ((kItemRows * row_bytes + scale_bytes) + 127u) & ~127u;
-  // parked partial sums: [item][warp][16 rows][tokp] for as many of a CTA's items as fit beside
-  // the ring (all of them for the usual layer sizes)
+  const int mt = (m > 8) ? 2 : 1;
+  const int num_chunks = w.in_dim / (i4 ? 128 : 64);
+  // Short rows (up to 1 KB of codes) keep few warps busy and their launches are short: eight warps on half an SM,
+  // so that the next launch's CTA sits beside this one with its copies done (1024 -> 1024, m = 1: 2.4 us a launch
+  // against 2.7).  Longer rows, and two token tiles, want the 16 warps: the launch is bound by the dequantization's
+  // instructions and their latencies, not by its start (4096 -> 14336, m = 1: 10.4 us, 11.4 with eight, 11.6 with 32).
+  l.warps = (num_chunks <= 16 && mt == 1) ? 8 : 16;
+  // Chunks a warp holds token fragments of at a time: as many as 64 registers take (a lane needs 16 of them per
+  // int4 chunk and token tile, 8 per int8 chunk), no more than the row has.
+  const int most = (i4 ? 4 : 8) / mt;
+  l.nch = 1;
+  while (l.nch < most && l.nch * l.warps < num_chunks)
+  {
+    l.nch *= 2;
+  }
+  const bool deep = !(mt == 2 && l.nch <= 2);
+  const uint32_t ring = static_cast<uint32_t>(l.warps) * (deep ? 8u : 6u) * 1024u;   // WARPS * DecodeCfg::WARP_RING
+  const uint32_t scales = i4 ? static_cast<uint32_t>(kTileRows * (w.in_dim / w.group_size) * 2) : 0u;
+  const uint32_t park = static_cast<uint32_t>(l.warps * kTileRows * tokp_for(m) * sizeof(float));
   const int quanta = (w.out_dim + kRowQuantum - 1) / kRowQuantum;
   int grid = sm_count();
   if (grid > quanta)
@@ -936,33 +923,30 @@ Layout layout_for(const caifq_weight &w, int64_t m)
     grid = quanta;
   }
   const int max_quanta = (quanta + grid - 1) / grid;
-  const int max_items = (max_quanta * kRowQuantum + kItemRows - 1) / kItemRows;
-  const uint32_t per_item = static_cast<uint32_t>(kWarps * kItemRows * tokp_for(m) * sizeof(float));
-  int stages = kRingDepth;
-  // Three items in flight per SM are enough to cover the latency of HBM.  More of them make the
-  // launch slower, not faster (measured on B200: 10.8 us per launch with three, 11.3 with four,
-  // 12.8 with six at in=4096, out=14336): every SM then asks for its whole share at once and the
-  // first item of each lands later.
-  while (stages > 2 && static_cast<uint32_t>(stages) * l.stage_bytes + per_item > kSmemBudget)
+  const int max_tiles = (max_quanta * kRowQuantum + kTileRows - 1) / kTileRows;
+  // all of a CTA's tiles in one round if they fit, else in several equal rounds
+  const uint32_t budget = l.warps == 8 ? kSmemHalf : kSmemFull;
+  auto align128 = [](uint32_t v) { return (v + 127u) & ~127u; };
+  auto bytes = [&](int tiles, int buffers)
+  { return ring + static_cast<uint32_t>(buffers) * align128(static_cast<uint32_t>(tiles) * scales) +
+           static_cast<uint32_t>(tiles) * park; };
+  int rounds = 1;
+  int tiles = max_tiles;
+  while (tiles > 1 && bytes(tiles, rounds > 1 ? 2 : 1) > budget)
   {
-    --stages;
+    ++rounds;
+    tiles = (max_tiles + rounds - 1) / rounds;
   }
-  if (static_cast<uint32_t>(stages) * l.stage_bytes + per_item > kSmemBudget)
+  const int buffers = (tiles < max_tiles) ? 2 : 1;
+  if (bytes(tiles, buffers) > kSmemFull)
   {
-    stages = 0;   // a row too long for two stages and one parked item
+    return l;
   }
-  int park = max_items;
-  if (stages > 0)
-  {
-    const int fit = static_cast<int>((kSmemBudget - static_cast<uint32_t>(stages) * l.stage_bytes) / per_item);
-    if (park > fit)
-    {
-      park = fit;
-    }
-  }
-  l.park_items = park;
-  l.partial_bytes = static_cast<uint32_t>(park) * per_item;
-  l.stages = stages;
+  l.round_tiles = tiles;
+  l.scale_offset = ring;
+  l.scale_bytes = align128(static_cast<uint32_t>(tiles) * scales);
+  l.park_offset = ring + static_cast<uint32_t>(buffers) * l.scale_bytes;
+  l.smem_bytes = bytes(tiles, buffers);
   return l;
 }
 
@@ -1004,7 +988,7 @@ bool decode_supported(const LinearArgs &args)
   const int64_t m = args.m;
   const int y_dtype = args.c_dtype;
   const int compute_dtype = args.compute_dtype;
-  if (args.backward || args.accumulate || args.a_prescale != 1.0f)
+  if (args.backward || args.a_prescale != 1.0f || (args.accumulate && args.num_peers > 0))
   {
     return false;
   }
@@ -1048,18 +1032,8 @@ bool decode_supported(const LinearArgs &args)
   {
     return false;
   }
-  {
-    // the token fragments of a warp's chunks must fit 64 registers
-    const int nch = chunks_per_warp(w);
-    const int xr = (w.storage == CAIFQ_I4) ? 16 : 8;
-    const int mt = (m > 8) ? 2 : 1;
-    if (nch * xr * mt > 64 || nch > 8)
-    {
-      return false;
-    }
-  }
-  // at least two ring stages must fit beside the parked partial sums
-  if (layout_for(w, m).stages < 2)
+  // a tile's scales and parked sums must fit beside the rings
+  if (layout_for(w, m).smem_bytes == 0)
   {
     return false;
   }
@@ -1122,15 +1096,7 @@ int launch_linear_decode(const LinearArgs &args, cudaStream_t s)
     p.y_col0 = 0;
   }
   p.y_dtype = y_dtype;
-  // four rows of one token as one 16-byte store: fp32 results whose rows of four start aligned
-  p.vec4 = (y_dtype == CAIFQ_F32 && (p.y_ld % 4) == 0 && (p.y_col0 % 4) == 0) ? 1 : 0;
-  for (int r = 0; r < p.num_y; ++r)
-  {
-    if ((reinterpret_cast<uintptr_t>(p.y[r]) & 15u) != 0)
-    {
-      p.vec4 = 0;
-    }
-  }
+  p.accumulate = args.accumulate ? 1 : 0;
   p.m = static_cast<int>(m);
   p.tokp = tokp_for(m);
   p.in_dim = w.in_dim;
@@ -1138,9 +1104,6 @@ int launch_linear_decode(const LinearArgs &args, cudaStream_t s)
   p.num_quanta = (w.out_dim + kRowQuantum - 1) / kRowQuantum;
   const bool i4 = (w.storage == CAIFQ_I4);
   p.row_bytes = i4 ? static_cast<uint32_t>(w.in_dim / 2) : static_cast<uint32_t>(w.in_dim);
-  // rows lie unpadded, as in memory, so one bulk copy fills a stage; the 2-way
-  // bank conflict on the four 16-byte reads per item is noise
-  p.row_stride = p.row_bytes;
   if (i4)
   {
     p.groups_per_row = w.in_dim / w.group_size;
@@ -1151,58 +1114,53 @@ int launch_linear_decode(const LinearArgs &args, cudaStream_t s)
     p.groups_per_row = 0;
     p.chunks_per_group = 1;
   }
+  p.num_chunks = w.in_dim / (i4 ? 128 : 64);
   const Layout lay = layout_for(w, m);
-  int stages = lay.stages;
-  if (const char *e = std::getenv("CAIFQ_DECODE_STAGES"))
+  if (lay.smem_bytes == 0)
   {
-    const int v = std::atoi(e);
-    if (v >= 2 && v < stages)
-    {
-      stages = v;
-    }
-  }
-  if (stages < 2)
-  {
-    set_error("frozen linear (decode): row too long for the shared-memory ring");
+    set_error("frozen linear (decode): row too long for the shared memory");
     return CAIFQ_ERR_UNSUPPORTED;
   }
-  p.stage_bytes = lay.stage_bytes;
-  p.stages = stages;
-  p.park_items = lay.park_items;
-  p.partial_offset = static_cast<uint32_t>(stages) * p.stage_bytes;
-  const uint32_t smem_bytes = p.partial_offset + lay.partial_bytes;
+  p.num_ksegs = (p.num_chunks + lay.nch * lay.warps - 1) / (lay.nch * lay.warps);
+  p.round_tiles = lay.round_tiles;
+  p.scale_offset = lay.scale_offset;
+  p.scale_bytes = lay.scale_bytes;
+  p.park_offset = lay.park_offset;
   p.spin_limit = kSpinLimit;
   p.stall_bytes = 0;
   if (t_stall_next)
   {
-    // self-test of the give-up path: the first item announces 16 bytes that never arrive
+    // self-test of the give-up path: the scales' wait announces 16 bytes that never arrive
     t_stall_next = false;
     p.spin_limit = kSpinLimitTest;
     p.stall_bytes = 16;
   }
 
-  const int nch = chunks_per_warp(w);
   const int mt = (m > 8) ? 2 : 1;
-#define CAIFQ_DECODE_CASE(B, M, N)                          \
-  if (nch <= N && mt == M)                                  \
-  {                                                         \
-    return launch_decode_inst<B, M, N>(p, smem_bytes, s);   \
+#define CAIFQ_DECODE_CASE(W, B, M, N)                                                      \
+  if (lay.warps == W && lay.nch == N && mt == M)                                           \
+  {                                                                                        \
+    return launch_decode_inst<W, B, M, N, (N > 1 ? 2 : 1)>(p, lay.smem_bytes, s);          \
   }
   if (i4)
   {
-    CAIFQ_DECODE_CASE(4, 1, 1)
-    CAIFQ_DECODE_CASE(4, 1, 2)
-    CAIFQ_DECODE_CASE(4, 1, 4)
-    CAIFQ_DECODE_CASE(4, 2, 1)
-    CAIFQ_DECODE_CASE(4, 2, 2)
+    CAIFQ_DECODE_CASE(8, 4, 1, 1)
+    CAIFQ_DECODE_CASE(8, 4, 1, 2)
+    CAIFQ_DECODE_CASE(16, 4, 1, 2)
+    CAIFQ_DECODE_CASE(16, 4, 1, 4)
+    CAIFQ_DECODE_CASE(16, 4, 2, 1)
+    CAIFQ_DECODE_CASE(16, 4, 2, 2)
   }
   else
   {
-    CAIFQ_DECODE_CASE(8, 1, 2)
-    CAIFQ_DECODE_CASE(8, 1, 4)
-    CAIFQ_DECODE_CASE(8, 1, 8)
-    CAIFQ_DECODE_CASE(8, 2, 2)
-    CAIFQ_DECODE_CASE(8, 2, 4)
+    CAIFQ_DECODE_CASE(8, 8, 1, 1)
+    CAIFQ_DECODE_CASE(8, 8, 1, 2)
+    CAIFQ_DECODE_CASE(16, 8, 1, 2)
+    CAIFQ_DECODE_CASE(16, 8, 1, 4)
+    CAIFQ_DECODE_CASE(16, 8, 1, 8)
+    CAIFQ_DECODE_CASE(16, 8, 2, 1)
+    CAIFQ_DECODE_CASE(16, 8, 2, 2)
+    CAIFQ_DECODE_CASE(16, 8, 2, 4)
   }
 #undef CAIFQ_DECODE_CASE
   set_error("frozen linear (decode): no kernel instance for in_dim=%d m=%lld", w.in_dim, static_cast<long long>(m));

@@ -163,6 +163,31 @@ def test_decode_shapes(storage, in_dim, out_dim, m, group):
     assert max_rel_err(y.cpu().numpy(), orc.frozen_linear_forward(x_np, wc)) <= TOL_F32
 
 
+@pytest.mark.parametrize("storage,in_dim,out_dim,m,sd", [
+    (orc.I4, 14336, 136, 5, orc.BF16),   # several passes over k, the last one partial
+    (orc.I4, 14336, 1000, 16, orc.F32),
+    (orc.I8, 14336, 72, 1, orc.BF16),
+    (orc.I8, 9280, 264, 16, orc.BF16),   # 145 chunks
+    (orc.I4, 8320, 9000, 9, orc.F32),    # passes over k and several rounds of parked sums
+    (orc.I4, 2048, 24, 8, orc.F16),      # eight-warp form, fewer rows than SMs
+])
+def test_decode_long_rows_and_the_residual_add(storage, in_dim, out_dim, m, sd):
+    rng = np.random.default_rng(in_dim + out_dim + m)
+    weight, codes, scales = make_weight(rng, out_dim, in_dim, storage)
+    wc = _oracle_w(weight, codes, scales, orc.F32)
+    x_np, x = act(rng, m, in_dim, orc.BF16)
+    res_np, res = act(rng, m, out_dim, sd)
+    want = orc.frozen_linear_forward(x_np, wc)
+    y = nv.linear_fwd(weight, x, torch.float32, orc.F32)
+    assert nv.last_path() == "decode"
+    assert max_rel_err(y.cpu().numpy(), want) <= TOL_F32
+    got = nv.linear_fwd_residual(weight, x, res.clone(), orc.F32)
+    assert nv.last_path() == "decode"
+    # the same bits as the product in the stream's dtype followed by an add there
+    sep = nv.linear_fwd(weight, x, TORCH_DTYPE[sd], orc.F32)
+    assert torch.equal(got, (sep.float() + res.float()).to(TORCH_DTYPE[sd]))
+
+
 def test_decode_int8_without_scales_and_bf16_out():
     rng = np.random.default_rng(77)
     weight, codes, scales = make_weight(rng, 256, 2048, orc.I8, with_scales=False)
