@@ -1,10 +1,14 @@
-"""ctypes binding of libcaifq.so (the C ABI in include/caifq.h) for torch tensors.
+"""Binding of libcaifq.so (the C ABI in include/caifq.h) for torch tensors.
 
 PyTorch is used for device memory and streams only: every function here hands
-raw device pointers to the shared library.  There is no fallback: if the
-library is missing or the call fails, a CaifqError is raised.
+raw device pointers to the shared library.  The calls that a program makes per
+layer and step go through a native extension (binding/torch_binding.cpp), the
+rest through ctypes.  There is no fallback: if the library or the extension is
+missing or the call fails, a CaifqError is raised.
 """
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 
 import torch
@@ -17,6 +21,7 @@ _CODE_TO_TORCH = {F32: torch.float32, F16: torch.float16, BF16: torch.bfloat16, 
 
 _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "libcaifq.so")
+BINDING_PATH = os.path.join(_PKG, "_torch_binding.so")
 
 
 class CaifqError(RuntimeError):
@@ -46,6 +51,7 @@ class CLora(ctypes.Structure):
 
 
 _lib = None
+_native = None
 
 _vp = ctypes.c_void_p
 _i32 = ctypes.c_int32
@@ -161,6 +167,21 @@ def lib():
     return _lib
 
 
+def _binding():
+    """The native extension, bound to the library; raises CaifqError when either has not been built."""
+    global _native
+    if _native is None:
+        lib()
+        if not os.path.exists(BINDING_PATH):
+            raise CaifqError("%s is missing: run `python -m caif_b200.build` (there is no fallback path)" % BINDING_PATH)
+        loader = importlib.machinery.ExtensionFileLoader("_torch_binding", BINDING_PATH)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_torch_binding", loader))
+        loader.exec_module(module)
+        module.load(LIB_PATH, CaifqError)
+        _native = module
+    return _native
+
+
 def _check(rc, what):
     if rc != 0:
         raise CaifqError("%s failed (%d): %s" % (what, rc, lib().caifq_last_error().decode()))
@@ -206,6 +227,7 @@ class Weight:
         self.out_dim = out_dim
         self.c = CWeight(codes.data_ptr(), scales.data_ptr() if scales is not None else None, storage, scheme,
                          group_size, in_dim, out_dim)
+        self._addr = ctypes.addressof(self.c)
 
     def ref(self):
         return ctypes.byref(self.c)
@@ -230,32 +252,15 @@ class Weight:
 # ---- quantize / dequantize ---------------------------------------------------
 
 def quantize_int8_per_tensor(x):
-    _need_cuda(x)
-    q = torch.empty(x.shape, dtype=torch.int8, device=x.device)
-    scale = torch.empty(1, dtype=torch.float32, device=x.device)
-    _check(lib().caifq_quantize_int8_per_tensor(_ptr(x), _ptr(q), _ptr(scale), x.numel(), _stream()),
-           "quantize_int8_per_tensor")
-    return q, scale
+    return (_native or _binding()).quantize_int8_per_tensor(x)
 
 
 def quantize_int8_per_channel(x):
-    _need_cuda(x)
-    rows, cols = x.shape
-    q = torch.empty(x.shape, dtype=torch.int8, device=x.device)
-    scales = torch.empty(cols, dtype=torch.float32, device=x.device)
-    _check(lib().caifq_quantize_int8_per_channel(_ptr(x), _ptr(q), _ptr(scales), rows, cols, _stream()),
-           "quantize_int8_per_channel")
-    return q, scales
+    return (_native or _binding()).quantize_int8_per_channel(x)
 
 
 def quantize_int4(x, group_size=128):
-    _need_cuda(x)
-    n = x.numel()
-    packed = torch.zeros((n + 1) // 2, dtype=torch.uint8, device=x.device)
-    scales = torch.zeros((n + group_size - 1) // group_size, dtype=torch.float16, device=x.device)
-    _check(lib().caifq_quantize_int4_per_group(_ptr(x), _ptr(packed), _ptr(scales), n, group_size, _stream()),
-           "quantize_int4_per_group")
-    return packed, scales
+    return (_native or _binding()).quantize_int4(x, group_size)
 
 
 def dequantize_int8_per_tensor(q, scale):
@@ -284,10 +289,7 @@ def dequantize_int4(packed, scales, n, group_size=128):
 
 
 def cast(x, dtype):
-    _need_cuda(x)
-    out = torch.empty(x.shape, dtype=dtype, device=x.device)
-    _check(lib().caifq_cast(_ptr(x), dtype_code(x), _ptr(out), dtype_code(dtype), x.numel(), _stream()), "cast")
-    return out
+    return (_native or _binding()).cast(x, dtype)
 
 
 def weight_materialize(w, dtype=torch.float32):
@@ -299,52 +301,24 @@ def weight_materialize(w, dtype=torch.float32):
 # ---- frozen linear -----------------------------------------------------------
 
 def linear_fwd(w, x, out_dtype=torch.float32, compute=F32, out=None):
-    _need_cuda(x)
-    m = x.numel() // w.in_dim
-    if out is None:
-        out = torch.empty(tuple(x.shape[:-1]) + (w.out_dim,), dtype=out_dtype, device=x.device)
-    _check(lib().caifq_linear_fwd(w.ref(), _ptr(x), dtype_code(x), m, _ptr(out), dtype_code(out), compute, _stream()),
-           "linear_fwd")
-    return out
+    return (_native or _binding()).linear_fwd(w, x, out_dtype, compute, out)
 
 
 def linear_fwd_residual(w, x, residual, compute=F32):
     """residual [m, out] += W-path(x) in place, with the roundings of cast-then-Add; returns residual."""
-    _need_cuda(x, residual)
-    m = x.numel() // w.in_dim
-    _check(lib().caifq_linear_fwd_residual(w.ref(), _ptr(x), dtype_code(x), m, _ptr(residual), dtype_code(residual),
-                                           compute, _stream()), "caifq_linear_fwd_residual")
-    return residual
+    return (_native or _binding()).linear_fwd_residual(w, x, residual, compute)
 
 
 def linear_fwd_multi(ws, x, out_dtype=torch.float32, compute=F32, out=None):
     """Few-token forward of several frozen linears that share x (q/k/v, gate/up) in one launch:
     y[m, sum out_i], weight i's outputs at columns sum_{j<i} out_j."""
-    _need_cuda(x)
-    m = x.numel() // ws[0].in_dim
-    total = sum(w.out_dim for w in ws)
-    y = out if out is not None else torch.empty((m, total), dtype=out_dtype, device=x.device)
-    arr = _weight_array(ws)
-    _check(lib().caifq_linear_fwd_multi(arr, len(ws), _ptr(x), dtype_code(x), m, _ptr(y), dtype_code(y), compute,
-                                        _stream()), "caifq_linear_fwd_multi")
-    return y
+    return (_native or _binding()).linear_fwd_multi(ws, x, out_dtype, compute, out)
 
 
 def linear_concat(ws, act, backward=False, out_dtype=torch.bfloat16, workspace=None):
     """Many-token product of several frozen linears that share their input as one launch over the concatenated
     weights: forward y[m, sum out_i] = x . [W_0; W_1; ...]^T, or backward dx[m, in] = dy[m, sum out_i] . [W_0; ...]."""
-    _need_cuda(act, workspace)
-    arr = _weight_array(ws)
-    total = sum(w.out_dim for w in ws)
-    need = lib().caifq_linear_concat_workspace_bytes(arr, len(ws))
-    if workspace is None:
-        workspace = torch.empty(need, dtype=torch.uint8, device=act.device)
-    m = act.numel() // (total if backward else ws[0].in_dim)
-    out = torch.empty((m, ws[0].in_dim if backward else total), dtype=out_dtype, device=act.device)
-    fn = lib().caifq_linear_dx_concat if backward else lib().caifq_linear_fwd_concat
-    _check(fn(arr, len(ws), _ptr(act), dtype_code(act), m, _ptr(out), dtype_code(out), BF16, _ptr(workspace),
-              workspace.numel(), _stream()), "caifq_linear_concat")
-    return out
+    return (_native or _binding()).linear_concat(ws, act, backward, out_dtype, workspace)
 
 
 def linear_fwd_gather(w, x, peer_ptrs, y_ld, y_col0, y_dtype=F32, compute=F32):
@@ -358,13 +332,7 @@ def linear_fwd_gather(w, x, peer_ptrs, y_ld, y_col0, y_dtype=F32, compute=F32):
 
 
 def linear_dx(w, dy, out_dtype=torch.float32, compute=F32, out=None):
-    _need_cuda(dy)
-    m = dy.numel() // w.out_dim
-    if out is None:
-        out = torch.empty(tuple(dy.shape[:-1]) + (w.in_dim,), dtype=out_dtype, device=dy.device)
-    _check(lib().caifq_linear_dx(w.ref(), _ptr(dy), dtype_code(dy), m, _ptr(out), dtype_code(out), compute, _stream()),
-           "linear_dx")
-    return out
+    return (_native or _binding()).linear_dx(w, dy, out_dtype, compute, out)
 
 
 # ---- LoRA --------------------------------------------------------------------
@@ -377,6 +345,7 @@ class Lora:
         self.alpha = float(alpha)
         self.rank = a.shape[0]
         self.c = CLora(a.data_ptr(), b.data_ptr(), dtype_code(a), self.rank, self.alpha)
+        self._addr = ctypes.addressof(self.c)
 
     def ref(self):
         return ctypes.byref(self.c)
@@ -398,41 +367,13 @@ def lora_linear_fwd(w, lora, x, compute=F32, out=None, hidden=None, workspace=No
     """y = W-path(x) + (alpha/r) . (x . A^T) . B^T.  `out`, `hidden` and `workspace` (a uint8 tensor of at
     least lora_fwd_workspace_bytes) may be passed in to keep the call free of allocations.  expanded=True
     uses the entry point that may expand the weight once per call into the (larger) workspace."""
-    _need_cuda(x)
-    m = x.numel() // w.in_dim
-    y = out if out is not None else torch.empty(tuple(x.shape[:-1]) + (w.out_dim,), dtype=x.dtype, device=x.device)
-    if hidden is None:
-        hidden = torch.empty((m, lora.rank), dtype=x.dtype, device=x.device)
-    ws_bytes = lora_fwd_workspace_bytes(w, lora, m, compute, expanded)
-    if workspace is None:
-        workspace = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=x.device)
-    elif workspace.numel() < ws_bytes:
-        raise CaifqError("lora_linear_fwd: workspace of %d bytes, %d needed" % (workspace.numel(), ws_bytes))
-    fn = lib().caifq_lora_linear_fwd_expanded if expanded else lib().caifq_lora_linear_fwd
-    _check(fn(w.ref(), lora.ref(), _ptr(x), m, _ptr(y), _ptr(hidden), _ptr(workspace), compute, _stream()),
-           "lora_linear_fwd")
-    return y, hidden
+    return (_native or _binding()).lora_linear_fwd(w, lora, x, compute, out, hidden, workspace, expanded)
 
 
 def lora_linear_bwd(w, lora, dy, x, hidden, compute=F32, dx=None, d_a=None, d_b=None, workspace=None,
                     expanded=False):
-    _need_cuda(dy, x, hidden)
-    m = dy.numel() // w.out_dim
-    if dx is None:
-        dx = torch.empty(tuple(dy.shape[:-1]) + (w.in_dim,), dtype=dy.dtype, device=dy.device)
-    if d_a is None:
-        d_a = torch.empty_like(lora.a)
-    if d_b is None:
-        d_b = torch.empty_like(lora.b)
-    ws_bytes = lora_bwd_workspace_bytes(w, lora, m, compute, expanded)
-    if workspace is None:
-        workspace = torch.empty(max(ws_bytes, 1), dtype=torch.uint8, device=dy.device)
-    elif workspace.numel() < ws_bytes:
-        raise CaifqError("lora_linear_bwd: workspace of %d bytes, %d needed" % (workspace.numel(), ws_bytes))
-    fn = lib().caifq_lora_linear_bwd_expanded if expanded else lib().caifq_lora_linear_bwd
-    _check(fn(w.ref(), lora.ref(), _ptr(dy), _ptr(x), _ptr(hidden), m, _ptr(dx), _ptr(d_a), _ptr(d_b),
-              _ptr(workspace), compute, _stream()), "lora_linear_bwd")
-    return dx, d_a, d_b
+    return (_native or _binding()).lora_linear_bwd(w, lora, lora.a, lora.b, dy, x, hidden, compute, dx, d_a, d_b,
+                                                  workspace, expanded)
 
 
 def lora_adamw_step(lora, d_a, d_b, m_a, v_a, m_b, v_b, lr, beta1, beta2, epsilon, weight_decay, step):
@@ -466,22 +407,11 @@ def lora_linear_bwd_noalloc(w, lora, dy, x, hidden, compute=F32):
 # ---- MoE ---------------------------------------------------------------------
 
 def moe_topk(probs, k):
-    _need_cuda(probs)
-    batch, dim = probs.shape
-    idx = torch.empty((batch, k), dtype=torch.int32, device=probs.device)
-    val = torch.empty((batch, k), dtype=probs.dtype, device=probs.device)
-    _check(lib().caifq_moe_topk(_ptr(probs), dtype_code(probs), _ptr(idx), _ptr(val), batch, dim, k, _stream()),
-           "moe_topk")
-    return idx, val
+    return (_native or _binding()).moe_topk(probs, k)
 
 
 def moe_normalize_rows(x):
-    _need_cuda(x)
-    batch, dim = x.shape
-    out = torch.empty_like(x)
-    _check(lib().caifq_moe_normalize_rows(_ptr(x), _ptr(out), dtype_code(x), batch, dim, _stream()),
-           "moe_normalize_rows")
-    return out
+    return (_native or _binding()).moe_normalize_rows(x)
 
 
 def moe_route_grouped(x, k, logits=True, bias=None, n_group=1, topk_group=1):
@@ -502,16 +432,8 @@ def moe_router_bwd(grad_weights, probs, indices, balance_bias=None, z_lse_scaled
                    normalize=True, scaling=1.0, exact_jacobian=False):
     """Gradient of the routing weights back to the router's logits: returns (grad_logits [tokens, experts],
     grad_topk [tokens, top_k])."""
-    _need_cuda(grad_weights, probs, indices, balance_bias, z_lse_scaled)
-    tokens, experts = probs.shape
-    top_k = indices.shape[1]
-    grad_logits = torch.empty_like(probs)
-    grad_topk = torch.empty_like(grad_weights)
-    _check(lib().caifq_moe_router_bwd(_ptr(grad_weights), _ptr(probs), _ptr(indices), _ptr(balance_bias),
-                                      _ptr(z_lse_scaled), _ptr(grad_topk), _ptr(grad_logits), dtype_code(probs),
-                                      tokens, experts, top_k, 1 if sigmoid_gate else 0, 1 if normalize else 0,
-                                      float(scaling), 1 if exact_jacobian else 0, _stream()), "moe_router_bwd")
-    return grad_logits, grad_topk
+    return (_native or _binding()).moe_router_bwd(grad_weights, probs, indices, balance_bias, z_lse_scaled,
+                                                 sigmoid_gate, normalize, scaling, exact_jacobian)
 
 
 def moe_aux_losses(logits, probs, expert_offsets, top_k, balance_weight, z_weight):
@@ -540,37 +462,17 @@ def moe_bias_update(bias, counts, rate, from_offsets=False):
 
 def rmsnorm_fwd(x, gamma, epsilon=1e-5):
     """Returns (y, rms_cache)."""
-    _need_cuda(x, gamma)
-    dim = x.shape[-1]
-    rows = x.numel() // dim
-    y = torch.empty_like(x)
-    rms = torch.empty(rows, dtype=torch.float32, device=x.device)
-    _check(lib().caifq_rmsnorm_fwd(_ptr(x), _ptr(gamma), _ptr(y), _ptr(rms), float(epsilon), dtype_code(x), rows, dim,
-                                   _stream()), "rmsnorm_fwd")
-    return y, rms
+    return (_native or _binding()).rmsnorm_fwd(x, gamma, epsilon)
 
 
 def rmsnorm_bwd(dy, x, gamma, rms_cache, grad_gamma=None):
     """Returns (dx, grad_gamma); grad_gamma is accumulated onto the tensor given (zeros when None)."""
-    _need_cuda(dy, x, gamma, rms_cache, grad_gamma)
-    dim = x.shape[-1]
-    rows = x.numel() // dim
-    dx = torch.empty_like(x)
-    if grad_gamma is None:
-        grad_gamma = torch.zeros(dim, dtype=torch.float32, device=x.device)
-    _check(lib().caifq_rmsnorm_bwd(_ptr(dy), _ptr(x), _ptr(gamma), _ptr(rms_cache), _ptr(dx), _ptr(grad_gamma),
-                                   dtype_code(x), rows, dim, _stream()), "rmsnorm_bwd")
-    return dx, grad_gamma
+    return (_native or _binding()).rmsnorm_bwd(dy, x, gamma, rms_cache, grad_gamma)
 
 
 def moe_softmax(logits, bias=None):
     """Router probabilities: softmax over the experts of each row, optional bias added first."""
-    _need_cuda(logits, bias)
-    rows, cols = logits.shape
-    probs = torch.empty_like(logits)
-    _check(lib().caifq_moe_router_softmax(_ptr(logits), _ptr(bias), _ptr(probs), dtype_code(logits), rows, cols,
-                                          _stream()), "moe_router_softmax")
-    return probs
+    return (_native or _binding()).moe_softmax(logits, bias)
 
 
 def scale(x, factor, out=None):
@@ -582,71 +484,32 @@ def scale(x, factor, out=None):
 
 
 def moe_build_dispatch(expert_indices, num_experts, capacity=0):
-    _need_cuda(expert_indices)
-    tokens, top_k = expert_indices.shape
-    dmap = torch.empty((tokens, top_k), dtype=torch.int32, device=expert_indices.device)
-    offsets = torch.empty(num_experts + 1, dtype=torch.int32, device=expert_indices.device)
-    _check(lib().caifq_moe_build_dispatch(_ptr(expert_indices), tokens, top_k, num_experts, capacity, _ptr(dmap),
-                                          _ptr(offsets), _stream()), "moe_build_dispatch")
-    return dmap, offsets
+    return (_native or _binding()).moe_build_dispatch(expert_indices, num_experts, capacity)
 
 
 def moe_dispatch(x, expert_indices, dispatch_map, expert_offsets, total_assigned):
-    _need_cuda(x, expert_indices, dispatch_map, expert_offsets)
-    tokens, dim = x.shape
-    top_k = expert_indices.shape[1]
     # every row below expert_offsets[E] is written exactly once; like the reference's layer
     # (src/caif_device_moe_layer.cpp:457-462, Uninitialized workspaces) the buffer is not cleared first
-    buf = torch.empty((total_assigned, dim), dtype=x.dtype, device=x.device)
-    _check(lib().caifq_moe_dispatch(_ptr(x), dtype_code(x), _ptr(expert_indices), _ptr(dispatch_map),
-                                    _ptr(expert_offsets), _ptr(buf), tokens, dim, top_k, _stream()), "moe_dispatch")
-    return buf
+    return (_native or _binding()).moe_dispatch(x, expert_indices, dispatch_map, expert_offsets, total_assigned)
 
 
 def moe_combine(buf, expert_indices, weights, dispatch_map, expert_offsets, num_tokens):
-    _need_cuda(buf, expert_indices, weights, dispatch_map, expert_offsets)
-    dim = buf.shape[1]
-    top_k = expert_indices.shape[1]
-    out = torch.empty((num_tokens, dim), dtype=buf.dtype, device=buf.device)
-    _check(lib().caifq_moe_combine(_ptr(buf), dtype_code(buf), _ptr(expert_indices), _ptr(weights),
-                                   _ptr(dispatch_map), _ptr(expert_offsets), _ptr(out), num_tokens, dim, top_k,
-                                   _stream()), "moe_combine")
-    return out
+    return (_native or _binding()).moe_combine(buf, expert_indices, weights, dispatch_map, expert_offsets, num_tokens)
 
 
 def moe_combine_bwd_grad_expert(grad_output, expert_indices, weights, dispatch_map, expert_offsets, total_assigned):
-    _need_cuda(grad_output, expert_indices, weights, dispatch_map, expert_offsets)
-    tokens, dim = grad_output.shape
-    top_k = expert_indices.shape[1]
-    gbuf = torch.empty((total_assigned, dim), dtype=grad_output.dtype, device=grad_output.device)   # as above (:723-728)
-    _check(lib().caifq_moe_combine_bwd_grad_expert(_ptr(grad_output), dtype_code(grad_output), _ptr(expert_indices),
-                                                   _ptr(weights), _ptr(dispatch_map), _ptr(expert_offsets),
-                                                   _ptr(gbuf), tokens, dim, top_k, _stream()),
-           "moe_combine_bwd_grad_expert")
-    return gbuf
+    # (not cleared first either, src/caif_device_moe_layer.cpp:723-728)
+    return (_native or _binding()).moe_combine_bwd_grad_expert(grad_output, expert_indices, weights, dispatch_map,
+                                                              expert_offsets, total_assigned)
 
 
 def moe_combine_bwd_grad_weights(grad_output, buf, expert_indices, dispatch_map, expert_offsets):
-    _need_cuda(grad_output, buf, expert_indices, dispatch_map, expert_offsets)
-    tokens, dim = grad_output.shape
-    top_k = expert_indices.shape[1]
-    gw = torch.empty((tokens, top_k), dtype=grad_output.dtype, device=grad_output.device)
-    _check(lib().caifq_moe_combine_bwd_grad_weights(_ptr(grad_output), _ptr(buf), dtype_code(grad_output),
-                                                    _ptr(expert_indices), _ptr(dispatch_map), _ptr(expert_offsets),
-                                                    _ptr(gw), tokens, dim, top_k, _stream()),
-           "moe_combine_bwd_grad_weights")
-    return gw
+    return (_native or _binding()).moe_combine_bwd_grad_weights(grad_output, buf, expert_indices, dispatch_map,
+                                                               expert_offsets)
 
 
 def moe_dispatch_bwd(grad_buf, expert_indices, dispatch_map, expert_offsets, num_tokens):
-    _need_cuda(grad_buf, expert_indices, dispatch_map, expert_offsets)
-    dim = grad_buf.shape[1]
-    top_k = expert_indices.shape[1]
-    gin = torch.empty((num_tokens, dim), dtype=grad_buf.dtype, device=grad_buf.device)
-    _check(lib().caifq_moe_dispatch_bwd(_ptr(grad_buf), dtype_code(grad_buf), _ptr(expert_indices),
-                                        _ptr(dispatch_map), _ptr(expert_offsets), _ptr(gin), num_tokens, dim, top_k,
-                                        _stream()), "moe_dispatch_bwd")
-    return gin
+    return (_native or _binding()).moe_dispatch_bwd(grad_buf, expert_indices, dispatch_map, expert_offsets, num_tokens)
 
 
 def _weight_array(ws):
@@ -665,57 +528,16 @@ def grouped_expert_expanded_bytes(gate, up, down, dtype=BF16, compute=F32):
 
 def grouped_expert_expand(gate, up, down, expanded, dtype=BF16, compute=F32):
     """Fill `expanded` (uint8 tensor of grouped_expert_expanded_bytes) with the bf16 copies, once per step."""
-    _need_cuda(expanded)
-    _check(lib().caifq_grouped_expert_expand(_weight_array(gate) if gate is not None else None, _weight_array(up),
-                                             _weight_array(down), len(up), _ptr(expanded), dtype, compute, _stream()),
-           "grouped_expert_expand")
-    return expanded
+    return (_native or _binding()).grouped_expert_expand(gate, up, down, expanded, dtype, compute)
 
 
 def grouped_expert_fwd(gate, up, down, offsets_host, x, compute=F32, expanded=None):
     """gate/up/down: lists of Weight (gate=None: experts without a gate projection; the gate output
     returned is then None); offsets_host: list of E+1 ints; x: packed [total, in].  expanded: the buffer
     grouped_expert_expand filled for these tables (the launches then read bf16 weight tiles from it)."""
-    _need_cuda(x)
-    n_exp = len(up)
-    total = int(offsets_host[-1])
-    hid = up[0].out_dim
-    out = torch.empty((total, up[0].in_dim), dtype=x.dtype, device=x.device)
-    gate_out = torch.empty((total, hid), dtype=x.dtype, device=x.device) if gate is not None else None
-    up_out = torch.empty((total, hid), dtype=x.dtype, device=x.device)
-    hidden = torch.empty((total, hid), dtype=x.dtype, device=x.device)
-    offs = (ctypes.c_int32 * (n_exp + 1))(*[int(v) for v in offsets_host])
-    if expanded is not None:
-        _check(lib().caifq_grouped_expert_fwd_expanded(_weight_array(gate) if gate is not None else None,
-                                                       _weight_array(up), _weight_array(down), n_exp, offs, _ptr(x),
-                                                       _ptr(out), _ptr(gate_out), _ptr(up_out), _ptr(hidden),
-                                                       _ptr(expanded), dtype_code(x), compute, _stream()),
-               "grouped_expert_fwd_expanded")
-        return out, gate_out, up_out
-    _check(lib().caifq_grouped_expert_fwd(_weight_array(gate) if gate is not None else None, _weight_array(up),
-                                          _weight_array(down), n_exp, offs,
-                                          _ptr(x), _ptr(out), _ptr(gate_out), _ptr(up_out), _ptr(hidden),
-                                          dtype_code(x), compute, _stream()), "grouped_expert_fwd")
-    return out, gate_out, up_out
+    return (_native or _binding()).grouped_expert_fwd(gate, up, down, offsets_host, x, compute, expanded)
 
 
 def grouped_expert_bwd(gate, up, down, offsets_host, dy, gate_out, up_out, compute=F32, expanded=None):
-    _need_cuda(dy, gate_out, up_out)
-    n_exp = len(up)
-    total = int(offsets_host[-1])
-    hid = up[0].out_dim
-    dx = torch.empty((total, up[0].in_dim), dtype=dy.dtype, device=dy.device)
-    ws = torch.empty((3, max(total, 1), hid), dtype=dy.dtype, device=dy.device)
-    offs = (ctypes.c_int32 * (n_exp + 1))(*[int(v) for v in offsets_host])
-    if expanded is not None:
-        _check(lib().caifq_grouped_expert_bwd_expanded(_weight_array(gate) if gate is not None else None,
-                                                       _weight_array(up), _weight_array(down), n_exp, offs, _ptr(dy),
-                                                       _ptr(gate_out), _ptr(up_out), _ptr(dx), _ptr(ws),
-                                                       _ptr(expanded), dtype_code(dy), compute, _stream()),
-               "grouped_expert_bwd_expanded")
-        return dx
-    _check(lib().caifq_grouped_expert_bwd(_weight_array(gate) if gate is not None else None, _weight_array(up),
-                                          _weight_array(down), n_exp, offs,
-                                          _ptr(dy), _ptr(gate_out), _ptr(up_out), _ptr(dx), _ptr(ws),
-                                          dtype_code(dy), compute, _stream()), "grouped_expert_bwd")
-    return dx
+    return (_native or _binding()).grouped_expert_bwd(gate, up, down, offsets_host, dy, gate_out, up_out, compute,
+                                                     expanded)
