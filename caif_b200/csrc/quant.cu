@@ -53,36 +53,59 @@ __device__ __forceinline__ float clamp_sym(float v, float lim)
 
 // scale[0] accumulates max|x| through an integer atomicMax on the bit pattern
 // (non-negative floats order like ints), as the reference does.
-__global__ void absmax_kernel(const float *__restrict__ x, float *scale, int64_t n)
+constexpr int kAbsmaxLoads = 8;   // 16-byte loads in flight per thread
+
+__global__ void __launch_bounds__(kBlock) absmax_kernel(const float *__restrict__ x, float *scale, int64_t n)
 {
   float m = 0.0f;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t n4 = n >> 2;
   if ((reinterpret_cast<uintptr_t>(x) & 15u) == 0)
   {
     const float4 *x4 = reinterpret_cast<const float4 *>(x);
-    for (int64_t j = i; j < n4; j += stride)
+    const int64_t n4 = n >> 2;
+    const int64_t step = static_cast<int64_t>(gridDim.x) * kBlock * kAbsmaxLoads;
+    for (int64_t base = static_cast<int64_t>(blockIdx.x) * (kBlock * kAbsmaxLoads) + threadIdx.x; base < n4; base += step)
     {
-      const float4 v = x4[j];
-      m = absmax_step(absmax_step(absmax_step(absmax_step(m, v.x), v.y), v.z), v.w);
+      float4 v[kAbsmaxLoads];
+#pragma unroll
+      for (int u = 0; u < kAbsmaxLoads; ++u)
+      {
+        const int64_t j = base + u * kBlock;
+        v[u] = j < n4 ? x4[j] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+#pragma unroll
+      for (int u = 0; u < kAbsmaxLoads; ++u)
+      {
+        m = absmax_step(absmax_step(absmax_step(absmax_step(m, v[u].x), v[u].y), v[u].z), v[u].w);
+      }
     }
-    for (int64_t j = (n4 << 2) + i; j < n; j += stride)
+    const int64_t rest = (n4 << 2) + threadIdx.x;
+    if (blockIdx.x == 0 && rest < n)
     {
-      m = absmax_step(m, x[j]);
+      m = absmax_step(m, x[rest]);
     }
   }
   else
   {
-    for (; i < n; i += stride)
+    const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+    for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
     {
       m = absmax_step(m, x[i]);
     }
   }
   m = warp_max(m);
-  if ((threadIdx.x & 31) == 0 && m > 0.0f)
+  __shared__ float part[kBlock / 32];
+  if ((threadIdx.x & 31) == 0)
   {
-    atomicMax(reinterpret_cast<int *>(scale), __float_as_int(m));
+    part[threadIdx.x >> 5] = m;
+  }
+  __syncthreads();
+  if (threadIdx.x < 32)
+  {
+    m = warp_max(threadIdx.x < kBlock / 32 ? part[threadIdx.x] : 0.0f);
+    if (threadIdx.x == 0 && m > 0.0f)
+    {
+      atomicMax(reinterpret_cast<int *>(scale), __float_as_int(m));
+    }
   }
 }
 
@@ -92,27 +115,62 @@ __global__ void finalize_scale_kernel(float *scale)
   scale[0] = (m > 0.0f) ? __fdiv_rn(m, 127.0f) : 1.0f;
 }
 
-__global__ void quantize_int8_pt_kernel(const float *__restrict__ x, int8_t *__restrict__ q,
-                                        const float *__restrict__ scale, int64_t n)
+__device__ __forceinline__ int quant_int8(float x, float inv)
+{
+  return static_cast<int>(rintf(clamp_sym(__fmul_rn(x, inv), 127.0f)));
+}
+
+__device__ __forceinline__ uint32_t quant_int8x4(const float4 v, const float4 inv)
+{
+  return (static_cast<uint32_t>(quant_int8(v.x, inv.x)) & 0xFFu) |
+         ((static_cast<uint32_t>(quant_int8(v.y, inv.y)) & 0xFFu) << 8) |
+         ((static_cast<uint32_t>(quant_int8(v.z, inv.z)) & 0xFFu) << 16) |
+         ((static_cast<uint32_t>(quant_int8(v.w, inv.w)) & 0xFFu) << 24);
+}
+
+// Four 16-byte loads in flight a thread, and the blocks take the elements from the end: the maximum's pass has just
+// left the last of them in L2.
+constexpr int kInt8Loads = 4;
+
+__global__ void __launch_bounds__(kBlock)
+quantize_int8_pt_kernel(const float *__restrict__ x, int8_t *__restrict__ q, const float *__restrict__ scale, int64_t n)
 {
   const float s = scale[0];
   const float inv = (s > 0.0f) ? __fdiv_rn(1.0f, s) : 0.0f;
-  const int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
-  if (i + 3 < n && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(q)) & 15u) == 0)
+  const int64_t block = static_cast<int64_t>(gridDim.x) - 1 - blockIdx.x;
+  if (((reinterpret_cast<uintptr_t>(x) & 15u) | (reinterpret_cast<uintptr_t>(q) & 3u)) == 0)
   {
-    const float4 v = *reinterpret_cast<const float4 *>(x + i);
-    char4 o;
-    o.x = static_cast<int8_t>(rintf(clamp_sym(__fmul_rn(v.x, inv), 127.0f)));
-    o.y = static_cast<int8_t>(rintf(clamp_sym(__fmul_rn(v.y, inv), 127.0f)));
-    o.z = static_cast<int8_t>(rintf(clamp_sym(__fmul_rn(v.z, inv), 127.0f)));
-    o.w = static_cast<int8_t>(rintf(clamp_sym(__fmul_rn(v.w, inv), 127.0f)));
-    *reinterpret_cast<char4 *>(q + i) = o;
+    const int64_t n4 = n >> 2;
+    const int64_t base = block * (kBlock * kInt8Loads) + threadIdx.x;
+    float4 v[kInt8Loads];
+#pragma unroll
+    for (int u = 0; u < kInt8Loads; ++u)
+    {
+      const int64_t j = base + u * kBlock;
+      v[u] = j < n4 ? __ldcs(reinterpret_cast<const float4 *>(x) + j) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+#pragma unroll
+    for (int u = 0; u < kInt8Loads; ++u)
+    {
+      const int64_t j = base + u * kBlock;
+      if (j < n4)
+      {
+        reinterpret_cast<uint32_t *>(q)[j] = quant_int8x4(v[u], make_float4(inv, inv, inv, inv));
+      }
+    }
+    const int64_t rest = (n4 << 2) + threadIdx.x;
+    if (block == 0 && rest < n)
+    {
+      q[rest] = static_cast<int8_t>(quant_int8(x[rest], inv));
+    }
   }
   else
   {
-    for (int64_t j = i; j < n && j < i + 4; ++j)
+    const int64_t first = block * (kBlock * kInt8Loads * 4);
+    const int64_t last = (first + kBlock * kInt8Loads * 4 < n) ? first + kBlock * kInt8Loads * 4 : n;
+    for (int64_t j = first + threadIdx.x; j < last; j += kBlock)
     {
-      q[j] = static_cast<int8_t>(rintf(clamp_sym(__fmul_rn(x[j], inv), 127.0f)));
+      q[j] = static_cast<int8_t>(quant_int8(x[j], inv));
     }
   }
 }
@@ -130,32 +188,144 @@ __global__ void dequantize_int8_pt_kernel(const int8_t *__restrict__ q, float *_
 
 // --------------------------------------------------------------- int8 / channel
 
-// One thread per column, rows walked in order: neighbouring threads read
-// neighbouring columns, so each row pass is coalesced.
-__global__ void channel_scale_kernel(const float *__restrict__ x, float *__restrict__ scales, int rows, int cols)
+// Column maxima.  A block takes 128 columns (a warp one row of them, 16 bytes a lane where rows are aligned) and a
+// slice of the rows; its eight warps' maxima meet in shared memory and go to scales[] as an integer atomicMax, which
+// the caller cleared.  (A thread that walked a whole column took 14336 dependent trips to memory.)
+constexpr int kPcCols = 128;
+
+__global__ void __launch_bounds__(kBlock)
+channel_absmax_kernel(const float *__restrict__ x, float *__restrict__ scales, int rows, int cols, int rows_per_block,
+                      int vec)
 {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= cols)
+  __shared__ float part[kBlock / 32][kPcCols];
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int c0 = blockIdx.x * kPcCols;
+  const int r_end = min(rows, (static_cast<int>(blockIdx.y) + 1) * rows_per_block);
+  float m[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  constexpr int U = 8;
+  for (int r = static_cast<int>(blockIdx.y) * rows_per_block + warp; r < r_end; r += U * (kBlock / 32))
   {
-    return;
+    float4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+    {
+      const int rr = r + u * (kBlock / 32);
+      v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (rr < r_end)
+      {
+        const float *row = x + static_cast<int64_t>(rr) * cols;
+        const int c = c0 + 4 * lane;
+        if (vec)
+        {
+          if (c < cols)
+          {
+            v[u] = *reinterpret_cast<const float4 *>(row + c);
+          }
+        }
+        else
+        {
+          v[u].x = (c + 0 < cols) ? row[c + 0] : 0.0f;
+          v[u].y = (c + 1 < cols) ? row[c + 1] : 0.0f;
+          v[u].z = (c + 2 < cols) ? row[c + 2] : 0.0f;
+          v[u].w = (c + 3 < cols) ? row[c + 3] : 0.0f;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+    {
+      m[0] = absmax_step(m[0], v[u].x);
+      m[1] = absmax_step(m[1], v[u].y);
+      m[2] = absmax_step(m[2], v[u].z);
+      m[3] = absmax_step(m[3], v[u].w);
+    }
   }
-  float m = 0.0f;
-  for (int r = 0; r < rows; ++r)
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
   {
-    m = absmax_step(m, x[static_cast<int64_t>(r) * cols + c]);
+    part[warp][4 * lane + i] = m[i];
   }
-  scales[c] = (m > 0.0f) ? __fdiv_rn(m, 127.0f) : 1.0f;
+  __syncthreads();
+  if (threadIdx.x < kPcCols && c0 + static_cast<int>(threadIdx.x) < cols)
+  {
+    float best = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kBlock / 32; ++w)
+    {
+      best = fmaxf(best, part[w][threadIdx.x]);
+    }
+    if (best > 0.0f)
+    {
+      atomicMax(reinterpret_cast<int *>(scales) + c0 + threadIdx.x, __float_as_int(best));
+    }
+  }
 }
 
-__global__ void quantize_int8_pc_kernel(const float *__restrict__ x, int8_t *__restrict__ q,
-                                        const float *__restrict__ scales, int64_t total, int cols)
+__global__ void finalize_channel_scales_kernel(float *scales, int cols)
 {
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride)
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < cols)
   {
-    const float s = scales[i % cols];
-    const float inv = (s > 0.0f) ? __fdiv_rn(1.0f, s) : 0.0f;
-    q[i] = static_cast<int8_t>(rintf(clamp_sym(__fmul_rn(x[i], inv), 127.0f)));
+    const float m = scales[c];
+    scales[c] = (m > 0.0f) ? __fdiv_rn(m, 127.0f) : 1.0f;
+  }
+}
+
+// Same shape of work: a lane keeps its columns' reciprocals and takes the rows of its slice, last slices first (they
+// are the ones the maxima's pass left in L2).
+__global__ void __launch_bounds__(kBlock)
+quantize_int8_pc_kernel(const float *__restrict__ x, int8_t *__restrict__ q, const float *__restrict__ scales, int rows,
+                        int cols, int rows_per_block, int vec)
+{
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int slice = static_cast<int>(gridDim.y) - 1 - static_cast<int>(blockIdx.y);
+  const int c = blockIdx.x * kPcCols + 4 * lane;
+  const int r_end = min(rows, (slice + 1) * rows_per_block);
+  float inv[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+  {
+    const float s = (c + i < cols) ? scales[c + i] : 0.0f;
+    inv[i] = (s > 0.0f) ? __fdiv_rn(1.0f, s) : 0.0f;
+  }
+  constexpr int U = 4;
+  for (int r = slice * rows_per_block + warp; r < r_end; r += U * (kBlock / 32))
+  {
+    if (vec)
+    {
+      float4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+      {
+        const int rr = r + u * (kBlock / 32);
+        v[u] = (rr < r_end && c < cols) ? __ldcs(reinterpret_cast<const float4 *>(x + static_cast<int64_t>(rr) * cols + c))
+                                        : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+      {
+        const int rr = r + u * (kBlock / 32);
+        if (rr < r_end && c < cols)
+        {
+          *reinterpret_cast<uint32_t *>(q + static_cast<int64_t>(rr) * cols + c) =
+              quant_int8x4(v[u], make_float4(inv[0], inv[1], inv[2], inv[3]));
+        }
+      }
+    }
+    else
+    {
+      for (int u = 0; u < U; ++u)
+      {
+        const int rr = r + u * (kBlock / 32);
+        for (int i = 0; i < 4 && rr < r_end && c + i < cols; ++i)
+        {
+          const int64_t at = static_cast<int64_t>(rr) * cols + c + i;
+          q[at] = static_cast<int8_t>(quant_int8(x[at], inv[i]));
+        }
+      }
+    }
   }
 }
 
@@ -176,7 +346,38 @@ __device__ __forceinline__ int quant_nibble(float x, float inv)
   return static_cast<int>(rintf(clamp_sym(__fmul_rn(x, inv), 7.0f))) & 0xF;
 }
 
-// Even group size: a warp per group, lanes take element pairs (one byte each).
+// one group, lanes take element pairs (one byte each)
+__device__ __forceinline__ void quantize_int4_group(const float *__restrict__ x, uint8_t *__restrict__ packed,
+                                                    __half *__restrict__ scales, int64_t n, int group, int64_t g,
+                                                    int lane)
+{
+  const int64_t start = g * group;
+  const int64_t end = (start + group < n) ? (start + group) : n;
+  float m = 0.0f;
+  for (int64_t i = start + 2 * lane; i < end; i += 64)
+  {
+    m = absmax_step(m, x[i]);
+    if (i + 1 < end)
+    {
+      m = absmax_step(m, x[i + 1]);
+    }
+  }
+  m = warp_max(m);
+  const float scale = (m == 0.0f) ? 0.0f : __fdiv_rn(m, 7.0f);
+  const float inv = (scale == 0.0f) ? 0.0f : __fdiv_rn(1.0f, scale);
+  if (lane == 0)
+  {
+    scales[g] = __float2half(scale);
+  }
+  for (int64_t i = start + 2 * lane; i < end; i += 64)
+  {
+    const int q0 = quant_nibble(x[i], inv);
+    const int q1 = (i + 1 < end) ? quant_nibble(x[i + 1], inv) : 0;
+    packed[i >> 1] = static_cast<uint8_t>(q0 | (q1 << 4));
+  }
+}
+
+// Even group size: a warp per group.
 __global__ void quantize_int4_warp_kernel(const float *__restrict__ x, uint8_t *__restrict__ packed,
                                           __half *__restrict__ scales, int64_t n, int group, int64_t num_groups)
 {
@@ -185,31 +386,89 @@ __global__ void quantize_int4_warp_kernel(const float *__restrict__ x, uint8_t *
   const int64_t warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   for (int64_t g = warp; g < num_groups; g += warps)
   {
-    const int64_t start = g * group;
-    const int64_t end = (start + group < n) ? (start + group) : n;
-    float m = 0.0f;
-    for (int64_t i = start + 2 * lane; i < end; i += 64)
+    quantize_int4_group(x, packed, scales, n, group, g, lane);
+  }
+}
+
+// Group sizes 32, 64, 128 and 256 on aligned buffers: a thread keeps eight elements (two 16-byte loads) in registers
+// between the maximum and the codes, LPG neighbouring lanes share a group, and kInt4Units such units a thread are
+// in flight.  Bound by HBM (4.5 bytes an element); the form above reads every element twice, eight bytes at a time,
+// one group in flight a warp (14336 x 4096: 128 us, this one 43).
+constexpr int kInt4Units = 4;
+
+template <int LPG>
+__global__ void __launch_bounds__(kBlock)
+quantize_int4_vec_kernel(const float4 *__restrict__ x, uint32_t *__restrict__ packed, __half *__restrict__ scales,
+                         int64_t n, int64_t full_groups)
+{
+  constexpr int GROUP = LPG * 8;
+  const int64_t units = full_groups * LPG;
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * (kBlock * kInt4Units) + threadIdx.x;
+  float4 v[kInt4Units][2];
+#pragma unroll
+  for (int u = 0; u < kInt4Units; ++u)
+  {
+    const int64_t i = base + u * kBlock;
+    if (i < units)
     {
-      m = absmax_step(m, x[i]);
-      if (i + 1 < end)
-      {
-        m = absmax_step(m, x[i + 1]);
-      }
+      v[u][0] = __ldcs(x + 2 * i);
+      v[u][1] = __ldcs(x + 2 * i + 1);
     }
-    m = warp_max(m);
-    const float scale = (m == 0.0f) ? 0.0f : __fdiv_rn(m, 7.0f);
-    const float inv = (scale == 0.0f) ? 0.0f : __fdiv_rn(1.0f, scale);
-    if (lane == 0)
+    else
     {
-      scales[g] = __float2half(scale);
-    }
-    for (int64_t i = start + 2 * lane; i < end; i += 64)
-    {
-      const int q0 = quant_nibble(x[i], inv);
-      const int q1 = (i + 1 < end) ? quant_nibble(x[i + 1], inv) : 0;
-      packed[i >> 1] = static_cast<uint8_t>(q0 | (q1 << 4));
+      v[u][0] = v[u][1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
   }
+#pragma unroll
+  for (int u = 0; u < kInt4Units; ++u)
+  {
+    const int64_t i = base + u * kBlock;
+    const float e[8] = {v[u][0].x, v[u][0].y, v[u][0].z, v[u][0].w, v[u][1].x, v[u][1].y, v[u][1].z, v[u][1].w};
+    float m = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+    {
+      m = absmax_step(m, e[k]);
+    }
+#pragma unroll
+    for (int o = LPG / 2; o > 0; o >>= 1)
+    {
+      m = fmaxf(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
+    }
+    const float scale = (m == 0.0f) ? 0.0f : __fdiv_rn(m, 7.0f);
+    const float inv = (scale == 0.0f) ? 0.0f : __fdiv_rn(1.0f, scale);
+    uint32_t w = 0u;
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+    {
+      w |= static_cast<uint32_t>(quant_nibble(e[k], inv)) << (4 * k);
+    }
+    if (i < units)
+    {
+      packed[i] = w;
+      if ((threadIdx.x & (LPG - 1)) == 0)
+      {
+        scales[i / LPG] = __float2half(scale);
+      }
+    }
+  }
+  // a last, shorter group
+  if (blockIdx.x == 0 && threadIdx.x < 32 && full_groups * GROUP < n)
+  {
+    quantize_int4_group(reinterpret_cast<const float *>(x), reinterpret_cast<uint8_t *>(packed), scales, n, GROUP,
+                        full_groups, static_cast<int>(threadIdx.x));
+  }
+}
+
+template <int LPG>
+void launch_int4_vec(const float *x, uint8_t *packed, uint16_t *scales, int64_t n, cudaStream_t s)
+{
+  const int64_t full = n / (LPG * 8);
+  const int64_t per_block = static_cast<int64_t>(kBlock) * kInt4Units;
+  const int64_t blocks = (full * LPG + per_block - 1) / per_block;
+  quantize_int4_vec_kernel<LPG><<<static_cast<unsigned>(blocks > 0 ? blocks : 1), kBlock, 0, s>>>(
+      reinterpret_cast<const float4 *>(x), reinterpret_cast<uint32_t *>(packed), reinterpret_cast<__half *>(scales), n,
+      full);
 }
 
 // Odd group size: groups share bytes; keep the reference's thread-per-group
@@ -353,12 +612,12 @@ int launch_quantize_int8_per_tensor(const float *x, int8_t *q, float *scale, int
     return CAIFQ_OK;
   }
   CAIFQ_CHECK_CUDA(cudaMemsetAsync(scale, 0, sizeof(float), s));
-  absmax_kernel<<<grid_for(n, 16), kBlock, 0, s>>>(x, scale, n);
+  absmax_kernel<<<grid_for(n, 4 * kAbsmaxLoads), kBlock, 0, s>>>(x, scale, n);
   CAIFQ_CHECK_LAUNCH();
   finalize_scale_kernel<<<1, 1, 0, s>>>(scale);
   CAIFQ_CHECK_LAUNCH();
-  const int64_t threads = (n + 3) / 4;
-  const int64_t grid = (threads + kBlock - 1) / kBlock;
+  const int64_t per_block = static_cast<int64_t>(kBlock) * kInt8Loads * 4;
+  const int64_t grid = (n + per_block - 1) / per_block;
   quantize_int8_pt_kernel<<<static_cast<unsigned>(grid), kBlock, 0, s>>>(x, q, scale, n);
   CAIFQ_CHECK_LAUNCH();
   return CAIFQ_OK;
@@ -381,10 +640,20 @@ int launch_quantize_int8_per_channel(const float *x, int8_t *q, float *scales, i
   {
     return CAIFQ_OK;
   }
-  channel_scale_kernel<<<(cols + kBlock - 1) / kBlock, kBlock, 0, s>>>(x, scales, rows, cols);
+  CAIFQ_CHECK_CUDA(cudaMemsetAsync(scales, 0, static_cast<size_t>(cols) * sizeof(float), s));
+  const int col_blocks = (cols + kPcCols - 1) / kPcCols;
+  // about eight blocks per SM over all columns, at least one trip of eight rows a warp each
+  int slices = (148 * 8 + col_blocks - 1) / col_blocks;
+  const int most = (rows + 63) / 64;
+  slices = slices < most ? slices : most;
+  const int per = (rows + slices - 1) / slices;
+  const dim3 grid(static_cast<unsigned>(col_blocks), static_cast<unsigned>((rows + per - 1) / per));
+  const int vec = (cols % 4) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(q) & 3u) == 0;
+  channel_absmax_kernel<<<grid, kBlock, 0, s>>>(x, scales, rows, cols, per, vec);
   CAIFQ_CHECK_LAUNCH();
-  const int64_t total = static_cast<int64_t>(rows) * cols;
-  quantize_int8_pc_kernel<<<grid_for(total), kBlock, 0, s>>>(x, q, scales, total, cols);
+  finalize_channel_scales_kernel<<<(cols + kBlock - 1) / kBlock, kBlock, 0, s>>>(scales, cols);
+  CAIFQ_CHECK_LAUNCH();
+  quantize_int8_pc_kernel<<<grid, kBlock, 0, s>>>(x, q, scales, rows, cols, per, vec);
   CAIFQ_CHECK_LAUNCH();
   return CAIFQ_OK;
 }
@@ -409,7 +678,24 @@ int launch_quantize_int4(const float *x, uint8_t *packed, uint16_t *scales, int6
     return CAIFQ_OK;
   }
   const int64_t num_groups = (n + group - 1) / group;
-  if ((group & 1) == 0)
+  const bool aligned = (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(packed) & 3u) == 0;
+  if (aligned && group == 128)
+  {
+    launch_int4_vec<16>(x, packed, scales, n, s);
+  }
+  else if (aligned && group == 64)
+  {
+    launch_int4_vec<8>(x, packed, scales, n, s);
+  }
+  else if (aligned && group == 32)
+  {
+    launch_int4_vec<4>(x, packed, scales, n, s);
+  }
+  else if (aligned && group == 256)
+  {
+    launch_int4_vec<32>(x, packed, scales, n, s);
+  }
+  else if ((group & 1) == 0)
   {
     const int64_t blocks = (num_groups + (kBlock / 32) - 1) / (kBlock / 32);
     const int64_t cap = 148 * 32;

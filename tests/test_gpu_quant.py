@@ -155,3 +155,31 @@ def test_oracle_matches_reference_kernels_on_routing():
     assert np.array_equal(_bits(rnorm), orc.normalize_rows(oval).view(np.int32))
     wide = torch.rand(7, 1000, generator=g).to(dev())
     assert np.array_equal(_bits(ref.normalize_rows(wide)), orc.normalize_rows(wide.cpu().numpy()).view(np.int32))
+
+
+@pytest.mark.parametrize("group,n", [(32, 8192 * 3 + 40), (64, 4096 * 5), (64, 100), (128, 8192 * 2 + 131), (256, 8192 + 257)])
+def test_int4_eight_elements_a_thread_bit_exact(group, n):
+    """Edges of a block's 8192 elements, a shorter last group, a buffer shorter than one group."""
+    g = torch.Generator().manual_seed(15)
+    x = torch.randn(n, generator=g) * 0.02
+    x[:min(n, group)] = 0.0
+    p, s = nv.quantize_int4(x.to(dev()), group)
+    op, os_ = orc.quantize_int4(x.numpy(), group)
+    assert np.array_equal(p.cpu().numpy(), op)
+    assert np.array_equal(_f16bits(s), os_)
+
+
+@pytest.mark.parametrize("shape", [(1000, 516), (4097, 130), (64, 128), (65, 131), (3, 4096)])
+def test_int8_slices_of_rows_bit_exact(shape):
+    """Per channel: several row slices, aligned and unaligned rows, a partial block of columns; per tensor: the same
+    elements, with and without a remainder of four."""
+    g = torch.Generator().manual_seed(16)
+    x = torch.randn(*shape, generator=g) * 0.02
+    q, s = nv.quantize_int8_per_channel(x.to(dev()))
+    oq, os_ = orc.quantize_int8_per_channel(x.numpy())
+    assert np.array_equal(q.cpu().numpy(), oq)
+    assert np.array_equal(_bits(s), os_.view(np.int32))
+    q, s = nv.quantize_int8_per_tensor(x.to(dev()))
+    oq, os_ = orc.quantize_int8_per_tensor(x.numpy())
+    assert np.array_equal(q.cpu().numpy(), oq)
+    assert np.array_equal(_bits(s), os_.view(np.int32))
