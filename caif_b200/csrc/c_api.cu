@@ -60,6 +60,15 @@ int device_sm_count()
   return v;
 }
 
+bool dependent_launches()
+{
+  static const bool on = []() {
+    const char *e = std::getenv("CAIFQ_PDL");
+    return e == nullptr || e[0] != '0';
+  }();
+  return on;
+}
+
 int persistent_ctas(const char *env_name)
 {
   int n = device_sm_count();

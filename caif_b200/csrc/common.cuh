@@ -47,6 +47,27 @@ constexpr int kMaxDevices = 64;
 int device_sm_count();
 int persistent_ctas(const char *env_name);
 
+// CAIFQ_PDL=0 turns programmatic dependent launches off (read once per process)
+bool dependent_launches();
+
+// Launch of a kernel that begins with griddepcontrol.wait: its CTAs may be placed while the previous kernel in the
+// stream still runs, which hides most of the launch's latency.
+template <typename... P, typename... A>
+inline cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, A... args)
+{
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = dependent_launches() ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 inline bool is_float_dtype(int d) { return d == CAIFQ_F32 || d == CAIFQ_F16 || d == CAIFQ_BF16; }
 
 inline size_t dtype_bytes(int d)

@@ -859,10 +859,6 @@ int launch_decode_inst(const DecodeParams &p, uint32_t smem, cudaStream_t s)
   {
     grid = p.num_quanta;
   }
-  static const bool pdl = []() {
-    const char *e = std::getenv("CAIFQ_PDL");
-    return e == nullptr || e[0] != '0';
-  }();
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
   cfg.blockDim = dim3(WARPS * 32);
@@ -874,7 +870,7 @@ int launch_decode_inst(const DecodeParams &p, uint32_t smem, cudaStream_t s)
   cfg.attrs = attr;
   // codes written just ahead in this stream by one of the library's own calls: a plain launch
   // orders the early copies behind that kernel
-  cfg.numAttrs = (pdl && !take_codes_written(s)) ? 1 : 0;
+  cfg.numAttrs = (dependent_launches() && !take_codes_written(s)) ? 1 : 0;
   CAIFQ_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
   CAIFQ_CHECK_LAUNCH();
   return CAIFQ_OK;

@@ -3,16 +3,14 @@
 // (src/caif_cuda_kernels_normalization.cu:46-119 forward, :129-203 backward) run one 256-thread block per row,
 // thread t owning columns t, t + 256, ..., and read the row twice from global memory with 2- or 4-byte loads.
 //
-// Here a CTA walks rows round robin; a row comes in once with 16-byte loads into shared memory, both passes
-// read it there, the result leaves with 16-byte stores, and the backward pass keeps its share of grad_gamma in
-// registers over all its rows and adds it with one atomic per column at the end (the reference issues one
-// atomic per element).  The usual case (even row length, 16-byte aligned rows) runs on 128 threads that each
-// play two adjacent threads of the reference's block; the kernels with one thread per reference thread take
-// the rest.  The arithmetic of y, rms and dx is the reference's, operation for
-// operation: the same columns per thread in the same order with a fused multiply-add per step, the same
-// shuffle-down tree inside a warp, the eight warp sums folded by the same tree, IEEE sqrt and divisions -- so
-// those three come out bit-identical.  grad_gamma is a sum over rows whose order the reference leaves to its
-// atomics; it agrees to rounding.
+// Here a row comes in once, with 4- to 16-byte loads, into the registers of the warps that own it, both passes read it
+// there, and the backward pass keeps its share of grad_gamma in registers over all its rows (the reference issues one
+// atomic per element).  A lane plays V adjacent threads of the reference's block.  The kernels with one thread per
+// reference thread take the rest (odd row lengths, unaligned rows, rows too long for the registers).  The arithmetic
+// of y, rms and dx is the reference's, operation for operation: the same columns per thread in the same order with a
+// fused multiply-add per step, the same shuffle-down tree inside a warp, the eight warp sums folded by the same tree,
+// IEEE sqrt and divisions -- so those three come out bit-identical.  grad_gamma is a sum over rows whose order the
+// reference leaves to its atomics; it agrees to rounding.
 #include "common.cuh"
 
 namespace caifq
@@ -153,123 +151,274 @@ rmsnorm_fwd_kernel(const T *__restrict__ input, const float *__restrict__ gamma,
   }
 }
 
-// ---- forward with two of the reference's threads per thread ----
-// Thread t of 128 plays threads 2t and 2t + 1 of the reference's 256-thread block: their columns are adjacent,
-// so one 4-byte (8-byte for fp32) shared-memory access serves both, and the instruction count per element
-// halves (the one-thread-per-reference-thread kernel above spent its time on shared-memory latency, not on
-// DRAM).  Each of the two partial sums runs over the same columns in the same order; the reference's
-// shuffle-down tree over 32 lanes becomes offsets 8, 4, 2, 1 over 16 threads for either sum followed by
-// sum0 += sum1, which adds the same pairs in the same order; the eight warp results are folded as before.
-constexpr int kPairThreads = 128;
+// ---- rows in registers: a lane plays V adjacent threads of the reference's block ----
+// A row is owned by 8 / V warps.  Lane q of virtual threads V q .. V q + V - 1 holds V adjacent columns of every stripe
+// of 256, so one access serves them; each of its V partial sums runs over the same columns in the same order as the
+// reference's thread.  The shuffle-down tree over 32 virtual threads becomes lane offsets 16 / V ... 1 and then the
+// same halving over the lane's own V sums, which adds the same pairs in the same order.
+// Bound by HBM for many rows (16-byte loads, one warp a row for 16-bit types, no barrier: 4096 x 4096 bf16 16 us a call, 20 before),
+// by latency for few (V = 2: four warps a row, all of it in flight at once).
+template <typename T, int V>
+struct alignas(V * sizeof(T) < 16 ? V * sizeof(T) : 16) Piece
+{
+  static constexpr int WORDS = V * static_cast<int>(sizeof(T)) / 4;
+  uint32_t w[WORDS];
 
-template <typename T>
-__device__ __forceinline__ void load2(const T *row, int i, float &a, float &b);
-template <>
-__device__ __forceinline__ void load2<float>(const float *row, int i, float &a, float &b)
+  __device__ __forceinline__ float get(int i) const
+  {
+    if constexpr (sizeof(T) == 4)
+    {
+      return __uint_as_float(w[i]);
+    }
+    else
+    {
+      const uint16_t h = static_cast<uint16_t>((i & 1) ? w[i >> 1] >> 16 : w[i >> 1]);
+      return nf<T>(*reinterpret_cast<const T *>(&h));
+    }
+  }
+
+  __device__ __forceinline__ void set(const float (&v)[V])
+  {
+#pragma unroll
+    for (int i = 0; i < WORDS; ++i)
+    {
+      if constexpr (sizeof(T) == 4)
+      {
+        w[i] = __float_as_uint(v[i]);
+      }
+      else
+      {
+        const T lo = nt<T>(v[2 * i]);
+        const T hi = nt<T>(v[2 * i + 1]);
+        w[i] = static_cast<uint32_t>(*reinterpret_cast<const uint16_t *>(&lo)) |
+               (static_cast<uint32_t>(*reinterpret_cast<const uint16_t *>(&hi)) << 16);
+      }
+    }
+  }
+
+  // the row stays packed between its two passes (the compiler would otherwise keep it as floats: twice the registers)
+  __device__ __forceinline__ void keep_packed()
+  {
+#pragma unroll
+    for (int i = 0; i < WORDS; ++i)
+    {
+      asm volatile("" : "+r"(w[i]));
+    }
+  }
+};
+
+template <typename T, int V>
+__device__ __forceinline__ Piece<T, V> zero_piece()
 {
-  const float2 v = reinterpret_cast<const float2 *>(row)[i];
-  a = v.x;
-  b = v.y;
-}
-template <>
-__device__ __forceinline__ void load2<__half>(const __half *row, int i, float &a, float &b)
-{
-  const __half2 h = reinterpret_cast<const __half2 *>(row)[i];
-  a = __low2float(h);
-  b = __high2float(h);
-}
-template <>
-__device__ __forceinline__ void load2<__nv_bfloat16>(const __nv_bfloat16 *row, int i, float &a, float &b)
-{
-  const uint32_t w = reinterpret_cast<const uint32_t *>(row)[i];
-  a = __uint_as_float(w << 16);
-  b = __uint_as_float(w & 0xFFFF0000u);
+  Piece<T, V> p;
+#pragma unroll
+  for (int i = 0; i < Piece<T, V>::WORDS; ++i)
+  {
+    p.w[i] = 0u;
+  }
+  return p;
 }
 
-template <typename T>
-__device__ __forceinline__ void store2(T *row, int i, float a, float b);
-template <>
-__device__ __forceinline__ void store2<float>(float *row, int i, float a, float b)
+template <int V>
+struct Gammas
 {
-  reinterpret_cast<float2 *>(row)[i] = make_float2(a, b);
-}
-template <>
-__device__ __forceinline__ void store2<__half>(__half *row, int i, float a, float b)
+  float e[V];
+};
+
+template <int V>
+__device__ __forceinline__ Gammas<V> load_gamma(const float *gamma, int c)
 {
-  reinterpret_cast<__half2 *>(row)[i] = __floats2half2_rn(a, b);
-}
-template <>
-__device__ __forceinline__ void store2<__nv_bfloat16>(__nv_bfloat16 *row, int i, float a, float b)
-{
-  reinterpret_cast<__nv_bfloat162 *>(row)[i] = __floats2bfloat162_rn(a, b);
+  Gammas<V> g;
+  if constexpr (V == 2)
+  {
+    const float2 v = __ldg(reinterpret_cast<const float2 *>(gamma + c));
+    g.e[0] = v.x;
+    g.e[1] = v.y;
+  }
+  else
+  {
+#pragma unroll
+    for (int i = 0; i < V; i += 4)
+    {
+      const float4 v = __ldg(reinterpret_cast<const float4 *>(gamma + c + i));
+      g.e[i] = v.x;
+      g.e[i + 1] = v.y;
+      g.e[i + 2] = v.z;
+      g.e[i + 3] = v.w;
+    }
+  }
+  return g;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kPairThreads, 16)
-rmsnorm_fwd_pair_kernel(const T *__restrict__ input, const float *__restrict__ gamma, T *__restrict__ output,
+// the reference's block sum of its 256 partial sums; every thread of the row gets it.  slots: [8] of this row.
+template <int V>
+__device__ __forceinline__ float row_sum(float (&v)[V], float *slots, int warp_in_row)
+{
+  constexpr int LANES = 32 / V;   // lanes of one virtual warp
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int off = LANES / 2; off > 0; off >>= 1)
+  {
+#pragma unroll
+    for (int i = 0; i < V; ++i)
+    {
+      v[i] += __shfl_down_sync(0xFFFFFFFFu, v[i], off, LANES);
+    }
+  }
+#pragma unroll
+  for (int off = V / 2; off > 0; off >>= 1)
+  {
+#pragma unroll
+    for (int i = 0; i < off; ++i)
+    {
+      v[i] += v[i + off];
+    }
+  }
+  float w[8];
+  if constexpr (V == 8)
+  {
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+    {
+      w[i] = __shfl_sync(0xFFFFFFFFu, v[0], i * LANES);
+    }
+  }
+  else
+  {
+    __syncthreads();   // the slots may still be read from the row before
+    if ((lane & (LANES - 1)) == 0)
+    {
+      slots[warp_in_row * V + lane / LANES] = v[0];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+    {
+      w[i] = slots[i];
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+  {
+    w[i] += 0.0f;   // lanes 8 to 31 of the reference's last tree
+  }
+  return ((w[0] + w[4]) + (w[2] + w[6])) + ((w[1] + w[5]) + (w[3] + w[7]));
+}
+
+// STRIPES: upper bound of ceil(dim / 256)
+template <typename T, int V, int STRIPES>
+__global__ void __launch_bounds__(kNormThreads)
+rmsnorm_fwd_rows_kernel(const T *input, const float *__restrict__ gamma, T *output,
                         float *__restrict__ rms_cache, float epsilon, int rows, int dim)
 {
-  extern __shared__ __align__(16) unsigned char norm_smem[];
-  __shared__ float warp_sums[kNormWarps + 1];
-  T *row = reinterpret_cast<T *>(norm_smem);
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int pairs = dim >> 1;
-  for (int r = blockIdx.x; r < rows; r += gridDim.x)
+  constexpr int WARPS = 8 / V;   // per row; V rows per CTA
+  __shared__ float sums[V][8];
+  // (launched ahead of the previous kernel's end; the next kernel may follow once that one is complete)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int slot = (threadIdx.x >> 5) / WARPS;
+  const int warp_in_row = (threadIdx.x >> 5) % WARPS;
+  const int r = blockIdx.x * V + slot;
+  const bool live = r < rows;
+  const int c0 = (warp_in_row * 32 + (threadIdx.x & 31)) * V;
+  const T *src = input + static_cast<int64_t>(live ? r : 0) * dim;
+  Piece<T, V> x[STRIPES];
+#pragma unroll
+  for (int j = 0; j < STRIPES; ++j)
   {
-    __syncthreads();   // the row buffer and the slot array are free again
-    row_in<kPairThreads>(row, input + static_cast<int64_t>(r) * dim, dim, true);
-    __syncthreads();
-    float s0 = 0.0f;
-    float s1 = 0.0f;
-    for (int i = tid; i < pairs; i += kPairThreads)
-    {
-      float a, b;
-      load2<T>(row, i, a, b);
-      s0 = __fmaf_rn(a, a, s0);
-      s1 = __fmaf_rn(b, b, s1);
-    }
+    const int c = c0 + 256 * j;
+    x[j] = (live && c < dim) ? *reinterpret_cast<const Piece<T, V> *>(src + c) : zero_piece<T, V>();
+  }
+  float part[V];
 #pragma unroll
-    for (int off = 8; off > 0; off >>= 1)
-    {
-      s0 += __shfl_down_sync(0xFFFFFFFFu, s0, off, 16);
-      s1 += __shfl_down_sync(0xFFFFFFFFu, s1, off, 16);
-    }
-    s0 += s1;
-    if ((tid & 15) == 0)
-    {
-      warp_sums[tid >> 4] = s0;   // lane 0 of the reference's warp tid / 16
-    }
-    __syncthreads();
-    if (tid < 32)
-    {
-      float v = lane < kNormWarps ? warp_sums[lane] : 0.0f;
+  for (int i = 0; i < V; ++i)
+  {
+    part[i] = 0.0f;
+  }
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1)
-      {
-        v += __shfl_down_sync(0xFFFFFFFFu, v, off);
-      }
-      if (lane == 0)
-      {
-        warp_sums[kNormWarps] = v;
-      }
-    }
-    __syncthreads();
-    const float rms = __fsqrt_rn(__fadd_rn(__fdiv_rn(warp_sums[kNormWarps], static_cast<float>(dim)), epsilon));
-    if (tid == 0 && rms_cache != nullptr)
+  for (int j = 0; j < STRIPES; ++j)
+  {
+#pragma unroll
+    for (int i = 0; i < V; ++i)
     {
-      rms_cache[r] = rms;
+      const float v = x[j].get(i);
+      part[i] = __fmaf_rn(v, v, part[i]);   // (columns past the row add +0 to a non-negative sum)
     }
-    const float rstd = __fdiv_rn(1.0f, rms);
-    for (int i = tid; i < pairs; i += kPairThreads)
+    x[j].keep_packed();
+  }
+  const float total = row_sum<V>(part, sums[slot], warp_in_row);
+  const float rms = __fsqrt_rn(__fadd_rn(__fdiv_rn(total, static_cast<float>(dim)), epsilon));
+  const float rstd = __fdiv_rn(1.0f, rms);
+  if (!live)
+  {
+    return;
+  }
+  if (c0 == 0 && rms_cache != nullptr)
+  {
+    rms_cache[r] = rms;
+  }
+  T *dst = output + static_cast<int64_t>(r) * dim;
+#pragma unroll
+  for (int j = 0; j < STRIPES; ++j)
+  {
+    const int c = c0 + 256 * j;
+    if (c < dim)
     {
-      float a, b;
-      load2<T>(row, i, a, b);
-      const float2 g = __ldg(reinterpret_cast<const float2 *>(gamma) + i);
-      store2<T>(row, i, __fmul_rn(__fmul_rn(a, rstd), g.x), __fmul_rn(__fmul_rn(b, rstd), g.y));
+      const Gammas<V> g = load_gamma<V>(gamma, c);
+      float v[V];
+#pragma unroll
+      for (int i = 0; i < V; ++i)
+      {
+        v[i] = __fmul_rn(__fmul_rn(x[j].get(i), rstd), g.e[i]);
+      }
+      Piece<T, V> y;
+      y.set(v);
+      *reinterpret_cast<Piece<T, V> *>(dst + c) = y;
     }
-    __syncthreads();
-    row_out<kPairThreads>(output + static_cast<int64_t>(r) * dim, row, dim, true);
+  }
+}
+
+template <typename T, int V, int STRIPES>
+void rows_fwd_inst(const void *input, const float *gamma, void *output, float *rms_cache, float epsilon, int rows,
+                   int dim, cudaStream_t s)
+{
+  launch_dependent(rmsnorm_fwd_rows_kernel<T, V, STRIPES>, dim3(static_cast<unsigned>((rows + V - 1) / V)),
+                   dim3(kNormThreads), 0, s, static_cast<const T *>(input), gamma, static_cast<T *>(output), rms_cache,
+                   epsilon, rows, dim);
+}
+
+template <typename T>
+void rows_fwd(const void *input, const float *gamma, void *output, float *rms_cache, float epsilon, int rows, int dim,
+              cudaStream_t s)
+{
+  constexpr int WIDE = 16 / static_cast<int>(sizeof(T));
+  // 16-byte pieces need eight (fp32: four) rows a CTA and up to 96 registers of row: from a CTA per SM on
+  if (rows >= 148 * WIDE && dim <= 256 * 24)
+  {
+    if (dim <= 256 * 8)
+    {
+      rows_fwd_inst<T, WIDE, 8>(input, gamma, output, rms_cache, epsilon, rows, dim, s);
+    }
+    else if (dim <= 256 * 16)
+    {
+      rows_fwd_inst<T, WIDE, 16>(input, gamma, output, rms_cache, epsilon, rows, dim, s);
+    }
+    else
+    {
+      rows_fwd_inst<T, WIDE, 24>(input, gamma, output, rms_cache, epsilon, rows, dim, s);
+    }
+  }
+  else if (dim <= 256 * 16)
+  {
+    rows_fwd_inst<T, 2, 16>(input, gamma, output, rms_cache, epsilon, rows, dim, s);
+  }
+  else if (dim <= 256 * 32)
+  {
+    rows_fwd_inst<T, 2, 32>(input, gamma, output, rms_cache, epsilon, rows, dim, s);
+  }
+  else
+  {
+    rows_fwd_inst<T, 2, 64>(input, gamma, output, rms_cache, epsilon, rows, dim, s);
   }
 }
 
@@ -337,107 +486,182 @@ rmsnorm_bwd_kernel(const T *__restrict__ grad_output, const T *__restrict__ inpu
   }
 }
 
-// backward with two of the reference's threads per thread (rows up to 4096 wide: a thread keeps 32 sums of
-// grad_gamma); same reading as the paired forward kernel
-constexpr int kPairMaxTrips = kNormMaxPerThread / 2;
+// Backward with rows in registers (V = 2: four warps a row, two rows at a time per CTA, two CTAs per SM).  The next
+// row's pieces are loaded while the current one is worked on where the registers allow it.  grad_gamma: 32 sums a
+// thread at 4096 columns, the CTA's two halves meet in shared memory and leave as one two-wide reduction per thread
+// and column pair; with one atomic per column and 888 CTAs those were a third of the time (4096 x 4096 bf16: 60 us,
+// now 31).
+template <typename T, int STRIPES>
+__global__ void __launch_bounds__(kNormThreads, 2)
+rmsnorm_bwd_rows_kernel(const T *__restrict__ grad_output, const T *__restrict__ input, const float *__restrict__ gamma,
+                        const float *__restrict__ rms_cache, T *__restrict__ grad_input, float *__restrict__ grad_gamma,
+                        int rows, int dim, int gamma_vec)
+{
+  constexpr int V = 2;
+  constexpr bool PREFETCH = STRIPES * sizeof(T) <= 32;
+  __shared__ float sums[V][8];
+  extern __shared__ __align__(16) unsigned char norm_smem[];   // [dim] sums of the second half
+  const int slot = threadIdx.x >> 7;
+  const int warp_in_row = (threadIdx.x >> 5) & 3;
+  const int c0 = (threadIdx.x & 127) * V;
+  Piece<T, V> x[STRIPES], d[STRIPES];
+  float gg[STRIPES][V];
+#pragma unroll
+  for (int j = 0; j < STRIPES; ++j)
+  {
+    gg[j][0] = gg[j][1] = 0.0f;
+  }
+  auto load = [&](int r, Piece<T, V> (&xr)[STRIPES], Piece<T, V> (&dr)[STRIPES])
+  {
+    const bool live = r < rows;
+    const int64_t base = static_cast<int64_t>(live ? r : 0) * dim;
+#pragma unroll
+    for (int j = 0; j < STRIPES; ++j)
+    {
+      const int c = c0 + 256 * j;
+      xr[j] = (live && c < dim) ? *reinterpret_cast<const Piece<T, V> *>(input + base + c) : zero_piece<T, V>();
+      dr[j] = (live && c < dim) ? *reinterpret_cast<const Piece<T, V> *>(grad_output + base + c) : zero_piece<T, V>();
+    }
+  };
+  const int step = gridDim.x * V;
+  if (PREFETCH)
+  {
+    load(blockIdx.x * V + slot, x, d);
+  }
+  // every thread makes the same trips: the row sum has barriers
+  for (int r0 = blockIdx.x * V; r0 < rows; r0 += step)
+  {
+    const int r = r0 + slot;
+    const bool live = r < rows;
+    Piece<T, V> nx[STRIPES], nd[STRIPES];
+    if (PREFETCH)
+    {
+      load(r + step, nx, nd);
+    }
+    else
+    {
+      load(r, x, d);
+    }
+    const float rstd = __fdiv_rn(1.0f, live ? __ldg(rms_cache + r) : 1.0f);
+    float part[V] = {0.0f, 0.0f};
+#pragma unroll
+    for (int j = 0; j < STRIPES; ++j)
+    {
+      const int c = c0 + 256 * j;
+      if (c < dim)
+      {
+        const Gammas<V> g = load_gamma<V>(gamma, c);
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+        {
+          part[i] = __fmaf_rn(__fmul_rn(d[j].get(i), g.e[i]), __fmul_rn(x[j].get(i), rstd), part[i]);
+        }
+      }
+      x[j].keep_packed();
+      d[j].keep_packed();
+    }
+    const float sum_term = __fdiv_rn(row_sum<V>(part, sums[slot], warp_in_row), static_cast<float>(dim));
+    T *dst = grad_input + static_cast<int64_t>(live ? r : 0) * dim;
+#pragma unroll
+    for (int j = 0; j < STRIPES; ++j)
+    {
+      const int c = c0 + 256 * j;
+      if (live && c < dim)
+      {
+        const Gammas<V> g = load_gamma<V>(gamma, c);
+        float v[V];
+#pragma unroll
+        for (int i = 0; i < V; ++i)
+        {
+          const float dv = d[j].get(i);
+          const float h = __fmul_rn(x[j].get(i), rstd);
+          gg[j][i] = __fmaf_rn(dv, h, gg[j][i]);
+          v[i] = __fmul_rn(rstd, __fmaf_rn(dv, g.e[i], -__fmul_rn(h, sum_term)));
+        }
+        Piece<T, V> o;
+        o.set(v);
+        *reinterpret_cast<Piece<T, V> *>(dst + c) = o;
+      }
+    }
+    if (PREFETCH)
+    {
+#pragma unroll
+      for (int j = 0; j < STRIPES; ++j)
+      {
+        x[j] = nx[j];
+        d[j] = nd[j];
+      }
+    }
+  }
+  if (grad_gamma == nullptr)
+  {
+    return;
+  }
+  float2 *half = reinterpret_cast<float2 *>(norm_smem);
+  if (slot == 1)
+  {
+#pragma unroll
+    for (int j = 0; j < STRIPES; ++j)
+    {
+      const int c = c0 + 256 * j;
+      if (c < dim)
+      {
+        half[c >> 1] = make_float2(gg[j][0], gg[j][1]);
+      }
+    }
+  }
+  __syncthreads();
+  if (slot == 0)
+  {
+#pragma unroll
+    for (int j = 0; j < STRIPES; ++j)
+    {
+      const int c = c0 + 256 * j;
+      if (c < dim)
+      {
+        const float2 o = half[c >> 1];
+        const float a = gg[j][0] + o.x;
+        const float b = gg[j][1] + o.y;
+        if (gamma_vec)
+        {
+          asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(grad_gamma + c), "f"(a), "f"(b) : "memory");
+        }
+        else
+        {
+          atomicAdd(grad_gamma + c, a);
+          atomicAdd(grad_gamma + c + 1, b);
+        }
+      }
+    }
+  }
+}
+
+template <typename T, int STRIPES>
+void rows_bwd_inst(const void *dy, const void *x, const float *gamma, const float *rms, void *dx, float *grad_gamma,
+                   int rows, int dim, cudaStream_t s)
+{
+  const int pairs = (rows + 1) / 2;
+  const int grid = pairs < 148 * 2 ? pairs : 148 * 2;
+  rmsnorm_bwd_rows_kernel<T, STRIPES><<<grid, kNormThreads, static_cast<size_t>(dim) * 4, s>>>(
+      static_cast<const T *>(dy), static_cast<const T *>(x), gamma, rms, static_cast<T *>(dx), grad_gamma, rows, dim,
+      (reinterpret_cast<uintptr_t>(grad_gamma) & 7u) == 0 ? 1 : 0);
+}
 
 template <typename T>
-__global__ void __launch_bounds__(kPairThreads, 6)
-rmsnorm_bwd_pair_kernel(const T *__restrict__ grad_output, const T *__restrict__ input,
-                        const float *__restrict__ gamma, const float *__restrict__ rms_cache,
-                        T *__restrict__ grad_input, float *__restrict__ grad_gamma, int rows, int dim)
+void rows_bwd(const void *dy, const void *x, const float *gamma, const float *rms, void *dx, float *grad_gamma,
+              int rows, int dim, cudaStream_t s)
 {
-  extern __shared__ __align__(16) unsigned char norm_smem[];
-  __shared__ float warp_sums[kNormWarps + 1];
-  T *xrow = reinterpret_cast<T *>(norm_smem);
-  T *grow = xrow + dim;
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int pairs = dim >> 1;
-  float gg[kNormMaxPerThread];
-#pragma unroll
-  for (int j = 0; j < kNormMaxPerThread; ++j)
+  if (dim <= 256 * 8)
   {
-    gg[j] = 0.0f;
+    rows_bwd_inst<T, 8>(dy, x, gamma, rms, dx, grad_gamma, rows, dim, s);
   }
-  for (int r = blockIdx.x; r < rows; r += gridDim.x)
+  else if (dim <= 256 * 16)
   {
-    __syncthreads();
-    row_in<kPairThreads>(xrow, input + static_cast<int64_t>(r) * dim, dim, true);
-    row_in<kPairThreads>(grow, grad_output + static_cast<int64_t>(r) * dim, dim, true);
-    __syncthreads();
-    const float rstd = __fdiv_rn(1.0f, __ldg(rms_cache + r));
-    float s0 = 0.0f;
-    float s1 = 0.0f;
-    for (int i = tid; i < pairs; i += kPairThreads)
-    {
-      float xa, xb, da, db;
-      load2<T>(xrow, i, xa, xb);
-      load2<T>(grow, i, da, db);
-      const float2 g = __ldg(reinterpret_cast<const float2 *>(gamma) + i);
-      s0 = __fmaf_rn(__fmul_rn(da, g.x), __fmul_rn(xa, rstd), s0);
-      s1 = __fmaf_rn(__fmul_rn(db, g.y), __fmul_rn(xb, rstd), s1);
-    }
-#pragma unroll
-    for (int off = 8; off > 0; off >>= 1)
-    {
-      s0 += __shfl_down_sync(0xFFFFFFFFu, s0, off, 16);
-      s1 += __shfl_down_sync(0xFFFFFFFFu, s1, off, 16);
-    }
-    s0 += s1;
-    if ((tid & 15) == 0)
-    {
-      warp_sums[tid >> 4] = s0;
-    }
-    __syncthreads();
-    if (tid < 32)
-    {
-      float v = lane < kNormWarps ? warp_sums[lane] : 0.0f;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1)
-      {
-        v += __shfl_down_sync(0xFFFFFFFFu, v, off);
-      }
-      if (lane == 0)
-      {
-        warp_sums[kNormWarps] = v;
-      }
-    }
-    __syncthreads();
-    const float sum_term = __fdiv_rn(warp_sums[kNormWarps], static_cast<float>(dim));
-#pragma unroll
-    for (int j = 0; j < kPairMaxTrips; ++j)
-    {
-      const int i = tid + j * kPairThreads;
-      if (i < pairs)
-      {
-        float xa, xb, da, db;
-        load2<T>(xrow, i, xa, xb);
-        load2<T>(grow, i, da, db);
-        const float2 g = __ldg(reinterpret_cast<const float2 *>(gamma) + i);
-        const float ha = __fmul_rn(xa, rstd);
-        const float hb = __fmul_rn(xb, rstd);
-        gg[2 * j] = __fmaf_rn(da, ha, gg[2 * j]);
-        gg[2 * j + 1] = __fmaf_rn(db, hb, gg[2 * j + 1]);
-        store2<T>(xrow, i, __fmul_rn(rstd, __fmaf_rn(da, g.x, -__fmul_rn(ha, sum_term))),
-                  __fmul_rn(rstd, __fmaf_rn(db, g.y, -__fmul_rn(hb, sum_term))));
-      }
-    }
-    __syncthreads();
-    row_out<kPairThreads>(grad_input + static_cast<int64_t>(r) * dim, xrow, dim, true);
+    rows_bwd_inst<T, 16>(dy, x, gamma, rms, dx, grad_gamma, rows, dim, s);
   }
-  if (grad_gamma != nullptr)
+  else if constexpr (sizeof(T) == 2)
   {
-#pragma unroll
-    for (int j = 0; j < kPairMaxTrips; ++j)
-    {
-      const int i = tid + j * kPairThreads;
-      if (i < pairs)
-      {
-        atomicAdd(grad_gamma + 2 * i, gg[2 * j]);
-        atomicAdd(grad_gamma + 2 * i + 1, gg[2 * j + 1]);
-      }
-    }
+    rows_bwd_inst<T, 24>(dy, x, gamma, rms, dx, grad_gamma, rows, dim, s);
   }
 }
 
@@ -463,35 +687,39 @@ int launch_rmsnorm_fwd(const void *input, const float *gamma, void *output, floa
     return CAIFQ_OK;
   }
   const size_t elem = (dtype == CAIFQ_F32) ? 4 : 2;
+  const int vec = rows_vectorizable(input, output, dim, elem) ? 1 : 0;
+  if (vec != 0 && dim <= 256 * 64 && (reinterpret_cast<uintptr_t>(gamma) & 15u) == 0)
+  {
+    if (dtype == CAIFQ_F32)
+    {
+      rows_fwd<float>(input, gamma, output, rms_cache, epsilon, rows, dim, s);
+    }
+    else if (dtype == CAIFQ_F16)
+    {
+      rows_fwd<__half>(input, gamma, output, rms_cache, epsilon, rows, dim, s);
+    }
+    else
+    {
+      rows_fwd<__nv_bfloat16>(input, gamma, output, rms_cache, epsilon, rows, dim, s);
+    }
+    CAIFQ_CHECK_LAUNCH();
+    return CAIFQ_OK;
+  }
   const size_t smem = static_cast<size_t>(dim) * elem;
   if (smem > 96 * 1024)
   {
     set_error("rmsnorm: rows of %d elements do not fit the row buffer", dim);
     return CAIFQ_ERR_UNSUPPORTED;
   }
-  const int vec = rows_vectorizable(input, output, dim, elem) ? 1 : 0;
-  const bool pair = vec != 0 && (dim % 2) == 0 && (reinterpret_cast<uintptr_t>(gamma) & 7u) == 0;
 #define CAIFQ_NORM_FWD(T)                                                                                        \
   {                                                                                                               \
     if (smem > 48 * 1024)                                                                                         \
     {                                                                                                             \
       cudaFuncSetAttribute(rmsnorm_fwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);        \
     }                                                                                                             \
-    if (pair)                                                                                                     \
-    {                                                                                                             \
-      if (smem > 48 * 1024)                                                                                       \
-      {                                                                                                           \
-        cudaFuncSetAttribute(rmsnorm_fwd_pair_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024); \
-      }                                                                                                           \
-      rmsnorm_fwd_pair_kernel<T><<<norm_grid(rows, 16), kPairThreads, smem, s>>>(                                 \
-          static_cast<const T *>(input), gamma, static_cast<T *>(output), rms_cache, epsilon, rows, dim);         \
-    }                                                                                                             \
-    else                                                                                                          \
-    {                                                                                                             \
-      rmsnorm_fwd_kernel<T><<<norm_grid(rows, 8), kNormThreads, smem, s>>>(static_cast<const T *>(input), gamma,  \
-                                                                           static_cast<T *>(output), rms_cache,   \
-                                                                           epsilon, rows, dim, vec);              \
-    }                                                                                                             \
+    rmsnorm_fwd_kernel<T><<<norm_grid(rows, 8), kNormThreads, smem, s>>>(static_cast<const T *>(input), gamma,    \
+                                                                         static_cast<T *>(output), rms_cache,     \
+                                                                         epsilon, rows, dim, vec);                \
   }
   if (dtype == CAIFQ_F32)
     CAIFQ_NORM_FWD(float)
@@ -521,26 +749,33 @@ int launch_rmsnorm_bwd(const void *grad_output, const void *input, const float *
   const int vec = (rows_vectorizable(input, grad_input, dim, elem) && rows_vectorizable(grad_output, grad_output, dim, elem))
                       ? 1
                       : 0;
-  const bool pair = vec != 0 && (dim % 2) == 0 && dim <= kPairThreads * 2 * kPairMaxTrips && smem <= 48 * 1024 &&
-                    (reinterpret_cast<uintptr_t>(gamma) & 7u) == 0;
+  // (fp32 rows of more than 4096 columns do not fit the registers beside their share of grad_gamma)
+  if (vec != 0 && dim <= 256 * (elem == 4 ? 16 : 24) && (reinterpret_cast<uintptr_t>(gamma) & 15u) == 0)
+  {
+    if (dtype == CAIFQ_F32)
+    {
+      rows_bwd<float>(grad_output, input, gamma, rms_cache, grad_input, grad_gamma, rows, dim, s);
+    }
+    else if (dtype == CAIFQ_F16)
+    {
+      rows_bwd<__half>(grad_output, input, gamma, rms_cache, grad_input, grad_gamma, rows, dim, s);
+    }
+    else
+    {
+      rows_bwd<__nv_bfloat16>(grad_output, input, gamma, rms_cache, grad_input, grad_gamma, rows, dim, s);
+    }
+    CAIFQ_CHECK_LAUNCH();
+    return CAIFQ_OK;
+  }
 #define CAIFQ_NORM_BWD(T)                                                                                        \
   {                                                                                                               \
-    if (pair)                                                                                                     \
+    if (smem > 48 * 1024)                                                                                         \
     {                                                                                                             \
-      rmsnorm_bwd_pair_kernel<T><<<norm_grid(rows, 6), kPairThreads, smem, s>>>(                                  \
-          static_cast<const T *>(grad_output), static_cast<const T *>(input), gamma, rms_cache,                   \
-          static_cast<T *>(grad_input), grad_gamma, rows, dim);                                                   \
+      cudaFuncSetAttribute(rmsnorm_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);        \
     }                                                                                                             \
-    else                                                                                                          \
-    {                                                                                                             \
-      if (smem > 48 * 1024)                                                                                       \
-      {                                                                                                           \
-        cudaFuncSetAttribute(rmsnorm_bwd_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);      \
-      }                                                                                                           \
-      rmsnorm_bwd_kernel<T><<<norm_grid(rows, 4), kNormThreads, smem, s>>>(                                       \
-          static_cast<const T *>(grad_output), static_cast<const T *>(input), gamma, rms_cache,                   \
-          static_cast<T *>(grad_input), grad_gamma, rows, dim, vec);                                              \
-    }                                                                                                             \
+    rmsnorm_bwd_kernel<T><<<norm_grid(rows, 4), kNormThreads, smem, s>>>(                                         \
+        static_cast<const T *>(grad_output), static_cast<const T *>(input), gamma, rms_cache,                     \
+        static_cast<T *>(grad_input), grad_gamma, rows, dim, vec);                                                \
   }
   if (dtype == CAIFQ_F32)
     CAIFQ_NORM_BWD(float)

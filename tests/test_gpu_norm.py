@@ -62,3 +62,34 @@ def test_rmsnorm_edge_cases():
     assert torch.equal(z, torch.zeros(2, 16, device="cuda")) and torch.all(rms == np.float32(1e-6) ** 0.5)
     with pytest.raises(nv.CaifqError, match="row buffer"):
         nv.rmsnorm_fwd(torch.zeros(1, 30000, device="cuda"), torch.ones(30000, device="cuda"))
+
+
+@pytest.mark.parametrize("dtype,rows,dim", [
+    (torch.bfloat16, 1, 2048), (torch.bfloat16, 5, 4096), (torch.bfloat16, 1185, 4096), (torch.bfloat16, 1190, 6144),
+    (torch.bfloat16, 1201, 1416), (torch.bfloat16, 7, 16384), (torch.float32, 600, 4096), (torch.float32, 3, 6144),
+    (torch.float16, 1184, 2056), (torch.bfloat16, 300, 264),
+])
+def test_rmsnorm_rows_in_registers_match_the_element_kernels(dtype, rows, dim):
+    """Edges of the register forms (rows per CTA, stripes of 256 columns, the last one partial) against the kernels
+    with one thread per column, which rows that do not start on 16 bytes take: the same bits."""
+    g = torch.Generator(device="cuda").manual_seed(rows + dim)
+    x = torch.randn(rows, dim, generator=g, device="cuda").to(dtype)
+    dy = torch.randn(rows, dim, generator=g, device="cuda").to(dtype)
+    gamma = torch.randn(dim, generator=g, device="cuda")
+
+    def shifted(t):
+        flat = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")
+        flat[1:] = t.reshape(-1)
+        return flat[1:].view(rows, dim)
+
+    y, rms = nv.rmsnorm_fwd(x, gamma)
+    if dim * x.element_size() <= 96 * 1024:
+        y2, rms2 = nv.rmsnorm_fwd(shifted(x), gamma)
+        assert torch.equal(y, y2) and torch.equal(rms, rms2)
+    want = x.float() / torch.sqrt(x.float().square().mean(-1, keepdim=True) + 1e-5) * gamma
+    assert float((y.float() - want).abs().max()) <= (1e-5 if dtype == torch.float32 else 5e-2) * float(want.abs().max())
+    if dim <= 8192:
+        dx, dg = nv.rmsnorm_bwd(dy, x, gamma, rms)
+        dx2, dg2 = nv.rmsnorm_bwd(shifted(dy), shifted(x), gamma, rms)
+        assert torch.equal(dx, dx2)
+        assert float((dg - dg2).abs().max()) <= 1e-4 * float(dg2.abs().max())
