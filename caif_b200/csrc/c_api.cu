@@ -260,6 +260,11 @@ int linear_any(const caifq_weight *w, bool backward, const void *a, int a_dtype,
     set_path("decode");
     return launch_linear_decode(args, s);
   }
+  if ((force == Force::None || force == Force::Decode) && rows_supported(args))
+  {
+    set_path("decode");
+    return launch_linear_rows(args, s);
+  }
   if ((force == Force::None || force == Force::Umma) && umma_supported(args))
   {
     set_path("umma");

@@ -345,6 +345,10 @@ void umma_stall_next_launch();
 bool decode_supported(const LinearArgs &args);
 int launch_linear_decode(const LinearArgs &args, cudaStream_t s);
 
+// bf16 weights, few rows (forward only)
+bool rows_supported(const LinearArgs &args);
+int launch_linear_rows(const LinearArgs &args, cudaStream_t s);
+
 // tcgen05 / TMEM tensor-core kernel for many tokens
 bool umma_supported(const LinearArgs &args);
 int launch_linear_umma(const LinearArgs &args, cudaStream_t s);

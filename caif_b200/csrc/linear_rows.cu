@@ -1,0 +1,152 @@
+// Forward product of a bf16 weight with few rows of bf16 activations:
+//
+//   y[m, out] = x[m, in] . W[out, in]^T  (+ y)        m <= 16, or 64 for a narrow weight
+//
+// The float-storage cell of CAIF_DeviceFrozenLinear (src/caif_device_frozen_linear.cpp:381-524) and the router's
+// product over the experts (src/caif_device_moe_router.cpp:233-260).  Bound by reading the weight once when it is
+// large, by latency when it is small: a router of 64 x 2048 on 16 tokens ran as ONE block of the fp32-FMA kernel that
+// walked all of k (219 us).  Here a CTA owns NT * 8 output columns and 16 rows, its eight warps split k and stream both
+// operands from global memory straight into bf16 tensor-core fragments, sixteen bytes a lane and operand (the order
+// of k inside a fragment is the same for both, which is all a dot product needs); the eight partial tiles meet in
+// shared memory.  Products are exact in fp32 and accumulate in fp32, so fp32 and bf16 compute are the same here.
+#include "common.cuh"
+
+namespace caifq
+{
+
+namespace
+{
+
+constexpr int kRowsWarps = 8;
+constexpr int kRowsUnroll = 4;   // k-steps of 32 whose loads are in flight per warp
+
+__device__ __forceinline__ void mma_rows(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
+                                         uint32_t b1)
+{
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+template <int NT>
+__global__ void __launch_bounds__(kRowsWarps * 32)
+linear_rows_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w, void *y, int y_dtype,
+                   int accumulate, int64_t m, int in_dim, int out_dim)
+{
+  __shared__ float part[kRowsWarps][16][NT * 8 + 1];
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int g = lane >> 2;
+  const int t = lane & 3;
+  const int64_t row0 = static_cast<int64_t>(blockIdx.y) * 16;
+  const int col0 = static_cast<int>(blockIdx.x) * NT * 8;
+  const bool lo_ok = row0 + g < m;
+  const bool hi_ok = row0 + g + 8 < m;
+  const int steps = in_dim / 32;
+  const int begin = (steps * warp) / kRowsWarps;
+  const int end = (steps * (warp + 1)) / kRowsWarps;
+  const uint4 *x_lo = reinterpret_cast<const uint4 *>(x + (lo_ok ? row0 + g : 0) * in_dim) + t;
+  const uint4 *x_hi = reinterpret_cast<const uint4 *>(x + (hi_ok ? row0 + g + 8 : 0) * in_dim) + t;
+  const uint4 *w_ptr[NT];
+  float c[NT][4];
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+  {
+    // columns past the last one read it again; they are not stored
+    const int col = min(col0 + nt * 8 + g, out_dim - 1);
+    w_ptr[nt] = reinterpret_cast<const uint4 *>(w + static_cast<int64_t>(col) * in_dim) + t;
+    c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.0f;
+  }
+  const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
+  for (int st = begin; st < end; st += kRowsUnroll)
+  {
+    uint4 xa[kRowsUnroll], xb[kRowsUnroll], wv[kRowsUnroll][NT];
+#pragma unroll
+    for (int u = 0; u < kRowsUnroll; ++u)
+    {
+      const bool in = st + u < end;
+      xa[u] = (in && lo_ok) ? __ldg(x_lo + (st + u) * 4) : zero4;
+      xb[u] = (in && hi_ok) ? __ldg(x_hi + (st + u) * 4) : zero4;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+      {
+        wv[u][nt] = in ? __ldg(w_ptr[nt] + (st + u) * 4) : zero4;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kRowsUnroll; ++u)
+    {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+      {
+        mma_rows(c[nt], xa[u].x, xb[u].x, xa[u].y, xb[u].y, wv[u][nt].x, wv[u][nt].y);
+        mma_rows(c[nt], xa[u].z, xb[u].z, xa[u].w, xb[u].w, wv[u][nt].z, wv[u][nt].w);
+      }
+    }
+  }
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt)
+  {
+    part[warp][g][nt * 8 + 2 * t] = c[nt][0];
+    part[warp][g][nt * 8 + 2 * t + 1] = c[nt][1];
+    part[warp][g + 8][nt * 8 + 2 * t] = c[nt][2];
+    part[warp][g + 8][nt * 8 + 2 * t + 1] = c[nt][3];
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < 16 * NT * 8; e += kRowsWarps * 32)
+  {
+    const int r = e / (NT * 8);
+    const int col = e % (NT * 8);
+    if (row0 + r >= m || col0 + col >= out_dim)
+    {
+      continue;
+    }
+    float v = 0.0f;
+#pragma unroll
+    for (int wi = 0; wi < kRowsWarps; ++wi)
+    {
+      v += part[wi][r][col];
+    }
+    const int64_t idx = (row0 + r) * out_dim + col0 + col;
+    if (accumulate)
+    {
+      v = round_through_rt(v, y_dtype) + load_as_float(y, idx, y_dtype);
+    }
+    store_from_float(y, idx, y_dtype, v);
+  }
+}
+
+}  // namespace
+
+// few tokens; for outputs narrower than a tensor-core tile (routers) up to 64, where that kernel's one tile is full enough
+bool rows_supported(const LinearArgs &g)
+{
+  return !g.backward && g.w.storage == CAIFQ_BF16 && g.a_dtype == CAIFQ_BF16 && g.a_prescale == 1.0f && g.m >= 1 &&
+         g.m <= (g.w.out_dim < 128 ? 64 : 16) && (g.compute_dtype == CAIFQ_F32 || g.compute_dtype == CAIFQ_BF16) && (g.w.in_dim % 32) == 0 &&
+         ((reinterpret_cast<uintptr_t>(g.a) | reinterpret_cast<uintptr_t>(g.w.codes)) & 15u) == 0 && g.num_peers == 0 &&
+         g.num_more == 0;
+}
+
+int launch_linear_rows(const LinearArgs &g, cudaStream_t s)
+{
+  const unsigned row_tiles = static_cast<unsigned>((g.m + 15) / 16);
+  const __nv_bfloat16 *x = static_cast<const __nv_bfloat16 *>(g.a);
+  const __nv_bfloat16 *w = static_cast<const __nv_bfloat16 *>(g.w.codes);
+  const int acc = g.accumulate ? 1 : 0;
+  // 32 columns a CTA share the activations' loads; narrow outputs take 8, for more CTAs
+  const int wide = (g.w.out_dim + 31) / 32;
+  if (wide * row_tiles >= 148)
+  {
+    linear_rows_kernel<4><<<dim3(static_cast<unsigned>(wide), row_tiles), kRowsWarps * 32, 0, s>>>(
+        x, w, g.c, g.c_dtype, acc, g.m, g.w.in_dim, g.w.out_dim);
+  }
+  else
+  {
+    linear_rows_kernel<1><<<dim3(static_cast<unsigned>((g.w.out_dim + 7) / 8), row_tiles), kRowsWarps * 32, 0, s>>>(
+        x, w, g.c, g.c_dtype, acc, g.m, g.w.in_dim, g.w.out_dim);
+  }
+  CAIFQ_CHECK_LAUNCH();
+  return CAIFQ_OK;
+}
+
+}  // namespace caifq

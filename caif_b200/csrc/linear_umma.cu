@@ -1608,7 +1608,9 @@ bool umma_supported(const LinearArgs &g)
   }
   const int n_total = g.backward ? w.in_dim : w.out_dim;
   const int k_total = g.backward ? w.out_dim : w.in_dim;
-  if ((n_total % 128) != 0 || (k_total % BK) != 0)
+  // (a bf16 weight's tiles are copies, zero past the matrix's edge: its last column tile may be partial, down to the
+  // 32 columns of an epilogue step, so that a router of 64 experts runs here too)
+  if ((n_total % (w.storage == CAIFQ_BF16 ? 32 : 128)) != 0 || (k_total % BK) != 0)
   {
     return false;
   }
@@ -1690,7 +1692,7 @@ int launch_linear_umma(const LinearArgs &g, cudaStream_t s)
   {
     bn = 128;   // a single CTA has 128-wide tiles only in the two-plane mode
   }
-  p.num_n_tiles = p.n_total / bn;
+  p.num_n_tiles = (p.n_total + bn - 1) / bn;
 
   CUtensorMap map_a;
   CUtensorMap map_b;
@@ -1780,7 +1782,8 @@ bool umma_grouped_supported(const GroupedLinearArgs &g)
     return false;
   }
   const caifq_weight &w0 = g.weights[0];
-  if (w0.storage != CAIFQ_I8 && w0.storage != CAIFQ_I4 && w0.storage != CAIFQ_BF16)
+  if ((w0.storage != CAIFQ_I8 && w0.storage != CAIFQ_I4 && w0.storage != CAIFQ_BF16) ||
+      ((g.backward ? w0.in_dim : w0.out_dim) % 128) != 0)
   {
     return false;
   }

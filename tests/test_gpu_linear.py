@@ -524,3 +524,34 @@ def test_layers_sharing_their_input_as_one_product_over_concatenated_weights(sto
     rc = nv.lib().caifq_linear_fwd_concat(arr, 3, nv._ptr(x), nv.BF16, m, nv._ptr(y2), nv.F32, nv.F32, nv._ptr(big),
                                           big.numel(), nv._stream())
     assert rc == 1 and b"BF16" in nv.lib().caifq_last_error()
+
+
+@pytest.mark.parametrize("m,in_dim,out_dim,sd", [
+    (1, 2048, 64, orc.F32), (16, 2048, 20, orc.F32), (17, 96, 8, orc.BF16), (64, 1056, 96, orc.F16), (9, 1056, 4096, orc.F16),
+    (40, 32, 33, orc.F32),     # fewer k-steps than warps, a ragged last column tile
+])
+def test_few_rows_on_a_bf16_weight(m, in_dim, out_dim, sd):
+    rng = np.random.default_rng(m + in_dim + out_dim)
+    weight, codes, _ = make_weight(rng, out_dim, in_dim, orc.BF16)
+    x_np, x = act(rng, m, in_dim, orc.BF16)
+    res_np, res = act(rng, m, out_dim, sd)
+    want = orc.frozen_linear_forward(x_np, _oracle_w(weight, codes, None, orc.F32))
+    y = nv.linear_fwd(weight, x, torch.float32, orc.F32)
+    assert nv.last_path() == "decode"
+    assert max_rel_err(y.cpu().numpy(), want) <= TOL_F32
+    got = nv.linear_fwd_residual(weight, x, res.clone(), orc.F32)
+    sep = nv.linear_fwd(weight, x, TORCH_DTYPE[sd], orc.F32)
+    assert torch.equal(got, (sep.float() + res.float()).to(TORCH_DTYPE[sd]))
+
+
+@pytest.mark.parametrize("m,in_dim,out_dim", [(65, 2048, 64), (300, 512, 96), (700, 256, 160)])
+def test_umma_bf16_weight_with_a_partial_last_column_tile(m, in_dim, out_dim):
+    weight, wc, x_np, x, dy_np, dy = _umma_case(orc.BF16, orc.F32, m, in_dim, out_dim, m + out_dim)
+    y = nv.linear_fwd(weight, x, torch.float32, orc.F32)
+    assert nv.last_path() == "umma"
+    assert max_rel_err(y.cpu().numpy(), orc.frozen_linear_forward(x_np, wc)) <= TOL_F32
+    if out_dim % 64 == 0:      # dX reduces over the output features, 64 at a time
+        weight, wc, x_np, x, dy_np, dy = _umma_case(orc.BF16, orc.F32, m, out_dim + 32, 128, m)
+        dx = nv.linear_dx(weight, dy, torch.float32, orc.F32)
+        assert nv.last_path() == "umma"
+        assert max_rel_err(dx.cpu().numpy(), orc.frozen_linear_backward(dy_np, wc)) <= TOL_F32
