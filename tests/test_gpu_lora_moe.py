@@ -164,6 +164,17 @@ def test_dispatch_map_bit_exact(tokens, top_k, experts, capacity):
     assert np.array_equal(dmap.cpu().numpy(), odmap)
 
 
+@pytest.mark.parametrize("entries,experts", [(1024, 3), (1025, 64), (148 * 1024, 9), (148 * 1024 + 5, 300)])
+def test_dispatch_map_over_slices_bit_exact(entries, experts):
+    """One slice, a second one of a single entry, a full set of one-chunk slices, slices of two chunks."""
+    rng = np.random.default_rng(entries + experts)
+    idx = rng.integers(-1, experts + 1, (entries, 1)).astype(np.int32)
+    dmap, off = nv.moe_build_dispatch(to_dev(idx), experts, 0)
+    odmap, ooff, _ = orc.build_dispatch_map(idx, experts, 0)
+    assert np.array_equal(off.cpu().numpy(), ooff)
+    assert np.array_equal(dmap.cpu().numpy(), odmap)
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_dispatch_and_combine(dtype):
     rng = np.random.default_rng(19)
