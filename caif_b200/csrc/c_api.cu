@@ -1077,15 +1077,10 @@ int concat_run(const caifq_weight *ws, int32_t count, bool backward, const void 
               who);
     return CAIFQ_ERR_UNSUPPORTED;
   }
-  uint8_t *dst = static_cast<uint8_t *>(workspace);
-  for (int i = 0; i < count; ++i)
+  rc = launch_weights_to_bf16_scaled(ws, count, workspace, s);
+  if (rc != CAIFQ_OK)
   {
-    rc = launch_weight_to_bf16_scaled(ws[i], dst, s);
-    if (rc != CAIFQ_OK)
-    {
-      return rc;
-    }
-    dst += static_cast<size_t>(ws[i].out_dim) * static_cast<size_t>(ws[i].in_dim) * 2;
+    return rc;
   }
   return linear_any(&cat, backward, a, a_dtype, 1.0f, m, c, c_dtype, false, compute_dtype, s, who);
 }

@@ -150,6 +150,36 @@ __device__ __forceinline__ uint4 expand_int4x8(const uint32_t w, const float sca
   return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
+// group of a flat weight index: a shift where the group size is a power of two (shift >= 0), else a division
+struct GroupOf
+{
+  int size;
+  int shift;
+
+  __host__ static GroupOf make(int size)
+  {
+    GroupOf g{size, -1};
+    for (int b = 0; b < 31; ++b)
+    {
+      if (size == (1 << b))
+      {
+        g.shift = b;
+      }
+    }
+    return g;
+  }
+
+  __device__ __forceinline__ int64_t operator()(int64_t flat) const { return shift >= 0 ? flat >> shift : flat / size; }
+};
+
+// sixteen bf16 values as one 32-byte store: a warp writes a contiguous kilobyte
+__device__ __forceinline__ void store_bf16x16(void *p, const uint4 a, const uint4 b)
+{
+  asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w),
+               "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+               : "memory");
+}
+
 // Round an fp32 value through a 16-bit float dtype (nearest even) and back.
 template <int DTYPE>
 __device__ __forceinline__ float round_through(float v)
@@ -224,6 +254,111 @@ __device__ __forceinline__ float weight_value(const caifq_weight &w, int64_t fla
   }
 }
 
+// int8 codes with the per-tensor scale inside the value: bf16(float(code) * scale)
+__device__ __forceinline__ uint4 expand_int8x8_scaled(const uint2 v, const float sc)
+{
+  const uint32_t w[2] = {v.x, v.y};
+  uint32_t o[4];
+#pragma unroll
+  for (int k = 0; k < 2; ++k)
+  {
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+    {
+      const float lo = __fmul_rn(static_cast<float>(static_cast<int8_t>((w[k] >> (16 * h)) & 0xFFu)), sc);
+      const float hi = __fmul_rn(static_cast<float>(static_cast<int8_t>((w[k] >> (16 * h + 8)) & 0xFFu)), sc);
+      asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[2 * k + h]) : "f"(hi), "f"(lo));
+    }
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+enum ExpandMode
+{
+  EXPAND_I8,         // exact integers, the scale is applied later
+  EXPAND_I8_SCALED,  // scales: one fp32
+  EXPAND_I4          // scales: fp16 per group
+};
+
+// Codes of one matrix -> bf16 (see expand_int8x8 / expand_int4x8), `units` eights of them, by the whole x dimension of
+// the grid.  A thread takes two neighbouring units and stores them as one 32-byte piece (dst is 32-byte aligned, codes
+// 16- / 8-byte); kPerTrip such pieces a trip, a block width apart, so that all the loads are in flight before the first
+// conversion and a warp's accesses stay contiguous.
+template <int MODE>
+__device__ __forceinline__ void expand_span(const void *codes, const void *scale_ptr, uint4 *dst, int64_t units,
+                                            GroupOf group_of)
+{
+  constexpr int kPerTrip = 4;
+  const __half *scales = static_cast<const __half *>(scale_ptr);
+  const float tensor_scale = (MODE == EXPAND_I8_SCALED) ? __ldg(static_cast<const float *>(scale_ptr)) : 1.0f;
+  auto int8x8 = [&](const uint2 v)
+  { return (MODE == EXPAND_I8_SCALED) ? expand_int8x8_scaled(v, tensor_scale) : expand_int8x8(v); };
+  const int64_t pairs = units >> 1;
+  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x * kPerTrip;
+  for (int64_t base = static_cast<int64_t>(blockIdx.x) * blockDim.x * kPerTrip + threadIdx.x; base < pairs; base += stride)
+  {
+    if constexpr (MODE != EXPAND_I4)
+    {
+      uint4 c[kPerTrip];
+#pragma unroll
+      for (int u = 0; u < kPerTrip; ++u)
+      {
+        const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
+        c[u] = (i < pairs) ? __ldg(static_cast<const uint4 *>(codes) + i) : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int u = 0; u < kPerTrip; ++u)
+      {
+        const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
+        if (i < pairs)
+        {
+          store_bf16x16(dst + 2 * i, int8x8(make_uint2(c[u].x, c[u].y)), int8x8(make_uint2(c[u].z, c[u].w)));
+        }
+      }
+    }
+    else
+    {
+      uint2 c[kPerTrip];
+      __half sc[kPerTrip][2];
+#pragma unroll
+      for (int u = 0; u < kPerTrip; ++u)
+      {
+        const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
+        c[u] = make_uint2(0u, 0u);
+        sc[u][0] = sc[u][1] = __half();
+        if (i < pairs)
+        {
+          c[u] = __ldg(static_cast<const uint2 *>(codes) + i);
+          sc[u][0] = __ldg(scales + group_of(16 * i));   // eight codes lie in one group
+          sc[u][1] = __ldg(scales + group_of(16 * i + 8));
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kPerTrip; ++u)
+      {
+        const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
+        if (i < pairs)
+        {
+          store_bf16x16(dst + 2 * i, expand_int4x8(c[u].x, __half2float(sc[u][0])),
+                        expand_int4x8(c[u].y, __half2float(sc[u][1])));
+        }
+      }
+    }
+  }
+  if ((units & 1) != 0 && blockIdx.x == 0 && threadIdx.x == 0)
+  {
+    const int64_t i = units - 1;
+    if constexpr (MODE != EXPAND_I4)
+    {
+      dst[i] = int8x8(static_cast<const uint2 *>(codes)[i]);
+    }
+    else
+    {
+      dst[i] = expand_int4x8(static_cast<const uint32_t *>(codes)[i], __half2float(scales[group_of(8 * i)]));
+    }
+  }
+}
+
 // ---- launchers implemented in the individual .cu files ----------------------
 
 int launch_quantize_int8_per_tensor(const float *x, int8_t *q, float *scale, int64_t n, cudaStream_t s);
@@ -238,9 +373,9 @@ int launch_cast(const void *src, int src_dtype, void *dst, int dst_dtype, int64_
 int launch_weight_materialize(const caifq_weight &w, void *dst, int dst_dtype, cudaStream_t s);
 // int8 / int4 codes -> a bf16 [out, in] matrix for the tensor core: int8 codes as exact integers (the scale
 // is left to the epilogue), int4 as bf16(scale * code), the reference's dequantize-then-cast value
-int launch_expand_to_bf16(const caifq_weight &w, void *dst, cudaStream_t s);
-// the weight as the bf16 matrix bf16 compute sees (scales inside the values): int4, int8 per-tensor, floats
-int launch_weight_to_bf16_scaled(const caifq_weight &w, void *dst, cudaStream_t s);
+// weights laid one under the other as the bf16 matrix bf16 compute sees (scales inside the values): int4, int8
+// per-tensor, floats
+int launch_weights_to_bf16_scaled(const caifq_weight *ws, int count, void *dst, cudaStream_t s);
 // the same for `count` experts of one shape in one launch; expert e lands at dst + e * out * in elements
 int launch_expand_grouped_to_bf16(const caifq_weight *ws, int count, void *dst, cudaStream_t s);
 

@@ -596,7 +596,7 @@ struct ExpandPrepare
   const __half *scales;
   uint4 *wb;
   int64_t units;      // weights / 8
-  int group_size;
+  GroupOf group_of;
   const __nv_bfloat16 *a;   // [r, n_a]
   const __nv_bfloat16 *b;   // [n_b, r]
   __nv_bfloat16 *bp;        // forward: [n_b, 64]
@@ -605,65 +605,14 @@ struct ExpandPrepare
   int n_a, n_b, r;
 };
 
-template <int STORAGE>
+template <int MODE>
 __global__ void expand_prepare_kernel(const ExpandPrepare p)
 {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t first = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (blockIdx.y == 0)
   {
-    // four units per thread and trip, a block width apart: the loads are all in flight before the first
-    // conversion and a warp's accesses stay contiguous
-    constexpr int kPerTrip = 4;
-    for (int64_t base = static_cast<int64_t>(blockIdx.x) * blockDim.x * kPerTrip + threadIdx.x; base < p.units;
-         base += stride * kPerTrip)
-    {
-      if (STORAGE == CAIFQ_I8)
-      {
-        uint2 c[kPerTrip];
-#pragma unroll
-        for (int u = 0; u < kPerTrip; ++u)
-        {
-          const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
-          c[u] = (i < p.units) ? __ldg(static_cast<const uint2 *>(p.codes) + i) : make_uint2(0u, 0u);
-        }
-#pragma unroll
-        for (int u = 0; u < kPerTrip; ++u)
-        {
-          const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
-          if (i < p.units)
-          {
-            p.wb[i] = expand_int8x8(c[u]);
-          }
-        }
-      }
-      else
-      {
-        uint32_t c[kPerTrip];
-        __half sc[kPerTrip];
-#pragma unroll
-        for (int u = 0; u < kPerTrip; ++u)
-        {
-          const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
-          c[u] = 0u;
-          sc[u] = __half();
-          if (i < p.units)
-          {
-            c[u] = __ldg(static_cast<const uint32_t *>(p.codes) + i);
-            sc[u] = __ldg(p.scales + (i * 8) / p.group_size);
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < kPerTrip; ++u)
-        {
-          const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
-          if (i < p.units)
-          {
-            p.wb[i] = expand_int4x8(c[u], __half2float(sc[u]));
-          }
-        }
-      }
-    }
+    expand_span<MODE>(p.codes, p.scales, p.wb, p.units, p.group_of);
     return;
   }
   const __nv_bfloat16 zero = __float2bfloat16(0.0f);
@@ -695,7 +644,7 @@ __global__ void expand_prepare_kernel(const ExpandPrepare p)
   }
 }
 
-// forward: bp != null; backward: bt and ap != null.  The weight must be one launch_expand_to_bf16 takes.
+// forward: bp != null; backward: bt and ap != null.  The weight must be one expand_span takes.
 int launch_expand_prepare(const caifq_weight &w, void *wb, const void *a, const void *b, void *bp, void *bt, void *ap,
                           int rank, cudaStream_t s)
 {
@@ -703,7 +652,7 @@ int launch_expand_prepare(const caifq_weight &w, void *wb, const void *a, const 
   const bool i8 = (w.storage == CAIFQ_I8);
   if ((total % 8) != 0 || (!i8 && !(w.storage == CAIFQ_I4 && w.scales != nullptr && w.group_size > 0 &&
                                     (w.group_size % 8) == 0)) ||
-      (reinterpret_cast<uintptr_t>(w.codes) & 7u) != 0)
+      (reinterpret_cast<uintptr_t>(w.codes) & 15u) != 0 || (reinterpret_cast<uintptr_t>(wb) & 31u) != 0)
   {
     set_error("expand_prepare: unsupported weight (storage %d)", w.storage);
     return CAIFQ_ERR_UNSUPPORTED;
@@ -713,7 +662,7 @@ int launch_expand_prepare(const caifq_weight &w, void *wb, const void *a, const 
   p.scales = static_cast<const __half *>(w.scales);
   p.wb = static_cast<uint4 *>(wb);
   p.units = total / 8;
-  p.group_size = w.group_size;
+  p.group_of = GroupOf::make(w.group_size);
   p.a = static_cast<const __nv_bfloat16 *>(a);
   p.b = static_cast<const __nv_bfloat16 *>(b);
   p.bp = static_cast<__nv_bfloat16 *>(bp);
@@ -725,11 +674,11 @@ int launch_expand_prepare(const caifq_weight &w, void *wb, const void *a, const 
   const dim3 grid(148 * 8, 2);
   if (i8)
   {
-    expand_prepare_kernel<CAIFQ_I8><<<grid, 256, 0, s>>>(p);
+    expand_prepare_kernel<EXPAND_I8><<<grid, 256, 0, s>>>(p);
   }
   else
   {
-    expand_prepare_kernel<CAIFQ_I4><<<grid, 256, 0, s>>>(p);
+    expand_prepare_kernel<EXPAND_I4><<<grid, 256, 0, s>>>(p);
   }
   CAIFQ_CHECK_LAUNCH();
   return CAIFQ_OK;

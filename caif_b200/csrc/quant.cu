@@ -747,195 +747,145 @@ int launch_cast(const void *src, int src_dtype, void *dst, int dst_dtype, int64_
 }
 
 // ---- codes -> bf16 operand matrix (many-token calls expand the weight once per call / step) ----
-// One thread per 16 bytes of OUTPUT (eight weights: 8 bytes of int8 codes or 4 bytes of int4 codes), so a
-// warp reads 256 / 128 contiguous bytes and writes 512 contiguous bytes per instruction.  int8: exact bf16
-// integers with byte permutes and one bf16 subtraction per pair.  int4: the offset-binary nibble is dropped
-// into the mantissa of 2^23 (exact), 2^23 + 8 subtracted (exact), the product with the group's fp16 scale
-// rounded once in fp32 and once to bf16 -- the value the reference's dequantize kernel followed by its cast
-// to bf16 gives (src/caif_cuda_kernels_quant.cu:364-420, src/caif_device_frozen_linear.cpp:319-334).
-// `units` = weights / 8 of one matrix; blockIdx.y selects the matrix (expert) of a stacked run
-constexpr int kExpandGroup = 64;
+// int8: exact bf16 integers with byte permutes and one bf16 subtraction per pair, or the scaled value.  int4: the
+// offset-binary nibble is dropped into the mantissa of 2^23 (exact), 2^23 + 8 subtracted (exact), the product with the
+// group's fp16 scale rounded once in fp32 and once to bf16 -- the value the reference's dequantize kernel followed by
+// its cast to bf16 gives (src/caif_cuda_kernels_quant.cu:364-420, src/caif_device_frozen_linear.cpp:319-334).
+// Bound by HBM (2.5 to 3 bytes a weight, most of them writes): 32-byte stores and a shift instead of a 64-bit division
+// per unit (64 experts of 2048 x 1408 int4: 101 us a projection before, 84 now).
+// blockIdx.y selects the matrix of a run; `units` = weights / 8.
+constexpr int kExpandRun = 64;
 struct ExpandTable
 {
-  const void *codes[kExpandGroup];
-  const __half *scales[kExpandGroup];
+  const void *codes[kExpandRun];
+  const void *scales[kExpandRun];
+  uint4 *dst[kExpandRun];
+  int64_t units[kExpandRun];
 };
 
-template <int STORAGE>
-__global__ void expand_kernel(const __grid_constant__ ExpandTable t, uint4 *dst, int64_t units, int group_size)
+template <int MODE>
+__global__ void expand_kernel(const __grid_constant__ ExpandTable t, GroupOf group_of)
 {
   const int e = blockIdx.y;
-  uint4 *out = dst + static_cast<int64_t>(e) * units;
-  // four units per thread and trip, a block width apart: all four loads are in flight before the first
-  // conversion, and a warp's accesses stay contiguous
-  constexpr int kPerTrip = 4;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x * kPerTrip;
-  for (int64_t base = static_cast<int64_t>(blockIdx.x) * blockDim.x * kPerTrip + threadIdx.x; base < units;
-       base += stride)
-  {
-    if (STORAGE == CAIFQ_I8)
-    {
-      uint2 c[kPerTrip];
-#pragma unroll
-      for (int u = 0; u < kPerTrip; ++u)
-      {
-        const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
-        c[u] = (i < units) ? __ldg(static_cast<const uint2 *>(t.codes[e]) + i) : make_uint2(0u, 0u);
-      }
-#pragma unroll
-      for (int u = 0; u < kPerTrip; ++u)
-      {
-        const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
-        if (i < units)
-        {
-          out[i] = expand_int8x8(c[u]);
-        }
-      }
-    }
-    else
-    {
-      uint32_t c[kPerTrip];
-      __half sc[kPerTrip];
-#pragma unroll
-      for (int u = 0; u < kPerTrip; ++u)
-      {
-        const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
-        c[u] = 0u;
-        sc[u] = __half();
-        if (i < units)
-        {
-          c[u] = __ldg(static_cast<const uint32_t *>(t.codes[e]) + i);
-          sc[u] = __ldg(t.scales[e] + (i * 8) / group_size);   // eight codes lie in one group
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < kPerTrip; ++u)
-      {
-        const int64_t i = base + static_cast<int64_t>(u) * blockDim.x;
-        if (i < units)
-        {
-          out[i] = expand_int4x8(c[u], __half2float(sc[u]));
-        }
-      }
-    }
-  }
+  expand_span<MODE>(t.codes[e], t.scales[e], t.dst[e], t.units[e], group_of);
 }
 
-int launch_expand_grouped_to_bf16(const caifq_weight *ws, int count, void *dst, cudaStream_t s)
+namespace
 {
-  const caifq_weight &w0 = ws[0];
-  const int64_t total = static_cast<int64_t>(w0.in_dim) * w0.out_dim;
-  const bool i8 = (w0.storage == CAIFQ_I8);
-  if ((total % 8) != 0 || (!i8 && !(w0.storage == CAIFQ_I4 && w0.group_size > 0 && (w0.group_size % 8) == 0)))
+template <int MODE>
+int launch_expand(const caifq_weight *ws, int count, uint8_t *dst, cudaStream_t s)
+{
+  for (int first = 0; first < count; first += kExpandRun)
   {
-    set_error("expand_to_bf16: unsupported weight (storage %d)", w0.storage);
-    return CAIFQ_ERR_UNSUPPORTED;
-  }
-  const int64_t units = total / 8;
-  for (int first = 0; first < count; first += kExpandGroup)
-  {
-    const int n = (count - first < kExpandGroup) ? (count - first) : kExpandGroup;
+    const int n = (count - first < kExpandRun) ? (count - first) : kExpandRun;
     ExpandTable t{};
+    int64_t most = 0;
     for (int e = 0; e < n; ++e)
     {
-      t.codes[e] = ws[first + e].codes;
-      t.scales[e] = static_cast<const __half *>(ws[first + e].scales);
-      if (!i8 && t.scales[e] == nullptr)
+      const caifq_weight &w = ws[first + e];
+      const int64_t total = static_cast<int64_t>(w.in_dim) * w.out_dim;
+      const bool bad_group = MODE == EXPAND_I4 && (w.scales == nullptr || w.group_size <= 0 || (w.group_size % 8) != 0 ||
+                                                   w.group_size != ws[0].group_size);
+      if ((total % 8) != 0 || bad_group || (MODE == EXPAND_I8_SCALED && w.scales == nullptr) ||
+          (reinterpret_cast<uintptr_t>(w.codes) & (MODE == EXPAND_I4 ? 7u : 15u)) != 0 ||
+          (reinterpret_cast<uintptr_t>(dst) & 31u) != 0)
       {
-        set_error("expand_to_bf16: int4 weight %d has no scales", first + e);
-        return CAIFQ_ERR_INVALID;
+        set_error("expand_to_bf16: unsupported weight %d (storage %d)", first + e, w.storage);
+        return CAIFQ_ERR_UNSUPPORTED;
       }
-      if ((reinterpret_cast<uintptr_t>(t.codes[e]) & 7u) != 0)
-      {
-        set_error("expand_to_bf16: codes of weight %d are not 8-byte aligned", first + e);
-        return CAIFQ_ERR_INVALID;
-      }
+      t.codes[e] = w.codes;
+      t.scales[e] = w.scales;
+      t.dst[e] = reinterpret_cast<uint4 *>(dst);
+      t.units[e] = total / 8;
+      most = t.units[e] > most ? t.units[e] : most;
+      dst += total * 2;
     }
-    int gx = grid_for(units);
+    int gx = grid_for(most, 2);
     const int cap = (148 * 8 + n - 1) / n;   // about eight CTAs per SM over all matrices
     if (gx > cap)
     {
       gx = cap;
     }
-    uint4 *out = static_cast<uint4 *>(dst) + static_cast<int64_t>(first) * units;
     const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(n));
-    if (i8)
-    {
-      expand_kernel<CAIFQ_I8><<<grid, kBlock, 0, s>>>(t, out, units, 0);
-    }
-    else
-    {
-      expand_kernel<CAIFQ_I4><<<grid, kBlock, 0, s>>>(t, out, units, w0.group_size);
-    }
+    expand_kernel<MODE><<<grid, kBlock, 0, s>>>(t, GroupOf::make(MODE == EXPAND_I4 ? ws[0].group_size : 1));
     CAIFQ_CHECK_LAUNCH();
   }
   return CAIFQ_OK;
 }
+}  // namespace
 
-int launch_expand_to_bf16(const caifq_weight &w, void *dst, cudaStream_t s) { return launch_expand_grouped_to_bf16(&w, 1, dst, s); }
-
-// ---- a weight as the bf16 matrix the reference's ConvertToComputeDtype would hold for bf16 compute ----
-// (src/caif_device_frozen_linear.cpp:288-378): int8 per-tensor bf16(float(code) * scale), int4 as
-// expand_int4x8, bf16 copied, fp32 / fp16 rounded to bf16.  Used where several layers' weights are laid one
-// under the other into one operand (fused q/k/v), so the scale has to be inside the values.
-__global__ void expand_int8_scaled_kernel(const uint2 *__restrict__ codes, const float *__restrict__ scale,
-                                          uint4 *__restrict__ dst, int64_t units)
+int launch_expand_grouped_to_bf16(const caifq_weight *ws, int count, void *dst, cudaStream_t s)
 {
-  const float sc = __ldg(scale);
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < units; i += stride)
-  {
-    const uint2 v = __ldg(codes + i);
-    const uint32_t w[2] = {v.x, v.y};
-    uint32_t o[4];
-#pragma unroll
-    for (int k = 0; k < 2; ++k)
-    {
-#pragma unroll
-      for (int h = 0; h < 2; ++h)
-      {
-        const float lo = __fmul_rn(static_cast<float>(static_cast<int8_t>((w[k] >> (16 * h)) & 0xFFu)), sc);
-        const float hi = __fmul_rn(static_cast<float>(static_cast<int8_t>((w[k] >> (16 * h + 8)) & 0xFFu)), sc);
-        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(o[2 * k + h]) : "f"(hi), "f"(lo));
-      }
-    }
-    dst[i] = make_uint4(o[0], o[1], o[2], o[3]);
-  }
+  return ws[0].storage == CAIFQ_I8 ? launch_expand<EXPAND_I8>(ws, count, static_cast<uint8_t *>(dst), s)
+                                   : launch_expand<EXPAND_I4>(ws, count, static_cast<uint8_t *>(dst), s);
 }
 
-int launch_weight_to_bf16_scaled(const caifq_weight &w, void *dst, cudaStream_t s)
+// ---- weights as the bf16 matrix the reference's ConvertToComputeDtype would hold for bf16 compute ----
+// (src/caif_device_frozen_linear.cpp:288-378): int8 per-tensor bf16(float(code) * scale), int4 as
+// expand_int4x8, bf16 copied, fp32 / fp16 rounded to bf16.  Used where several layers' weights are laid one
+// under the other into one operand (fused q/k/v), so the scale has to be inside the values.  Neighbours of one
+// storage share a launch.
+int launch_weights_to_bf16_scaled(const caifq_weight *ws, int count, void *dst, cudaStream_t s)
 {
-  const int64_t total = static_cast<int64_t>(w.in_dim) * w.out_dim;
-  if (w.storage == CAIFQ_I4)
+  uint8_t *out = static_cast<uint8_t *>(dst);
+  for (int i = 0; i < count;)
   {
-    return launch_expand_to_bf16(w, dst, s);
-  }
-  if (w.storage == CAIFQ_I8)
-  {
-    if (w.scheme != CAIFQ_PER_TENSOR || w.scales == nullptr || (total % 8) != 0 ||
-        (reinterpret_cast<uintptr_t>(w.codes) & 7u) != 0)
+    int n = 1;
+    while (i + n < count && ws[i + n].storage == ws[i].storage && ws[i + n].group_size == ws[i].group_size)
     {
-      set_error("weight_to_bf16: int8 needs one per-tensor scale, 8-byte aligned codes and a multiple of 8 weights");
-      return CAIFQ_ERR_UNSUPPORTED;
+      ++n;
     }
-    const int64_t units = total / 8;
-    expand_int8_scaled_kernel<<<grid_for(units), kBlock, 0, s>>>(static_cast<const uint2 *>(w.codes),
-                                                               static_cast<const float *>(w.scales),
-                                                               static_cast<uint4 *>(dst), units);
-    CAIFQ_CHECK_LAUNCH();
-    return CAIFQ_OK;
-  }
-  if (w.storage == CAIFQ_BF16)
-  {
-    const cudaError_t err = cudaMemcpyAsync(dst, w.codes, static_cast<size_t>(total) * 2, cudaMemcpyDeviceToDevice, s);
-    if (err != cudaSuccess)
+    int rc = CAIFQ_OK;
+    bool aligned = true;
+    for (int k = i; k < i + n; ++k)
     {
-      set_error("weight_to_bf16: copy failed: %s", cudaGetErrorString(err));
-      return CAIFQ_ERR_CUDA;
+      aligned = aligned && (reinterpret_cast<uintptr_t>(ws[k].codes) & 15u) == 0;
     }
-    return CAIFQ_OK;
+    if (!aligned)
+    {
+      n = 1;   // a view of codes that 16-byte loads cannot read
+      rc = launch_weight_materialize(ws[i], out, CAIFQ_BF16, s);
+    }
+    else if (ws[i].storage == CAIFQ_I4)
+    {
+      rc = launch_expand<EXPAND_I4>(ws + i, n, out, s);
+    }
+    else if (ws[i].storage == CAIFQ_I8)
+    {
+      for (int k = i; k < i + n; ++k)
+      {
+        if (ws[k].scheme != CAIFQ_PER_TENSOR)
+        {
+          set_error("weight_to_bf16: int8 needs one per-tensor scale");
+          return CAIFQ_ERR_UNSUPPORTED;
+        }
+      }
+      rc = launch_expand<EXPAND_I8_SCALED>(ws + i, n, out, s);
+    }
+    else
+    {
+      n = 1;
+      const int64_t total = static_cast<int64_t>(ws[i].in_dim) * ws[i].out_dim;
+      if (ws[i].storage == CAIFQ_BF16)
+      {
+        CAIFQ_CHECK_CUDA(cudaMemcpyAsync(out, ws[i].codes, static_cast<size_t>(total) * 2, cudaMemcpyDeviceToDevice, s));
+      }
+      else
+      {
+        rc = launch_cast(ws[i].codes, ws[i].storage, out, CAIFQ_BF16, total, s);
+      }
+    }
+    if (rc != CAIFQ_OK)
+    {
+      return rc;
+    }
+    for (int k = i; k < i + n; ++k)
+    {
+      out += static_cast<size_t>(ws[k].in_dim) * static_cast<size_t>(ws[k].out_dim) * 2;
+    }
+    i += n;
   }
-  return launch_cast(w.codes, w.storage, dst, CAIFQ_BF16, total, s);
+  return CAIFQ_OK;
 }
 
 int launch_weight_materialize(const caifq_weight &w, void *dst, int dst_dtype, cudaStream_t s)
