@@ -270,6 +270,11 @@ int linear_any(const caifq_weight *w, bool backward, const void *a, int a_dtype,
     set_path("umma");
     return launch_linear_umma(args, s);
   }
+  if (force == Force::None && f32_supported(args))
+  {
+    set_path("umma");
+    return launch_linear_f32(args, s);
+  }
   if (force == Force::Umma || force == Force::Decode)
   {
     set_error("%s: forced kernel family does not support this call", who);

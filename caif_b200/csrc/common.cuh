@@ -484,6 +484,10 @@ int launch_linear_decode(const LinearArgs &args, cudaStream_t s);
 bool rows_supported(const LinearArgs &args);
 int launch_linear_rows(const LinearArgs &args, cudaStream_t s);
 
+// fp32 activations, int8 / int4 weights, fp32 compute
+bool f32_supported(const LinearArgs &args);
+int launch_linear_f32(const LinearArgs &args, cudaStream_t s);
+
 // tcgen05 / TMEM tensor-core kernel for many tokens
 bool umma_supported(const LinearArgs &args);
 int launch_linear_umma(const LinearArgs &args, cudaStream_t s);

@@ -555,3 +555,27 @@ def test_umma_bf16_weight_with_a_partial_last_column_tile(m, in_dim, out_dim):
         dx = nv.linear_dx(weight, dy, torch.float32, orc.F32)
         assert nv.last_path() == "umma"
         assert max_rel_err(dx.cpu().numpy(), orc.frozen_linear_backward(dy_np, wc)) <= TOL_F32
+
+
+@pytest.mark.parametrize("storage,group", [(orc.I8, 128), (orc.I4, 128), (orc.I4, 64)])
+@pytest.mark.parametrize("m,in_dim,out_dim", [(1, 1024, 128), (64, 1024, 1024), (65, 128, 64), (130, 64, 192), (1000, 384, 2048)])
+def test_fp32_activations_on_the_tensor_core(storage, group, m, in_dim, out_dim):
+    """Three bf16 terms per activation: tile edges in m, one block of k, every split of k over a cluster.  Held to an
+    fp32 GEMM's own error, far below the layer's bound."""
+    if storage == orc.I4 and in_dim % group:
+        pytest.skip("groups straddle rows: the generic kernel's")
+    rng = np.random.default_rng(m + in_dim + out_dim + group)
+    weight, codes, scales = make_weight(rng, out_dim, in_dim, storage, group=group)
+    wc = _oracle_w(weight, codes, scales, orc.F32)
+    x_np, x = act(rng, m, in_dim, orc.F32)
+    dy_np, dy = act(rng, m, out_dim, orc.F32)
+    y = nv.linear_fwd(weight, x)
+    assert nv.last_path() == "umma"
+    want = x_np.astype(np.float64) @ wc.astype(np.float64).T
+    assert np.linalg.norm(y.cpu().numpy() - want) <= 1e-6 * np.linalg.norm(want)
+    dx = nv.linear_dx(weight, dy)
+    assert nv.last_path() == "umma"
+    want = dy_np.astype(np.float64) @ wc.astype(np.float64)
+    assert np.linalg.norm(dx.cpu().numpy() - want) <= 1e-6 * np.linalg.norm(want)
+    res_np, res = act(rng, m, out_dim, orc.F32)
+    assert torch.equal(nv.linear_fwd_residual(weight, x, res.clone()), y + res)
