@@ -16,6 +16,7 @@ namespace caifq
 // each kernel file owns its flag and the code that reads it (device symbols are per translation unit)
 int take_decode_timeout_flag();
 int take_umma_timeout_flag();
+int take_stream_timeout_flag();
 
 namespace
 {
@@ -265,6 +266,11 @@ int linear_any(const caifq_weight *w, bool backward, const void *a, int a_dtype,
     set_path("decode");
     return launch_linear_rows(args, s);
   }
+  if ((force == Force::None || force == Force::Umma) && stream_supported(args))
+  {
+    set_path("umma");
+    return launch_linear_stream(args, s);
+  }
   if ((force == Force::None || force == Force::Umma) && umma_supported(args))
   {
     set_path("umma");
@@ -424,12 +430,13 @@ int caifq_device_status(void)
   }
   const int decode_flag = take_decode_timeout_flag();
   const int umma_flag = take_umma_timeout_flag();
-  if (decode_flag < 0 || umma_flag < 0)
+  const int stream_flag = take_stream_timeout_flag();
+  if (decode_flag < 0 || umma_flag < 0 || stream_flag < 0)
   {
     set_error("caifq_device_status: %s", cudaGetErrorString(cudaGetLastError()));
     return -1;
   }
-  return (decode_flag ? 1 : 0) | (umma_flag ? 2 : 0);
+  return (decode_flag ? 1 : 0) | ((umma_flag || stream_flag) ? 2 : 0);
 }
 
 void caifq_selftest_stall_next_decode(void) { decode_stall_next_launch(); }
@@ -1352,6 +1359,76 @@ int grouped_linear(const caifq_weight *ws, int num_experts, const int32_t *offse
   return CAIFQ_OK;
 }
 
+// Experts that see few rows each (decoding): their products are bound by reading the codes, and run on the kernel that
+// streams them -- gate and up of all experts as one launch, then the activation, then down.
+const int kFewRowsPerExpert = 64;
+
+static bool few_rows(int num_experts, const int32_t *offsets, int dtype)
+{
+  static const bool grouping = []() {
+    const char *e = std::getenv("CAIFQ_GROUPED");
+    return e == nullptr || e[0] != '0';
+  }();
+  return grouping && forced_path() == Force::None && dtype == CAIFQ_BF16 &&
+         static_cast<int64_t>(offsets[num_experts]) <= static_cast<int64_t>(kFewRowsPerExpert) * num_experts;
+}
+
+// One launch per run of `sets` weight lists over the experts' rows: list i writes to outs[i].  CAIFQ_ERR_UNSUPPORTED
+// (nothing launched, no message) when the kernel does not take them.
+static int stream_experts(const caifq_weight *const *lists, void *const *outs, int sets, int num_experts,
+                          const int32_t *offsets, const void *a, int dtype, int compute_dtype, cudaStream_t s)
+{
+  constexpr int kRun = 160;
+  const int per_run = kRun / sets;
+  caifq_weight ws[kRun];
+  int32_t row_begin[kRun];
+  int32_t row_end[kRun];
+  void *c[kRun];
+  for (int pass = 0; pass < 2; ++pass)   // first look at every run, then launch
+  {
+    for (int first = 0; first < num_experts; first += per_run)
+    {
+      const int n = (num_experts - first < per_run) ? (num_experts - first) : per_run;
+      GroupedStreamArgs g{};
+      for (int i = 0; i < sets; ++i)
+      {
+        for (int e = 0; e < n; ++e)
+        {
+          ws[g.count] = lists[i][first + e];
+          row_begin[g.count] = offsets[first + e];
+          row_end[g.count] = offsets[first + e + 1];
+          c[g.count] = outs[i];
+          ++g.count;
+        }
+      }
+      g.weights = ws;
+      g.row_begin = row_begin;
+      g.row_end = row_end;
+      g.c = c;
+      g.a = a;
+      g.total_rows = offsets[num_experts];
+      g.c_dtype = dtype;
+      g.accumulate = false;
+      g.compute_dtype = compute_dtype;
+      if (pass == 0)
+      {
+        if (!stream_grouped_supported(g))
+        {
+          return CAIFQ_ERR_UNSUPPORTED;
+        }
+        continue;
+      }
+      const int rc = launch_linear_stream_grouped(g, s);
+      if (rc != CAIFQ_OK)
+      {
+        return rc;
+      }
+    }
+  }
+  set_path("umma-grouped");
+  return CAIFQ_OK;
+}
+
 int caifq_grouped_expert_fwd(const caifq_weight *gate, const caifq_weight *up, const caifq_weight *down,
                              int32_t num_experts, const int32_t *expert_offsets_host, const void *x, void *out,
                              void *gate_out, void *up_out, void *hidden_ws, int32_t dtype, int32_t compute_dtype,
@@ -1373,6 +1450,27 @@ int caifq_grouped_expert_fwd(const caifq_weight *gate, const caifq_weight *up, c
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int64_t hid = up[0].out_dim;
   int r = CAIFQ_OK;
+  if (few_rows(num_experts, expert_offsets_host, dtype))
+  {
+    const caifq_weight *lists[2] = {up, gate};
+    void *outs[2] = {up_out, gate_out};
+    r = stream_experts(lists, outs, gate != nullptr ? 2 : 1, num_experts, expert_offsets_host, x, dtype, compute_dtype, s);
+    if (r == CAIFQ_OK)
+    {
+      r = gate != nullptr ? launch_swiglu_fwd(gate_out, up_out, hidden_ws, dtype, total * hid, s)
+                          : launch_silu_fwd(up_out, hidden_ws, dtype, total * hid, s);
+      if (r == CAIFQ_OK)
+      {
+        const caifq_weight *list = down;
+        r = stream_experts(&list, &out, 1, num_experts, expert_offsets_host, hidden_ws, dtype, compute_dtype, s);
+      }
+    }
+    if (r != CAIFQ_ERR_UNSUPPORTED)
+    {
+      return r;
+    }
+    r = CAIFQ_OK;
+  }
   if (gate == nullptr)
   {
     // hidden = SiLU(up(x)), src/caif_device_moe_frozen_expert.cpp:158-162

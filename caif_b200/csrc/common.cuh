@@ -170,6 +170,7 @@ struct GroupOf
   }
 
   __device__ __forceinline__ int64_t operator()(int64_t flat) const { return shift >= 0 ? flat >> shift : flat / size; }
+  __device__ __forceinline__ uint32_t operator()(uint32_t k) const { return shift >= 0 ? k >> shift : k / static_cast<uint32_t>(size); }
 };
 
 // sixteen bf16 values as one 32-byte store: a warp writes a contiguous kilobyte
@@ -487,6 +488,27 @@ int launch_linear_rows(const LinearArgs &args, cudaStream_t s);
 // fp32 activations, int8 / int4 weights, fp32 compute
 bool f32_supported(const LinearArgs &args);
 int launch_linear_f32(const LinearArgs &args, cudaStream_t s);
+
+// tcgen05 kernel that streams the weight past few hundred tokens (forward): one layer, or experts of few rows each
+struct GroupedStreamArgs
+{
+  // entry e: rows [row_begin[e], row_end[e]) of the packed buffer, c[e][row, :] = a[row, :] . weights[e]^T
+  const caifq_weight *weights;
+  const int32_t *row_begin;
+  const int32_t *row_end;
+  void *const *c;
+  int count;
+  const void *a;
+  int64_t total_rows;
+  int c_dtype;
+  bool accumulate;
+  int compute_dtype;
+};
+bool stream_supported(const LinearArgs &args);
+int launch_linear_stream(const LinearArgs &args, cudaStream_t s);
+bool stream_grouped_supported(const GroupedStreamArgs &args);
+int launch_linear_stream_grouped(const GroupedStreamArgs &args, cudaStream_t s);
+bool take_umma_stall();   // self-test hook of the tensor-core kernels' waits
 
 // tcgen05 / TMEM tensor-core kernel for many tokens
 bool umma_supported(const LinearArgs &args);

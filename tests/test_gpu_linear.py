@@ -579,3 +579,46 @@ def test_fp32_activations_on_the_tensor_core(storage, group, m, in_dim, out_dim)
     assert np.linalg.norm(dx.cpu().numpy() - want) <= 1e-6 * np.linalg.norm(want)
     res_np, res = act(rng, m, out_dim, orc.F32)
     assert torch.equal(nv.linear_fwd_residual(weight, x, res.clone()), y + res)
+
+
+@pytest.mark.parametrize("storage,compute,group", [(orc.I8, orc.BF16, 128), (orc.I4, orc.BF16, 32), (orc.I4, orc.F32, 128)])
+@pytest.mark.parametrize("m,in_dim,out_dim", [
+    (17, 128, 128),        # one stage of k
+    (33, 320, 128),        # an odd 64 k at the end, a box of tokens with one row
+    (64, 384, 19072),      # more tiles than SMs: both accumulator sets, tiles of one unit
+    (128, 2048, 256),      # k over clusters of eight
+    (129, 1408, 640),      # clusters of four; one accumulator set, or two tiles of tokens
+    (257, 1152, 6272), (512, 4096, 128), (768, 256, 384),
+])
+def test_tens_to_hundreds_of_tokens(storage, compute, group, m, in_dim, out_dim):
+    if in_dim % group:
+        pytest.skip("groups straddle rows: the generic kernel's")
+    weight, wc, x_np, x, dy_np, dy = _umma_case(storage, compute, m, in_dim, out_dim, m + in_dim, group)
+    y = nv.linear_fwd(weight, x, torch.float32, compute)
+    assert nv.last_path() == "umma"
+    want = x_np.astype(np.float64) @ wc.astype(np.float64).T
+    assert np.abs(y.cpu().numpy() - want).max() <= (TOL_F32 if compute == orc.F32 else 5e-3) * np.abs(want).max()
+    for sd in (orc.BF16, orc.F32):
+        res_np, res = act(np.random.default_rng(m), m, out_dim, sd)
+        got = nv.linear_fwd_residual(weight, x, res.clone(), compute)
+        sep = nv.linear_fwd(weight, x, TORCH_DTYPE[sd], compute)
+        assert torch.equal(got, (sep.float() + res.float()).to(TORCH_DTYPE[sd]))
+    assert nv.lib().caifq_device_status() == 0
+
+
+@pytest.mark.parametrize("m,out_dim", [(64, 1024), (512, 14336)])
+def test_streaming_wait_that_runs_out_raises_the_flag_and_returns(m, out_dim):
+    import time
+
+    weight, wc, x_np, x, dy_np, dy = _umma_case(orc.I4, orc.BF16, m, 1024, out_dim, 4243)
+    y = nv.linear_fwd(weight, x, torch.float32, orc.BF16)
+    assert nv.lib().caifq_device_status() == 0
+    nv.lib().caifq_selftest_stall_next_umma()
+    t0 = time.time()
+    nv.linear_fwd(weight, x, torch.float32, orc.BF16)
+    torch.cuda.synchronize()
+    assert time.time() - t0 < 1.0
+    assert nv.lib().caifq_device_status() & 2
+    y2 = nv.linear_fwd(weight, x, torch.float32, orc.BF16)
+    assert nv.lib().caifq_device_status() == 0
+    assert torch.equal(y, y2)

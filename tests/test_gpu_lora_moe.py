@@ -837,3 +837,30 @@ def test_dense_gated_ffn_is_the_grouped_call_with_one_expert(storage):
     want_dx = orc.frozen_expert_backward(dy_np[sample], g, u, oracle_ws[0], oracle_ws[1], oracle_ws[2], orc.BF16,
                                          orc.BF16)
     assert max_rel_err(dx[sample].float().cpu().numpy(), want_dx) <= 2e-2
+
+
+@pytest.mark.parametrize("storage,compute", [(orc.I4, orc.BF16), (orc.I8, orc.BF16), (orc.I4, orc.F32)])
+@pytest.mark.parametrize("counts", [[0, 1, 0, 2, 5, 0], [300, 0, 17, 1, 2, 3, 4], [64] * 3])
+@pytest.mark.parametrize("gated", [True, False])
+def test_experts_of_few_rows(storage, compute, counts, gated):
+    """Decode-sized experts: gate and up of all of them in one launch; experts without rows, and one with several tiles of
+    tokens beside experts of a row or two."""
+    rng = np.random.default_rng(sum(counts))
+    in_dim, hid, sd = 512, 384, orc.BF16
+    offsets = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    ws = [[make_weight(rng, o, i, storage, std=0.05) for _ in counts]
+          for (o, i) in ((hid, in_dim), (hid, in_dim), (in_dim, hid))]
+    ref = [[orc.weight_to_compute(c, s, storage, w.in_dim, w.out_dim, compute, w.scheme, w.group_size) for (w, c, s) in l]
+           for l in ws]
+    gate, up, down = [[w for (w, _, _) in l] for l in ws]
+    x_np, x = act(rng, int(offsets[-1]), in_dim, sd)
+    out, gate_out, up_out = nv.grouped_expert_fwd(gate if gated else None, up, down, offsets.tolist(), x, compute)
+    assert nv.last_path() == "umma-grouped"
+    assert nv.lib().caifq_device_status() == 0
+    for e in range(len(counts)):
+        lo, hi = offsets[e], offsets[e + 1]
+        if lo == hi:
+            continue
+        want, g, u = orc.frozen_expert_forward(x_np[lo:hi], ref[0][e] if gated else None, ref[1][e], ref[2][e], compute, sd)
+        assert max_rel_err(out[lo:hi].float().cpu().numpy(), want) <= 2e-2
+        assert max_rel_err(up_out[lo:hi].float().cpu().numpy(), u) <= 2e-2
