@@ -82,6 +82,7 @@ constexpr int BM_SUB = 128;          // rows of one MMA
 constexpr int MT = 2;                // MMAs (row sub-tiles) per weight tile
 constexpr int BM = BM_SUB * MT;      // 256
 // BN (columns of the output tile, N of one MMA) is a template parameter: 128 or 256
+constexpr int kBand = 8;             // row tiles of a band of the schedule
 constexpr int BK = 64;               // one 128-byte swizzle span of bf16
 constexpr int UMMA_K = 16;
 constexpr int A_SUB_BYTES = BM_SUB * BK * 2;       // 16 KB
@@ -92,6 +93,7 @@ constexpr int NUM_WARPS = 14;
 constexpr int NUM_THREADS = NUM_WARPS * 32;
 constexpr int DEQ_WARP0 = 6;
 constexpr int DEQ_THREADS = 8 * 32;
+constexpr int B_WARP = 10;           // bf16 weights: the warp that copies their tiles
 // Teams of dequant warps (see the dequantization role): two for a single CTA's tile; four for a CTA pair,
 // whose k-blocks take half as long while a conversion's latency chain (wait, loads, ~150 instructions,
 // stores, proxy fence, arrive) stays the same (two teams: 750-830 TFLOP/s on 4096 x 4096 int8, four: 980-1150).
@@ -134,6 +136,9 @@ struct UmmaParams
   int groups_per_row;  // int4: in_dim / group_size
   int num_m_tiles;
   int num_n_tiles;
+  int band;            // row tiles of a band of the schedule (see locate_tile)
+  int wide_stores;     // outputs (and what the SwiGLU backward reads) are 32-byte aligned
+  int bn;              // bf16 weights on CTA pairs: columns of a tile, 64 .. 256 in steps of 32 (see choose_pair_width)
   const uint8_t *lora_rhs;  // null = no LoRA k-block
   const float *c_scale;     // bf16 weights only: factor of the fp32 accumulator in the epilogue (null = 1)
   int expert_rows;          // grouped bf16 weights: rows of one expert's matrix in the stacked [E * rows, in] matrix
@@ -209,12 +214,18 @@ __device__ __forceinline__ TileWork locate_tile(int tile, const UmmaParams &p, c
 template <>
 __device__ __forceinline__ TileWork locate_tile<false>(int tile, const UmmaParams &p, const NoGroupTable &)
 {
-  // column tiles fastest: the CTAs running at one time share a few row tiles of the activations
-  // (read from memory once) and sweep the weight, which stays in L2
+  // In bands of p.band row tiles, row tiles fastest: the CTAs running at one time then work on a near-square block of
+  // the output (74 pairs: 8 x 9 tiles), which takes the fewest operand bytes.  With column tiles fastest every band of
+  // 256 tokens swept the whole weight, and one that does not fit L2 was read from memory again each time
+  // (4096 -> 14336, 2047 tokens: 198 us, with the bands 165).
   TileWork t;
   t.expert = 0;
-  t.n_tile = tile % p.num_n_tiles;
-  t.row0 = static_cast<int64_t>(tile / p.num_n_tiles) * BM;
+  const int per_band = p.band * p.num_n_tiles;
+  const int band0 = tile / per_band * p.band;
+  const int rows = min(p.band, p.num_m_tiles - band0);
+  const int local = tile - band0 * p.num_n_tiles;
+  t.n_tile = local / rows;
+  t.row0 = static_cast<int64_t>(band0 + local % rows) * BM;
   t.row_end = p.m;
   t.codes = p.codes;
   t.scales = p.scales;
@@ -253,6 +264,38 @@ __device__ __forceinline__ TileWork locate_tile<true>(int tile, const UmmaParams
   return t;
 }
 
+// 32 bytes of an output row: one store where alignment allows.  A lane owns a row, so every store instruction touches 32
+// lines; with 16-byte stores their number, not the bytes, bounded the epilogue (4800 cycles a 256-wide tile).
+__device__ __forceinline__ void store_row32(void *p, const uint32_t (&v)[8], bool wide)
+{
+  if (wide)
+  {
+    store_bf16x16(p, make_uint4(v[0], v[1], v[2], v[3]), make_uint4(v[4], v[5], v[6], v[7]));
+  }
+  else
+  {
+    static_cast<uint4 *>(p)[0] = make_uint4(v[0], v[1], v[2], v[3]);
+    static_cast<uint4 *>(p)[1] = make_uint4(v[4], v[5], v[6], v[7]);
+  }
+}
+
+__device__ __forceinline__ void load_row32(const void *p, uint32_t (&v)[8], bool wide)
+{
+  if (wide)
+  {
+    asm volatile("ld.global.nc.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "l"(p));
+  }
+  else
+  {
+    const uint4 a = __ldg(static_cast<const uint4 *>(p));
+    const uint4 b = __ldg(static_cast<const uint4 *>(p) + 1);
+    v[0] = a.x, v[1] = a.y, v[2] = a.z, v[3] = a.w;
+    v[4] = b.x, v[5] = b.y, v[6] = b.z, v[7] = b.w;
+  }
+}
+
 template <int WMODE, bool BWD, int BN, bool GROUPED, bool PAIR>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -273,6 +316,11 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   constexpr int ACC_COLS = Cfg::ACC_COLS;
   constexpr int ACC_BUFS = Cfg::ACC_BUFS;
   constexpr uint32_t CTAS = PAIR ? 2u : 1u;   // CTAs that work on one tile
+  // columns of a tile, and weight rows of it that this CTA stages: chosen per launch where the weight is fed by copies
+  // alone (the places in shared and tensor memory are those of the widest tile)
+  constexpr bool ANY_WIDTH = PAIR && WMODE == W_BF16;
+  const int bn = ANY_WIDTH ? p.bn : BN;
+  const int bnc = ANY_WIDTH ? p.bn / 2 : BNC;
   // A bf16 weight needs no dequant warps: four of them join the epilogue, so every quarter of the accumulator's
   // lanes is drained by two warps that take alternate 32-column chunks.
   constexpr int EPI_GROUPS = (WMODE == W_BF16) ? 2 : 1;
@@ -324,7 +372,7 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     for (int s = 0; s < STAGES; ++s)
     {
       mbar_init(a_full(s), 1);
-      mbar_init(b_full(s), (WMODE == W_BF16) ? 1 : (8 / DEQ_TEAMS) * CTAS);
+      mbar_init(b_full(s), (8 / DEQ_TEAMS) * CTAS);   // (a bf16 weight's copies arrive on a_full)
       mbar_init(empty(s), 1);
     }
     for (int a = 0; a < ACC_BUFS; ++a)
@@ -360,101 +408,65 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   }
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
+  // nothing above reads or writes what another kernel does: all of it runs beside the end of the previous one
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   const int num_tiles = p.num_m_tiles * p.num_n_tiles;
   const int num_kb = p.k_total / BK;
   // with a LoRA product the loop runs one more k-block whose operands are the padded factors
   const int num_kb_all = (p.dual_k ? 2 * num_kb : num_kb) + ((p.lora_rhs != nullptr) ? 1 : 0);
 
+  // One thread copies the activation tiles and, where the weight is bf16, another the weight tiles: waiting for a place,
+  // announcing the bytes and issuing both copies took one thread 460 cycles a k-block, more than most tiles' MMAs take.
+  // (pair: the leader announces both CTAs' bytes; the other CTA's copies may complete first, the phase cannot end before
+  // the leader's arrival)
+  const uint32_t lead_bar0 = lead(bar0);
+  auto load = [&](uint32_t dst, const CUtensorMap *map, int c0, int c1, int stage)
+  {
+    if (PAIR)
+    {
+      tma_load_2d_pair(dst, map, c0, c1, lead_bar0 + static_cast<uint32_t>(stage) * 8u);
+    }
+    else
+    {
+      tma_load_2d(dst, map, c0, c1, a_full(stage));
+    }
+  };
+
   if (warp == 0)
   {
-    // ------------------------------------------------------------ TMA producer
-    if (lane == 0)
+    // ------------------------------------------------------------ TMA producer: activations
+    auto produce = [&]()
     {
+      // (a bf16 weight's tile arrives on the same barrier)
+      const uint32_t b_bytes = BWD ? static_cast<uint32_t>((bnc + 63) / 64) * 8192u : static_cast<uint32_t>(bnc) * 128u;
+      const uint32_t bytes = (A_STAGE + (WMODE == W_BF16 ? b_bytes : 0u)) * CTAS;
+      uint32_t stall = p.stall_bytes;
       int s = 0;
       uint32_t par = 0;
       for (int tile = worker; tile < num_tiles; tile += workers)
       {
         const TileWork tw = locate_tile<GROUPED>(tile, p, gt);
-        const int n_tile = tw.n_tile;
         const int row_tile = static_cast<int>(tw.row0) + static_cast<int>(rank) * BM_SUB;   // pair: this CTA's half
         for (int kb = 0; kb < num_kb_all; ++kb)
         {
           if (!wait(empty(s), par ^ 1u))
           {
-            tile = num_tiles;   // nothing new is started once a wait has run out
-            break;
+            return;   // nothing new is started once a wait has run out
           }
-          // (pair: the leader announces both CTAs' bytes; the other CTA's copies may complete first, the
-          // phase cannot end before the leader's arrival)
-          auto load = [&](uint32_t dst, const CUtensorMap *map, int c0, int c1, uint32_t bar)
-          {
-            if (PAIR)
-            {
-              tma_load_2d_pair(dst, map, c0, c1, lead(bar));
-            }
-            else
-            {
-              tma_load_2d(dst, map, c0, c1, bar);
-            }
-          };
           if (rank == 0)
           {
-            mbar_expect_tx(a_full(s), A_STAGE * CTAS + ((tile == worker && kb == 0) ? p.stall_bytes : 0u));
+            mbar_expect_tx(a_full(s), bytes + stall);
+            stall = 0;
           }
+          // from num_kb on: the LoRA k-block's activation-side operand, or the second operand pair's k-blocks
+          const CUtensorMap *map = (kb < num_kb) ? &map_a : &map_h;
+          const int kc = (kb < num_kb) ? kb * BK : (kb - num_kb) * BK;
 #pragma unroll
           for (int mt = 0; mt < MTK; ++mt)
           {
-            if (kb < num_kb)
-            {
-              load(a_addr(s, mt), &map_a, kb * BK, row_tile + mt * BM_SUB, a_full(s));
-            }
-            else
-            {
-              // the LoRA k-block's activation-side operand, or the second operand pair's k-block
-              load(a_addr(s, mt), &map_h, p.dual_k ? (kb - num_kb) * BK : 0, row_tile + mt * BM_SUB, a_full(s));
-            }
-          }
-          if (WMODE == W_BF16)
-          {
-            const int nc0 = n_tile * BN + static_cast<int>(rank) * BNC;   // this CTA's weight rows
-            if (rank == 0)
-            {
-              mbar_expect_tx(b_full(s), B_STAGE_BYTES * CTAS);
-            }
-            // the LoRA k-block (number num_kb) takes its weight-side operand, the padded factor, from map_l
-            const CUtensorMap *bmap = (kb < num_kb) ? &map_b : &map_l;
-            const int kc = (kb < num_kb) ? kb * BK : (p.dual_k ? (kb - num_kb) * BK : 0);
-            // grouped: the experts' matrices lie stacked in one [E * rows, in] matrix
-            const int erow = GROUPED ? tw.expert * p.expert_rows : 0;
-            if (!BWD && p.swiglu)
-            {
-              // HALF features of the gate projection (map_b) and the same features of the up projection (map_l)
-              constexpr int HALF = BN / 2;
-              const int f0 = erow + n_tile * HALF;
-              if (PAIR)
-              {
-                load(b_addr(s), (rank == 0) ? &map_b : &map_l, kc, f0, b_full(s));
-              }
-              else
-              {
-                load(b_addr(s), &map_b, kc, f0, b_full(s));
-                load(b_addr(s) + static_cast<uint32_t>(HALF) * 128u, &map_l, kc, f0, b_full(s));
-              }
-            }
-            else if (BWD)
-            {
-              // [k rows][n cols]: boxes of 64 n x 64 k land as the MN-major blocks
-#pragma unroll
-              for (int nb = 0; nb < BNC / 64; ++nb)
-              {
-                load(b_addr(s) + static_cast<uint32_t>(nb) * 8192u, bmap, nc0 + nb * 64, erow + kc, b_full(s));
-              }
-            }
-            else
-            {
-              load(b_addr(s), bmap, kc, erow + nc0, b_full(s));
-            }
+            load(a_addr(s, mt), map, kc, row_tile + mt * BM_SUB, s);
           }
           if (++s == STAGES)
           {
@@ -463,16 +475,90 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           }
         }
       }
+    };
+    if (lane == 0)
+    {
+      produce();
+    }
+  }
+  else if (WMODE == W_BF16 && warp == B_WARP)
+  {
+    // ------------------------------------------------------------ TMA producer: bf16 weight
+    auto produce = [&]()
+    {
+      int s = 0;
+      uint32_t par = 0;
+      for (int tile = worker; tile < num_tiles; tile += workers)
+      {
+        const TileWork tw = locate_tile<GROUPED>(tile, p, gt);
+        const int nc0 = tw.n_tile * bn + static_cast<int>(rank) * bnc;   // this CTA's weight rows
+        // grouped: the experts' matrices lie stacked in one [E * rows, in] matrix
+        const int erow = GROUPED ? tw.expert * p.expert_rows : 0;
+        for (int kb = 0; kb < num_kb_all; ++kb)
+        {
+          if (!wait(empty(s), par ^ 1u))
+          {
+            return;
+          }
+          // from num_kb on: the padded LoRA factor, or the second operand pair's weight
+          const CUtensorMap *map = (kb < num_kb) ? &map_b : &map_l;
+          const int kc = (kb < num_kb) ? kb * BK : (kb - num_kb) * BK;
+          if (!BWD && p.swiglu)
+          {
+            // HALF features of the gate projection (map_b) and the same features of the up projection (map_l)
+            constexpr int HALF = BN / 2;
+            const int f0 = erow + tw.n_tile * HALF;
+            if (PAIR)
+            {
+              load(b_addr(s), (rank == 0) ? &map_b : &map_l, kc, f0, s);
+            }
+            else
+            {
+              load(b_addr(s), &map_b, kc, f0, s);
+              load(b_addr(s) + static_cast<uint32_t>(HALF) * 128u, &map_l, kc, f0, s);
+            }
+          }
+          else if (BWD)
+          {
+            // [k rows][n cols]: boxes of 64 n x 64 k land as the MN-major blocks
+#pragma unroll
+            for (int nb = 0; nb < BNC / 64; ++nb)
+            {
+              if (ANY_WIDTH && nb * 64 >= bnc)
+              {
+                break;
+              }
+              load(b_addr(s) + static_cast<uint32_t>(nb) * 8192u, map, nc0 + nb * 64, erow + kc, s);
+            }
+          }
+          else
+          {
+            load(b_addr(s), map, kc, erow + nc0, s);
+          }
+          if (++s == STAGES)
+          {
+            s = 0;
+            par ^= 1u;
+          }
+        }
+      }
+    };
+    if (lane == 0)
+    {
+      produce();
     }
   }
   else if (warp == 1)
   {
     // -------------------------------------------------------------- MMA issuer
-    // The whole warp runs the loop, so addresses and descriptors are warp-uniform values;
-    // one elected lane issues the MMAs and the commits.  (Pair: the leader CTA's warp only.)
-    if (rank == 0)
+    // One elected lane does it all (of the leader CTA's warp in a pair), with as few instructions as it takes: the loop's
+    // own latency, not the tensor core, bounded the kernel while the whole warp ran it with an election and a warp
+    // barrier per k-block (560 cycles a k-block at any tile width; 512 is what a 256-wide tile's MMAs take).
+    // After a wait that ran out it stops: a barrier that still expects bytes must not be armed again, and the producer
+    // arms one only after its stage has been committed here.
+    auto multiply = [&]()
     {
-      constexpr uint32_t idesc = make_idesc(BWD, BN, PAIR ? 2 * BM_SUB : BM_SUB);
+      const uint32_t idesc = make_idesc(BWD, bn, PAIR ? 2 * BM_SUB : BM_SUB);
       auto mma = [&](uint32_t d, uint64_t a, uint64_t b, uint32_t accumulate)
       {
         if (PAIR)
@@ -495,67 +581,68 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           umma_commit(bar);
         }
       };
+      const uint64_t adesc_base = make_desc(a_addr(0, 0), 16, 1024);
+      const uint64_t bdesc_base = BWD ? make_desc(b_addr(0), 8192, 1024) : make_desc(b_addr(0), 16, 1024);
       int s = 0;
       uint32_t par = 0;
       int acc = 0;
       uint32_t acc_par = 0;
-      // After a wait that ran out nothing is committed any more: a barrier that still expects bytes must not be armed
-      // again, and the producer arms one only after its stage has been committed here.
-      bool gave_up = false;
       for (int tile = worker; tile < num_tiles; tile += workers)
       {
-        gave_up |= !wait(acc_empty(acc), acc_par ^ 1u);
-        tc_fence_after();
+        if (!wait(acc_empty(acc), acc_par ^ 1u))
+        {
+          return;
+        }
+        const uint32_t d0 = tmem_base + static_cast<uint32_t>(acc * ACC_COLS);
+        uint32_t accumulate = 0;
         for (int kb = 0; kb < num_kb_all; ++kb)
         {
-          gave_up |= !wait(a_full(s), par);
-          gave_up |= !wait(b_full(s), par);
+          if (!wait(a_full(s), par) || (WMODE != W_BF16 && !wait(b_full(s), par)))
+          {
+            return;
+          }
           tc_fence_after();
-          const uint64_t adesc0 = make_desc(a_addr(s, 0), 16, 1024);
-          const uint64_t bdesc0 = BWD ? make_desc(b_addr(s), 8192, 1024) : make_desc(b_addr(s), 16, 1024);
-          const uint32_t d0 = tmem_base + static_cast<uint32_t>(acc * ACC_COLS);
-          if (elect_one() && !gave_up)
+          // descriptor address fields count 16-byte units
+          const uint64_t stage = static_cast<uint64_t>(s) * (STAGE_BYTES >> 4);
+#pragma unroll
+          for (int mt = 0; mt < MTK; ++mt)
           {
 #pragma unroll
-            for (int mt = 0; mt < MTK; ++mt)
+            for (int k16 = 0; k16 < BK / UMMA_K; ++k16)
             {
-#pragma unroll
-              for (int k16 = 0; k16 < BK / UMMA_K; ++k16)
+              const uint64_t adesc = adesc_base + stage + static_cast<uint64_t>((mt * A_SUB_BYTES + k16 * (UMMA_K * 2)) >> 4);
+              const uint64_t bdesc = bdesc_base + stage + static_cast<uint64_t>((BWD ? k16 * 2048 : k16 * (UMMA_K * 2)) >> 4);
+              mma(d0 + static_cast<uint32_t>(mt * BN), adesc, bdesc, (k16 == 0) ? accumulate : 1u);
+              if (PLANES == 2 && kb < num_kb)
               {
-                // descriptor address fields count 16-byte units
-                const uint64_t adesc = adesc0 + static_cast<uint64_t>((mt * A_SUB_BYTES + k16 * (UMMA_K * 2)) >> 4);
-                const uint64_t bdesc = bdesc0 + static_cast<uint64_t>((BWD ? k16 * 2048 : k16 * (UMMA_K * 2)) >> 4);
-                mma(d0 + static_cast<uint32_t>(mt * BN), adesc, bdesc, (kb > 0 || k16 > 0) ? 1u : 0u);
-                if (PLANES == 2 && kb < num_kb)
-                {
-                  // the low-order term of the weights (the LoRA k-block has one plane only)
-                  mma(d0 + static_cast<uint32_t>(mt * BN), adesc, bdesc + static_cast<uint64_t>(B_PLANE_BYTES >> 4), 1u);
-                }
+                // the low-order term of the weights (the LoRA k-block has one plane only)
+                mma(d0 + static_cast<uint32_t>(mt * BN), adesc, bdesc + static_cast<uint64_t>(B_PLANE_BYTES >> 4), 1u);
               }
             }
-            commit(empty(s));
           }
-          __syncwarp();
+          commit(empty(s));
+          accumulate = 1;
           if (++s == STAGES)
           {
             s = 0;
             par ^= 1u;
           }
         }
-        if (elect_one() && !gave_up)
-        {
-          commit(acc_full(acc));
-        }
-        __syncwarp();
+        commit(acc_full(acc));
         if (++acc == ACC_BUFS)
         {
           acc = 0;
           acc_par ^= 1u;
         }
       }
+    };
+    if (rank == 0 && elect_one())
+    {
+      multiply();
     }
+    __syncwarp();
   }
-  else if (warp < DEQ_WARP0 + 4 * (EPI_GROUPS - 1))
+  else if (warp >= 2 && warp < DEQ_WARP0 + 4 * (EPI_GROUPS - 1))
   {
     // ---------------------------------------------------------------- epilogue
     const int quarter = warp & 3;  // TMEM lanes 32*quarter .. +31 are the ones this warp may read
@@ -612,11 +699,11 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
               uint4 *du = reinterpret_cast<uint4 *>(static_cast<uint16_t *>(p.c_up) + off);
               uint4 *dh = reinterpret_cast<uint4 *>(static_cast<uint16_t *>(p.c_hidden) + off);
 #pragma unroll
-              for (int q = 0; q < 4; ++q)
+              for (int q = 0; q < 2; ++q)
               {
-                uint32_t pg[4], pu[4], ph[4];
+                uint32_t pg[8], pu[8], ph[8];
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
+                for (int e = 0; e < 8; ++e)
                 {
                   float g2[2], u2[2], h2[2];
 #pragma unroll
@@ -624,8 +711,8 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                   {
                     // the separate kernels' roundings: projection outputs to the storage dtype,
                     // silu(gate) to the storage dtype, then the product
-                    g2[z] = round_through<CAIFQ_BF16>(__uint_as_float(rg[8 * q + 2 * e + z]) * out_scale);
-                    u2[z] = round_through<CAIFQ_BF16>(__uint_as_float(ru[8 * q + 2 * e + z]) * up_scale);
+                    g2[z] = round_through<CAIFQ_BF16>(__uint_as_float(rg[16 * q + 2 * e + z]) * out_scale);
+                    u2[z] = round_through<CAIFQ_BF16>(__uint_as_float(ru[16 * q + 2 * e + z]) * up_scale);
                     const float act = round_through<CAIFQ_BF16>(g2[z] / (1.0f + expf(-g2[z])));
                     h2[z] = act * u2[z];
                   }
@@ -633,10 +720,64 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                   pu[e] = pack_bf16x2(u2[0], u2[1]);
                   ph[e] = pack_bf16x2(h2[0], h2[1]);
                 }
-                dg[q] = make_uint4(pg[0], pg[1], pg[2], pg[3]);
-                du[q] = make_uint4(pu[0], pu[1], pu[2], pu[3]);
-                dh[q] = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+                store_row32(dg + 2 * q, pg, p.wide_stores != 0);
+                store_row32(du + 2 * q, pu, p.wide_stores != 0);
+                store_row32(dh + 2 * q, ph, p.wide_stores != 0);
               }
+            }
+          }
+        }
+      }
+      else if (BWD && p.sb_gate != nullptr)
+      {
+        // g_hidden = round(acc); g_up = round(g_hidden * round(silu(gate))); g_gate = round(round(g_hidden *
+        // up) * silu'(gate)): the separate kernel's rounding points (see swiglu_bwd_kernel).  Sixteen columns at a time:
+        // 32-byte loads and stores, and no more registers than that takes.
+#pragma unroll
+        for (int mt = 0; mt < MTK; ++mt)
+        {
+          const int64_t row = tw.row0 + static_cast<int64_t>(rank) * BM_SUB + mt * BM_SUB + quarter * 32 + lane;
+          for (int cb = epi_group; cb < bn / 16; cb += EPI_GROUPS)
+          {
+            const int64_t off = row * p.n_total + static_cast<int64_t>(n_tile) * bn + cb * 16;
+            const bool mine = row < tw.row_end && n_tile * bn + cb * 16 < p.n_total;
+            uint32_t gw[8] = {}, uw[8] = {};
+            if (mine)
+            {
+              load_row32(static_cast<const uint16_t *>(p.sb_gate) + off, gw, p.wide_stores != 0);
+              load_row32(static_cast<const uint16_t *>(p.sb_up) + off, uw, p.wide_stores != 0);
+            }
+            uint32_t r[16];
+            tmem_ld16(tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) +
+                          static_cast<uint32_t>(acc * ACC_COLS + mt * BN + cb * 16),
+                      r);
+            tmem_ld_wait();
+            if (mine)
+            {
+#pragma unroll
+              for (int e = 0; e < 8; ++e)
+              {
+                float og[2], ou[2];
+#pragma unroll
+                for (int z = 0; z < 2; ++z)
+                {
+                  const float x = z ? __uint_as_float(gw[e] & 0xFFFF0000u) : __uint_as_float(gw[e] << 16);
+                  const float uv = z ? __uint_as_float(uw[e] & 0xFFFF0000u) : __uint_as_float(uw[e] << 16);
+                  const float gh = round_through<CAIFQ_BF16>(__uint_as_float(r[2 * e + z]) * out_scale);
+                  // one fast exponential and one fast reciprocal per element: 256 x 128 elements per tile must
+                  // fit beside the next tile's MMAs (the exact expf and two IEEE divisions did not: 2x slower);
+                  // fp32 relative error ~1e-6 before the bf16 roundings
+                  const float sg = __fdividef(1.0f, 1.0f + __expf(-x));
+                  const float act = round_through<CAIFQ_BF16>(x * sg);
+                  ou[z] = gh * act;
+                  const float gv = round_through<CAIFQ_BF16>(gh * uv);
+                  og[z] = gv * sg * fmaf(x, 1.0f - sg, 1.0f);
+                }
+                gw[e] = pack_bf16x2(og[0], og[1]);
+                uw[e] = pack_bf16x2(ou[0], ou[1]);
+              }
+              store_row32(static_cast<uint16_t *>(p.c) + off, gw, p.wide_stores != 0);
+              store_row32(static_cast<uint16_t *>(p.sb_g_up) + off, uw, p.wide_stores != 0);
             }
           }
         }
@@ -649,7 +790,7 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 #pragma unroll
         for (int cb = 0; cb < BN / 32; ++cb)
         {
-          if (EPI_GROUPS > 1 && (cb % EPI_GROUPS) != epi_group)
+          if ((EPI_GROUPS > 1 && (cb % EPI_GROUPS) != epi_group) || (ANY_WIDTH && cb * 32 >= bn))
           {
             continue;
           }
@@ -660,93 +801,56 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           tmem_ld_wait();
           // (the last column tile may reach past the output's width when the width is not a multiple of the
           // tile's: those columns, computed on zero or foreign weight rows, are not stored)
-          if (row < tw.row_end && n_tile * BN + cb * 32 < p.n_total)
+          if (row < tw.row_end && n_tile * bn + cb * 32 < p.n_total)
           {
-            const int64_t off = row * p.n_total + static_cast<int64_t>(n_tile) * BN + cb * 32;
-            if (BWD && p.sb_gate != nullptr)
-            {
-              // g_hidden = round(acc); g_up = round(g_hidden * round(silu(gate))); g_gate = round(round(g_hidden *
-              // up) * silu'(gate)): the separate kernel's rounding points (see swiglu_bwd_kernel)
-              const uint4 *gt4 = reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(p.sb_gate) + off);
-              const uint4 *up4 = reinterpret_cast<const uint4 *>(static_cast<const uint16_t *>(p.sb_up) + off);
-              uint4 *dg = reinterpret_cast<uint4 *>(static_cast<uint16_t *>(p.c) + off);
-              uint4 *du = reinterpret_cast<uint4 *>(static_cast<uint16_t *>(p.sb_g_up) + off);
-#pragma unroll
-              for (int q = 0; q < 4; ++q)
-              {
-                const uint4 gq = __ldg(gt4 + q);
-                const uint4 uq = __ldg(up4 + q);
-                const uint32_t gw[4] = {gq.x, gq.y, gq.z, gq.w};
-                const uint32_t uw[4] = {uq.x, uq.y, uq.z, uq.w};
-                uint32_t pg[4], pu[4];
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                {
-                  float og[2], ou[2];
-#pragma unroll
-                  for (int z = 0; z < 2; ++z)
-                  {
-                    const float x = z ? __uint_as_float(gw[e] & 0xFFFF0000u) : __uint_as_float(gw[e] << 16);
-                    const float uv = z ? __uint_as_float(uw[e] & 0xFFFF0000u) : __uint_as_float(uw[e] << 16);
-                    const float gh = round_through<CAIFQ_BF16>(__uint_as_float(r[8 * q + 2 * e + z]) * out_scale);
-                    // one fast exponential and one fast reciprocal per element: 256 x 128 elements per tile must
-                    // fit beside the next tile's MMAs (the exact expf and two IEEE divisions did not: 2x slower);
-                    // fp32 relative error ~1e-6 before the bf16 roundings
-                    const float sg = __fdividef(1.0f, 1.0f + __expf(-x));
-                    const float act = round_through<CAIFQ_BF16>(x * sg);
-                    ou[z] = gh * act;
-                    const float gv = round_through<CAIFQ_BF16>(gh * uv);
-                    og[z] = gv * sg * fmaf(x, 1.0f - sg, 1.0f);
-                  }
-                  pg[e] = pack_bf16x2(og[0], og[1]);
-                  pu[e] = pack_bf16x2(ou[0], ou[1]);
-                }
-                dg[q] = make_uint4(pg[0], pg[1], pg[2], pg[3]);
-                du[q] = make_uint4(pu[0], pu[1], pu[2], pu[3]);
-              }
-            }
-            else if (p.c_dtype == CAIFQ_F32)
+            const int64_t off = row * p.n_total + static_cast<int64_t>(n_tile) * bn + cb * 32;
+            if (p.c_dtype == CAIFQ_F32)
             {
               float4 *dst = reinterpret_cast<float4 *>(static_cast<float *>(p.c) + off);
 #pragma unroll
-              for (int q = 0; q < 8; ++q)
+              for (int q = 0; q < 4; ++q)
               {
-                float4 v;
-                v.x = __uint_as_float(r[4 * q + 0]) * out_scale;
-                v.y = __uint_as_float(r[4 * q + 1]) * out_scale;
-                v.z = __uint_as_float(r[4 * q + 2]) * out_scale;
-                v.w = __uint_as_float(r[4 * q + 3]) * out_scale;
+                uint32_t v[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                {
+                  v[e] = __float_as_uint(__uint_as_float(r[8 * q + e]) * out_scale);
+                }
                 if (p.accumulate)
                 {
-                  const float4 o = dst[q];
-                  v.x += o.x;
-                  v.y += o.y;
-                  v.z += o.z;
-                  v.w += o.w;
+                  const float4 o0 = dst[2 * q];
+                  const float4 o1 = dst[2 * q + 1];
+                  const float o[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
+#pragma unroll
+                  for (int e = 0; e < 8; ++e)
+                  {
+                    v[e] = __float_as_uint(__uint_as_float(v[e]) + o[e]);
+                  }
                 }
-                dst[q] = v;
+                store_row32(dst + 2 * q, v, p.wide_stores != 0);
               }
             }
             else
             {
-              // 16-bit outputs: 32 values = 64 bytes = four 16-byte stores
+              // 16-bit outputs: 32 values = 64 bytes = two 32-byte stores
               uint4 *dst = reinterpret_cast<uint4 *>(static_cast<uint16_t *>(p.c) + off);
 #pragma unroll
-              for (int q = 0; q < 4; ++q)
+              for (int q = 0; q < 2; ++q)
               {
-                float v[8];
+                float v[16];
 #pragma unroll
-                for (int e = 0; e < 8; ++e)
+                for (int e = 0; e < 16; ++e)
                 {
-                  v[e] = __uint_as_float(r[8 * q + e]) * out_scale;
+                  v[e] = __uint_as_float(r[16 * q + e]) * out_scale;
                 }
-                uint32_t packed[4];
+                uint32_t packed[8];
                 if (p.accumulate)
                 {
-                  const uint4 o = dst[q];
-                  const uint32_t ow[4] = {o.x, o.y, o.z, o.w};
+                  const uint4 o0 = dst[2 * q];
+                  const uint4 o1 = dst[2 * q + 1];
+                  const uint32_t ow[8] = {o0.x, o0.y, o0.z, o0.w, o1.x, o1.y, o1.z, o1.w};
 #pragma unroll
-                  for (int e = 0; e < 4; ++e)
+                  for (int e = 0; e < 8; ++e)
                   {
                     float lo;
                     float hi;
@@ -766,7 +870,7 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                   }
                 }
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
+                for (int e = 0; e < 8; ++e)
                 {
                   if (p.c_dtype == CAIFQ_BF16)
                   {
@@ -778,7 +882,7 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
                     packed[e] = *reinterpret_cast<const uint32_t *>(&h);
                   }
                 }
-                dst[q] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
+                store_row32(dst + 2 * q, packed, p.wide_stores != 0);
               }
             }
           }
@@ -1172,11 +1276,13 @@ int launch_inst(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtens
     cfg.blockDim = dim3(NUM_THREADS, 1, 1);
     cfg.dynamicSmemBytes = SMEM_BYTES;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = 2;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     // The grid is persistent, so it must not hold more pairs than the device keeps resident at a time (a
@@ -1201,12 +1307,12 @@ int launch_inst(const CUtensorMap &map_a, const CUtensorMap &map_b, const CUtens
       pairs = static_cast<int>(tiles);
     }
     cfg.gridDim = dim3(static_cast<unsigned>(2 * pairs), 1, 1);
+    cfg.numAttrs = dependent_launches() ? 2 : 1;
     CAIFQ_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, map_a, map_b, map_h, map_l, p, gt));
     return CAIFQ_OK;
   }
   const int grid = tiles < sm_count_umma() ? static_cast<int>(tiles) : sm_count_umma();
-  kernel<<<grid, NUM_THREADS, SMEM_BYTES, s>>>(map_a, map_b, map_h, map_l, p, gt);
-  CAIFQ_CHECK_LAUNCH();
+  CAIFQ_CHECK_CUDA(launch_dependent(kernel, dim3(grid), dim3(NUM_THREADS), SMEM_BYTES, s, map_a, map_b, map_h, map_l, p, gt));
   return CAIFQ_OK;
 }
 
@@ -1222,6 +1328,39 @@ int umma_pair_capacity()
   }
   return g_pair_capacity[dev].load(std::memory_order_relaxed);
 }
+
+namespace
+{
+
+// Columns of a pair's tile for a bf16 weight.  The grid is persistent, so a launch takes as many waves as the busiest pair
+// has tiles, and a last wave of a few tiles costs as much as a full one: 8 x 56 tiles of 256 are 6.05 waves of 74 pairs,
+// 8 x 64 tiles of 224 are 6.92 (2047 tokens of 4096 -> 14336: 165 and 153 us).  A wave's time is near linear in the width
+// with a constant that is the copies' (measured per wave: 15.6 us at 128 columns, 17.0 at 160, 18.4 at 192, 21.9 at 224,
+// 23.5 at 256); few tiles (1 wave at any width) so take the narrowest.
+int choose_pair_width(int m_tiles, int n_total, int pairs)
+{
+  constexpr int kWaveConstant = 120;   // columns
+  const int widest = n_total < 256 ? (n_total + 31) & ~31 : 256;
+  int best = 0;
+  int64_t best_cost = 0;
+  for (int bn = widest; bn >= 64; bn -= 32)
+  {
+    const int64_t tiles = static_cast<int64_t>(m_tiles) * ((n_total + bn - 1) / bn);
+    const int64_t cost = (tiles + pairs - 1) / pairs * (bn + kWaveConstant);
+    if (best == 0 || cost < best_cost)
+    {
+      best = bn;
+      best_cost = cost;
+    }
+    if (bn <= 128)
+    {
+      break;   // below, the copies are all there is to a wave
+    }
+  }
+  return best == 0 ? 64 : best;
+}
+
+}  // namespace
 
 bool umma_supported(const LinearArgs &g)
 {
@@ -1294,28 +1433,48 @@ int launch_linear_umma(const LinearArgs &g, cudaStream_t s)
   p.group_size = w.group_size;
   p.groups_per_row = (w.group_size > 0) ? w.in_dim / w.group_size : 0;
   p.num_m_tiles = static_cast<int>((g.m + BM - 1) / BM);
+  p.band = kBand;
+  p.wide_stores = (reinterpret_cast<uintptr_t>(g.c) & 31u) == 0;
   // 256-wide tiles feed the tensor core better per shared-memory byte; 128-wide ones keep a
   // second accumulator set so the epilogue overlaps the next tile.  CAIFQ_UMMA_BN overrides.
   // A 256-wide tile goes to a CTA pair (half the operand bytes per SM and flop, two accumulator sets) when
   // there are enough tiles for the pairs, else to a single CTA when there are enough for the SMs.
   const int mode = wmode_of(w, g.compute_dtype);
-  const bool pair = pairs_enabled(mode) && (p.n_total % 256) == 0 &&
-                    static_cast<int64_t>(p.num_m_tiles) * (p.n_total / 256) >= pair_count_umma();
-  int bn = (pair || ((p.n_total % 256) == 0 &&
-                     static_cast<int64_t>(p.num_m_tiles) * (p.n_total / 256) >= sm_count_umma()))
-               ? 256
-               : 128;
-  if (const char *e = std::getenv("CAIFQ_UMMA_BN"))
+  const char *forced = std::getenv("CAIFQ_UMMA_BN");
+  int bn = 128;
+  bool pair = false;
+  if (mode == W_BF16)
   {
-    const int v = std::atoi(e);
-    if (v == 128 || (v == 256 && (p.n_total % 256) == 0))
+    p.bn = pairs_enabled(mode) ? choose_pair_width(p.num_m_tiles, p.n_total, pair_count_umma()) : 0;
+    if (forced != nullptr && p.bn != 0)
     {
-      bn = v;
+      p.bn = std::atoi(forced) & ~31;
+      p.bn = p.bn < 64 ? 64 : (p.bn > 256 ? 256 : p.bn);
     }
+    pair = p.bn != 0;
+    bn = pair ? p.bn : 128;
   }
-  if (w.storage == CAIFQ_I4 && g.compute_dtype == CAIFQ_F32 && !(pair && bn == 256))
+  else
   {
-    bn = 128;   // a single CTA has 128-wide tiles only in the two-plane mode
+    pair = pairs_enabled(mode) && (p.n_total % 256) == 0 &&
+           static_cast<int64_t>(p.num_m_tiles) * (p.n_total / 256) >= pair_count_umma();
+    bn = (pair || ((p.n_total % 256) == 0 &&
+                   static_cast<int64_t>(p.num_m_tiles) * (p.n_total / 256) >= sm_count_umma()))
+             ? 256
+             : 128;
+    if (forced != nullptr)
+    {
+      const int v = std::atoi(forced);
+      if (v == 128 || (v == 256 && (p.n_total % 256) == 0))
+      {
+        bn = v;
+      }
+    }
+    if (mode == W_I4S && !(pair && bn == 256))
+    {
+      bn = 128;   // a single CTA has 128-wide tiles only in the two-plane mode
+    }
+    pair = pair && bn == 256;
   }
   p.num_n_tiles = (p.n_total + bn - 1) / bn;
 
@@ -1330,7 +1489,7 @@ int launch_linear_umma(const LinearArgs &g, cudaStream_t s)
   {
     // the [out, in] weight itself: forward boxes are 64 k x 128 n rows, backward 64 n x 64 k rows
     rc = make_map_bf16(&map_b, w.codes, static_cast<uint64_t>(w.in_dim), static_cast<uint64_t>(w.out_dim),
-                       g.backward ? BK : ((pair && bn == 256) ? 128 : bn));
+                       g.backward ? BK : (pair ? bn / 2 : bn));
     if (rc != CAIFQ_OK)
     {
       return rc;
@@ -1357,7 +1516,7 @@ int launch_linear_umma(const LinearArgs &g, cudaStream_t s)
       // [64, N] (backward, boxes of 64 n x 64 k), like the weight itself
       rc = g.backward ? make_map_bf16(&map_l, g.lora_rhs, static_cast<uint64_t>(p.n_total), 64, BK)
                       : make_map_bf16(&map_l, g.lora_rhs, 64, static_cast<uint64_t>(p.n_total),
-                                      (pair && bn == 256) ? 128 : bn);
+                                      pair ? bn / 2 : bn);
       if (rc != CAIFQ_OK)
       {
         return rc;
@@ -1365,7 +1524,7 @@ int launch_linear_umma(const LinearArgs &g, cudaStream_t s)
     }
   }
 #define CAIFQ_UMMA_PAIR_CASE(MODE)                                                                      \
-  if (mode == MODE && bn == 256 && pair)                                                                \
+  if (mode == MODE && pair)                                                                \
   {                                                                                                     \
     return g.backward ? launch_inst<MODE, true, 256, false, true>(map_a, map_b, map_h, map_l, p, NoGroupTable{}, s)   \
                       : launch_inst<MODE, false, 256, false, true>(map_a, map_b, map_h, map_l, p, NoGroupTable{}, s); \
@@ -1465,6 +1624,8 @@ int launch_linear_umma_grouped(const GroupedLinearArgs &g, cudaStream_t s)
   p.c = g.c;
   p.c_dtype = g.c_dtype;
   p.accumulate = g.accumulate ? 1 : 0;
+  p.wide_stores = ((reinterpret_cast<uintptr_t>(g.c) | reinterpret_cast<uintptr_t>(g.sb_g_up) |
+                    reinterpret_cast<uintptr_t>(g.sb_gate) | reinterpret_cast<uintptr_t>(g.sb_up)) & 31u) == 0;
   p.m = total_rows;
   p.n_total = g.backward ? w0.in_dim : w0.out_dim;
   p.k_total = g.backward ? w0.out_dim : w0.in_dim;
@@ -1517,6 +1678,7 @@ int launch_linear_umma_grouped(const GroupedLinearArgs &g, cudaStream_t s)
       // half is masked in the epilogue, 9 % of wasted MMAs against 62 -> 85 % tensor activity)
       const int wide_tiles = (p.n_total + 255) / 256;
       const bool wide = static_cast<int64_t>(tiles) * wide_tiles >= pair_count_umma() && pairs_enabled(mode);
+      p.bn = 256;
       p.num_n_tiles = wide ? wide_tiles : p.n_total / 128;
       p.expert_rows = w0.out_dim;
       CUtensorMap map_b;
@@ -1662,6 +1824,8 @@ int launch_linear_umma_swiglu(const GroupedSwigluArgs &g, cudaStream_t s)
   p.c_hidden = g.hidden;
   p.c_dtype = g.dtype;
   p.accumulate = 0;
+  p.wide_stores = ((reinterpret_cast<uintptr_t>(g.gate_out) | reinterpret_cast<uintptr_t>(g.up_out) |
+                    reinterpret_cast<uintptr_t>(g.hidden)) & 31u) == 0;
   p.m = total_rows;
   p.n_total = 2 * w0.out_dim;   // gate and up features side by side in every tile
   p.k_total = w0.in_dim;
@@ -1669,6 +1833,7 @@ int launch_linear_umma_swiglu(const GroupedSwigluArgs &g, cudaStream_t s)
   p.group_size = w0.group_size;
   p.groups_per_row = (w0.group_size > 0) ? w0.in_dim / w0.group_size : 0;
   p.swiglu = 1;
+  p.bn = 256;
   CUtensorMap map_a;
   int rc = make_map_bf16(&map_a, g.x, static_cast<uint64_t>(p.k_total), static_cast<uint64_t>(total_rows), BM_SUB);
   if (rc != CAIFQ_OK)
