@@ -30,7 +30,7 @@ PyObject *g_error = nullptr;   // native.CaifqError
 
 // entry points, looked up in the library that native.py loaded
 #define CAIFQ_BOUND(X)                                                                                                \
-  X(linear_fwd) X(linear_fwd_residual) X(linear_fwd_multi) X(linear_dx) X(linear_concat_workspace_bytes)              \
+  X(linear_fwd) X(linear_fwd_residual) X(linear_fwd_multi) X(linear_dx) X(linear_workspace_bytes) X(linear_fwd_ws) X(linear_dx_ws) X(linear_concat_workspace_bytes)              \
   X(linear_fwd_concat) X(linear_dx_concat) X(lora_fwd_workspace_bytes) X(lora_fwd_workspace_bytes_expanded)           \
   X(lora_bwd_workspace_bytes) X(lora_bwd_workspace_bytes_expanded) X(lora_linear_fwd) X(lora_linear_fwd_expanded)     \
   X(lora_linear_bwd) X(lora_linear_bwd_expanded) X(rmsnorm_fwd) X(rmsnorm_bwd) X(cast) X(quantize_int8_per_tensor)    \
@@ -322,6 +322,19 @@ int unlocked(F &&f)
   return rc;
 }
 
+// Scratch that a call can do without: undefined when the device has no memory left for it.
+at::Tensor scratch(size_t bytes, const at::Tensor &like)
+{
+  try
+  {
+    return empty({static_cast<int64_t>(bytes)}, at::kByte, like);
+  }
+  catch (const c10::OutOfMemoryError &)
+  {
+    return at::Tensor();
+  }
+}
+
 // ---- frozen linear ------------------------------------------------------------------------------------------
 
 // (weight, act, out_dtype, compute, out | None): forward or dX
@@ -336,8 +349,12 @@ PyObject *linear(Args &a, bool backward)
   at::Tensor y = out != nullptr ? *out : empty(shape_with_last(x, backward ? w->in_dim : w->out_dim), out_dtype, x);
   const int xc = code_of(x), yc = code_of(y);
   void *s = stream();
-  auto fn = backward ? api.linear_dx : api.linear_fwd;
-  check(unlocked([&] { return fn(w, ptr(x), xc, m, ptr(y), yc, compute, s); }), backward ? "linear_dx" : "linear_fwd");
+  const size_t need = api.linear_workspace_bytes(w, backward ? 1 : 0, xc, m, compute);
+  const at::Tensor work = need > 0 ? scratch(need, x) : at::Tensor();
+  void *scratch_ptr = work.defined() ? ptr(work) : nullptr;
+  auto fn = backward ? api.linear_dx_ws : api.linear_fwd_ws;
+  check(unlocked([&] { return fn(w, ptr(x), xc, m, ptr(y), yc, compute, scratch_ptr, scratch_ptr ? need : 0, s); }),
+        backward ? "linear_dx" : "linear_fwd");
   return wrap(std::move(y));
 }
 

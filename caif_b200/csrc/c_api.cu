@@ -342,11 +342,12 @@ bool fused_lora_ok(const caifq_weight *w, const caifq_lora *l, const void *act, 
 // Many-token calls may expand the weight once per call into a bf16 matrix in the caller's workspace and feed
 // it to the tensor core with plain tile copies on CTA pairs (1.43-1.55 PFLOP/s per launch at 4096 x 4096,
 // 8192 tokens) instead of converting every tile again in the dequant warps of every CTA (1.1-1.3): the
-// conversion is then done once per weight, not once per weight and 256 rows of tokens.  Worth its 10-15 us
-// from a few thousand tokens on.  int4 needs bf16 compute (fp32 compute keeps the two-term form).
+// conversion is then done once per weight, not once per weight and 256 rows of tokens.  The expansion takes 2.5 bytes
+// of HBM a weight (4096 x 4096: 7 us), the in-kernel conversion at least 40 us at any number of tokens, so it pays
+// from half a tile of tokens on.  int4 needs bf16 compute (fp32 compute keeps the two-term form).
 bool expand_ok(const caifq_weight *w, const caifq_lora *l, const void *act, int64_t m, int compute_dtype)
 {
-  if (m < 4096 || !fused_lora_ok(w, l, act, m, compute_dtype))
+  if (m < 128 || !fused_lora_ok(w, l, act, m, compute_dtype))
   {
     return false;
   }
@@ -354,7 +355,33 @@ bool expand_ok(const caifq_weight *w, const caifq_lora *l, const void *act, int6
   {
     return false;
   }
-  return (w->in_dim % 256) == 0 && (w->out_dim % 256) == 0;
+  return true;
+}
+
+// A plain product (no adapter) that expands its weight into the caller's workspace first.  The conversion inside the
+// tensor-core kernels is repeated for every 256 tokens and bounds them from about 700 tokens on; the expansion costs 2.5
+// bytes of HBM a weight once (4096 x 14336 int4: 22 us).  Forward calls of up to kStreamMostTokens tokens are the
+// streaming kernel's.  dX has no such kernel: the expansion pays from half a tile of tokens on (4096 x 14336, 256 rows:
+// 103 us converting in the kernel, 27 + 55 expanded).  int4 with fp32 compute keeps its two operand terms.
+bool expand_linear_ok(const caifq_weight *w, bool backward, const void *a, int a_dtype, int64_t m, const void *c,
+                      int c_dtype, int compute_dtype)
+{
+  if (forced_path() != Force::None || (w->storage != CAIFQ_I8 && w->storage != CAIFQ_I4) ||
+      (w->storage == CAIFQ_I4 && (compute_dtype != CAIFQ_BF16 || (w->group_size % 32) != 0)) || m < 128)
+  {
+    return false;
+  }
+  LinearArgs probe{};
+  probe.w = *w;
+  probe.a = a;
+  probe.a_dtype = a_dtype;
+  probe.a_prescale = 1.0f;
+  probe.m = m;
+  probe.c = const_cast<void *>(c);
+  probe.c_dtype = c_dtype;
+  probe.compute_dtype = compute_dtype;
+  probe.backward = backward;
+  return umma_supported(probe) && !stream_supported(probe);
 }
 
 size_t expanded_weight_bytes(const caifq_weight *w)
@@ -541,6 +568,61 @@ int caifq_linear_fwd(const caifq_weight *w, const void *x, int32_t x_dtype, int6
 {
   return linear_any(w, false, x, x_dtype, 1.0f, m, y, y_dtype, false, compute_dtype,
                     static_cast<cudaStream_t>(stream), "caifq_linear_fwd");
+}
+
+}  // extern "C"
+
+static int linear_ws(const caifq_weight *w, bool backward, const void *a, int a_dtype, int64_t m, void *c, int c_dtype,
+                     int compute_dtype, void *workspace, size_t workspace_bytes, cudaStream_t s, const char *who)
+{
+  const int rc = check_weight(w, who);
+  if (rc != CAIFQ_OK)
+  {
+    return rc;
+  }
+  if (workspace == nullptr || a == nullptr || c == nullptr || workspace_bytes < expanded_weight_bytes(w) ||
+      (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0 ||
+      !expand_linear_ok(w, backward, a, a_dtype, m, c, c_dtype, compute_dtype))
+  {
+    return linear_any(w, backward, a, a_dtype, 1.0f, m, c, c_dtype, false, compute_dtype, s, who);
+  }
+  const int r = launch_expand_prepare(*w, workspace, nullptr, nullptr, nullptr, nullptr, nullptr, 0, s);
+  if (r != CAIFQ_OK)
+  {
+    return r;
+  }
+  const caifq_weight wbf = float_weight(workspace, CAIFQ_BF16, w->out_dim, w->in_dim);
+  return linear_any(&wbf, backward, a, a_dtype, 1.0f, m, c, c_dtype, false, compute_dtype, s, who, nullptr, nullptr,
+                    epilogue_scale_ptr(w));
+}
+
+extern "C" {
+
+size_t caifq_linear_workspace_bytes(const caifq_weight *w, int32_t backward, int32_t a_dtype, int64_t m,
+                                    int32_t compute_dtype)
+{
+  if (w == nullptr || w->codes == nullptr || w->in_dim <= 0 || w->out_dim <= 0)
+  {
+    return 0;
+  }
+  const void *aligned = reinterpret_cast<const void *>(static_cast<uintptr_t>(256));   // only alignment is looked at
+  return expand_linear_ok(w, backward != 0, aligned, a_dtype, m, aligned, CAIFQ_BF16, compute_dtype)
+             ? expanded_weight_bytes(w)
+             : 0;
+}
+
+int caifq_linear_fwd_ws(const caifq_weight *w, const void *x, int32_t x_dtype, int64_t m, void *y, int32_t y_dtype,
+                        int32_t compute_dtype, void *workspace, size_t workspace_bytes, void *stream)
+{
+  return linear_ws(w, false, x, x_dtype, m, y, y_dtype, compute_dtype, workspace, workspace_bytes,
+                   static_cast<cudaStream_t>(stream), "caifq_linear_fwd");
+}
+
+int caifq_linear_dx_ws(const caifq_weight *w, const void *dy, int32_t dy_dtype, int64_t m, void *dx, int32_t dx_dtype,
+                       int32_t compute_dtype, void *workspace, size_t workspace_bytes, void *stream)
+{
+  return linear_ws(w, true, dy, dy_dtype, m, dx, dx_dtype, compute_dtype, workspace, workspace_bytes,
+                   static_cast<cudaStream_t>(stream), "caifq_linear_dx");
 }
 
 int caifq_linear_fwd_residual(const caifq_weight *w, const void *x, int32_t x_dtype, int64_t m, void *y_inout,

@@ -86,6 +86,11 @@ _SIGNATURES = {
     "caifq_linear_fwd_gather": (ctypes.c_int, [ctypes.POINTER(CWeight), _vp, _i32, _i64, ctypes.POINTER(_vp), _i32,
                                                _i64, _i64, _i32, _i32, _vp]),
     "caifq_linear_dx": (ctypes.c_int, [ctypes.POINTER(CWeight), _vp, _i32, _i64, _vp, _i32, _i32, _vp]),
+    "caifq_linear_workspace_bytes": (ctypes.c_size_t, [ctypes.POINTER(CWeight), _i32, _i32, _i64, _i32]),
+    "caifq_linear_fwd_ws": (ctypes.c_int, [ctypes.POINTER(CWeight), _vp, _i32, _i64, _vp, _i32, _i32, _vp,
+                                           ctypes.c_size_t, _vp]),
+    "caifq_linear_dx_ws": (ctypes.c_int, [ctypes.POINTER(CWeight), _vp, _i32, _i64, _vp, _i32, _i32, _vp,
+                                          ctypes.c_size_t, _vp]),
     "caifq_lora_fwd_workspace_bytes": (ctypes.c_size_t, [ctypes.POINTER(CWeight), ctypes.POINTER(CLora), _i64]),
     "caifq_lora_linear_fwd": (ctypes.c_int, [ctypes.POINTER(CWeight), ctypes.POINTER(CLora), _vp, _i64, _vp, _vp,
                                              _vp, _i32, _vp]),

@@ -179,6 +179,21 @@ CAIFQ_API int caifq_linear_dx(const caifq_weight *w, const void *dy, int32_t dy_
                     int32_t compute_dtype, void *stream);
 
 /*
+ * The same two calls with a scratch for many tokens: with a workspace of caifq_linear_workspace_bytes(...) bytes, 256-byte
+ * aligned, the weight is expanded once per call into a bf16 [out, in] matrix there (int8 codes as exact integers whose
+ * scale is applied to the sum, int4 codes times their group scale, rounded once) and the tensor core reads plain tiles,
+ * instead of converting every tile again for every 256 tokens.  A size of 0 means that these calls do not expand; with a
+ * null or smaller workspace they are the plain calls.  The workspace is scratch: nothing in it outlives the call.
+ */
+CAIFQ_API size_t caifq_linear_workspace_bytes(const caifq_weight *w, int32_t backward, int32_t a_dtype, int64_t m,
+                                              int32_t compute_dtype);
+CAIFQ_API int caifq_linear_fwd_ws(const caifq_weight *w, const void *x, int32_t x_dtype, int64_t m, void *y, int32_t y_dtype,
+                                  int32_t compute_dtype, void *workspace, size_t workspace_bytes, void *stream);
+CAIFQ_API int caifq_linear_dx_ws(const caifq_weight *w, const void *dy, int32_t dy_dtype, int64_t m, void *dx,
+                                 int32_t dx_dtype, int32_t compute_dtype, void *workspace, size_t workspace_bytes,
+                                 void *stream);
+
+/*
  * Column-parallel forward with the all-gather of Y fused into the kernel's stores, for layers
  * sharded by output features over the GPUs of one box (the reference itself has no multi-GPU
  * linear; this replaces ForwardImpl followed by an NCCL all-gather of the slices).

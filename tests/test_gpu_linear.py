@@ -622,3 +622,44 @@ def test_streaming_wait_that_runs_out_raises_the_flag_and_returns(m, out_dim):
     y2 = nv.linear_fwd(weight, x, torch.float32, orc.BF16)
     assert nv.lib().caifq_device_status() == 0
     assert torch.equal(y, y2)
+
+
+@pytest.mark.parametrize("width", ["64", "96", "128", "160", "192", "224", "256", None])
+@pytest.mark.parametrize("m,in_dim,out_dim", [(300, 320, 480), (2305, 128, 1088)])   # partial tiles both ways; 10 row tiles
+def test_umma_bf16_tile_widths(width, m, in_dim, out_dim, monkeypatch):
+    if width is not None:
+        monkeypatch.setenv("CAIFQ_UMMA_BN", width)
+    out_dx = (out_dim + 63) // 64 * 64      # dX reduces over the output features, 64 at a time
+    weight, wc, x_np, x, dy_np, dy = _umma_case(orc.BF16, orc.F32, m, in_dim, out_dim, m + out_dim)
+    y = nv.linear_fwd(weight, x, torch.float32, orc.F32)
+    assert nv.last_path() == "umma"
+    assert max_rel_err(y.cpu().numpy(), x_np.astype(np.float64) @ wc.astype(np.float64).T) <= TOL_F32
+    out = torch.empty(m * out_dim + 8, dtype=torch.bfloat16, device="cuda")[8:].view(m, out_dim)   # 16-byte aligned only
+    nv.linear_fwd(weight, x, torch.bfloat16, orc.F32, out=out)
+    assert torch.equal(out, y.to(torch.bfloat16))
+    weight, wc, x_np, x, dy_np, dy = _umma_case(orc.BF16, orc.F32, m, in_dim, out_dx, m + out_dx)
+    dx = nv.linear_dx(weight, dy, torch.float32, orc.F32)
+    assert max_rel_err(dx.cpu().numpy(), dy_np.astype(np.float64) @ wc.astype(np.float64)) <= TOL_F32
+    assert nv.lib().caifq_device_status() == 0
+
+
+@pytest.mark.parametrize("storage,compute,group", [(orc.I8, orc.F32, 128), (orc.I8, orc.BF16, 128), (orc.I4, orc.BF16, 32),
+                                                   (orc.I4, orc.BF16, 96)])
+@pytest.mark.parametrize("m,in_dim,out_dim", [(128, 384, 640), (769, 1152, 384), (1025, 768, 128)])
+def test_many_tokens_through_an_expanded_weight(storage, compute, group, m, in_dim, out_dim):
+    """The binding hands linear_fwd / linear_dx a scratch for the weight as bf16; without one (the plain C calls) the same
+    values come from the in-kernel conversion.  int4: code times scale rounded once, so the bound is a bf16 GEMM's own."""
+    weight, wc, x_np, x, dy_np, dy = _umma_case(storage, compute, m, in_dim, out_dim, m + out_dim, group)
+    need = nv.lib().caifq_linear_workspace_bytes
+    assert need(weight.ref(), 1, nv.BF16, m, compute) == in_dim * out_dim * 2
+    assert (need(weight.ref(), 0, nv.BF16, m, compute) > 0) == (m > 768)
+    assert need(weight.ref(), 1, nv.F32, m, compute) == 0 and need(weight.ref(), 1, nv.BF16, 127, compute) == 0
+    tol = TOL_F32 if compute == orc.F32 else 4e-3
+    y = nv.linear_fwd(weight, x, torch.float32, compute)
+    dx = nv.linear_dx(weight, dy, torch.float32, compute)
+    assert nv.last_path() == "umma"
+    assert max_rel_err(y.cpu().numpy(), x_np.astype(np.float64) @ wc.astype(np.float64).T) <= tol
+    assert max_rel_err(dx.cpu().numpy(), dy_np.astype(np.float64) @ wc.astype(np.float64)) <= tol
+    plain = torch.empty_like(dx)
+    rc = nv.lib().caifq_linear_dx(weight.ref(), dy.data_ptr(), nv.BF16, m, plain.data_ptr(), nv.F32, compute, nv._stream())
+    assert rc == 0 and max_rel_err(plain.cpu().numpy(), dx.cpu().numpy()) <= 2 * tol
