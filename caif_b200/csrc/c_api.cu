@@ -145,14 +145,11 @@ int launch_lora_adamw(void *a, void *b, const void *d_a, const void *d_b, float 
                       cudaStream_t s);
 bool skinny_supported(int dtype, int rank, int k);
 int launch_skinny_nt(const void *x, const void *a, void *h, void *hs, float x_prescale, float hs_mul,
-                     const float *hs_div, int64_t m, int k, int rank, cudaStream_t s);
-int launch_skinny_tn(const void *u, const void *v, void *c, float *scratch, float u_prescale, int64_t m, int big,
-                     int rank, bool transpose_out, cudaStream_t s);
-int launch_lora_pad_b(const void *b, void *bp, int n, int rank, cudaStream_t s);
-int launch_lora_transpose_b(const void *b, void *bt, int n, int rank, cudaStream_t s);
-int launch_lora_pad_a(const void *a, void *ap, int n, int rank, cudaStream_t s);
+                     const float *hs_div, int64_t m, int k, int rank, bool independent, cudaStream_t s);
+int launch_skinny_tn(const void *dy, const void *h, void *db, float prescale, int out, const void *x, const void *dh,
+                     void *da, int in, float *sums, int64_t m, int rank, cudaStream_t s);
 int launch_expand_prepare(const caifq_weight &w, void *wb, const void *a, const void *b, void *bp, void *bt, void *ap,
-                          int rank, cudaStream_t s);
+                          float *zero, int64_t zeros, int rank, cudaStream_t s);
 
 namespace
 {
@@ -414,7 +411,7 @@ LoraFwdWs lora_fwd_ws(const caifq_weight *w, int64_t m)
 struct LoraBwdWs
 {
   size_t d_hidden;  // [m, r] in <= 4-byte elements
-  size_t scratch;   // fp32 [max(in,out), r]
+  size_t scratch;   // fp32 [in + out, r]
   size_t bt;        // [r, out] bf16
   size_t dhs;       // [m, 64] bf16
   size_t ap;        // [64, in] bf16
@@ -424,10 +421,10 @@ struct LoraBwdWs
 LoraBwdWs lora_bwd_ws(const caifq_weight *w, const caifq_lora *l, int64_t m)
 {
   LoraBwdWs o{};
-  const size_t big = static_cast<size_t>(w->in_dim > w->out_dim ? w->in_dim : w->out_dim);
+  const size_t both = static_cast<size_t>(w->in_dim) + static_cast<size_t>(w->out_dim);
   o.d_hidden = 0;
   o.scratch = align256(static_cast<size_t>(m) * static_cast<size_t>(l->rank) * 4);
-  o.bt = o.scratch + align256(big * static_cast<size_t>(l->rank) * sizeof(float));
+  o.bt = o.scratch + align256(both * static_cast<size_t>(l->rank) * sizeof(float));
   o.dhs = o.bt + align256(static_cast<size_t>(l->rank) * w->out_dim * 2);
   o.ap = o.dhs + align256(static_cast<size_t>(m) * 64 * 2);
   o.total = o.ap + align256(static_cast<size_t>(64) * w->in_dim * 2);
@@ -586,7 +583,7 @@ static int linear_ws(const caifq_weight *w, bool backward, const void *a, int a_
   {
     return linear_any(w, backward, a, a_dtype, 1.0f, m, c, c_dtype, false, compute_dtype, s, who);
   }
-  const int r = launch_expand_prepare(*w, workspace, nullptr, nullptr, nullptr, nullptr, nullptr, 0, s);
+  const int r = launch_expand_prepare(*w, workspace, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, 0, 0, s);
   if (r != CAIFQ_OK)
   {
     return r;
@@ -785,12 +782,12 @@ int lora_fwd_impl(const caifq_weight *w, const caifq_lora *lora, const void *x, 
     const bool expand = may_expand && expand_ok(w, lora, x, m, compute_dtype);
     void *wb = base + ws.total;   // (expanded calls) the weight as a bf16 matrix behind the other scratch
     // the padded B factor, and with it the expansion of the weight where the call expands: one launch
-    int r = expand ? launch_expand_prepare(*w, wb, lora->a, lora->b, base + ws.bp, nullptr, nullptr, lora->rank, s)
-                   : launch_lora_pad_b(lora->b, base + ws.bp, w->out_dim, lora->rank, s);
+    int r = launch_expand_prepare(*w, expand ? wb : nullptr, lora->a, lora->b, base + ws.bp, nullptr, nullptr, nullptr, 0,
+                                  lora->rank, s);
     if (r == CAIFQ_OK)
     {
       r = launch_skinny_nt(x, lora->a, hidden, base + ws.hs, 1.0f, scale, epilogue_scale_ptr(w), m, w->in_dim,
-                           lora->rank, s);
+                           lora->rank, true, s);
     }
     if (r != CAIFQ_OK)
     {
@@ -894,33 +891,18 @@ int lora_bwd_impl(const caifq_weight *w, const caifq_lora *lora, const void *dy,
     // dH = (scale . dy) . B through the transposed copy of B; dHs = dH / epilogue scale, padded
     const bool expand = may_expand && expand_ok(w, lora, dy, m, compute_dtype);
     void *wb = wbase + ws.total;
-    int r = CAIFQ_OK;
-    if (expand)
-    {
-      // transposed B, padded A and the expansion of the weight in one launch
-      r = launch_expand_prepare(*w, wb, lora->a, lora->b, nullptr, wbase + ws.bt, wbase + ws.ap, lora->rank, s);
-    }
-    else
-    {
-      r = launch_lora_transpose_b(lora->b, wbase + ws.bt, w->out_dim, lora->rank, s);
-      if (r == CAIFQ_OK)
-      {
-        r = launch_lora_pad_a(lora->a, wbase + ws.ap, w->in_dim, lora->rank, s);
-      }
-    }
+    // transposed B, padded A, zeros for the gradients' sums and the expansion of the weight in one launch
+    int r = launch_expand_prepare(*w, expand ? wb : nullptr, lora->a, lora->b, nullptr, wbase + ws.bt, wbase + ws.ap,
+                                  scratch, (static_cast<int64_t>(w->in_dim) + w->out_dim) * lora->rank, lora->rank, s);
     if (r == CAIFQ_OK)
     {
       r = launch_skinny_nt(dy, wbase + ws.bt, d_hidden, wbase + ws.dhs, scale, 1.0f, epilogue_scale_ptr(w), m,
-                           w->out_dim, lora->rank, s);
+                           w->out_dim, lora->rank, false, s);
     }
     // dB[out, r] = (scale . dy)^T . hidden;  dA[r, in] = dH^T . x
     if (r == CAIFQ_OK)
     {
-      r = launch_skinny_tn(dy, hidden, d_b, scratch, scale, m, w->out_dim, lora->rank, false, s);
-    }
-    if (r == CAIFQ_OK)
-    {
-      r = launch_skinny_tn(x, d_hidden, d_a, scratch, 1.0f, m, w->in_dim, lora->rank, true, s);
+      r = launch_skinny_tn(dy, hidden, d_b, scale, w->out_dim, x, d_hidden, d_a, w->in_dim, scratch, m, lora->rank, s);
     }
     if (r != CAIFQ_OK)
     {

@@ -6,7 +6,7 @@
 // products accumulate in fp32, the result is rounded once to the storage dtype.
 #include <cstdlib>
 
-#include "common.cuh"
+#include "umma.cuh"
 
 namespace caifq
 {
@@ -148,11 +148,16 @@ __device__ __forceinline__ uint32_t scale2(uint32_t v, float s)
 // for X and A, which is all a dot product needs).  Optionally also writes
 //   Hs[m, 64] = bf16( float(H) * hs_mul / *hs_div ), zero beyond column R,
 // the padded operand the tensor-core kernel consumes as one extra k-block.
+// Bound by latency, not by the 16 to 120 MB of X: few tokens leave most SMs idle and long rows make a warp's chain of
+// loads long, so k is split once more over the CTAs of a cluster, whose sums meet through distributed shared memory in
+// rank order (1000 x 14336: 23 us, with eight CTAs a row tile 13, most of them beside the expansion).
+// `after` = 1: nothing here depends on the kernel before this one in the stream (the weight's expansion), which is only
+// waited for at the end, for the kernels that follow.
 template <int NT>  // NT = R / 8
 __global__ void __launch_bounds__(256)
 skinny_nt_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ a,
                  __nv_bfloat16 *__restrict__ h, __nv_bfloat16 *__restrict__ hs, float x_prescale, float hs_mul,
-                 const float *__restrict__ hs_div, int64_t m, int k)
+                 const float *__restrict__ hs_div, int64_t m, int k, int cluster, int after)
 {
   // a CTA owns 16 rows; its 8 warps split K and add their partial tiles through shared memory
   __shared__ float part[8][16][NT * 8 + 1];
@@ -160,14 +165,20 @@ skinny_nt_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__res
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2;
   const int t = lane & 3;
-  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * 16;
+  if (!after)
+  {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int rank = cluster > 1 ? static_cast<int>(cluster_ctarank()) : 0;
+  const int64_t row0 = static_cast<int64_t>(blockIdx.x / cluster) * 16;
   const int64_t r_lo = row0 + g;
   const int64_t r_hi = row0 + g + 8;
   const bool lo_ok = r_lo < m;
   const bool hi_ok = r_hi < m;
   const int steps = k / 32;  // 32 k per step: 4 lanes x 8
-  const int st_begin = (steps * warp) / 8;
-  const int st_end = (steps * (warp + 1)) / 8;
+  const int st_begin = (steps * (rank * 8 + warp)) / (8 * cluster);
+  const int st_end = (steps * (rank * 8 + warp + 1)) / (8 * cluster);
   const uint4 *x_lo = reinterpret_cast<const uint4 *>(x + (lo_ok ? r_lo : 0) * k) + t;
   const uint4 *x_hi = reinterpret_cast<const uint4 *>(x + (hi_ok ? r_hi : 0) * k) + t;
   const uint4 *a_ptr[NT];
@@ -218,10 +229,51 @@ skinny_nt_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__res
   {
     mul = __fdividef(hs_mul, hs_div[0]);
   }
-  // 16 rows x 64 padded columns, one element pair per thread-iteration
-  for (int e = threadIdx.x; e < 16 * 32; e += 256)
+  // the CTA's eight partial tiles become one, in the first of them
+  float2 sum[(16 * (R / 2) + 255) / 256];
+#pragma unroll
+  for (int i = 0; i < (16 * (R / 2) + 255) / 256; ++i)
   {
-    const int rr = e >> 5;
+    const int e = threadIdx.x + i * 256;
+    sum[i] = make_float2(0.0f, 0.0f);
+    if (e < 16 * (R / 2))
+    {
+#pragma unroll
+      for (int w = 0; w < 8; ++w)
+      {
+        sum[i].x += part[w][e / (R / 2)][e % (R / 2) * 2];
+        sum[i].y += part[w][e / (R / 2)][e % (R / 2) * 2 + 1];
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < (16 * (R / 2) + 255) / 256; ++i)
+  {
+    const int e = threadIdx.x + i * 256;
+    if (e < 16 * (R / 2))
+    {
+      part[0][e / (R / 2)][e % (R / 2) * 2] = sum[i].x;
+      part[0][e / (R / 2)][e % (R / 2) * 2 + 1] = sum[i].y;
+    }
+  }
+  if (cluster > 1)
+  {
+    cluster_sync_all();
+  }
+  else
+  {
+    __syncthreads();
+  }
+  if (after)
+  {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
+  // this CTA's share of the 16 rows x 64 padded columns, one element pair per thread-iteration
+  const int rows = 16 / cluster;
+  for (int e = threadIdx.x; e < rows * 32; e += 256)
+  {
+    const int rr = rank * rows + (e >> 5);
     const int col = (e & 31) * 2;
     const int64_t row = row0 + rr;
     if (row >= m)
@@ -230,13 +282,19 @@ skinny_nt_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__res
     }
     if (col < R)
     {
-      float v0 = 0.0f;
-      float v1 = 0.0f;
-#pragma unroll
-      for (int w = 0; w < 8; ++w)
+      float v0 = part[0][rr][col];
+      float v1 = part[0][rr][col + 1];
+      if (cluster > 1)
       {
-        v0 += part[w][rr][col];
-        v1 += part[w][rr][col + 1];
+        v0 = 0.0f;
+        v1 = 0.0f;
+        const uint32_t mine = static_cast<uint32_t>(__cvta_generic_to_shared(&part[0][rr][col]));
+        for (int c2 = 0; c2 < cluster; ++c2)
+        {
+          const uint32_t theirs = map_to_cta(mine, static_cast<uint32_t>(c2));
+          v0 += __uint_as_float(ld_shared_cluster(theirs));
+          v1 += __uint_as_float(ld_shared_cluster(theirs + 4u));
+        }
       }
       const uint32_t packed = pack2(v0, v1);
       *reinterpret_cast<uint32_t *>(h + row * R + col) = packed;
@@ -249,6 +307,10 @@ skinny_nt_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__res
     {
       *reinterpret_cast<uint32_t *>(hs + row * 64 + col) = 0u;
     }
+  }
+  if (cluster > 1)
+  {
+    cluster_sync_all();   // nobody's shared memory is read after this
   }
 }
 
@@ -279,11 +341,30 @@ constexpr int STN_THREADS = (TN_COLS / 16) * 32;
 constexpr int TN_ROWS = 64;
 constexpr int TN_UPITCH = TN_COLS + 8;  // bf16 elements: 144-byte rows keep ldmatrix conflict-free
 
+// Both gradients of an adapter are one launch: column tiles [0, tiles0) are dB's, the others dA's.
+struct SkinnyTn
+{
+  const __nv_bfloat16 *u;
+  const __nv_bfloat16 *v;
+  float *acc;
+  float prescale;
+  int big;
+  int transpose_out;
+};
+
 template <int NT>  // R = 8 * NT
 __global__ void __launch_bounds__(STN_THREADS)
-skinny_tn_kernel(const __nv_bfloat16 *__restrict__ u, const __nv_bfloat16 *__restrict__ v, float *__restrict__ acc,
-                 float u_prescale, int64_t m, int big, int transpose_out)
+skinny_tn_kernel(const SkinnyTn job0, const SkinnyTn job1, int tiles0, int64_t m)
 {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const bool second = static_cast<int>(blockIdx.x) >= tiles0;
+  const __nv_bfloat16 *__restrict__ u = second ? job1.u : job0.u;
+  const __nv_bfloat16 *__restrict__ v = second ? job1.v : job0.v;
+  float *__restrict__ acc = second ? job1.acc : job0.acc;
+  const float u_prescale = second ? job1.prescale : job0.prescale;
+  const int big = second ? job1.big : job0.big;
+  const int transpose_out = second ? job1.transpose_out : job0.transpose_out;
   constexpr int R = 8 * NT;
   constexpr int VPITCH = R + 8;
   __shared__ __align__(16) __nv_bfloat16 su[TN_ROWS][TN_UPITCH];
@@ -293,7 +374,7 @@ skinny_tn_kernel(const __nv_bfloat16 *__restrict__ u, const __nv_bfloat16 *__res
   const int lane = tid & 31;
   const int g = lane >> 2;
   const int t = lane & 3;
-  const int c0 = blockIdx.x * TN_COLS;
+  const int c0 = (static_cast<int>(blockIdx.x) - (second ? tiles0 : 0)) * TN_COLS;
   const int64_t per = ((m + gridDim.y - 1) / gridDim.y + TN_ROWS - 1) / TN_ROWS * TN_ROWS;
   const int64_t m_begin = per * blockIdx.y;
   const int64_t m_end = (m_begin + per < m) ? (m_begin + per) : m;
@@ -407,40 +488,25 @@ skinny_tn_kernel(const __nv_bfloat16 *__restrict__ u, const __nv_bfloat16 *__res
   }
 }
 
-// Bp[n, 64] = B[n, R] padded with zeros (forward), or Bt[R, n] = B[n, R]^T (backward).
-__global__ void lora_pad_b_kernel(const __nv_bfloat16 *__restrict__ b, __nv_bfloat16 *__restrict__ bp, int n, int r)
+// fp32 sums of both gradients -> bf16 (the sums lie one behind the other)
+__global__ void round_pair_kernel(const float2 *__restrict__ acc, __nv_bfloat162 *__restrict__ c0,
+                                  __nv_bfloat162 *__restrict__ c1, int64_t n0, int64_t n)
 {
-  const int64_t total = static_cast<int64_t>(n) * 64;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i < n)
   {
-    const int col = static_cast<int>(i & 63);
-    const int64_t row = i >> 6;
-    bp[i] = (col < r) ? b[row * r + col] : __float2bfloat16(0.0f);
-  }
-}
-
-__global__ void lora_transpose_b_kernel(const __nv_bfloat16 *__restrict__ b, __nv_bfloat16 *__restrict__ bt, int n,
-                                        int r)
-{
-  const int64_t total = static_cast<int64_t>(n) * r;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride)
-  {
-    const int64_t j = i / n;   // output row (rank index)
-    const int64_t o = i % n;   // output column
-    bt[i] = b[o * r + j];
-  }
-}
-
-// Ap[64, n] = A[R, n] followed by zero rows.
-__global__ void lora_pad_a_kernel(const __nv_bfloat16 *__restrict__ a, __nv_bfloat16 *__restrict__ ap, int n, int r)
-{
-  const int64_t total = static_cast<int64_t>(64) * n;
-  const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride)
-  {
-    ap[i] = (i < static_cast<int64_t>(r) * n) ? a[i] : __float2bfloat16(0.0f);
+    const float2 v = acc[i];
+    const __nv_bfloat162 r = __floats2bfloat162_rn(v.x, v.y);
+    if (i < n0)
+    {
+      c0[i] = r;
+    }
+    else
+    {
+      c1[i - n0] = r;
+    }
   }
 }
 
@@ -495,93 +561,98 @@ bool skinny_supported(int dtype, int rank, int k)
 }
 
 int launch_skinny_nt(const void *x, const void *a, void *h, void *hs, float x_prescale, float hs_mul,
-                     const float *hs_div, int64_t m, int k, int rank, cudaStream_t s)
+                     const float *hs_div, int64_t m, int k, int rank, bool independent, cudaStream_t s)
 {
   if (m <= 0)
   {
     return CAIFQ_OK;
   }
-  const unsigned grid = static_cast<unsigned>((m + 15) / 16);
-  const __nv_bfloat16 *xp = static_cast<const __nv_bfloat16 *>(x);
-  const __nv_bfloat16 *ap = static_cast<const __nv_bfloat16 *>(a);
-  __nv_bfloat16 *hp = static_cast<__nv_bfloat16 *>(h);
-  __nv_bfloat16 *hsp = static_cast<__nv_bfloat16 *>(hs);
+  // CTAs a row tile: enough that four to eight are on every SM, with at least four 32-k steps for every warp
+  const int64_t tiles = (m + 15) / 16;
+  int cluster = 1;
+  while (cluster < 8 && tiles * cluster < 4 * 148 && k / 32 >= 2 * cluster * 8 * 4)
+  {
+    cluster *= 2;
+  }
+  void (*kernel)(const __nv_bfloat16 *, const __nv_bfloat16 *, __nv_bfloat16 *, __nv_bfloat16 *, float, float,
+                 const float *, int64_t, int, int, int) = nullptr;
   switch (rank)
   {
     case 8:
-      skinny_nt_kernel<1><<<grid, 256, 0, s>>>(xp, ap, hp, hsp, x_prescale, hs_mul, hs_div, m, k);
+      kernel = skinny_nt_kernel<1>;
       break;
     case 16:
-      skinny_nt_kernel<2><<<grid, 256, 0, s>>>(xp, ap, hp, hsp, x_prescale, hs_mul, hs_div, m, k);
+      kernel = skinny_nt_kernel<2>;
       break;
     case 32:
-      skinny_nt_kernel<4><<<grid, 256, 0, s>>>(xp, ap, hp, hsp, x_prescale, hs_mul, hs_div, m, k);
+      kernel = skinny_nt_kernel<4>;
       break;
     case 64:
-      skinny_nt_kernel<8><<<grid, 256, 0, s>>>(xp, ap, hp, hsp, x_prescale, hs_mul, hs_div, m, k);
+      kernel = skinny_nt_kernel<8>;
       break;
     default:
       set_error("LoRA fast path: unsupported rank %d", rank);
       return CAIFQ_ERR_UNSUPPORTED;
   }
-  CAIFQ_CHECK_LAUNCH();
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(static_cast<unsigned>(tiles * cluster));
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = dependent_launches() ? 2 : 1;
+  CAIFQ_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<const __nv_bfloat16 *>(x),
+                                      static_cast<const __nv_bfloat16 *>(a), static_cast<__nv_bfloat16 *>(h),
+                                      static_cast<__nv_bfloat16 *>(hs), x_prescale, hs_mul, hs_div, m, k, cluster,
+                                      independent ? 1 : 0));
   return CAIFQ_OK;
 }
 
-// C = (prescale . U)^T . V with U [m, big], V [m, rank]; C is [big, rank] or, transposed, [rank, big].
-int launch_skinny_tn(const void *u, const void *v, void *c, float *scratch, float u_prescale, int64_t m, int big,
-                     int rank, bool transpose_out, cudaStream_t s)
+// The two reductions over tokens of an adapter's backward, with U [m, big] and V [m, rank]:
+//   db[out, rank] = (prescale . dy)^T . h       da[rank, in] = dh^T . x
+// `sums`: (out + in) x rank floats, zero.
+int launch_skinny_tn(const void *dy, const void *h, void *db, float prescale, int out, const void *x, const void *dh,
+                     void *da, int in, float *sums, int64_t m, int rank, cudaStream_t s)
 {
-  const int64_t n = static_cast<int64_t>(big) * rank;
-  if (n <= 0)
+  const int64_t n0 = static_cast<int64_t>(out) * rank;
+  const int64_t n = n0 + static_cast<int64_t>(in) * rank;
+  const int tiles0 = (out + TN_COLS - 1) / TN_COLS;
+  const int tiles = tiles0 + (in + TN_COLS - 1) / TN_COLS;
+  int64_t slices = (148 * 8 + tiles - 1) / tiles;   // ~8 CTAs of 128 threads per SM
+  const int64_t max_slices = (m + TN_ROWS - 1) / TN_ROWS;
+  slices = slices > max_slices ? max_slices : slices;
+  const SkinnyTn job0{static_cast<const __nv_bfloat16 *>(dy), static_cast<const __nv_bfloat16 *>(h), sums, prescale, out, 0};
+  const SkinnyTn job1{static_cast<const __nv_bfloat16 *>(x), static_cast<const __nv_bfloat16 *>(dh), sums + n0, 1.0f, in, 1};
+  const dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(slices));
+  cudaError_t err = cudaSuccess;
+  switch (rank)
   {
-    return CAIFQ_OK;
+    case 8:
+      err = launch_dependent(skinny_tn_kernel<1>, grid, dim3(STN_THREADS), 0, s, job0, job1, tiles0, m);
+      break;
+    case 16:
+      err = launch_dependent(skinny_tn_kernel<2>, grid, dim3(STN_THREADS), 0, s, job0, job1, tiles0, m);
+      break;
+    case 32:
+      err = launch_dependent(skinny_tn_kernel<4>, grid, dim3(STN_THREADS), 0, s, job0, job1, tiles0, m);
+      break;
+    case 64:
+      err = launch_dependent(skinny_tn_kernel<8>, grid, dim3(STN_THREADS), 0, s, job0, job1, tiles0, m);
+      break;
+    default:
+      set_error("LoRA fast path: unsupported rank %d", rank);
+      return CAIFQ_ERR_UNSUPPORTED;
   }
-  CAIFQ_CHECK_CUDA(cudaMemsetAsync(scratch, 0, static_cast<size_t>(n) * sizeof(float), s));
-  if (m > 0)
-  {
-    const int col_tiles = (big + TN_COLS - 1) / TN_COLS;
-    int64_t slices = (148 * 8 + col_tiles - 1) / col_tiles;   // ~8 CTAs of 128 threads per SM
-    const int64_t max_slices = (m + TN_ROWS - 1) / TN_ROWS;
-    if (slices > max_slices)
-    {
-      slices = max_slices;
-    }
-    if (slices < 1)
-    {
-      slices = 1;
-    }
-    dim3 grid(col_tiles, static_cast<unsigned>(slices));
-    const __nv_bfloat16 *up = static_cast<const __nv_bfloat16 *>(u);
-    const __nv_bfloat16 *vp = static_cast<const __nv_bfloat16 *>(v);
-    const int tr = transpose_out ? 1 : 0;
-    switch (rank)
-    {
-      case 8:
-        skinny_tn_kernel<1><<<grid, STN_THREADS, 0, s>>>(up, vp, scratch, u_prescale, m, big, tr);
-        break;
-      case 16:
-        skinny_tn_kernel<2><<<grid, STN_THREADS, 0, s>>>(up, vp, scratch, u_prescale, m, big, tr);
-        break;
-      case 32:
-        skinny_tn_kernel<4><<<grid, STN_THREADS, 0, s>>>(up, vp, scratch, u_prescale, m, big, tr);
-        break;
-      case 64:
-        skinny_tn_kernel<8><<<grid, STN_THREADS, 0, s>>>(up, vp, scratch, u_prescale, m, big, tr);
-        break;
-      default:
-        set_error("LoRA fast path: unsupported rank %d", rank);
-        return CAIFQ_ERR_UNSUPPORTED;
-    }
-    CAIFQ_CHECK_LAUNCH();
-  }
-  int64_t g = (n + 255) / 256;
-  if (g > 148 * 8)
-  {
-    g = 148 * 8;
-  }
-  round_out_kernel<<<static_cast<unsigned>(g), 256, 0, s>>>(scratch, c, CAIFQ_BF16, n);
-  CAIFQ_CHECK_LAUNCH();
+  CAIFQ_CHECK_CUDA(err);
+  CAIFQ_CHECK_CUDA(launch_dependent(round_pair_kernel, dim3(static_cast<unsigned>((n / 2 + 255) / 256)), dim3(256), 0, s,
+                                    reinterpret_cast<const float2 *>(sums), static_cast<__nv_bfloat162 *>(db),
+                                    static_cast<__nv_bfloat162 *>(da), n0 / 2, n / 2));
   return CAIFQ_OK;
 }
 
@@ -589,7 +660,8 @@ int launch_skinny_tn(const void *u, const void *v, void *c, float *scratch, floa
 // (they are independent of each other and each of them alone is mostly launch latency):
 //   blockIdx.y == 0: the expansion (8 weights per thread and step);
 //   blockIdx.y == 1: Bp = pad(B) [n_b, 64]      (forward), or
-//                    Bt = B^T [r, n_b] and Ap = pad(A) [64, n_a]   (backward).
+//                    Bt = B^T [r, n_b] and Ap = pad(A) [64, n_a], and zeros for the gradients' sums   (backward).
+// Calls that do not expand launch the second part alone.
 struct ExpandPrepare
 {
   const void *codes;
@@ -602,6 +674,8 @@ struct ExpandPrepare
   __nv_bfloat16 *bp;        // forward: [n_b, 64]
   __nv_bfloat16 *bt;        // backward: [r, n_b]
   __nv_bfloat16 *ap;        // backward: [64, n_a]
+  float *zero;              // backward
+  int64_t zeros;
   int n_a, n_b, r;
 };
 
@@ -610,7 +684,8 @@ __global__ void expand_prepare_kernel(const ExpandPrepare p)
 {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t first = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (blockIdx.y == 0)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (blockIdx.y == 0 && p.wb != nullptr)
   {
     expand_span<MODE>(p.codes, p.scales, p.wb, p.units, p.group_of);
     return;
@@ -633,6 +708,10 @@ __global__ void expand_prepare_kernel(const ExpandPrepare p)
       p.bt[i] = p.b[(i % p.n_b) * p.r + i / p.n_b];
     }
   }
+  for (int64_t i = first; i < p.zeros; i += stride)
+  {
+    p.zero[i] = 0.0f;
+  }
   if (p.ap != nullptr)
   {
     const int64_t total = static_cast<int64_t>(64) * p.n_a;
@@ -644,15 +723,16 @@ __global__ void expand_prepare_kernel(const ExpandPrepare p)
   }
 }
 
-// forward: bp != null; backward: bt and ap != null.  The weight must be one expand_span takes.
+// forward: bp != null; backward: bt and ap != null.  Where wb is not null the weight must be one expand_span takes.
 int launch_expand_prepare(const caifq_weight &w, void *wb, const void *a, const void *b, void *bp, void *bt, void *ap,
-                          int rank, cudaStream_t s)
+                          float *zero, int64_t zeros, int rank, cudaStream_t s)
 {
   const int64_t total = static_cast<int64_t>(w.in_dim) * w.out_dim;
   const bool i8 = (w.storage == CAIFQ_I8);
-  if ((total % 8) != 0 || (!i8 && !(w.storage == CAIFQ_I4 && w.scales != nullptr && w.group_size > 0 &&
+  if (wb != nullptr &&
+      ((total % 8) != 0 || (!i8 && !(w.storage == CAIFQ_I4 && w.scales != nullptr && w.group_size > 0 &&
                                     (w.group_size % 8) == 0)) ||
-      (reinterpret_cast<uintptr_t>(w.codes) & 15u) != 0 || (reinterpret_cast<uintptr_t>(wb) & 31u) != 0)
+      (reinterpret_cast<uintptr_t>(w.codes) & 15u) != 0 || (reinterpret_cast<uintptr_t>(wb) & 31u) != 0))
   {
     set_error("expand_prepare: unsupported weight (storage %d)", w.storage);
     return CAIFQ_ERR_UNSUPPORTED;
@@ -662,7 +742,9 @@ int launch_expand_prepare(const caifq_weight &w, void *wb, const void *a, const 
   p.scales = static_cast<const __half *>(w.scales);
   p.wb = static_cast<uint4 *>(wb);
   p.units = total / 8;
-  p.group_of = GroupOf::make(w.group_size);
+  p.group_of = GroupOf::make(w.group_size > 0 ? w.group_size : 1);
+  p.zero = zero;
+  p.zeros = zeros;
   p.a = static_cast<const __nv_bfloat16 *>(a);
   p.b = static_cast<const __nv_bfloat16 *>(b);
   p.bp = static_cast<__nv_bfloat16 *>(bp);
@@ -671,7 +753,8 @@ int launch_expand_prepare(const caifq_weight &w, void *wb, const void *a, const 
   p.n_a = w.in_dim;
   p.n_b = w.out_dim;
   p.r = rank;
-  const dim3 grid(148 * 8, 2);
+  const bool factors = bp != nullptr || bt != nullptr;
+  const dim3 grid(wb != nullptr ? 148 * 8 : 148 * 2, wb != nullptr && factors ? 2 : 1);
   if (i8)
   {
     expand_prepare_kernel<EXPAND_I8><<<grid, 256, 0, s>>>(p);
@@ -680,30 +763,6 @@ int launch_expand_prepare(const caifq_weight &w, void *wb, const void *a, const 
   {
     expand_prepare_kernel<EXPAND_I4><<<grid, 256, 0, s>>>(p);
   }
-  CAIFQ_CHECK_LAUNCH();
-  return CAIFQ_OK;
-}
-
-int launch_lora_pad_b(const void *b, void *bp, int n, int rank, cudaStream_t s)
-{
-  lora_pad_b_kernel<<<148 * 2, 256, 0, s>>>(static_cast<const __nv_bfloat16 *>(b), static_cast<__nv_bfloat16 *>(bp), n,
-                                           rank);
-  CAIFQ_CHECK_LAUNCH();
-  return CAIFQ_OK;
-}
-
-int launch_lora_transpose_b(const void *b, void *bt, int n, int rank, cudaStream_t s)
-{
-  lora_transpose_b_kernel<<<148, 256, 0, s>>>(static_cast<const __nv_bfloat16 *>(b), static_cast<__nv_bfloat16 *>(bt),
-                                             n, rank);
-  CAIFQ_CHECK_LAUNCH();
-  return CAIFQ_OK;
-}
-
-int launch_lora_pad_a(const void *a, void *ap, int n, int rank, cudaStream_t s)
-{
-  lora_pad_a_kernel<<<148 * 2, 256, 0, s>>>(static_cast<const __nv_bfloat16 *>(a), static_cast<__nv_bfloat16 *>(ap), n,
-                                           rank);
   CAIFQ_CHECK_LAUNCH();
   return CAIFQ_OK;
 }

@@ -864,3 +864,21 @@ def test_experts_of_few_rows(storage, compute, counts, gated):
         want, g, u = orc.frozen_expert_forward(x_np[lo:hi], ref[0][e] if gated else None, ref[1][e], ref[2][e], compute, sd)
         assert max_rel_err(out[lo:hi].float().cpu().numpy(), want) <= 2e-2
         assert max_rel_err(up_out[lo:hi].float().cpu().numpy(), u) <= 2e-2
+
+
+@pytest.mark.parametrize("rank", [8, 16, 64])
+@pytest.mark.parametrize("m,in_dim,out_dim", [(33, 14336, 128), (128, 2048, 1152), (1000, 640, 4096)])
+def test_lora_products_split_over_clusters(rank, m, in_dim, out_dim):
+    """Row tiles whose reduction is split over one to eight CTAs, with and without the expansion; both gradients of the
+    factors come from one launch."""
+    rng = np.random.default_rng(rank + m)
+    weight, codes, scales, a, b, x_np, x, dy_np, dy, lora = _lora_case(rng, orc.I8, orc.BF16, in_dim, out_dim, m, rank, 32.0)
+    y, h = nv.lora_linear_fwd(weight, lora, x, orc.F32, expanded=True)
+    dx, da, db = nv.lora_linear_bwd(weight, lora, dy, x, h, orc.F32, expanded=True)
+    assert nv.lib().caifq_device_status() == 0
+    af, bf, xf, dyf = (t.double() for t in (lora.a, lora.b, x, dy))
+    hf = xf @ af.T
+    assert max_rel_err(h.float().cpu().numpy(), hf.cpu().numpy()) <= 1e-2
+    dh = (dyf * (32.0 / rank)) @ bf
+    assert max_rel_err(da.float().cpu().numpy(), (dh.T @ xf).cpu().numpy()) <= 2e-2
+    assert max_rel_err(db.float().cpu().numpy(), (dyf.T @ h.double() * (32.0 / rank)).cpu().numpy()) <= 2e-2
