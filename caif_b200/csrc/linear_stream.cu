@@ -32,7 +32,6 @@
 // Every wait is bounded; a wait that runs out sets a flag that the host can read and lets the kernel finish (with wrong
 // numbers) instead of hanging.
 #include <atomic>
-#include <vector>
 
 #include "umma.cuh"
 
@@ -73,6 +72,7 @@ constexpr int MAX_B = 6;                    // activation stages (128 k each) in
 constexpr int DONE = 8;                     // ring of "stage multiplied" barriers
 constexpr int TMEM_COLUMNS = 512;
 constexpr uint32_t SMEM_LIMIT = 226u * 1024u;
+constexpr uint32_t SCALES_LIMIT = 40u * 1024u;   // more would cost the activations their places
 // Most tokens for which a tile's conversion, repeated for every 256 tokens, is not yet more than the many-token kernel's,
 // repeated for every 256 of its rows: 768 tokens of 4096 -> 14336 take 94 us against 119, 1024 take 124 against 120.
 constexpr int kStreamMostTokens = 768;
@@ -106,6 +106,8 @@ struct StreamParams
   GroupOf group_of;      // int4
   int groups_per_row;
   int group_size;
+  uint32_t scales_at;    // their place in shared memory
+  uint32_t scale_bytes;  // int4: of a tile's 128 rows, where they are copied to shared memory; 0 = read from global memory
   int num_tiles;
   int splits;            // CTAs of a cluster (k ranges)
   int box;               // tokens per activation copy
@@ -212,7 +214,7 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
   constexpr uint32_t STAGE_COLUMNS = PLANE_COLUMNS * PLANES;
   constexpr uint32_t PLACES = 256u / STAGE_COLUMNS;   // stages of the weight operand: 4, or 2 of two planes
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t bars[4 + DONE + MAX_B + 4];
+  __shared__ uint64_t bars[4 + DONE + MAX_B + 4 + 2];
   __shared__ uint64_t drain_bar;   // give-up path only: the MMAs issued so far have completed
   __shared__ uint32_t tmem_base_slot;
   __shared__ uint32_t cta_abort;   // a wait of this CTA has run out
@@ -231,6 +233,11 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
   auto b_full = [&](uint32_t s) { return bar0 + (4u + DONE + s) * 8u; };
   auto acc_full = [&](int a) { return bar0 + static_cast<uint32_t>(4 + DONE + MAX_B + a) * 8u; };
   auto acc_empty = [&](int a) { return bar0 + static_cast<uint32_t>(4 + DONE + MAX_B + 2 + a) * 8u; };
+  auto sc_full = [&](int i) { return bar0 + static_cast<uint32_t>(4 + DONE + MAX_B + 4 + (i & 1)) * 8u; };
+  // int4: the scales of tile i (its rows' are contiguous), in one of two places after the tile records
+  auto scales_at = [&](int i) { return p.scales_at + smem_base + static_cast<uint32_t>(i & 1) * p.scale_bytes; };
+  // (the warps' arrivals and the copies' bytes have separate barriers: after a wait that ran out the warps run on, and an
+  // arrival beyond the count of a barrier that still expects bytes is a fault)
   volatile uint32_t *abort_word = &cta_abort;
   auto wait = [&](uint32_t bar, uint32_t parity)
   { return mbar_wait(bar, parity, abort_word, p.spin_limit, &g_stream_timeout_flag); };
@@ -263,6 +270,7 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
     for (int a = 0; a < 2; ++a)
     {
       mbar_init(acc_full(a), 1);
+      mbar_init(sc_full(a), 1);
       mbar_init(acc_empty(a), CODE_WARPS);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -348,8 +356,23 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
       int acc = 0;
       uint32_t acc_par = 0;
       const uint64_t bdesc_base = make_desc(smem_base, 16, 1024);
+      auto copy_scales = [&](int tile)
+      {
+        // (not once a wait has run out: the place's barrier may still expect bytes)
+        if (IS_I4 && p.scale_bytes != 0u && tile < num_tiles && *abort_word == 0u)
+        {
+          mbar_expect_tx(sc_full(tile), p.scale_bytes);
+          asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                           scales_at(tile)),
+                       "l"(tiles[tile].scales), "r"(p.scale_bytes), "r"(sc_full(tile))
+                       : "memory");
+        }
+      };
+      copy_scales(0);
       for (int tile = 0; tile < num_tiles; ++tile)
       {
+        // (everything of the tile before this one has been converted, so its scales' place is free)
+        copy_scales(tile + 1);
         const uint32_t idesc = make_idesc(false, (tiles[tile].tokens + 15) & ~15, ROWS);
         const uint32_t d = tmem_base + static_cast<uint32_t>(acc * 128);
         if (!wait(acc_empty(acc), acc_par ^ 1u))
@@ -529,7 +552,7 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
         f_last = f_left > 0 && at + static_cast<uint32_t>(last) * STAGE_CODES < p.row_bytes &&
                  first + last + static_cast<int>(piece_stage) < stages;
         f_src = tiles[f_tile].codes + static_cast<size_t>(wq * 32 + static_cast<int>(copy_row)) * p.row_bytes + at;
-        if (IS_I4)
+        if (IS_I4 && p.scale_bytes == 0u)
         {
           // the scales of this lane's row are on their way to L2 before the first of them is used
           const char *sc = static_cast<const char *>(tiles[f_tile].scales) +
@@ -563,35 +586,41 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
     const uint32_t ring_sw = static_cast<uint32_t>((lane >> 1) & 3);
     const uint32_t dst = tmem_base + (static_cast<uint32_t>(wq * 32) << 16) + A_COLUMN0 +
                          static_cast<uint32_t>(half) * SUB_COLUMNS;
-    // int4: the scales of a unit's 32-code pieces, loaded while the unit before it is converted
-    uint16_t next_sc[IS_I4 ? 4 : 1];
+    // int4: the scales of a unit's 32-code pieces.  A lane owns a row, so reading them from global memory touches 32 lines
+    // a time: they are copied to shared memory a tile ahead, unless the rows are too long for that (14336 -> 4096,
+    // 17 tokens: 23.4 us without, 21.9 with; two operand planes, 4096 -> 14336, 512 tokens: 114 and 109).
     const bool pairs = (p.group_size % KB) == 0;   // both pieces of a stage have one scale
-    auto load_scales = [&](const uint16_t *row_scales, int first, int unit)
+    auto load_scales = [&](int tile, int first, int unit, uint16_t (&sc)[4])
     {
-      if constexpr (IS_I4)
-      {
+      const uint16_t *global =
+          static_cast<const uint16_t *>(tiles[tile].scales) + static_cast<int64_t>(wq * 32 + lane) * p.groups_per_row;
+      const uint32_t shared = scales_at(tile) + static_cast<uint32_t>((wq * 32 + lane) * p.groups_per_row) * 2u;
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 4; ++i)
+      {
+        if ((i & 1) && pairs)
         {
-          if ((i & 1) && pairs)
+          sc[i] = sc[i - 1];
+        }
+        else
+        {
+          const int k = ((st_begin + first + 2 * (UNIT_STAGES * unit + (i >> 1))) * 2 + half) * KB + (i & 1) * 32;
+          const uint32_t group = p.group_of(static_cast<uint32_t>(min(k, p.k_total - 1)));
+          if (p.scale_bytes != 0u)
           {
-            next_sc[i] = next_sc[i - 1];
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(sc[i]) : "r"(shared + group * 2u));
           }
           else
           {
-            const int k = ((st_begin + first + 2 * (UNIT_STAGES * unit + (i >> 1))) * 2 + half) * KB + (i & 1) * 32;
-            next_sc[i] = __ldg(row_scales + p.group_of(static_cast<uint32_t>(min(k, p.k_total - 1))));
+            sc[i] = __ldg(global + group);
           }
         }
       }
     };
-    auto scales_of = [&](int i)
-    { return static_cast<const uint16_t *>(tiles[i].scales) + static_cast<int64_t>(wq * 32 + lane) * p.groups_per_row; };
-    const uint16_t *row_scales = nullptr;
-    if (IS_I4 && num_tiles > 0)
+    uint16_t next_sc[4];   // read from global memory: loaded while the unit before is converted
+    if (IS_I4 && p.scale_bytes == 0u && num_tiles > 0)
     {
-      row_scales = scales_of(0);
-      load_scales(row_scales, first_stage(0), 0);
+      load_scales(0, first_stage(0), 0, next_sc);
     }
     int undrained = -1;   // a tile whose accumulators still wait
     bool released = false;
@@ -635,6 +664,14 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
         float sc[IS_I4 ? 4 : 1];
         if constexpr (IS_I4)
         {
+          if (p.scale_bytes != 0u)
+          {
+            if (unit == 0)
+            {
+              wait(sc_full(tile), static_cast<uint32_t>(tile >> 1) & 1u);
+            }
+            load_scales(tile, first, unit, next_sc);
+          }
 #pragma unroll
           for (int i = 0; i < 4; ++i)
           {
@@ -645,16 +682,15 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
         fetch(slot);
         slot += UNIT_BYTES;
         slot = slot == ring_end ? ring : slot;
-        if constexpr (IS_I4)
+        if (IS_I4 && p.scale_bytes == 0u)
         {
           if (unit + 1 < units)
           {
-            load_scales(row_scales, first, unit + 1);
+            load_scales(tile, first, unit + 1, next_sc);
           }
           else if (tile + 1 < num_tiles)
           {
-            row_scales = scales_of(tile + 1);
-            load_scales(row_scales, first_stage(tile + 1), 0);
+            load_scales(tile + 1, first_stage(tile + 1), 0, next_sc);
           }
         }
 #pragma unroll
@@ -804,19 +840,27 @@ int stream_ctas() { return persistent_ctas("CAIFQ_UMMA_CTAS"); }
 bool choose_depths(StreamParams &p, uint32_t &smem)
 {
   const int ctas = stream_ctas();
-  const uint32_t records = static_cast<uint32_t>((p.num_tiles + ctas - 1) / ctas) * static_cast<uint32_t>(sizeof(StreamTile));
+  const uint32_t per_cta = static_cast<uint32_t>((p.num_tiles + ctas - 1) / ctas);
+  const uint32_t records = per_cta * static_cast<uint32_t>(sizeof(StreamTile));
+  const uint32_t scales = p.scale_bytes * (per_cta > 1 ? 2u : 1u);
+  if (scales > SCALES_LIMIT)
+  {
+    p.scale_bytes = 0;
+  }
   const int want = p.b_stage_bytes <= 16384 ? 4 : (p.b_stage_bytes <= 32768 ? 3 : 2);
   for (int least = want; least >= 2; --least)
   {
     for (int depth : {3, 2})   // units of codes per warp
     {
-      const uint32_t fixed = static_cast<uint32_t>(CODE_WARPS * depth) * UNIT_BYTES + records + 1024u;
+      const uint32_t fixed = static_cast<uint32_t>(CODE_WARPS * depth) * UNIT_BYTES + ((records + 15u) & ~15u) + (p.scale_bytes != 0u ? scales : 0u) + 1024u;
       if (fixed + static_cast<uint32_t>(least) * p.b_stage_bytes <= SMEM_LIMIT)
       {
         const int fit = static_cast<int>((SMEM_LIMIT - fixed) / p.b_stage_bytes);
         p.depth = depth;
         p.b_stages = fit < MAX_B ? fit : MAX_B;
         smem = fixed + static_cast<uint32_t>(p.b_stages) * p.b_stage_bytes;
+        p.scales_at = static_cast<uint32_t>(p.b_stages) * p.b_stage_bytes +
+                      static_cast<uint32_t>(CODE_WARPS * depth) * UNIT_BYTES + ((records + 15u) & ~15u);
         return true;
       }
     }
@@ -880,7 +924,7 @@ int launch_stream_inst(const CUtensorMap &map_b, StreamParams &p, const StreamTa
     for (int c : {8, 4, 3, 2})
     {
       if (p.num_tiles * c <= stream_ctas() && num_kb >= 4 * c && p.num_tiles <= resident_clusters(kernel, dev, c) &&
-          p.b_sub_bytes * 4u + sizeof(StreamTile) + 1024u <= smem)
+          p.b_sub_bytes * 4u + 32u + p.scale_bytes + 1024u <= smem)
       {
         p.splits = c;
         break;
@@ -942,7 +986,8 @@ bool weight_streams(const caifq_weight &w, int compute_dtype)
 // (two operand planes leave tensor memory for two accumulator sets of 128 tokens)
 int tile_tokens(int mode) { return mode == W_I4S ? 128 : TOKENS; }
 
-StreamParams common_params(const caifq_weight &w, int mode, int c_dtype, bool accumulate, int most_rows)
+StreamParams common_params(const caifq_weight &w, int mode, int c_dtype, bool accumulate, int most_rows,
+                           bool scales_aligned)
 {
   StreamParams p{};
   p.c_dtype = c_dtype;
@@ -953,6 +998,7 @@ StreamParams common_params(const caifq_weight &w, int mode, int c_dtype, bool ac
   p.group_of = GroupOf::make(w.group_size > 0 ? w.group_size : 1);
   p.group_size = w.group_size;
   p.groups_per_row = w.storage == CAIFQ_I4 ? w.in_dim / w.group_size : 0;
+  p.scale_bytes = scales_aligned ? static_cast<uint32_t>(p.groups_per_row) * (ROWS * 2u) : 0u;
   p.splits = 1;
   p.tile_tokens = tile_tokens(mode);
   const int most_tokens = most_rows < p.tile_tokens ? most_rows : p.tile_tokens;
@@ -994,7 +1040,7 @@ int launch_linear_stream(const LinearArgs &g, cudaStream_t s)
   const caifq_weight &w = g.w;
   const int mode = wmode_of(w, g.compute_dtype);
   const int m = static_cast<int>(g.m);
-  StreamParams p = common_params(w, mode, g.c_dtype, g.accumulate, m);
+  StreamParams p = common_params(w, mode, g.c_dtype, g.accumulate, m, (reinterpret_cast<uintptr_t>(w.scales) & 15u) == 0);
   StreamTable<1> table{};
   table.count = 1;
   table.e[0].codes = static_cast<const uint8_t *>(w.codes);
@@ -1047,6 +1093,7 @@ int launch_linear_stream_grouped(const GroupedStreamArgs &g, cudaStream_t s)
   static thread_local StreamTable<MAX_ENTRIES> table;
   int most = 0;
   int tiles = 0;
+  bool scales_aligned = true;
   table.count = 0;
   for (int e = 0; e < g.count; ++e)
   {
@@ -1058,6 +1105,7 @@ int launch_linear_stream_grouped(const GroupedStreamArgs &g, cudaStream_t s)
     StreamEntry &t = table.e[table.count++];
     t.codes = static_cast<const uint8_t *>(g.weights[e].codes);
     t.scales = g.weights[e].scales;
+    scales_aligned = scales_aligned && (reinterpret_cast<uintptr_t>(t.scales) & 15u) == 0;
     t.c = g.c[e];
     t.row0 = g.row_begin[e];
     t.rows = rows;
@@ -1069,7 +1117,7 @@ int launch_linear_stream_grouped(const GroupedStreamArgs &g, cudaStream_t s)
   {
     return CAIFQ_OK;
   }
-  StreamParams p = common_params(w0, mode, g.c_dtype, g.accumulate, most);
+  StreamParams p = common_params(w0, mode, g.c_dtype, g.accumulate, most, scales_aligned);
   p.num_tiles = tiles;
   uint32_t smem = 0;
   if (!choose_depths(p, smem))
