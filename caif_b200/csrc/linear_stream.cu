@@ -10,12 +10,12 @@
 // Here the roles are swapped: 128 weight rows are the M of the MMA and the tokens its N, 16 to 256 in steps of 16.  The
 // converted weight goes to tensor memory as the A operand, which leaves shared memory's bandwidth to the codes and the
 // activations (256 tokens: 50 us with A in shared memory, 40 with it here).
-// 4096 -> 14336 int4, us a call, many-token kernel / this one: 17 tokens 42 / 23, 96 tokens 42 / 27, 256 tokens 44 / 36,
-// 512 tokens 79 / 64; 4096 -> 4096: 38 / 11, 38 / 13, 41 / 20, 41 / 30; 64 experts of 2048 x 1408, 16 tokens top-6, three
-// products: 249 / 138.
+// 4096 -> 14336 int4, us a call, many-token kernel / this one: 17 tokens 42 / 20, 96 tokens 42 / 22, 256 tokens 44 / 33,
+// 512 tokens 79 / 61; 4096 -> 4096: 38 / 11, 38 / 13, 41 / 19, 41 / 28; 64 experts of 2048 x 1408, 16 tokens top-6, three
+// products: 249 / 121.
 //
-// One persistent CTA per SM, 18 warps, over tiles of 128 weight rows x up to 256 tokens:
-//   warp 0      TMA producer for the activation tiles, in boxes of 16 to 64 tokens, as many as the tile has
+// One persistent CTA per SM, 19 warps, over tiles of 128 weight rows x up to 256 tokens:
+//   warps 0, 18 TMA producers for the activation tiles
 //   warp 1      TMEM allocation, MMA issue (one elected lane)
 //   warps 2-17  codes: two teams of eight warps take alternate stages of 128 k, so one converts while the other's stage
 //               is multiplied; a warp owns 32 rows x 64 k of a stage, copies its pieces into its own ring (cp.async,
@@ -64,9 +64,10 @@ constexpr int KB = 64;               // k of an operand tile: one 128-byte swizz
 constexpr uint32_t A_COLUMN0 = 256;
 constexpr uint32_t SUB_COLUMNS = 32;
 constexpr uint32_t PLANE_COLUMNS = 2 * SUB_COLUMNS;   // of a stage (128 k)
-constexpr int WARPS = 18;
+constexpr int WARPS = 19;
 constexpr int CODE_WARP0 = 2;
 constexpr int CODE_WARPS = 16;
+constexpr int SECOND_COPY_WARP = CODE_WARP0 + CODE_WARPS;
 constexpr uint32_t UNIT_BYTES = 32 * 64;    // a warp's 32 rows x 64 bytes of codes
 constexpr int MAX_B = 6;                    // activation stages (128 k each) in flight
 constexpr int DONE = 8;                     // ring of "stage multiplied" barriers
@@ -295,9 +296,12 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
   const int stages = (all_stages * (rank + 1)) / p.splits - st_begin;
   const int num_kb = min(all_kb - 2 * st_begin, 2 * stages);
 
-  if (warp == 0)
+  if (warp == 0 || warp == SECOND_COPY_WARP)
   {
     // ------------------------------------------------------- activation tiles
+    // Two threads, each copies the tile of one 64-k half of every stage: one that waited, announced the bytes and issued
+    // both copies needed 700 cycles a stage and kept the MMAs waiting.
+    const int half = warp == 0 ? 0 : 1;
     auto produce = [&]()
     {
       asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -320,13 +324,17 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
             }
           }
           const int subs = min(2, num_kb - 2 * st);
-          mbar_expect_tx(b_full(s), static_cast<uint32_t>(subs * boxes) * box_bytes + (g == 0 ? p.stall_bytes : 0u));
-          for (int h = 0; h < subs; ++h)
+          if (half == 0)
           {
+            mbar_expect_tx(b_full(s), static_cast<uint32_t>(subs * boxes) * box_bytes + (g == 0 ? p.stall_bytes : 0u));
+          }
+          if (half < subs)
+          {
+            const uint32_t to = b_addr(s) + static_cast<uint32_t>(half) * p.b_sub_bytes;
             for (int b = 0; b < boxes; ++b)
             {
-              tma_load_2d(b_addr(s) + static_cast<uint32_t>(h) * p.b_sub_bytes + static_cast<uint32_t>(b) * box_bytes, &map_b,
-                          (2 * (st_begin + st) + h) * KB, w.token0 + b * p.box, b_full(s));
+              tma_load_2d(to + static_cast<uint32_t>(b) * box_bytes, &map_b, (2 * (st_begin + st) + half) * KB,
+                          w.token0 + b * p.box, b_full(s));
             }
           }
           if (++s == static_cast<uint32_t>(p.b_stages))
@@ -987,7 +995,7 @@ bool weight_streams(const caifq_weight &w, int compute_dtype)
 int tile_tokens(int mode) { return mode == W_I4S ? 128 : TOKENS; }
 
 StreamParams common_params(const caifq_weight &w, int mode, int c_dtype, bool accumulate, int most_rows,
-                           bool scales_aligned)
+                           bool scales_aligned, bool grouped)
 {
   StreamParams p{};
   p.c_dtype = c_dtype;
@@ -1002,9 +1010,9 @@ StreamParams common_params(const caifq_weight &w, int mode, int c_dtype, bool ac
   p.splits = 1;
   p.tile_tokens = tile_tokens(mode);
   const int most_tokens = most_rows < p.tile_tokens ? most_rows : p.tile_tokens;
-  // few copies per stage for full tiles, little over-fetch for small ones
   p.acc_bufs = most_tokens <= 128 ? 2 : 1;
-  p.box = most_tokens <= 16 ? 16 : (most_tokens <= 128 ? 32 : 64);
+  // one copy a tile where the tiles are alike, little over-fetch where experts have a row here and hundreds there
+  p.box = (!grouped || most_tokens <= 32) ? (most_tokens + 15) & ~15 : (most_tokens <= 128 ? 32 : 64);
   p.b_sub_bytes = static_cast<uint32_t>((most_tokens + p.box - 1) / p.box * p.box) * 128u;
   p.b_stage_bytes = 2u * p.b_sub_bytes;
   p.spin_limit = kSpinLimit;
@@ -1040,7 +1048,7 @@ int launch_linear_stream(const LinearArgs &g, cudaStream_t s)
   const caifq_weight &w = g.w;
   const int mode = wmode_of(w, g.compute_dtype);
   const int m = static_cast<int>(g.m);
-  StreamParams p = common_params(w, mode, g.c_dtype, g.accumulate, m, (reinterpret_cast<uintptr_t>(w.scales) & 15u) == 0);
+  StreamParams p = common_params(w, mode, g.c_dtype, g.accumulate, m, (reinterpret_cast<uintptr_t>(w.scales) & 15u) == 0, false);
   StreamTable<1> table{};
   table.count = 1;
   table.e[0].codes = static_cast<const uint8_t *>(w.codes);
@@ -1117,7 +1125,7 @@ int launch_linear_stream_grouped(const GroupedStreamArgs &g, cudaStream_t s)
   {
     return CAIFQ_OK;
   }
-  StreamParams p = common_params(w0, mode, g.c_dtype, g.accumulate, most, scales_aligned);
+  StreamParams p = common_params(w0, mode, g.c_dtype, g.accumulate, most, scales_aligned, true);
   p.num_tiles = tiles;
   uint32_t smem = 0;
   if (!choose_depths(p, smem))

@@ -272,8 +272,8 @@ CAIFQ_API int caifq_lora_linear_bwd(const caifq_weight *w, const caifq_lora *lor
 
 /*
  * The same two calls for hosts that can spare a larger workspace (no counterpart in the reference, whose
- * cache_fp32 keeps an fp32 copy of every weight for good).  From a few thousand tokens on (m >= 4096, bf16
- * adapter on an int8 base, or on an int4 base under bf16 compute, in_dim and out_dim multiples of 256) the
+ * cache_fp32 keeps an fp32 copy of every weight for good).  From 128 tokens on (bf16
+ * adapter on an int8 base, or on an int4 base under bf16 compute, in_dim and out_dim multiples of 128) the
  * weight is expanded ONCE per call into a bf16 [out, in] matrix behind the other scratch -- int8 codes as
  * exact integers with the per-tensor scale left to the epilogue, int4 as bf16(scale * code), the value the
  * reference's dequantize-then-cast gives -- and the tensor core is fed from it by plain tile copies on CTA
