@@ -411,7 +411,7 @@ LoraFwdWs lora_fwd_ws(const caifq_weight *w, int64_t m)
 struct LoraBwdWs
 {
   size_t d_hidden;  // [m, r] in <= 4-byte elements
-  size_t scratch;   // fp32 [in + out, r]
+  size_t scratch;   // fp32 [max(in,out), r]
   size_t bt;        // [r, out] bf16
   size_t dhs;       // [m, 64] bf16
   size_t ap;        // [64, in] bf16
@@ -421,14 +421,21 @@ struct LoraBwdWs
 LoraBwdWs lora_bwd_ws(const caifq_weight *w, const caifq_lora *l, int64_t m)
 {
   LoraBwdWs o{};
-  const size_t both = static_cast<size_t>(w->in_dim) + static_cast<size_t>(w->out_dim);
+  const size_t big = static_cast<size_t>(w->in_dim > w->out_dim ? w->in_dim : w->out_dim);
   o.d_hidden = 0;
   o.scratch = align256(static_cast<size_t>(m) * static_cast<size_t>(l->rank) * 4);
-  o.bt = o.scratch + align256(both * static_cast<size_t>(l->rank) * sizeof(float));
+  o.bt = o.scratch + align256(big * static_cast<size_t>(l->rank) * sizeof(float));
   o.dhs = o.bt + align256(static_cast<size_t>(l->rank) * w->out_dim * 2);
   o.ap = o.dhs + align256(static_cast<size_t>(m) * 64 * 2);
   o.total = o.ap + align256(static_cast<size_t>(64) * w->in_dim * 2);
   return o;
+}
+
+// (expanded calls) the sums of both factors' gradients, behind the weight: fp32 [in + out, r]
+size_t lora_sums_bytes(const caifq_weight *w, const caifq_lora *l)
+{
+  return align256((static_cast<size_t>(w->in_dim) + static_cast<size_t>(w->out_dim)) * static_cast<size_t>(l->rank) *
+                  sizeof(float));
 }
 
 }  // namespace
@@ -892,17 +899,27 @@ int lora_bwd_impl(const caifq_weight *w, const caifq_lora *lora, const void *dy,
     const bool expand = may_expand && expand_ok(w, lora, dy, m, compute_dtype);
     void *wb = wbase + ws.total;
     // transposed B, padded A, zeros for the gradients' sums and the expansion of the weight in one launch
-    int r = launch_expand_prepare(*w, expand ? wb : nullptr, lora->a, lora->b, nullptr, wbase + ws.bt, wbase + ws.ap,
-                                  scratch, (static_cast<int64_t>(w->in_dim) + w->out_dim) * lora->rank, lora->rank, s);
+    const int64_t n_b = static_cast<int64_t>(w->out_dim) * lora->rank;
+    const int64_t n_a = static_cast<int64_t>(w->in_dim) * lora->rank;
+    float *sums = expand ? reinterpret_cast<float *>(static_cast<char *>(wb) + expanded_weight_bytes(w)) : scratch;
+    int r = launch_expand_prepare(*w, expand ? wb : nullptr, lora->a, lora->b, nullptr, wbase + ws.bt, wbase + ws.ap, sums,
+                                  expand ? n_b + n_a : n_b, lora->rank, s);
     if (r == CAIFQ_OK)
     {
       r = launch_skinny_nt(dy, wbase + ws.bt, d_hidden, wbase + ws.dhs, scale, 1.0f, epilogue_scale_ptr(w), m,
                            w->out_dim, lora->rank, false, s);
     }
-    // dB[out, r] = (scale . dy)^T . hidden;  dA[r, in] = dH^T . x
+    // dB[out, r] = (scale . dy)^T . hidden;  dA[r, in] = dH^T . x: one launch, or, where the scratch holds the sums of one
+    // of them at a time, one after the other
     if (r == CAIFQ_OK)
     {
-      r = launch_skinny_tn(dy, hidden, d_b, scale, w->out_dim, x, d_hidden, d_a, w->in_dim, scratch, m, lora->rank, s);
+      r = launch_skinny_tn(dy, hidden, d_b, scale, w->out_dim, x, d_hidden, d_a, expand ? w->in_dim : 0, sums, m,
+                           lora->rank, s);
+    }
+    if (r == CAIFQ_OK && !expand)
+    {
+      CAIFQ_CHECK_CUDA(cudaMemsetAsync(sums, 0, static_cast<size_t>(n_a) * sizeof(float), s));
+      r = launch_skinny_tn(nullptr, nullptr, nullptr, 1.0f, 0, x, d_hidden, d_a, w->in_dim, sums, m, lora->rank, s);
     }
     if (r != CAIFQ_OK)
     {
@@ -965,7 +982,9 @@ size_t caifq_lora_bwd_workspace_bytes_expanded(const caifq_weight *w, const caif
     return 0;
   }
   const size_t plain = lora_bwd_ws(w, lora, m).total;
-  return expand_ok(w, lora, kAlignedProbe, m, compute_dtype) ? plain + expanded_weight_bytes(w) : plain;
+  return expand_ok(w, lora, kAlignedProbe, m, compute_dtype)
+             ? plain + expanded_weight_bytes(w) + lora_sums_bytes(w, lora)
+             : plain;
 }
 
 int caifq_lora_linear_bwd_expanded(const caifq_weight *w, const caifq_lora *lora, const void *dy, const void *x,

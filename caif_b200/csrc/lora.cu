@@ -616,7 +616,7 @@ int launch_skinny_nt(const void *x, const void *a, void *h, void *hs, float x_pr
 
 // The two reductions over tokens of an adapter's backward, with U [m, big] and V [m, rank]:
 //   db[out, rank] = (prescale . dy)^T . h       da[rank, in] = dh^T . x
-// `sums`: (out + in) x rank floats, zero.
+// `sums`: (out + in) x rank floats, zero.  A product of no columns is left out.
 int launch_skinny_tn(const void *dy, const void *h, void *db, float prescale, int out, const void *x, const void *dh,
                      void *da, int in, float *sums, int64_t m, int rank, cudaStream_t s)
 {
