@@ -10,8 +10,8 @@
 // Here the roles are swapped: 128 weight rows are the M of the MMA and the tokens its N, 16 to 256 in steps of 16.  The
 // converted weight goes to tensor memory as the A operand, which leaves shared memory's bandwidth to the codes and the
 // activations (256 tokens: 50 us with A in shared memory, 40 with it here).
-// 4096 -> 14336 int4, us a call, many-token kernel / this one: 17 tokens 42 / 20, 96 tokens 42 / 22, 256 tokens 44 / 33,
-// 512 tokens 79 / 61; 4096 -> 4096: 38 / 11, 38 / 13, 41 / 19, 41 / 28; 64 experts of 2048 x 1408, 16 tokens top-6, three
+// 4096 -> 14336 int4, us a call, many-token kernel / this one: 17 tokens 42 / 20, 96 tokens 42 / 22, 256 tokens 44 / 30,
+// 512 tokens 79 / 55; 4096 -> 4096: 38 / 11, 38 / 13, 41 / 19, 41 / 27; 64 experts of 2048 x 1408, 16 tokens top-6, three
 // products: 249 / 121.
 //
 // One persistent CTA per SM, 19 warps, over tiles of 128 weight rows x up to 256 tokens:
@@ -113,7 +113,8 @@ struct StreamParams
   int splits;            // CTAs of a cluster (k ranges)
   int box;               // tokens per activation copy
   int tile_tokens;       // most tokens of a tile
-  int b_stages;
+  int b_stages;          // places for activations: of 128 k, or of 64 k where `halves` is set
+  int halves;
   int acc_bufs;          // accumulator sets: 2 of 128 columns, or 1 of 256
   int depth;             // units in flight per code warp: 2 or 3
   uint32_t b_sub_bytes;  // 64 k of the activations
@@ -203,7 +204,7 @@ __device__ __forceinline__ void umma_bf16_tmem(uint32_t tmem_d, uint32_t tmem_a,
       : "memory");
 }
 
-template <int WMODE, int N>
+template <int WMODE, int N, bool HALVES>
 __global__ void __launch_bounds__(WARPS * 32, 1)
 linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_constant__ StreamParams p,
                      const __grid_constant__ StreamTable<N> table)
@@ -215,7 +216,7 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
   constexpr uint32_t STAGE_COLUMNS = PLANE_COLUMNS * PLANES;
   constexpr uint32_t PLACES = 256u / STAGE_COLUMNS;   // stages of the weight operand: 4, or 2 of two planes
   extern __shared__ uint8_t smem_raw[];
-  __shared__ uint64_t bars[4 + DONE + MAX_B + 4 + 2];
+  __shared__ uint64_t bars[4 + DONE + 2 * MAX_B + 4 + 2];
   __shared__ uint64_t drain_bar;   // give-up path only: the MMAs issued so far have completed
   __shared__ uint32_t tmem_base_slot;
   __shared__ uint32_t cta_abort;   // a wait of this CTA has run out
@@ -223,8 +224,9 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  auto b_addr = [&](uint32_t s) { return smem_base + s * p.b_stage_bytes; };
-  const uint32_t ring_base = smem_base + static_cast<uint32_t>(p.b_stages) * p.b_stage_bytes;
+  const uint32_t b_place_bytes = HALVES ? p.b_sub_bytes : p.b_stage_bytes;
+  auto b_addr = [&](uint32_t s) { return smem_base + s * b_place_bytes; };
+  const uint32_t ring_base = smem_base + static_cast<uint32_t>(p.b_stages) * b_place_bytes;
   const uint32_t bar0 = smem_u32(bars);
   const uint32_t tiles_base = ring_base + static_cast<uint32_t>(CODE_WARPS * p.depth) * UNIT_BYTES;
   const StreamTile *tiles = reinterpret_cast<const StreamTile *>(smem_raw + (tiles_base - smem_u32(smem_raw)));
@@ -232,9 +234,10 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
   auto done = [&](uint32_t g) { return bar0 + (4u + g % DONE) * 8u; };
   auto done_parity = [&](uint32_t g) { return (g / DONE) & 1u; };
   auto b_full = [&](uint32_t s) { return bar0 + (4u + DONE + s) * 8u; };
-  auto acc_full = [&](int a) { return bar0 + static_cast<uint32_t>(4 + DONE + MAX_B + a) * 8u; };
-  auto acc_empty = [&](int a) { return bar0 + static_cast<uint32_t>(4 + DONE + MAX_B + 2 + a) * 8u; };
-  auto sc_full = [&](int i) { return bar0 + static_cast<uint32_t>(4 + DONE + MAX_B + 4 + (i & 1)) * 8u; };
+  auto b_empty = [&](uint32_t s) { return bar0 + (4u + DONE + MAX_B + s) * 8u; };   // halves only
+  auto acc_full = [&](int a) { return bar0 + static_cast<uint32_t>(4 + DONE + 2 * MAX_B + a) * 8u; };
+  auto acc_empty = [&](int a) { return bar0 + static_cast<uint32_t>(4 + DONE + 2 * MAX_B + 2 + a) * 8u; };
+  auto sc_full = [&](int i) { return bar0 + static_cast<uint32_t>(4 + DONE + 2 * MAX_B + 4 + (i & 1)) * 8u; };
   // int4: the scales of tile i (its rows' are contiguous), in one of two places after the tile records
   auto scales_at = [&](int i) { return p.scales_at + smem_base + static_cast<uint32_t>(i & 1) * p.scale_bytes; };
   // (the warps' arrivals and the copies' bytes have separate barriers: after a wait that ran out the warps run on, and an
@@ -267,6 +270,7 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
     for (uint32_t s = 0; s < MAX_B; ++s)
     {
       mbar_init(b_full(s), 1);
+      mbar_init(b_empty(s), 1);
     }
     for (int a = 0; a < 2; ++a)
     {
@@ -301,12 +305,18 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
     // ------------------------------------------------------- activation tiles
     // Two threads, each copies the tile of one 64-k half of every stage: one that waited, announced the bytes and issued
     // both copies needed 700 cycles a stage and kept the MMAs waiting.
+    // HALVES: tiles of more than 128 tokens (64 KB a stage) have places of 64 k, freed one by one: two places of 128 k
+    // left the MMAs waiting for 570 of 1380 cycles a stage (256 tokens: 33 us, now 30).  Half h has every other place.
+    // Fewer tokens keep whole stages: there the one thread that issues the MMAs is the limit, and a wait and a commit more
+    // a stage cost 7 %.
     const int half = warp == 0 ? 0 : 1;
+    const uint32_t own = static_cast<uint32_t>(p.b_stages) / 2u;
     auto produce = [&]()
     {
       asm volatile("griddepcontrol.wait;" ::: "memory");
       uint32_t s = 0;
       uint32_t g = 0;
+      uint32_t n = 0;   // halves copied so far
       for (int tile = 0; tile < num_tiles; ++tile)
       {
         const StreamTile w = tiles[tile];
@@ -314,6 +324,26 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
         const uint32_t box_bytes = static_cast<uint32_t>(p.box) * 128u;
         for (int st = 0; st < stages; ++st, ++g)
         {
+          const int subs = min(2, num_kb - 2 * st);
+          if (HALVES)
+          {
+            if (half < subs)
+            {
+              const uint32_t at = 2u * (n % own) + static_cast<uint32_t>(half);
+              if (n >= own && !wait(b_empty(at), (n / own - 1u) & 1u))
+              {
+                return;
+              }
+              mbar_expect_tx(b_full(at), static_cast<uint32_t>(boxes) * box_bytes + (g == 0 && half == 0 ? p.stall_bytes : 0u));
+              for (int b = 0; b < boxes; ++b)
+              {
+                tma_load_2d(b_addr(at) + static_cast<uint32_t>(b) * box_bytes, &map_b, (2 * (st_begin + st) + half) * KB,
+                            w.token0 + b * p.box, b_full(at));
+              }
+              ++n;
+            }
+            continue;
+          }
           // the place of the stage b_stages before this one: it must have been multiplied
           if (g >= static_cast<uint32_t>(p.b_stages))
           {
@@ -323,7 +353,6 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
               return;   // nothing new is started once a wait has run out
             }
           }
-          const int subs = min(2, num_kb - 2 * st);
           if (half == 0)
           {
             mbar_expect_tx(b_full(s), static_cast<uint32_t>(subs * boxes) * box_bytes + (g == 0 ? p.stall_bytes : 0u));
@@ -361,6 +390,8 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
     {
       uint32_t g = 0;    // stages multiplied so far
       uint32_t sb = 0, b_par = 0;
+      uint32_t halves[2] = {0, 0};   // multiplied so far
+      const uint32_t own = static_cast<uint32_t>(p.b_stages) / 2u;
       int acc = 0;
       uint32_t acc_par = 0;
       const uint64_t bdesc_base = make_desc(smem_base, 16, 1024);
@@ -391,8 +422,8 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
         for (int st = 0; st < stages; ++st, ++g)
         {
           const uint32_t a0 = tmem_base + A_COLUMN0 + (g % PLACES) * STAGE_COLUMNS;
-          const uint64_t bdesc0 = bdesc_base + static_cast<uint64_t>((sb * p.b_stage_bytes) >> 4);
-          if (!wait(b_full(sb), b_par) || !wait(a_full(g % PLACES), (g / PLACES) & 1u))
+          uint64_t bdesc0 = bdesc_base + static_cast<uint64_t>((sb * p.b_stage_bytes) >> 4);
+          if ((!HALVES && !wait(b_full(sb), b_par)) || !wait(a_full(g % PLACES), (g / PLACES) & 1u))
           {
             return;
           }
@@ -402,6 +433,18 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
           {
             if (h == 0 || 2 * st + 1 < num_kb)
             {
+              uint32_t at = 0;
+              if (HALVES)
+              {
+                at = 2u * (halves[h] % own) + static_cast<uint32_t>(h);
+                if (!wait(b_full(at), (halves[h] / own) & 1u))
+                {
+                  return;
+                }
+                tc_fence_after();
+                ++halves[h];
+                bdesc0 = bdesc_base + static_cast<uint64_t>((b_addr(at) - smem_base - (h ? p.b_sub_bytes : 0u)) >> 4);
+              }
 #pragma unroll
               for (int k16 = 0; k16 < KB / 16; ++k16)
               {
@@ -412,6 +455,10 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
                 {
                   umma_bf16_tmem(d, a + PLANE_COLUMNS, bdesc, idesc, 1u);
                 }
+              }
+              if (HALVES)
+              {
+                umma_commit(b_empty(at));
               }
             }
           }
@@ -855,19 +902,22 @@ bool choose_depths(StreamParams &p, uint32_t &smem)
   {
     p.scale_bytes = 0;
   }
-  const int want = p.b_stage_bytes <= 16384 ? 4 : (p.b_stage_bytes <= 32768 ? 3 : 2);
+  p.halves = p.acc_bufs == 1 ? 1 : 0;   // more than 128 tokens
+  const uint32_t place = p.halves ? p.b_sub_bytes : p.b_stage_bytes;
+  const int want = (p.halves || place <= 16384) ? 4 : (place <= 32768 ? 3 : 2);
   for (int least = want; least >= 2; --least)
   {
     for (int depth : {3, 2})   // units of codes per warp
     {
       const uint32_t fixed = static_cast<uint32_t>(CODE_WARPS * depth) * UNIT_BYTES + ((records + 15u) & ~15u) + (p.scale_bytes != 0u ? scales : 0u) + 1024u;
-      if (fixed + static_cast<uint32_t>(least) * p.b_stage_bytes <= SMEM_LIMIT)
+      if (fixed + static_cast<uint32_t>(least) * place <= SMEM_LIMIT)
       {
-        const int fit = static_cast<int>((SMEM_LIMIT - fixed) / p.b_stage_bytes);
+        int fit = static_cast<int>((SMEM_LIMIT - fixed) / place);
+        fit = p.halves ? fit & ~1 : fit;
         p.depth = depth;
         p.b_stages = fit < MAX_B ? fit : MAX_B;
-        smem = fixed + static_cast<uint32_t>(p.b_stages) * p.b_stage_bytes;
-        p.scales_at = static_cast<uint32_t>(p.b_stages) * p.b_stage_bytes +
+        smem = fixed + static_cast<uint32_t>(p.b_stages) * place;
+        p.scales_at = static_cast<uint32_t>(p.b_stages) * place +
                       static_cast<uint32_t>(CODE_WARPS * depth) * UNIT_BYTES + ((records + 15u) & ~15u);
         return true;
       }
@@ -906,11 +956,11 @@ int resident_clusters(K kernel, int dev, int size)
   return n;
 }
 
-template <int WMODE, int N>
+template <int WMODE, int N, bool HALVES>
 int launch_stream_inst(const CUtensorMap &map_b, StreamParams &p, const StreamTable<N> &table, uint32_t smem,
                        bool dependent, cudaStream_t s)
 {
-  auto kernel = linear_stream_kernel<WMODE, N>;
+  auto kernel = linear_stream_kernel<WMODE, N, HALVES>;
   static std::atomic<bool> configured[kMaxDevices];
   int dev = 0;
   CAIFQ_CHECK_CUDA(cudaGetDevice(&dev));
@@ -968,11 +1018,13 @@ int launch_stream(int mode, const CUtensorMap &map_b, StreamParams &p, const Str
   switch (mode)
   {
     case W_I8:
-      return launch_stream_inst<W_I8, N>(map_b, p, table, smem, dependent, s);
+      return p.halves ? launch_stream_inst<W_I8, N, true>(map_b, p, table, smem, dependent, s)
+                      : launch_stream_inst<W_I8, N, false>(map_b, p, table, smem, dependent, s);
     case W_I4:
-      return launch_stream_inst<W_I4, N>(map_b, p, table, smem, dependent, s);
+      return p.halves ? launch_stream_inst<W_I4, N, true>(map_b, p, table, smem, dependent, s)
+                      : launch_stream_inst<W_I4, N, false>(map_b, p, table, smem, dependent, s);
     default:
-      return launch_stream_inst<W_I4S, N>(map_b, p, table, smem, dependent, s);
+      return launch_stream_inst<W_I4S, N, false>(map_b, p, table, smem, dependent, s);
   }
 }
 
