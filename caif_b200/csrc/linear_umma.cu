@@ -12,8 +12,8 @@
 // memory, one k-block ahead of the MMA warp.
 //
 // One persistent CTA per SM, 14 warps:
-//   warp 0      TMA producer for the activation tiles (and the weight tiles when
-//               the weight is already bf16)
+//   warp 0      TMA producer for the activation tiles (warp 10 for the weight tiles
+//               when the weight is already bf16)
 //   warp 1      TMEM allocation, MMA issue (one elected lane)
 //   warps 2-5   epilogue: TMEM -> registers -> scale -> global
 //   warps 6-13  dequantization of the weight tile
@@ -1435,10 +1435,10 @@ int launch_linear_umma(const LinearArgs &g, cudaStream_t s)
   p.num_m_tiles = static_cast<int>((g.m + BM - 1) / BM);
   p.band = kBand;
   p.wide_stores = (reinterpret_cast<uintptr_t>(g.c) & 31u) == 0;
-  // 256-wide tiles feed the tensor core better per shared-memory byte; 128-wide ones keep a
-  // second accumulator set so the epilogue overlaps the next tile.  CAIFQ_UMMA_BN overrides.
-  // A 256-wide tile goes to a CTA pair (half the operand bytes per SM and flop, two accumulator sets) when
-  // there are enough tiles for the pairs, else to a single CTA when there are enough for the SMs.
+  // A bf16 weight's tiles go to CTA pairs (half the operand bytes per SM and flop, two accumulator sets), in the width
+  // that choose_pair_width picks.  Of a quantized weight's, 256-wide ones feed the tensor core better per shared-memory
+  // byte and are taken when there are enough for the SMs; 128-wide ones keep a second accumulator set so the epilogue
+  // overlaps the next tile.  CAIFQ_UMMA_BN overrides.
   const int mode = wmode_of(w, g.compute_dtype);
   const char *forced = std::getenv("CAIFQ_UMMA_BN");
   int bn = 128;
@@ -1547,8 +1547,12 @@ int launch_linear_umma(const LinearArgs &g, cudaStream_t s)
   }
   CAIFQ_UMMA_CASE(W_I8)
   CAIFQ_UMMA_CASE(W_I4)
-  CAIFQ_UMMA_CASE(W_BF16)
 #undef CAIFQ_UMMA_CASE
+  if (mode == W_BF16)
+  {
+    return g.backward ? launch_inst<W_BF16, true, 128, false>(map_a, map_b, map_h, map_l, p, NoGroupTable{}, s)
+                      : launch_inst<W_BF16, false, 128, false>(map_a, map_b, map_h, map_l, p, NoGroupTable{}, s);
+  }
   if (mode == W_I4S)   // two operand planes: 128-wide tiles only
   {
     return g.backward ? launch_inst<W_I4S, true, 128, false>(map_a, map_b, map_h, map_l, p, NoGroupTable{}, s)
