@@ -1,14 +1,18 @@
-// Forward product of a bf16 weight with few rows of bf16 activations:
+// Forward product of a bf16 weight with few rows of bf16 activations, or into few columns:
 //
-//   y[m, out] = x[m, in] . W[out, in]^T  (+ y)        m <= 16, or 64 for a narrow weight
+//   y[m, out] = x[m, in] . W[out, in]^T  (+ y)        m <= 16, or any m where out is not a multiple of 128
 //
 // The float-storage cell of CAIF_DeviceFrozenLinear (src/caif_device_frozen_linear.cpp:381-524) and the router's
 // product over the experts (src/caif_device_moe_router.cpp:233-260).  Bound by reading the weight once when it is
 // large, by latency when it is small: a router of 64 x 2048 on 16 tokens ran as ONE block of the fp32-FMA kernel that
-// walked all of k (219 us).  Here a CTA owns NT * 8 output columns and 16 rows, its eight warps split k and stream both
-// operands from global memory straight into bf16 tensor-core fragments, sixteen bytes a lane and operand (the order
-// of k inside a fragment is the same for both, which is all a dot product needs); the eight partial tiles meet in
-// shared memory.  Products are exact in fp32 and accumulate in fp32, so fp32 and bf16 compute are the same here.
+// walked all of k (191 us, 7.7 here), by L2 for many rows (16384 tokens: 48 us, the FMA kernel 270).  Here a CTA owns
+// NT * 8 output columns and 16 rows, its eight warps split k and stream both operands from global memory straight into
+// bf16 tensor-core fragments, sixteen bytes a lane and operand (the order of k inside a fragment is the same for both,
+// which is all a dot product needs); the eight partial tiles meet in shared memory.  Products are exact in fp32 and
+// accumulate in fp32, so fp32 and bf16 compute are the same here.  The tensor core truncates where it adds, so a chain of
+// MMAs is 128 k long and the chains meet in IEEE additions: closer to 64 bits than the FMA kernel at every k (one chain a
+// warp was not, from k = 8192 on; the many-token kernel's one chain over all of k is five to twelve times further off:
+// 12 us for the 16384 tokens, but 2.1e-6 where this and the FMA kernel have 1.3e-7 and 3.9e-7).
 #include "common.cuh"
 
 namespace caifq
@@ -19,6 +23,7 @@ namespace
 
 constexpr int kRowsWarps = 8;
 constexpr int kRowsUnroll = 4;   // k-steps of 32 whose loads are in flight per warp
+constexpr int64_t kRowsMost = 16 * 65535;   // rows of a launch: the grid's second dimension
 
 __device__ __forceinline__ void mma_rows(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                          uint32_t b1)
@@ -48,14 +53,14 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__r
   const uint4 *x_lo = reinterpret_cast<const uint4 *>(x + (lo_ok ? row0 + g : 0) * in_dim) + t;
   const uint4 *x_hi = reinterpret_cast<const uint4 *>(x + (hi_ok ? row0 + g + 8 : 0) * in_dim) + t;
   const uint4 *w_ptr[NT];
-  float c[NT][4];
+  float sum[NT][4];
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt)
   {
     // columns past the last one read it again; they are not stored
     const int col = min(col0 + nt * 8 + g, out_dim - 1);
     w_ptr[nt] = reinterpret_cast<const uint4 *>(w + static_cast<int64_t>(col) * in_dim) + t;
-    c[nt][0] = c[nt][1] = c[nt][2] = c[nt][3] = 0.0f;
+    sum[nt][0] = sum[nt][1] = sum[nt][2] = sum[nt][3] = 0.0f;
   }
   const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
   for (int st = begin; st < end; st += kRowsUnroll)
@@ -73,6 +78,7 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__r
         wv[u][nt] = in ? __ldg(w_ptr[nt] + (st + u) * 4) : zero4;
       }
     }
+    float c[NT][4] = {};
 #pragma unroll
     for (int u = 0; u < kRowsUnroll; ++u)
     {
@@ -83,14 +89,23 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__r
         mma_rows(c[nt], xa[u].z, xb[u].z, xa[u].w, xb[u].w, wv[u][nt].z, wv[u][nt].w);
       }
     }
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+    {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+      {
+        sum[nt][i] += c[nt][i];
+      }
+    }
   }
 #pragma unroll
   for (int nt = 0; nt < NT; ++nt)
   {
-    part[warp][g][nt * 8 + 2 * t] = c[nt][0];
-    part[warp][g][nt * 8 + 2 * t + 1] = c[nt][1];
-    part[warp][g + 8][nt * 8 + 2 * t] = c[nt][2];
-    part[warp][g + 8][nt * 8 + 2 * t + 1] = c[nt][3];
+    part[warp][g][nt * 8 + 2 * t] = sum[nt][0];
+    part[warp][g][nt * 8 + 2 * t + 1] = sum[nt][1];
+    part[warp][g + 8][nt * 8 + 2 * t] = sum[nt][2];
+    part[warp][g + 8][nt * 8 + 2 * t + 1] = sum[nt][3];
   }
   __syncthreads();
   for (int e = threadIdx.x; e < 16 * NT * 8; e += kRowsWarps * 32)
@@ -118,11 +133,12 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__r
 
 }  // namespace
 
-// few tokens; for outputs narrower than a tensor-core tile (routers) up to 64, where that kernel's one tile is full enough
+// Few tokens; and any number of them where the output is not made of the tensor-core kernel's 128-column tiles (routers).
 bool rows_supported(const LinearArgs &g)
 {
   return !g.backward && g.w.storage == CAIFQ_BF16 && g.a_dtype == CAIFQ_BF16 && g.a_prescale == 1.0f && g.m >= 1 &&
-         g.m <= (g.w.out_dim < 128 ? 64 : 16) && (g.compute_dtype == CAIFQ_F32 || g.compute_dtype == CAIFQ_BF16) && (g.w.in_dim % 32) == 0 &&
+         g.m <= ((g.w.out_dim % 128) != 0 ? kRowsMost : 16) && (g.compute_dtype == CAIFQ_F32 || g.compute_dtype == CAIFQ_BF16) &&
+         (g.w.in_dim % 32) == 0 &&
          ((reinterpret_cast<uintptr_t>(g.a) | reinterpret_cast<uintptr_t>(g.w.codes)) & 15u) == 0 && g.num_peers == 0 &&
          g.num_more == 0;
 }

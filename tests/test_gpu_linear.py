@@ -544,17 +544,32 @@ def test_few_rows_on_a_bf16_weight(m, in_dim, out_dim, sd):
     assert torch.equal(got, (sep.float() + res.float()).to(TORCH_DTYPE[sd]))
 
 
-@pytest.mark.parametrize("m,in_dim,out_dim", [(65, 2048, 64), (300, 512, 96), (700, 256, 160)])
-def test_umma_bf16_weight_with_a_partial_last_column_tile(m, in_dim, out_dim):
-    weight, wc, x_np, x, dy_np, dy = _umma_case(orc.BF16, orc.F32, m, in_dim, out_dim, m + out_dim)
-    y = nv.linear_fwd(weight, x, torch.float32, orc.F32)
-    assert nv.last_path() == "umma"
-    assert max_rel_err(y.cpu().numpy(), orc.frozen_linear_forward(x_np, wc)) <= TOL_F32
-    if out_dim % 64 == 0:      # dX reduces over the output features, 64 at a time
-        weight, wc, x_np, x, dy_np, dy = _umma_case(orc.BF16, orc.F32, m, out_dim + 32, 128, m)
-        dx = nv.linear_dx(weight, dy, torch.float32, orc.F32)
-        assert nv.last_path() == "umma"
-        assert max_rel_err(dx.cpu().numpy(), orc.frozen_linear_backward(dy_np, wc)) <= TOL_F32
+@pytest.mark.parametrize("compute", [orc.F32, orc.BF16])
+@pytest.mark.parametrize("m,in_dim,out_dim", [
+    (65, 2048, 64), (300, 512, 96), (700, 256, 160), (17, 14336, 8),
+    (2500, 4096, 33),      # more rows than a wave of CTAs, a ragged last column tile
+    (16, 14336, 4096), (257, 8192, 4104),
+])
+def test_bf16_weight_outside_the_tensor_core_tiles_keeps_fp32_precision(m, in_dim, out_dim, compute, monkeypatch):
+    """Products of bf16 values are exact in fp32 and the sums are fp32's: no further from 64 bits than the fp32-FMA kernel."""
+    g = torch.Generator(device="cuda").manual_seed(m + in_dim + out_dim)
+    w = (torch.randn(out_dim, in_dim, generator=g, device="cuda") / in_dim ** 0.5).bfloat16()
+    x = torch.randn(m, in_dim, generator=g, device="cuda").bfloat16()
+    weight = nv.Weight(w, nv.BF16, in_dim, out_dim)
+    want = x.double() @ w.double().T
+    y = nv.linear_fwd(weight, x, torch.float32, compute)
+    assert nv.last_path() == "decode"
+    monkeypatch.setenv("CAIFQ_FORCE_PATH", "generic")
+    fma = nv.linear_fwd(weight, x, torch.float32, compute)
+    assert nv.last_path() == "generic"
+    assert (y.double() - want).norm() <= 1.02 * (fma.double() - want).norm()
+
+
+def test_layers_over_ragged_widths_are_refused_as_one_product():
+    """The concatenated product needs whole 128-column tiles: 96 + 64 output features are not."""
+    ws = [make_weight(np.random.default_rng(o), o, 256, orc.I8)[0] for o in (96, 64)]
+    with pytest.raises(nv.CaifqError, match="tensor-core path"):
+        nv.linear_concat(ws, torch.zeros(64, 256, dtype=torch.bfloat16, device="cuda"))
 
 
 @pytest.mark.parametrize("storage,group", [(orc.I8, 128), (orc.I4, 128), (orc.I4, 64)])
@@ -625,11 +640,10 @@ def test_streaming_wait_that_runs_out_raises_the_flag_and_returns(m, out_dim):
 
 
 @pytest.mark.parametrize("width", ["64", "96", "128", "160", "192", "224", "256", None])
-@pytest.mark.parametrize("m,in_dim,out_dim", [(300, 320, 480), (2305, 128, 1088)])   # partial tiles both ways; 10 row tiles
+@pytest.mark.parametrize("m,in_dim,out_dim", [(300, 320, 384), (2305, 128, 1152)])   # partial tiles both ways; 10 row tiles
 def test_umma_bf16_tile_widths(width, m, in_dim, out_dim, monkeypatch):
     if width is not None:
         monkeypatch.setenv("CAIFQ_UMMA_BN", width)
-    out_dx = (out_dim + 63) // 64 * 64      # dX reduces over the output features, 64 at a time
     weight, wc, x_np, x, dy_np, dy = _umma_case(orc.BF16, orc.F32, m, in_dim, out_dim, m + out_dim)
     y = nv.linear_fwd(weight, x, torch.float32, orc.F32)
     assert nv.last_path() == "umma"
@@ -637,8 +651,10 @@ def test_umma_bf16_tile_widths(width, m, in_dim, out_dim, monkeypatch):
     out = torch.empty(m * out_dim + 8, dtype=torch.bfloat16, device="cuda")[8:].view(m, out_dim)   # 16-byte aligned only
     nv.linear_fwd(weight, x, torch.bfloat16, orc.F32, out=out)
     assert torch.equal(out, y.to(torch.bfloat16))
-    weight, wc, x_np, x, dy_np, dy = _umma_case(orc.BF16, orc.F32, m, in_dim, out_dx, m + out_dx)
+    in_dx = (in_dim + 127) // 128 * 128      # dX has in_dim columns: whole 128-column tiles
+    weight, wc, x_np, x, dy_np, dy = _umma_case(orc.BF16, orc.F32, m, in_dx, out_dim, m + out_dim)
     dx = nv.linear_dx(weight, dy, torch.float32, orc.F32)
+    assert nv.last_path() == "umma"
     assert max_rel_err(dx.cpu().numpy(), dy_np.astype(np.float64) @ wc.astype(np.float64)) <= TOL_F32
     assert nv.lib().caifq_device_status() == 0
 
