@@ -240,11 +240,12 @@ struct DecodeParams
   uint32_t stall_bytes;   // self-test only: bytes the first wait announces but never receives
 };
 
-// int4 codes are turned into the bf16 integers 136 + q (q in [-8,7]): the
-// nibble, flipped to offset binary, is dropped into the mantissa of 128.0.  The
-// constant is taken out again by starting each accumulator at -136 * (sum of x
-// over the same 128 elements), so no subtract runs per weight.
-constexpr uint32_t kMinus136x2 = 0xC308C308u;
+// int4 codes are turned into the bf16 integers 24 + q (q in [-8,7]): the nibble, flipped to offset binary, is dropped
+// into the upper mantissa bits of 16.0.  The constant is taken out again by starting each accumulator at -24 * (sum of x
+// over the same 128 elements), so no subtract runs per weight.  The accumulator holds both for a while, so the constant
+// sets the rounding: 136 + q (the nibble in the lower bits) saves a shift per eight weights, and was further from 64
+// bits than an fp32 GEMM (4096 -> 4096, 5 tokens: 1.35e-6 against 7.4e-7; now 1.6e-7).
+constexpr uint32_t kMinus24x2 = 0xC1C0C1C0u;
 
 // WARPS: 8 or 16.  BITS: 4 or 8.  MT: token tiles of 8 (1 -> m <= 8, 2 -> m <= 16).
 // NCH: chunks (64 bytes of one row: a quad of lanes x 16 bytes) per warp and pass; PCH of them per ring slot.
@@ -266,6 +267,32 @@ struct DecodeCfg
 __device__ __forceinline__ uint32_t park_swizzle(int row, int tokp)
 {
   return tokp == 16 ? static_cast<uint32_t>((row >> 1) & 3) : (tokp == 8 ? static_cast<uint32_t>((row >> 2) & 1) : 0u);
+}
+
+// An output as a plain fp32 sum of products: for tokens with an infinity or NaN, and where sums overflow only before the
+// scale.  (Called without inlining it cost the 16-token forms 1.3 to 3 us a launch, registers being spilled around it.)
+template <int BITS>
+__device__ __forceinline__ float plain_sum(const DecodeParams &p, int row, int token)
+{
+  int sg = 0;
+  while (sg + 1 < p.num_seg && row >= p.seg_row0[sg + 1])
+  {
+    ++sg;
+  }
+  row -= p.seg_row0[sg];
+  const uint8_t *codes = p.codes[sg] + static_cast<size_t>(row) * p.row_bytes;
+  const __half *group_scales = static_cast<const __half *>(p.scales[sg]) + static_cast<size_t>(row) * p.groups_per_row;
+  const float tensor_scale = (BITS == 8 && p.scales[sg] != nullptr) ? *static_cast<const float *>(p.scales[sg]) : 1.0f;
+  const __nv_bfloat16 *x = p.x + static_cast<size_t>(token) * p.in_dim;
+  float sum = 0.0f;
+#pragma unroll 1
+  for (int k = 0; k < p.in_dim; ++k)
+  {
+    const int q = (BITS == 4) ? sign_extend_nibble((codes[k >> 1] >> (4 * (k & 1))) & 0xF) : static_cast<int8_t>(codes[k]);
+    const float s = (BITS == 4) ? __half2float(group_scales[k / (128 * p.chunks_per_group)]) : tensor_scale;
+    sum = fmaf(__fmul_rn(static_cast<float>(q), s), __bfloat162float(x[k]), sum);
+  }
+  return sum;
 }
 
 template <int WARPS, int BITS, int MT, int NCH, int PCH>
@@ -413,7 +440,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
   //   int4, word wi: (8wi+0, 8wi+4) (8wi+2, 8wi+6) (8wi+1, 8wi+5) (8wi+3, 8wi+7)
   //   int8, word wi: (4wi+0, 4wi+2) (4wi+1, 4wi+3)
   uint32_t xf[NCH][MT][XR];
-  float sx[NCH][MT][4];     // int4: -136 * (sum of x over the chunk's 128 elements) as an accumulator fragment
+  float sx[NCH][MT][4];     // int4: -24 * (sum of x over the chunk's 128 elements) as an accumulator fragment
   uint32_t scale_off[NCH];  // byte offset of row g's scale for the chunk inside a tile's scales
   auto load_x = [&](int kseg)
   {
@@ -465,7 +492,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
             f[2 * wi + 1] = __byte_perm(r0, r1, 0x7632);
           }
         }
-        // the sums come from the tensor core too: the accumulators of weight rows whose codes are all -136
+        // the sums come from the tensor core too: the accumulators of weight rows whose codes are all -24
         float c0[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (BITS == 4)
         {
@@ -473,8 +500,8 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
 #pragma unroll
           for (int j = 0; j < XR / 2; j += 2)
           {
-            mma_bf16_16816(c0, kMinus136x2, kMinus136x2, kMinus136x2, kMinus136x2, f[2 * j], f[2 * j + 1], c0);
-            mma_bf16_16816(c1, kMinus136x2, kMinus136x2, kMinus136x2, kMinus136x2, f[2 * j + 2], f[2 * j + 3], c1);
+            mma_bf16_16816(c0, kMinus24x2, kMinus24x2, kMinus24x2, kMinus24x2, f[2 * j], f[2 * j + 1], c0);
+            mma_bf16_16816(c1, kMinus24x2, kMinus24x2, kMinus24x2, kMinus24x2, f[2 * j + 2], f[2 * j + 3], c1);
           }
 #pragma unroll
           for (int i = 0; i < 4; ++i)
@@ -588,20 +615,20 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
                   uint32_t a_lo[4];
                   uint32_t a_hi[4];
                   {
-                    const uint32_t ev = lop3_and_xor(wlo[wi], 0x0F0F0F0Fu, 0x08080808u);
-                    const uint32_t od = lop3_and_xor(wlo[wi] >> 4, 0x0F0F0F0Fu, 0x08080808u);
-                    a_lo[0] = __byte_perm(ev, 0x43434343u, 0x4240);
-                    a_lo[1] = __byte_perm(ev, 0x43434343u, 0x4341);
-                    a_lo[2] = __byte_perm(od, 0x43434343u, 0x4240);
-                    a_lo[3] = __byte_perm(od, 0x43434343u, 0x4341);
+                    const uint32_t ev = lop3_and_xor(wlo[wi] << 3, 0x78787878u, 0xC0C0C0C0u);
+                    const uint32_t od = lop3_and_xor(wlo[wi] >> 1, 0x78787878u, 0xC0C0C0C0u);
+                    a_lo[0] = __byte_perm(ev, 0x41414141u, 0x4240);
+                    a_lo[1] = __byte_perm(ev, 0x41414141u, 0x4341);
+                    a_lo[2] = __byte_perm(od, 0x41414141u, 0x4240);
+                    a_lo[3] = __byte_perm(od, 0x41414141u, 0x4341);
                   }
                   {
-                    const uint32_t ev = lop3_and_xor(whi[wi], 0x0F0F0F0Fu, 0x08080808u);
-                    const uint32_t od = lop3_and_xor(whi[wi] >> 4, 0x0F0F0F0Fu, 0x08080808u);
-                    a_hi[0] = __byte_perm(ev, 0x43434343u, 0x4240);
-                    a_hi[1] = __byte_perm(ev, 0x43434343u, 0x4341);
-                    a_hi[2] = __byte_perm(od, 0x43434343u, 0x4240);
-                    a_hi[3] = __byte_perm(od, 0x43434343u, 0x4341);
+                    const uint32_t ev = lop3_and_xor(whi[wi] << 3, 0x78787878u, 0xC0C0C0C0u);
+                    const uint32_t od = lop3_and_xor(whi[wi] >> 1, 0x78787878u, 0xC0C0C0C0u);
+                    a_hi[0] = __byte_perm(ev, 0x41414141u, 0x4240);
+                    a_hi[1] = __byte_perm(ev, 0x41414141u, 0x4341);
+                    a_hi[2] = __byte_perm(od, 0x41414141u, 0x4240);
+                    a_hi[3] = __byte_perm(od, 0x41414141u, 0x4341);
                   }
 #pragma unroll
                   for (int h = 0; h < 2; ++h)
@@ -750,6 +777,24 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
           }
         }
         const int live = min(4, p.m - 4 * tq);
+        // (summed before the scale, and int4 with an offset that turns an infinity into infinity - infinity)
+        if (__builtin_expect(!(fabsf(acc[0]) + fabsf(acc[1]) + fabsf(acc[2]) + fabsf(acc[3]) <= 3.402823466e38f), 0))
+        {
+#pragma unroll 1
+          for (int i = 0; i < live; ++i)
+          {
+            const float sum = i == 0 ? acc[0] : (i == 1 ? acc[1] : (i == 2 ? acc[2] : acc[3]));
+            if (fabsf(sum) <= 3.402823466e38f)
+            {
+              continue;
+            }
+            const float v = plain_sum<BITS>(p, row, 4 * tq + i);
+            acc[0] = i == 0 ? v : acc[0];
+            acc[1] = i == 1 ? v : acc[1];
+            acc[2] = i == 2 ? v : acc[2];
+            acc[3] = i == 3 ? v : acc[3];
+          }
+        }
         int64_t idx = static_cast<int64_t>(4 * tq) * p.y_ld + p.y_col0 + row;
         if (p.y_dtype == CAIFQ_F32 && !p.accumulate && p.num_y == 1)
         {

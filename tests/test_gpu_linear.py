@@ -188,6 +188,51 @@ def test_decode_long_rows_and_the_residual_add(storage, in_dim, out_dim, m, sd):
     assert torch.equal(got, (sep.float() + res.float()).to(TORCH_DTYPE[sd]))
 
 
+@pytest.mark.parametrize("storage", [orc.I4, orc.I8])
+@pytest.mark.parametrize("in_dim,out_dim,m", [(1024, 1024, 4), (4096, 1000, 9), (14336, 520, 1), (14336, 136, 16), (9216, 72, 5)])
+def test_decode_is_as_close_to_64_bits_as_the_fma_kernel(storage, in_dim, out_dim, m, monkeypatch):
+    rng = np.random.default_rng(in_dim + out_dim + m)
+    weight, codes, scales = make_weight(rng, out_dim, in_dim, storage)
+    w = torch.from_numpy(_oracle_w(weight, codes, scales, orc.F32)).double().cuda()
+    x = torch.from_numpy(rng.standard_normal((m, in_dim)).astype(np.float32)).cuda().bfloat16()
+    want = x.double() @ w.T
+    y = nv.linear_fwd(weight, x, torch.float32, orc.F32)
+    assert nv.last_path() == "decode"
+    monkeypatch.setenv("CAIFQ_FORCE_PATH", "generic")
+    fma = nv.linear_fwd(weight, x, torch.float32, orc.F32)
+    assert (y.double() - want).norm() <= 1.02 * (fma.double() - want).norm()
+
+
+@pytest.mark.parametrize("storage", [orc.I4, orc.I8])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.0e38])
+@pytest.mark.parametrize("in_dim,m", [(512, 1), (4096, 3), (14336, 12)])
+def test_decode_infinities_and_nans_reach_only_their_token(storage, value, in_dim, m, monkeypatch):
+    """An infinity times a weight is an infinity of that sign (NaN for a zero), as in a plain fp32 product; and large values
+    overflow only where the product itself does.  Three layers in one launch."""
+    rng = np.random.default_rng(in_dim + m)
+    ws = [make_weight(rng, o, in_dim, storage)[0] for o in (264, 64, 40)]
+    x = torch.from_numpy(rng.standard_normal((m, in_dim)).astype(np.float32)).cuda().bfloat16()
+    clean = nv.linear_fwd_multi(ws, x, torch.float32, orc.F32)
+    x[m // 2, 77] = value
+    x[m // 2, in_dim - 1] = value
+    y = nv.linear_fwd_multi(ws, x, torch.float32, orc.F32)
+    one = nv.linear_fwd(ws[0], x, torch.float32, orc.F32)
+    assert nv.last_path() == "decode"
+    monkeypatch.setenv("CAIFQ_FORCE_PATH", "generic")
+    want = torch.cat([nv.linear_fwd(w, x, torch.float32, orc.F32) for w in ws], 1)
+    others = [t for t in range(m) if t != m // 2]
+    assert torch.equal(y[others], clean[others]) and torch.equal(one[others], y[others, :264])
+    for got, ref in ((y[m // 2], want[m // 2]), (one[m // 2], want[m // 2, :264])):
+        assert torch.equal(torch.isnan(got), torch.isnan(ref))
+        live = ~torch.isnan(ref)
+        assert torch.equal(torch.isinf(got[live]), torch.isinf(ref[live]))
+        if live.any():
+            # (two huge terms may cancel: the bound is that of the terms, not of the sum)
+            scale = ref[live].abs()[torch.isfinite(ref[live])].max() if torch.isfinite(ref[live]).any() else 0.0
+            same = got[live] == ref[live]
+            assert (same | ((got[live] - ref[live]).abs() <= 1e-5 * scale)).all()
+
+
 def test_decode_int8_without_scales_and_bf16_out():
     rng = np.random.default_rng(77)
     weight, codes, scales = make_weight(rng, 256, 2048, orc.I8, with_scales=False)
