@@ -24,7 +24,8 @@
 //               their first stage of the next tile; a token's 32 rows leave as one contiguous store.
 // Few row tiles (narrow layers) split k over the CTAs of a cluster; their partial tiles meet through distributed shared
 // memory in rank order: no scratch, no atomics, the same bits every time.
-// The codes' copies start before the kernel waits for the previous one in the stream (programmatic dependent launch).
+// The codes' copies start before the kernel waits for the previous one in the stream (programmatic dependent launch); so
+// do the first places' conversions.
 //
 // Operands and roundings are those of the many-token kernel: int8 codes exact in bf16 with the scale in the epilogue,
 // int4 times its group scale rounded to bf16, or as two bf16 terms for fp32 compute.
@@ -408,6 +409,8 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
         }
       };
       copy_scales(0);
+      // (the activations come after the previous kernel: the limit of a wait must not run while that one does)
+      asm volatile("griddepcontrol.wait;" ::: "memory");
       for (int tile = 0; tile < num_tiles; ++tile)
       {
         // (everything of the tile before this one has been converted, so its scales' place is free)
@@ -678,7 +681,17 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
       load_scales(0, first_stage(0), 0, next_sc);
     }
     int undrained = -1;   // a tile whose accumulators still wait
+    // Before the first wait on what follows from an MMA, and before anything is written: the kernel before this one has
+    // ended.  Until then its time would count against the wait's limit, and it may read what is written here.
     bool released = false;
+    auto after_previous = [&]()
+    {
+      if (!released)
+      {
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+        released = true;
+      }
+    };
     // one trip more than there are tiles, to drain the last one
     for (int tile = 0; tile <= num_tiles; ++tile, g_before += static_cast<uint32_t>(stages))
     {
@@ -689,11 +702,7 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
         // (with one accumulator set before anything of the next tile, which could not be multiplied)
         if (undrained >= 0 && (unit >= 1 || units <= 1 || p.acc_bufs == 1))
         {
-          if (!released)
-          {
-            asm volatile("griddepcontrol.wait;" ::: "memory");   // the kernel before this one may read what is written
-            released = true;
-          }
+          after_previous();
           epilogue(undrained);
           undrained = -1;
         }
@@ -723,6 +732,10 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
           {
             if (unit == 0)
             {
+              if (tile > 0)   // (the first tile's scales are on their way at once)
+              {
+                after_previous();
+              }
               wait(sc_full(tile), static_cast<uint32_t>(tile >> 1) & 1u);
             }
             load_scales(tile, first, unit, next_sc);
@@ -798,6 +811,7 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
                 placed = true;
                 if (g >= PLACES)
                 {
+                  after_previous();
                   wait(done(g - PLACES), done_parity(g - PLACES));
                   tc_fence_after();
                 }

@@ -684,6 +684,34 @@ def test_streaming_wait_that_runs_out_raises_the_flag_and_returns(m, out_dim):
     assert torch.equal(y, y2)
 
 
+@pytest.mark.parametrize("storage,m,out_dim", [(orc.I4, 64, 1024), (orc.I8, 96, 14336), (orc.I4, 300, 19072)])
+def test_streaming_launch_behind_a_long_kernel_waits_for_it(storage, m, out_dim):
+    """A launch that is placed beside the end of a long one (here one CTA's, a few hundred ms) must not count that one's
+    time as its own waiting."""
+    weight, wc, x_np, x, dy_np, dy = _umma_case(storage, orc.BF16, m, 256, out_dim, 4321)
+    want = nv.linear_fwd(weight, x, torch.float32, orc.BF16)
+    assert nv.lib().caifq_device_status() == 0
+    rng = np.random.default_rng(3)
+    big, _, _ = make_weight(rng, 2048, 4096, orc.I8)
+    rows = torch.ones(131072, 4096, dtype=torch.bfloat16, device="cuda")
+    y_big = torch.empty(131072, 2048, dtype=torch.bfloat16, device="cuda")
+    y = torch.empty_like(want)
+    start, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    nv.lib().caifq_set_cta_limit(1)
+    try:
+        start.record()
+        # (the plain entry point: the weight is converted in the kernel, which takes a single CTA)
+        assert nv.lib().caifq_linear_fwd(big.ref(), nv._ptr(rows), nv.BF16, rows.shape[0], nv._ptr(y_big), nv.BF16, nv.BF16,
+                                         nv._stream()) == 0
+    finally:
+        nv.lib().caifq_set_cta_limit(0)
+    assert nv.lib().caifq_linear_fwd(weight.ref(), nv._ptr(x), nv.BF16, m, nv._ptr(y), nv.F32, nv.BF16, nv._stream()) == 0
+    end.record()
+    assert nv.lib().caifq_device_status() == 0
+    assert start.elapsed_time(end) > 150.0
+    assert torch.equal(y, want)
+
+
 @pytest.mark.parametrize("width", ["64", "96", "128", "160", "192", "224", "256", None])
 @pytest.mark.parametrize("m,in_dim,out_dim", [(300, 320, 384), (2305, 128, 1152)])   # partial tiles both ways; 10 row tiles
 def test_umma_bf16_tile_widths(width, m, in_dim, out_dim, monkeypatch):
