@@ -488,9 +488,10 @@ skinny_tn_kernel(const SkinnyTn job0, const SkinnyTn job1, int tiles0, int64_t m
   }
 }
 
-// fp32 sums of both gradients -> bf16 (the sums lie one behind the other)
-__global__ void round_pair_kernel(const float2 *__restrict__ acc, __nv_bfloat162 *__restrict__ c0,
-                                  __nv_bfloat162 *__restrict__ c1, int64_t n0, int64_t n)
+// fp32 sums of both gradients -> bf16 (the sums lie one behind the other), two elements a thread.  A gradient may be a
+// view that starts on any element of a larger buffer: `pairs0` / `pairs1` say which of them takes 4-byte stores.
+__global__ void round_pair_kernel(const float2 *__restrict__ acc, __nv_bfloat16 *__restrict__ c0,
+                                  __nv_bfloat16 *__restrict__ c1, int64_t n0, int64_t n, int pairs0, int pairs1)
 {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -499,13 +500,15 @@ __global__ void round_pair_kernel(const float2 *__restrict__ acc, __nv_bfloat162
   {
     const float2 v = acc[i];
     const __nv_bfloat162 r = __floats2bfloat162_rn(v.x, v.y);
-    if (i < n0)
+    __nv_bfloat16 *dst = i < n0 ? c0 + 2 * i : c1 + 2 * (i - n0);
+    if (i < n0 ? pairs0 : pairs1)
     {
-      c0[i] = r;
+      *reinterpret_cast<__nv_bfloat162 *>(dst) = r;
     }
     else
     {
-      c1[i - n0] = r;
+      dst[0] = r.x;
+      dst[1] = r.y;
     }
   }
 }
@@ -651,8 +654,10 @@ int launch_skinny_tn(const void *dy, const void *h, void *db, float prescale, in
   }
   CAIFQ_CHECK_CUDA(err);
   CAIFQ_CHECK_CUDA(launch_dependent(round_pair_kernel, dim3(static_cast<unsigned>((n / 2 + 255) / 256)), dim3(256), 0, s,
-                                    reinterpret_cast<const float2 *>(sums), static_cast<__nv_bfloat162 *>(db),
-                                    static_cast<__nv_bfloat162 *>(da), n0 / 2, n / 2));
+                                    reinterpret_cast<const float2 *>(sums), static_cast<__nv_bfloat16 *>(db),
+                                    static_cast<__nv_bfloat16 *>(da), n0 / 2, n / 2,
+                                    (reinterpret_cast<uintptr_t>(db) & 3u) == 0 ? 1 : 0,
+                                    (reinterpret_cast<uintptr_t>(da) & 3u) == 0 ? 1 : 0));
   return CAIFQ_OK;
 }
 

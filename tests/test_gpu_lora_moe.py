@@ -882,3 +882,27 @@ def test_lora_products_split_over_clusters(rank, m, in_dim, out_dim):
     dh = (dyf * (32.0 / rank)) @ bf
     assert max_rel_err(da.float().cpu().numpy(), (dh.T @ xf).cpu().numpy()) <= 2e-2
     assert max_rel_err(db.float().cpu().numpy(), (dyf.T @ h.double() * (32.0 / rank)).cpu().numpy()) <= 2e-2
+
+
+@pytest.mark.parametrize("expanded", [False, True])
+@pytest.mark.parametrize("rank,m", [(8, 64), (16, 200)])
+def test_lora_gradients_into_views_on_any_element(rank, m, expanded):
+    """d_a and d_b as views into one flat gradient buffer, behind an odd number of elements: the same values, and nothing
+    written around them."""
+    rng = np.random.default_rng(rank + m)
+    in_dim, out_dim = 256, 384
+    weight, codes, scales, a, b, x_np, x, dy_np, dy, lora = _lora_case(rng, orc.I8, orc.BF16, in_dim, out_dim, m, rank, 32.0)
+    y, h = nv.lora_linear_fwd(weight, lora, x, orc.F32, expanded=expanded)
+    dx, da, db = nv.lora_linear_bwd(weight, lora, dy, x, h, orc.F32, expanded=expanded)
+    for shift_a, shift_b in ((1, 0), (0, 1), (1, 1)):
+        n_a, n_b = rank * in_dim, out_dim * rank
+        flat_a = torch.full((n_a + 3,), 7.0, dtype=torch.bfloat16, device="cuda")
+        flat_b = torch.full((n_b + 3,), 7.0, dtype=torch.bfloat16, device="cuda")
+        va = flat_a[shift_a:shift_a + n_a].view(rank, in_dim)
+        vb = flat_b[shift_b:shift_b + n_b].view(out_dim, rank)
+        nv.lora_linear_bwd(weight, lora, dy, x, h, orc.F32, d_a=va, d_b=vb, expanded=expanded)
+        # (the sums over tokens meet in atomic additions, in any order)
+        assert max_rel_err(va.float().cpu().numpy(), da.float().cpu().numpy()) <= 1e-2
+        assert max_rel_err(vb.float().cpu().numpy(), db.float().cpu().numpy()) <= 1e-2
+        for flat, shift, n in ((flat_a, shift_a, n_a), (flat_b, shift_b, n_b)):
+            assert torch.all(flat[:shift] == 7.0) and torch.all(flat[shift + n:] == 7.0)
