@@ -1241,6 +1241,10 @@ std::atomic<int> g_pair_capacity[kMaxDevices];
 // is the limit.  So pairs are the default for bf16 weights only; CAIFQ_UMMA_PAIR=1 / 0 forces them on / off.
 bool pairs_enabled(int mode)
 {
+  if (pair_count_umma() < 1)
+  {
+    return false;   // a limit of one CTA leaves no pair
+  }
   const char *e = std::getenv("CAIFQ_UMMA_PAIR");
   if (e == nullptr)
   {

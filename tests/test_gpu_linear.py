@@ -752,3 +752,41 @@ def test_many_tokens_through_an_expanded_weight(storage, compute, group, m, in_d
     plain = torch.empty_like(dx)
     rc = nv.lib().caifq_linear_dx(weight.ref(), dy.data_ptr(), nv.BF16, m, plain.data_ptr(), nv.F32, compute, nv._stream())
     assert rc == 0 and max_rel_err(plain.cpu().numpy(), dx.cpu().numpy()) <= 2 * tol
+
+
+@pytest.mark.parametrize("limit", [1, 3])
+def test_products_under_a_limit_of_few_ctas(limit):
+    """One CTA leaves no pair, three leave one: the same numbers from the expanded products, plain and with an adapter, and
+    from experts."""
+    weight, wc, x_np, x, dy_np, dy = _umma_case(orc.I8, orc.BF16, 1025, 256, 384, 11)
+    dense = nv.Weight(torch.randn(384, 256, device="cuda").bfloat16(), nv.BF16, 256, 384)
+    lora = nv.Lora(torch.randn(16, 256, device="cuda").bfloat16() / 16, torch.randn(384, 16, device="cuda").bfloat16() / 16, 32.0)
+    rng = np.random.default_rng(12)
+    gate, up, down = ([make_weight(rng, o, i, orc.I4)[0] for _ in range(2)] for o, i in ((384, 256), (384, 256), (256, 384)))
+    offsets = [0, 700, 1025]
+    need = nv.grouped_expert_expanded_bytes(gate, up, down, nv.BF16, nv.BF16)
+    expanded = torch.empty(need, dtype=torch.uint8, device="cuda")
+
+    def products():
+        y = nv.linear_fwd(weight, x, torch.bfloat16, orc.BF16)
+        dx = nv.linear_dx(weight, dy, torch.bfloat16, orc.BF16)
+        few = nv.linear_fwd(weight, x[:64], torch.bfloat16, orc.BF16)
+        d = nv.linear_fwd(dense, x, torch.bfloat16, orc.BF16)
+        ly, h = nv.lora_linear_fwd(weight, lora, x, orc.F32, expanded=True)
+        ldx, _, _ = nv.lora_linear_bwd(weight, lora, dy, x, h, orc.F32, expanded=True)
+        nv.grouped_expert_expand(gate, up, down, expanded, nv.BF16, nv.BF16)
+        out, g, u = nv.grouped_expert_fwd(gate, up, down, offsets, x, nv.BF16, expanded)
+        edx = nv.grouped_expert_bwd(gate, up, down, offsets, x, g, u, nv.BF16, expanded)
+        out2, g2, u2 = nv.grouped_expert_fwd(gate, up, down, offsets, x, nv.BF16)
+        edx2 = nv.grouped_expert_bwd(gate, up, down, offsets, x, g2, u2, nv.BF16)
+        return [y, dx, few, d, ly, h, ldx, out, g, u, edx, out2, edx2]
+
+    want = products()
+    nv.lib().caifq_set_cta_limit(limit)
+    try:
+        got = products()
+        assert nv.lib().caifq_device_status() == 0
+    finally:
+        nv.lib().caifq_set_cta_limit(0)
+    for a, b in zip(got, want):
+        assert max_rel_err(a.float().cpu().numpy(), b.float().cpu().numpy()) <= 1e-2
