@@ -290,6 +290,16 @@ std::vector<int64_t> shape_with_last(const at::Tensor &x, int64_t last)
   return s;
 }
 
+// numel // width as Python has it: a width of zero is an exception there, and the end of the process in C
+int64_t rows_of(const at::Tensor &t, int64_t width)
+{
+  if (width == 0)
+  {
+    raise(PyExc_ZeroDivisionError, "integer division or modulo by zero");
+  }
+  return t.numel() / width;
+}
+
 PyObject *wrap(at::Tensor t) { return THPVariable_Wrap(std::move(t)); }
 
 PyObject *wrap_or_none(const at::Tensor &t)
@@ -345,7 +355,7 @@ PyObject *linear(Args &a, bool backward)
   const at::ScalarType out_dtype = a.dtype();
   const int compute = static_cast<int>(a.integer());
   const at::Tensor *out = a.buffer();
-  const int64_t m = x.numel() / (backward ? w->out_dim : w->in_dim);
+  const int64_t m = rows_of(x, backward ? w->out_dim : w->in_dim);
   at::Tensor y = out != nullptr ? *out : empty(shape_with_last(x, backward ? w->in_dim : w->out_dim), out_dtype, x);
   const int xc = code_of(x), yc = code_of(y);
   void *s = stream();
@@ -367,7 +377,7 @@ PyObject *linear_fwd_residual(Args &a)
   const at::Tensor &x = *a.tensor();
   const at::Tensor &res = *a.tensor();
   const int compute = static_cast<int>(a.integer());
-  const int64_t m = x.numel() / w->in_dim;
+  const int64_t m = rows_of(x, w->in_dim);
   const int xc = code_of(x), rc = code_of(res);
   void *s = stream();
   check(unlocked([&] { return api.linear_fwd_residual(w, ptr(x), xc, m, ptr(res), rc, compute, s); }),
@@ -386,7 +396,7 @@ PyObject *linear_fwd_multi(Args &a)
   const at::ScalarType out_dtype = a.dtype();
   const int compute = static_cast<int>(a.integer());
   const at::Tensor *out = a.buffer();
-  const int64_t m = x.numel() / ws[0].in_dim;
+  const int64_t m = rows_of(x, ws[0].in_dim);
   int64_t total = 0;
   for (const caifq_weight &w : ws)
   {
@@ -422,7 +432,7 @@ PyObject *linear_concat(Args &a)
   at::Tensor work = given != nullptr ? *given
                                      : empty({static_cast<int64_t>(api.linear_concat_workspace_bytes(ws.data(), count))},
                                              at::kByte, act);
-  const int64_t m = act.numel() / (backward ? total : ws[0].in_dim);
+  const int64_t m = rows_of(act, backward ? total : ws[0].in_dim);
   at::Tensor out = empty({m, backward ? ws[0].in_dim : total}, out_dtype, act);
   const int ac = code_of(act), oc = code_of(out);
   void *s = stream();
@@ -461,7 +471,7 @@ PyObject *lora_linear_fwd(Args &a)
   const at::Tensor *hid = a.buffer();
   const at::Tensor *given = a.buffer();
   const bool expanded = a.truth();
-  const int64_t m = x.numel() / w->in_dim;
+  const int64_t m = rows_of(x, w->in_dim);
   at::Tensor y = out != nullptr ? *out : empty(shape_with_last(x, w->out_dim), x.scalar_type(), x);
   at::Tensor hidden = hid != nullptr ? *hid : empty({m, l->rank}, x.scalar_type(), x);
   const size_t need =
@@ -488,7 +498,7 @@ PyObject *lora_linear_bwd(Args &a)
   const at::Tensor *db_given = a.buffer();
   const at::Tensor *given = a.buffer();
   const bool expanded = a.truth();
-  const int64_t m = dy.numel() / w->out_dim;
+  const int64_t m = rows_of(dy, w->out_dim);
   at::Tensor dx = dx_given != nullptr ? *dx_given : empty(shape_with_last(dy, w->in_dim), dy.scalar_type(), dy);
   at::Tensor da = da_given != nullptr ? *da_given : empty_like(*la);
   at::Tensor db = db_given != nullptr ? *db_given : empty_like(*lb);
@@ -512,7 +522,7 @@ PyObject *rmsnorm_fwd(Args &a)
   const at::Tensor &gamma = *a.tensor();
   const float eps = static_cast<float>(a.real());
   const int64_t dim = x.size(-1);
-  const int64_t rows = x.numel() / dim;
+  const int64_t rows = rows_of(x, dim);
   at::Tensor y = empty_like(x);
   at::Tensor rms = empty({rows}, at::kFloat, x);
   const int xc = code_of(x);
@@ -533,7 +543,7 @@ PyObject *rmsnorm_bwd(Args &a)
   const at::Tensor &rms = *a.tensor();
   const at::Tensor *given = a.tensor(true);
   const int64_t dim = x.size(-1);
-  const int64_t rows = x.numel() / dim;
+  const int64_t rows = rows_of(x, dim);
   at::Tensor dx = empty_like(x);
   at::Tensor dg = given != nullptr ? *given : empty({dim}, at::kFloat, x).zero_();
   const int xc = code_of(x);

@@ -1,0 +1,33 @@
+"""What the Python entry points refuse, and with which exception."""
+import pytest
+import torch
+
+from caif_b200 import native as nv
+
+pytestmark = pytest.mark.gpu
+
+
+def _int8(out_dim, in_dim):
+    return nv.Weight(torch.zeros(max(1, out_dim * in_dim), dtype=torch.int8, device="cuda"), nv.I8, in_dim, out_dim,
+                     torch.ones(1, device="cuda"))
+
+
+@pytest.mark.parametrize("call", [
+    lambda x, w, l: nv.rmsnorm_fwd(x, x.float()),
+    lambda x, w, l: nv.rmsnorm_bwd(x, x, x.float(), x.float()),
+    lambda x, w, l: nv.linear_fwd(w, x),
+    lambda x, w, l: nv.linear_dx(w, x),
+    lambda x, w, l: nv.linear_fwd_residual(w, x, x),
+    lambda x, w, l: nv.linear_fwd_multi([w, w], x),
+    lambda x, w, l: nv.linear_concat([w, w], x, workspace=x),
+    lambda x, w, l: nv.linear_concat([w, w], x, backward=True, workspace=x),
+    lambda x, w, l: nv.lora_linear_fwd(w, l, x),
+    lambda x, w, l: nv.lora_linear_bwd(w, l, x, x, x),
+])
+def test_rows_of_no_elements_are_a_division_by_zero(call):
+    x = torch.empty(3, 0, dtype=torch.bfloat16, device="cuda")
+    w = _int8(0, 0)
+    lora = nv.Lora(torch.zeros(8, 0, dtype=torch.bfloat16, device="cuda"),
+                   torch.zeros(0, 8, dtype=torch.bfloat16, device="cuda"), 8.0)
+    with pytest.raises(ZeroDivisionError):
+        call(x, w, lora)
