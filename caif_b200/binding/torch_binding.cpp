@@ -290,6 +290,17 @@ std::vector<int64_t> shape_with_last(const at::Tensor &x, int64_t last)
   return s;
 }
 
+// an [rows, columns] operand: another rank would be read as one of the wrong width
+void need_matrix(const at::Tensor &t, const char *who)
+{
+  if (t.dim() != 2)
+  {
+    PyErr_Format(PyExc_ValueError, "%s: a [rows, columns] tensor expected, got %lld dimensions", who,
+                 static_cast<long long>(t.dim()));
+    throw Raised{};
+  }
+}
+
 // numel // width as Python has it: a width of zero is an exception there, and the end of the process in C
 int64_t rows_of(const at::Tensor &t, int64_t width)
 {
@@ -585,10 +596,7 @@ PyObject *quantize_int8_per_tensor(Args &a)
 PyObject *quantize_int8_per_channel(Args &a)
 {
   const at::Tensor &x = *a.tensor();
-  if (x.dim() != 2)
-  {
-    raise(PyExc_ValueError, "quantize_int8_per_channel: a [rows, cols] tensor");
-  }
+  need_matrix(x, "quantize_int8_per_channel");
   const int64_t rows = x.size(0), cols = x.size(1);
   at::Tensor q = empty(x.sizes(), at::kChar, x);
   at::Tensor scales = empty({cols}, at::kFloat, x);
@@ -631,6 +639,7 @@ PyObject *moe_topk(Args &a)
 {
   const at::Tensor &probs = *a.tensor();
   const int64_t k = a.integer();
+  need_matrix(probs, "moe_topk");
   const int64_t batch = probs.size(0), dim = probs.size(1);
   at::Tensor idx = empty({batch, k}, at::kInt, probs);
   at::Tensor val = empty({batch, k}, probs.scalar_type(), probs);
@@ -647,6 +656,7 @@ PyObject *moe_topk(Args &a)
 PyObject *moe_normalize_rows(Args &a)
 {
   const at::Tensor &x = *a.tensor();
+  need_matrix(x, "moe_normalize_rows");
   at::Tensor out = empty_like(x);
   const int xc = code_of(x);
   void *s = stream();
@@ -662,6 +672,7 @@ PyObject *moe_softmax(Args &a)
 {
   const at::Tensor &x = *a.tensor();
   const at::Tensor *bias = a.tensor(true);
+  need_matrix(x, "moe_softmax");
   at::Tensor out = empty_like(x);
   const int xc = code_of(x);
   void *s = stream();
@@ -678,6 +689,7 @@ PyObject *moe_build_dispatch(Args &a)
   const at::Tensor &idx = *a.tensor();
   const int64_t experts = a.integer();
   const int64_t capacity = a.integer();
+  need_matrix(idx, "moe_build_dispatch");
   const int64_t tokens = idx.size(0), k = idx.size(1);
   at::Tensor map = empty({tokens, k}, at::kInt, idx);
   at::Tensor offsets = empty({experts + 1}, at::kInt, idx);
@@ -700,6 +712,7 @@ PyObject *moe_dispatch(Args &a)
   const at::Tensor &map = *a.tensor();
   const at::Tensor &offs = *a.tensor();
   const int64_t total = a.integer();
+  need_matrix(x, "moe_dispatch");
   at::Tensor buf = empty({total, x.size(1)}, x.scalar_type(), x);
   const int xc = code_of(x);
   void *s = stream();
@@ -740,6 +753,7 @@ PyObject *moe_combine_bwd_grad_expert(Args &a)
   const at::Tensor &map = *a.tensor();
   const at::Tensor &offs = *a.tensor();
   const int64_t total = a.integer();
+  need_matrix(g, "moe_combine_bwd_grad_expert");
   at::Tensor buf = empty({total, g.size(1)}, g.scalar_type(), g);
   const int gc = code_of(g);
   void *s = stream();
@@ -759,6 +773,7 @@ PyObject *moe_combine_bwd_grad_weights(Args &a)
   const at::Tensor &idx = *a.tensor();
   const at::Tensor &map = *a.tensor();
   const at::Tensor &offs = *a.tensor();
+  need_matrix(g, "moe_combine_bwd_grad_weights");
   at::Tensor out = empty({g.size(0), idx.size(1)}, g.scalar_type(), g);
   const int gc = code_of(g);
   void *s = stream();
@@ -801,6 +816,7 @@ PyObject *moe_router_bwd(Args &a)
   const bool normalize = a.truth();
   const float scaling = static_cast<float>(a.real());
   const bool exact = a.truth();
+  need_matrix(probs, "moe_router_bwd");
   at::Tensor gl = empty_like(probs);
   at::Tensor gt = empty_like(gw);
   const int pc = code_of(probs);

@@ -31,3 +31,21 @@ def test_rows_of_no_elements_are_a_division_by_zero(call):
                    torch.zeros(0, 8, dtype=torch.bfloat16, device="cuda"), 8.0)
     with pytest.raises(ZeroDivisionError):
         call(x, w, lora)
+
+
+@pytest.mark.parametrize("call", [
+    lambda x, i: nv.moe_topk(x, 2),
+    lambda x, i: nv.moe_normalize_rows(x),
+    lambda x, i: nv.moe_softmax(x),
+    lambda x, i: nv.moe_build_dispatch(i, 4),
+    lambda x, i: nv.moe_dispatch(x, i[0], i[0], i[0, 0], 8),
+    lambda x, i: nv.moe_combine_bwd_grad_expert(x, i[0], x[0], i[0], i[0, 0], 8),
+    lambda x, i: nv.moe_combine_bwd_grad_weights(x, x, i[0], i[0], i[0, 0]),
+    lambda x, i: nv.moe_router_bwd(x[0], x, i[0]),
+    lambda x, i: nv.quantize_int8_per_channel(x),
+])
+def test_operands_of_another_rank_than_two_are_refused(call):
+    x = torch.rand(2, 4, 8, device="cuda")
+    idx = torch.zeros(2, 4, 2, dtype=torch.int32, device="cuda")
+    with pytest.raises(ValueError):
+        call(x, idx)
