@@ -14,6 +14,7 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <dlfcn.h>
@@ -948,9 +949,10 @@ PyObject *entry(PyObject *, PyObject *const *args, Py_ssize_t n)
   {
     return nullptr;
   }
-  catch (const std::exception &e)
+  catch (...)
   {
-    PyErr_SetString(PyExc_RuntimeError, e.what());
+    // the Python types torch's own functions raise: torch.OutOfMemoryError, IndexError, ...
+    torch::translate_exception_to_python(std::current_exception());
     return nullptr;
   }
 }

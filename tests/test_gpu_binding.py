@@ -49,3 +49,14 @@ def test_operands_of_another_rank_than_two_are_refused(call):
     idx = torch.zeros(2, 4, 2, dtype=torch.int32, device="cuda")
     with pytest.raises(ValueError):
         call(x, idx)
+
+
+def test_exceptions_are_the_ones_torch_raises():
+    x = torch.rand(2, 4, device="cuda")
+    idx = torch.zeros(2, 1, dtype=torch.int32, device="cuda")
+    with pytest.raises(torch.OutOfMemoryError):
+        nv.moe_combine(x, idx, x[:, :1].contiguous(), idx, idx.view(-1), 10 ** 12)
+    with pytest.raises(IndexError):
+        nv.rmsnorm_fwd(torch.zeros((), device="cuda"), torch.ones(1, device="cuda"))
+    with pytest.raises(IndexError):
+        nv.moe_combine(x.view(-1), idx, x, idx, idx.view(-1), 2)
