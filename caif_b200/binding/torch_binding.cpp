@@ -357,6 +357,19 @@ at::Tensor scratch(size_t bytes, const at::Tensor &like)
   }
 }
 
+// A call that is given its result allocates nothing while its stream is captured: the capture may be the caller's own, and
+// scratch from the caching allocator would be somebody else's when that graph is replayed.  (With no result given the call
+// takes that from the allocator too, so the capture must be one that torch knows of.)
+bool may_take_scratch(const at::Tensor *out, void *s)
+{
+  if (out == nullptr)
+  {
+    return true;
+  }
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(static_cast<cudaStream_t>(s), &status) == cudaSuccess && status == cudaStreamCaptureStatusNone;
+}
+
 // ---- frozen linear ------------------------------------------------------------------------------------------
 
 // (weight, act, out_dtype, compute, out | None): forward or dX
@@ -372,7 +385,7 @@ PyObject *linear(Args &a, bool backward)
   const int xc = code_of(x), yc = code_of(y);
   void *s = stream();
   const size_t need = api.linear_workspace_bytes(w, backward ? 1 : 0, xc, m, compute);
-  const at::Tensor work = need > 0 ? scratch(need, x) : at::Tensor();
+  const at::Tensor work = need > 0 && may_take_scratch(out, s) ? scratch(need, x) : at::Tensor();
   void *scratch_ptr = work.defined() ? ptr(work) : nullptr;
   auto fn = backward ? api.linear_dx_ws : api.linear_fwd_ws;
   check(unlocked([&] { return fn(w, ptr(x), xc, m, ptr(y), yc, compute, scratch_ptr, scratch_ptr ? need : 0, s); }),

@@ -1,4 +1,6 @@
 """What the Python entry points refuse, and with which exception."""
+import ctypes
+
 import pytest
 import torch
 
@@ -60,3 +62,42 @@ def test_exceptions_are_the_ones_torch_raises():
         nv.rmsnorm_fwd(torch.zeros((), device="cuda"), torch.ones(1, device="cuda"))
     with pytest.raises(IndexError):
         nv.moe_combine(x.view(-1), idx, x, idx, idx.view(-1), 2)
+
+
+def test_calls_with_their_result_allocate_nothing_under_a_capture():
+    """A graph captured without torch's knowledge: what its launches use must still be theirs when it is replayed."""
+    x = torch.randn(1025, 256, device="cuda").bfloat16()
+    w = _int8(384, 256)
+    w.codes.random_(-127, 128)
+    dy = torch.randn(1025, 384, device="cuda").bfloat16()
+    y, dx = torch.empty(1025, 384, device="cuda"), torch.empty(1025, 256, device="cuda")
+    stream = torch.cuda.Stream()
+    rt = ctypes.CDLL(None)
+    if not hasattr(rt, "cudaStreamBeginCapture"):
+        import glob
+        import os
+        rt = ctypes.CDLL((glob.glob(os.path.join(os.path.dirname(torch.__file__), "..", "nvidia", "cuda_runtime", "lib",
+                                                 "libcudart.so*")) or ["libcudart.so"])[0])
+    handle, graph, executable = ctypes.c_void_p(stream.cuda_stream), ctypes.c_void_p(), ctypes.c_void_p()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        for _ in range(2):      # (what is set up once is set up now, and the allocator has blocks to give)
+            nv.linear_fwd(w, x, torch.float32, nv.BF16, out=y)
+            nv.linear_dx(w, dy, torch.float32, nv.BF16, out=dx)
+        torch.cuda.synchronize()
+        want = y.clone(), dx.clone()
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_stats()["allocation.all.allocated"]
+        assert rt.cudaStreamBeginCapture(handle, 1) == 0
+        nv.linear_fwd(w, x, torch.float32, nv.BF16, out=y)
+        nv.linear_dx(w, dy, torch.float32, nv.BF16, out=dx)
+        assert rt.cudaStreamEndCapture(handle, ctypes.byref(graph)) == 0
+        assert torch.cuda.memory_stats()["allocation.all.allocated"] == before
+        assert rt.cudaGraphInstantiate(ctypes.byref(executable), graph, ctypes.c_ulonglong(0)) == 0
+        y.zero_()
+        dx.zero_()
+        assert rt.cudaGraphLaunch(executable, handle) == 0
+        torch.cuda.synchronize()
+        rt.cudaGraphExecDestroy(executable)
+        rt.cudaGraphDestroy(graph)
+    assert torch.equal(y, want[0]) and torch.equal(dx, want[1])
