@@ -345,21 +345,23 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
             }
             continue;
           }
-          // the place of the stage b_stages before this one: it must have been multiplied
-          if (g >= static_cast<uint32_t>(p.b_stages))
-          {
-            const uint32_t old = g - static_cast<uint32_t>(p.b_stages);
-            if (!wait(done(old), done_parity(old)))
-            {
-              return;   // nothing new is started once a wait has run out
-            }
-          }
-          if (half == 0)
-          {
-            mbar_expect_tx(b_full(s), static_cast<uint32_t>(subs * boxes) * box_bytes + (g == 0 ? p.stall_bytes : 0u));
-          }
+          // (A stage of one half is multiplied without the second thread, which must then not wait for it either: the
+          // stages may be DONE ahead of it by the time it looks, and the parity it waits for past.)
           if (half < subs)
           {
+            // the place of the stage b_stages before this one: it must have been multiplied
+            if (g >= static_cast<uint32_t>(p.b_stages))
+            {
+              const uint32_t old = g - static_cast<uint32_t>(p.b_stages);
+              if (!wait(done(old), done_parity(old)))
+              {
+                return;   // nothing new is started once a wait has run out
+              }
+            }
+            if (half == 0)
+            {
+              mbar_expect_tx(b_full(s), static_cast<uint32_t>(subs * boxes) * box_bytes + (g == 0 ? p.stall_bytes : 0u));
+            }
             const uint32_t to = b_addr(s) + static_cast<uint32_t>(half) * p.b_sub_bytes;
             for (int b = 0; b < boxes; ++b)
             {

@@ -644,6 +644,7 @@ def test_fp32_activations_on_the_tensor_core(storage, group, m, in_dim, out_dim)
 @pytest.mark.parametrize("storage,compute,group", [(orc.I8, orc.BF16, 128), (orc.I4, orc.BF16, 32), (orc.I4, orc.F32, 128)])
 @pytest.mark.parametrize("m,in_dim,out_dim", [
     (17, 128, 128),        # one stage of k
+    (17, 64, 192512),      # half a stage of k, more tiles a CTA than there are barriers for them
     (33, 320, 128),        # an odd 64 k at the end, a box of tokens with one row
     (64, 384, 19072),      # more tiles than SMs: both accumulator sets, tiles of one unit
     (128, 2048, 256),      # k over clusters of eight
