@@ -943,12 +943,11 @@ bool choose_depths(StreamParams &p, uint32_t &smem)
 }
 
 // Clusters of `size` CTAs (one per SM) that run at the same time: GPCs are not multiples of every size, and a few of their
-// SMs may be missing, so this is asked for, once per device.
+// SMs may be missing, so this is asked for, once per kernel and device.  A query that fails counts as none for its call.
 template <typename K>
-int resident_clusters(K kernel, int dev, int size)
+int resident_clusters(K kernel, std::atomic<int> &known, int size)
 {
-  static std::atomic<int> known[kMaxDevices][9];
-  int n = known[dev][size].load(std::memory_order_relaxed);
+  int n = known.load(std::memory_order_relaxed);
   if (n == 0)
   {
     cudaLaunchConfig_t cfg{};
@@ -965,9 +964,9 @@ int resident_clusters(K kernel, int dev, int size)
     if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1)
     {
       cudaGetLastError();
-      n = -1;
+      return 0;
     }
-    known[dev][size].store(n, std::memory_order_relaxed);
+    known.store(n, std::memory_order_relaxed);
   }
   return n;
 }
@@ -994,10 +993,11 @@ int launch_stream_inst(const CUtensorMap &map_b, StreamParams &p, const StreamTa
   {
     // k is split where all clusters run at once, with at least four 64-k tiles for every CTA and room for the partial tile
     // in shared memory
+    static std::atomic<int> clusters[kMaxDevices][9];   // by size; of this kernel
     const int num_kb = p.k_total / KB;
     for (int c : {8, 4, 3, 2})
     {
-      if (p.num_tiles * c <= stream_ctas() && num_kb >= 4 * c && p.num_tiles <= resident_clusters(kernel, dev, c) &&
+      if (p.num_tiles * c <= stream_ctas() && num_kb >= 4 * c && p.num_tiles <= resident_clusters(kernel, clusters[dev][c], c) &&
           p.b_sub_bytes * 4u + 32u + p.scale_bytes + 1024u <= smem)
       {
         p.splits = c;
