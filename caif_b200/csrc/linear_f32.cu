@@ -68,13 +68,14 @@ __device__ __forceinline__ void f32_ldmatrix_trans(uint32_t (&r)[4], uint32_t ad
 }
 
 // Two fp32 values -> three bf16x2 terms whose sum they are: the upper halves of the value, of what that leaves, and of
-// what that leaves (which has eight bits or fewer).  An infinity or NaN is its own first term.
+// what that leaves (which has eight bits or fewer).  An infinity is its own first term; a NaN is one in the second at least
+// (one whose payload lies in the lower half has the upper half of an infinity).
 __device__ __forceinline__ void f32_split(float a, float b, uint32_t &hi, uint32_t &mid, uint32_t &lo)
 {
   auto rest = [](float v)
   {
     const float r = v - __uint_as_float(__float_as_uint(v) & 0xFFFF0000u);
-    return fabsf(v) <= 3.402823466e38f ? r : 0.0f;
+    return fabsf(v) == __int_as_float(0x7F800000) ? 0.0f : r;   // (NaN - x: NaN)
   };
   auto upper = [](float x, float y) { return __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632); };
   hi = upper(a, b);

@@ -641,6 +641,27 @@ def test_fp32_activations_on_the_tensor_core(storage, group, m, in_dim, out_dim)
     assert torch.equal(nv.linear_fwd_residual(weight, x, res.clone()), y + res)
 
 
+@pytest.mark.parametrize("bits", [0x7FC00000, 0x7F800001, 0xFF80FFFF, 0x7F800000, 0xFF800000])
+def test_fp32_activations_that_are_not_finite(bits, monkeypatch):
+    """A NaN of any payload stays one; an infinity gives what the fp32-FMA kernel gives; other rows keep their bits."""
+    rng = np.random.default_rng(99)
+    weight, codes, scales = make_weight(rng, 192, 128, orc.I8)
+    for f, width in ((nv.linear_fwd, 128), (nv.linear_dx, 192)):
+        x = torch.randn(5, width, device="cuda")
+        clean = f(weight, x)
+        x.view(torch.int32)[2, 9] = bits - (1 << 32) if bits >= 1 << 31 else bits
+        y = f(weight, x)
+        assert nv.last_path() == "umma"
+        monkeypatch.setenv("CAIFQ_FORCE_PATH", "generic")
+        want = f(weight, x)
+        monkeypatch.delenv("CAIFQ_FORCE_PATH")
+        rest = [0, 1, 3, 4]
+        assert torch.equal(y[rest], clean[rest])
+        assert torch.equal(torch.isnan(y[2]), torch.isnan(want[2]))
+        live = ~torch.isnan(want[2])
+        assert torch.equal(y[2][live], want[2][live])
+
+
 @pytest.mark.parametrize("storage,compute,group", [(orc.I8, orc.BF16, 128), (orc.I4, orc.BF16, 32), (orc.I4, orc.F32, 128)])
 @pytest.mark.parametrize("m,in_dim,out_dim", [
     (17, 128, 128),        # one stage of k
