@@ -336,6 +336,8 @@ bool fused_lora_ok(const caifq_weight *w, const caifq_lora *l, const void *act, 
   return umma_supported(probe);
 }
 
+inline bool aligned_to(const void *p, uintptr_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; }
+
 // Many-token calls may expand the weight once per call into a bf16 matrix in the caller's workspace and feed
 // it to the tensor core with plain tile copies on CTA pairs (1.43-1.55 PFLOP/s per launch at 4096 x 4096,
 // 8192 tokens) instead of converting every tile again in the dequant warps of every CTA (1.1-1.3): the
@@ -779,8 +781,9 @@ int lora_fwd_impl(const caifq_weight *w, const caifq_lora *lora, const void *x, 
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const int sd = lora->dtype;
   const float scale = lora->alpha / static_cast<float>(lora->rank);
-  if (workspace != nullptr && fused_lora_ok(w, lora, x, m, compute_dtype) &&
-      (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0)
+  // (the thin product reads rows of A sixteen bytes at a time and writes pairs of H)
+  if (workspace != nullptr && fused_lora_ok(w, lora, x, m, compute_dtype) && aligned_to(workspace, 256) &&
+      aligned_to(lora->a, 16) && aligned_to(hidden, 4))
   {
     // hidden = x . A^T (bf16), Hs = hidden * (alpha/r) / epilogue scale, padded to 64 columns;
     // then one tensor-core launch computes x . W^T and Hs . Bp^T into the same accumulators.
@@ -893,7 +896,9 @@ int lora_bwd_impl(const caifq_weight *w, const caifq_lora *lora, const void *dy,
   char *wbase = static_cast<char *>(workspace);
   void *d_hidden = wbase + ws.d_hidden;
   float *scratch = reinterpret_cast<float *>(wbase + ws.scratch);
-  if (fused_lora_ok(w, lora, dy, m, compute_dtype) && (reinterpret_cast<uintptr_t>(workspace) & 255u) == 0)
+  // (the reductions over tokens read rows of x and H sixteen bytes at a time)
+  if (fused_lora_ok(w, lora, dy, m, compute_dtype) && aligned_to(workspace, 256) && aligned_to(x, 16) &&
+      aligned_to(hidden, 16))
   {
     // dH = (scale . dy) . B through the transposed copy of B; dHs = dH / epilogue scale, padded
     const bool expand = may_expand && expand_ok(w, lora, dy, m, compute_dtype);

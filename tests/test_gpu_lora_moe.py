@@ -906,3 +906,26 @@ def test_lora_gradients_into_views_on_any_element(rank, m, expanded):
         assert max_rel_err(vb.float().cpu().numpy(), db.float().cpu().numpy()) <= 1e-2
         for flat, shift, n in ((flat_a, shift_a, n_a), (flat_b, shift_b, n_b)):
             assert torch.all(flat[:shift] == 7.0) and torch.all(flat[shift + n:] == 7.0)
+
+
+def test_lora_operands_that_start_on_any_element():
+    """x, H and the down factor as views that 16-byte loads cannot read go to the general kernels: the same values."""
+    rng = np.random.default_rng(5)
+    in_dim, out_dim, m, rank = 256, 384, 200, 16
+    weight, codes, scales, a, b, x_np, x, dy_np, dy, lora = _lora_case(rng, orc.I8, orc.BF16, in_dim, out_dim, m, rank, 32.0)
+
+    def shifted(t):
+        flat = torch.empty(t.numel() + 1, dtype=t.dtype, device="cuda")
+        flat[1:] = t.reshape(-1)
+        return flat[1:].view(t.shape)
+
+    y, h = nv.lora_linear_fwd(weight, lora, x, orc.F32, expanded=True)
+    grads = nv.lora_linear_bwd(weight, lora, dy, x, h, orc.F32, expanded=True)
+    odd = nv.Lora(shifted(lora.a), shifted(lora.b), lora.alpha)
+    for x2, h2, l2 in ((x, shifted(h), lora), (x, h, odd)):
+        y2, h3 = nv.lora_linear_fwd(weight, l2, x2, orc.F32, hidden=shifted(h) if l2 is lora else None, expanded=True)
+        assert max_rel_err(y2.float().cpu().numpy(), y.float().cpu().numpy()) <= 2e-2
+        assert max_rel_err(h3.float().cpu().numpy(), h.float().cpu().numpy()) <= 1e-2
+    for x2, h2, l2 in ((shifted(x), h, lora), (x, shifted(h), lora), (x, h, odd)):
+        for got, want in zip(nv.lora_linear_bwd(weight, l2, dy, x2, h2, orc.F32, expanded=True), grads):
+            assert max_rel_err(got.float().cpu().numpy(), want.float().cpu().numpy()) <= 2e-2
