@@ -839,7 +839,14 @@ int launch_weights_to_bf16_scaled(const caifq_weight *ws, int count, void *dst, 
     bool aligned = true;
     for (int k = i; k < i + n; ++k)
     {
-      aligned = aligned && (reinterpret_cast<uintptr_t>(ws[k].codes) & 15u) == 0;
+      const caifq_weight &w = ws[k];
+      if ((w.storage == CAIFQ_I8 && (w.scheme != CAIFQ_PER_TENSOR || w.scales == nullptr)) ||
+          (w.storage == CAIFQ_I4 && (w.scales == nullptr || w.group_size <= 0 || (w.group_size % 8) != 0)))
+      {
+        set_error("weight_to_bf16: int8 needs one per-tensor scale, int4 groups of a multiple of 8");
+        return CAIFQ_ERR_UNSUPPORTED;
+      }
+      aligned = aligned && (reinterpret_cast<uintptr_t>(w.codes) & 15u) == 0;
     }
     if (!aligned)
     {
@@ -852,14 +859,6 @@ int launch_weights_to_bf16_scaled(const caifq_weight *ws, int count, void *dst, 
     }
     else if (ws[i].storage == CAIFQ_I8)
     {
-      for (int k = i; k < i + n; ++k)
-      {
-        if (ws[k].scheme != CAIFQ_PER_TENSOR)
-        {
-          set_error("weight_to_bf16: int8 needs one per-tensor scale");
-          return CAIFQ_ERR_UNSUPPORTED;
-        }
-      }
       rc = launch_expand<EXPAND_I8_SCALED>(ws + i, n, out, s);
     }
     else

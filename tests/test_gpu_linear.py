@@ -617,6 +617,21 @@ def test_layers_over_ragged_widths_are_refused_as_one_product():
         nv.linear_concat(ws, torch.zeros(64, 256, dtype=torch.bfloat16, device="cuda"))
 
 
+@pytest.mark.parametrize("offset", [0, 8])
+def test_layers_as_one_product_take_what_one_scale_inside_the_values_can_hold(offset):
+    """Codes that start on 16 bytes or on 8: the same values, and the same refusals."""
+    codes = torch.randint(-127, 128, (offset + 128 * 256,), dtype=torch.int8, device="cuda")[offset:]
+    scales = torch.rand(128, device="cuda") * 0.01 + 0.01
+    x = torch.randn(64, 256, device="cuda").bfloat16()
+    good = nv.Weight(codes, nv.I8, 256, 128, scales[:1].contiguous())
+    want = x.double() @ (codes.view(128, 256).float() * scales[0]).bfloat16().double().T
+    y = nv.linear_concat([good, good], x, out_dtype=torch.float32)
+    assert (y.double() - torch.cat([want, want], 1)).norm() <= 1e-5 * (2 ** 0.5) * want.norm()
+    for bad in (nv.Weight(codes, nv.I8, 256, 128), nv.Weight(codes, nv.I8, 256, 128, scales, scheme=nv.PER_CHANNEL)):
+        with pytest.raises(nv.CaifqError, match="per-tensor scale"):
+            nv.linear_concat([bad, bad], x)
+
+
 @pytest.mark.parametrize("storage,group", [(orc.I8, 128), (orc.I4, 128), (orc.I4, 64)])
 @pytest.mark.parametrize("m,in_dim,out_dim", [(1, 1024, 128), (64, 1024, 1024), (65, 128, 64), (130, 64, 192), (1000, 384, 2048)])
 def test_fp32_activations_on_the_tensor_core(storage, group, m, in_dim, out_dim):
