@@ -907,6 +907,13 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap map_b, const __grid_con
 // ------------------------------------------------------------------ host side
 int stream_ctas() { return persistent_ctas("CAIFQ_UMMA_CTAS"); }
 
+// A CTA keeps a record of each of its tiles in shared memory.  With at most 1024 of them (32 KB) two places for
+// activations and the codes in flight always fit beside them; one CTA of a large layer (a host that leaves this library few
+// SMs) may have more, and is the many-token kernel's.
+constexpr int64_t kMostTilesPerCta = 1024;
+
+bool records_fit(int64_t tiles) { return tiles <= kMostTilesPerCta * stream_ctas(); }
+
 // What shares the memory of an SM: codes in flight and activation tiles.
 bool choose_depths(StreamParams &p, uint32_t &smem)
 {
@@ -1108,7 +1115,8 @@ bool stream_supported(const LinearArgs &g)
   }
   return !g.backward && g.a_dtype == CAIFQ_BF16 && g.a_prescale == 1.0f && g.m >= 17 && g.m <= kStreamMostTokens &&
          g.lora_lhs == nullptr && g.num_peers == 0 && g.num_more == 0 && is_float_dtype(g.c_dtype) &&
-         (reinterpret_cast<uintptr_t>(g.a) & 15u) == 0 && weight_streams(g.w, g.compute_dtype);
+         (reinterpret_cast<uintptr_t>(g.a) & 15u) == 0 && weight_streams(g.w, g.compute_dtype) &&
+         records_fit((g.w.out_dim / ROWS) * ((g.m + 127) / 128));
 }
 
 int launch_linear_stream(const LinearArgs &g, cudaStream_t s)
@@ -1150,6 +1158,7 @@ bool stream_grouped_supported(const GroupedStreamArgs &g)
     return false;
   }
   const caifq_weight &w0 = g.weights[0];
+  int64_t tiles = 0;
   for (int e = 0; e < g.count; ++e)
   {
     const caifq_weight &w = g.weights[e];
@@ -1158,8 +1167,9 @@ bool stream_grouped_supported(const GroupedStreamArgs &g)
     {
       return false;
     }
+    tiles += (w0.out_dim / ROWS) * ((static_cast<int64_t>(g.row_end[e]) - g.row_begin[e] + 127) / 128);
   }
-  return true;
+  return records_fit(tiles);
 }
 
 int launch_linear_stream_grouped(const GroupedStreamArgs &g, cudaStream_t s)

@@ -827,3 +827,19 @@ def test_products_under_a_limit_of_few_ctas(limit):
         nv.lib().caifq_set_cta_limit(0)
     for a, b in zip(got, want):
         assert max_rel_err(a.float().cpu().numpy(), b.float().cpu().numpy()) <= 1e-2
+
+
+def test_a_wide_layer_on_one_cta():
+    """More tiles than a CTA can keep records of go to the kernel that needs none."""
+    out_dim, in_dim, m = 128 * 4800, 64, 17
+    codes = torch.randint(-127, 128, (out_dim, in_dim), dtype=torch.int8, device="cuda")
+    weight = nv.Weight(codes, nv.I8, in_dim, out_dim, torch.full((1,), 0.01, device="cuda"))
+    x = torch.randn(m, in_dim, device="cuda").bfloat16()
+    want = nv.linear_fwd(weight, x, torch.bfloat16, orc.BF16)
+    nv.lib().caifq_set_cta_limit(1)
+    try:
+        got = nv.linear_fwd(weight, x, torch.bfloat16, orc.BF16)
+        assert nv.lib().caifq_device_status() == 0
+    finally:
+        nv.lib().caifq_set_cta_limit(0)
+    assert torch.equal(got, want)
