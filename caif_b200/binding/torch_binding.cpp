@@ -151,9 +151,14 @@ public:
     return &THPVariable_Unpack(o);
   }
 
+  // None: torch's default, as in torch.empty
   at::ScalarType dtype()
   {
     PyObject *o = next();
+    if (o == Py_None)
+    {
+      return c10::get_default_dtype_as_scalartype();
+    }
     if (!THPDtype_Check(o))
     {
       raise(PyExc_TypeError, "expected a torch.dtype");

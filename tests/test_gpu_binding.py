@@ -101,3 +101,16 @@ def test_calls_with_their_result_allocate_nothing_under_a_capture():
         rt.cudaGraphExecDestroy(executable)
         rt.cudaGraphDestroy(graph)
     assert torch.equal(y, want[0]) and torch.equal(dx, want[1])
+
+
+def test_no_output_type_is_the_default_one():
+    w = _int8(128, 64)
+    w.codes.random_(-127, 128)
+    x = torch.randn(4, 64, device="cuda").bfloat16()
+    want = nv.linear_fwd(w, x)
+    assert want.dtype == torch.float32
+    assert torch.equal(nv.linear_fwd(w, x, None), want)
+    out = torch.empty(4, 128, dtype=torch.bfloat16, device="cuda")
+    assert nv.linear_fwd(w, x, None, out=out) is out and torch.equal(out, want.bfloat16())
+    assert nv.linear_dx(w, want.bfloat16(), out_dtype=None).dtype == torch.float32
+    assert nv.linear_fwd_multi([w, w], x, None).dtype == torch.float32
