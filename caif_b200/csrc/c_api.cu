@@ -341,9 +341,10 @@ inline bool aligned_to(const void *p, uintptr_t bytes) { return (reinterpret_cas
 // Many-token calls may expand the weight once per call into a bf16 matrix in the caller's workspace and feed
 // it to the tensor core with plain tile copies on CTA pairs (1.43-1.55 PFLOP/s per launch at 4096 x 4096,
 // 8192 tokens) instead of converting every tile again in the dequant warps of every CTA (1.1-1.3): the
-// conversion is then done once per weight, not once per weight and 256 rows of tokens.  The expansion takes 2.5 bytes
-// of HBM a weight (4096 x 4096: 7 us), the in-kernel conversion at least 40 us at any number of tokens, so it pays
-// from half a tile of tokens on.  int4 needs bf16 compute (fp32 compute keeps the two-term form).
+// conversion is then done once per weight, not once per weight and 256 rows of tokens.  This says whether a call of m
+// rows may; it is monotone in m, so that a workspace sized for the most rows serves fewer.  Whether it does is
+// umma_expansion_pays.  (17 to 127 rows, one tile too, have not been compared: they convert.)  int4 needs bf16 compute
+// (fp32 compute keeps the two-term form).
 bool expand_ok(const caifq_weight *w, const caifq_lora *l, const void *act, int64_t m, int compute_dtype)
 {
   if (m < 128 || !fused_lora_ok(w, l, act, m, compute_dtype))
@@ -357,11 +358,18 @@ bool expand_ok(const caifq_weight *w, const caifq_lora *l, const void *act, int6
   return true;
 }
 
-// A plain product (no adapter) that expands its weight into the caller's workspace first.  The conversion inside the
-// tensor-core kernels is repeated for every 256 tokens and bounds them from about 700 tokens on; the expansion costs 2.5
-// bytes of HBM a weight once (4096 x 14336 int4: 22 us).  Forward calls of up to kStreamMostTokens tokens are the
-// streaming kernel's.  dX has no such kernel: the expansion pays from half a tile of tokens on (4096 x 14336, 256 rows:
-// 103 us converting in the kernel, 27 + 55 expanded).  int4 with fp32 compute keeps its two operand terms.
+bool expansion_pays(const caifq_weight *w, bool backward, int64_t m)
+{
+  LinearArgs probe{};
+  probe.w = *w;
+  probe.m = m;
+  probe.backward = backward;
+  return umma_expansion_pays(probe);
+}
+
+// A plain product (no adapter) that expands its weight into the caller's workspace first: dX from half a tile of tokens on,
+// forward calls above the streaming kernel's range (up to kStreamMostTokens), where umma_expansion_pays.  int4 with fp32
+// compute keeps its two operand terms.
 bool expand_linear_ok(const caifq_weight *w, bool backward, const void *a, int a_dtype, int64_t m, const void *c,
                       int c_dtype, int compute_dtype)
 {
@@ -380,7 +388,7 @@ bool expand_linear_ok(const caifq_weight *w, bool backward, const void *a, int a
   probe.c_dtype = c_dtype;
   probe.compute_dtype = compute_dtype;
   probe.backward = backward;
-  return umma_supported(probe) && !stream_supported(probe);
+  return umma_supported(probe) && !stream_supported(probe) && umma_expansion_pays(probe);
 }
 
 size_t expanded_weight_bytes(const caifq_weight *w)
@@ -789,7 +797,7 @@ int lora_fwd_impl(const caifq_weight *w, const caifq_lora *lora, const void *x, 
     // then one tensor-core launch computes x . W^T and Hs . Bp^T into the same accumulators.
     const LoraFwdWs ws = lora_fwd_ws(w, m);
     char *base = static_cast<char *>(workspace);
-    const bool expand = may_expand && expand_ok(w, lora, x, m, compute_dtype);
+    const bool expand = may_expand && expand_ok(w, lora, x, m, compute_dtype) && expansion_pays(w, false, m);
     void *wb = base + ws.total;   // (expanded calls) the weight as a bf16 matrix behind the other scratch
     // the padded B factor, and with it the expansion of the weight where the call expands: one launch
     int r = launch_expand_prepare(*w, expand ? wb : nullptr, lora->a, lora->b, base + ws.bp, nullptr, nullptr, nullptr, 0,
@@ -901,7 +909,7 @@ int lora_bwd_impl(const caifq_weight *w, const caifq_lora *lora, const void *dy,
       aligned_to(hidden, 16))
   {
     // dH = (scale . dy) . B through the transposed copy of B; dHs = dH / epilogue scale, padded
-    const bool expand = may_expand && expand_ok(w, lora, dy, m, compute_dtype);
+    const bool expand = may_expand && expand_ok(w, lora, dy, m, compute_dtype) && expansion_pays(w, true, m);
     void *wb = wbase + ws.total;
     // transposed B, padded A, zeros for the gradients' sums and the expansion of the weight in one launch
     const int64_t n_b = static_cast<int64_t>(w->out_dim) * lora->rank;

@@ -512,6 +512,7 @@ bool take_umma_stall();   // self-test hook of the tensor-core kernels' waits
 
 // tcgen05 / TMEM tensor-core kernel for many tokens
 bool umma_supported(const LinearArgs &args);
+bool umma_expansion_pays(const LinearArgs &args);   // of a product that may expand its int8 / int4 weight first
 int launch_linear_umma(const LinearArgs &args, cudaStream_t s);
 
 }  // namespace caifq

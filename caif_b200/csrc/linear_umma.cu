@@ -1340,17 +1340,24 @@ namespace
 // has tiles, and a last wave of a few tiles costs as much as a full one: 8 x 56 tiles of 256 are 6.05 waves of 74 pairs,
 // 8 x 64 tiles of 224 are 6.92 (2047 tokens of 4096 -> 14336: 165 and 153 us).  A wave's time is near linear in the width
 // with a constant that is the copies' (measured per wave: 15.6 us at 128 columns, 17.0 at 160, 18.4 at 192, 21.9 at 224,
-// 23.5 at 256); few tiles (1 wave at any width) so take the narrowest.
+// 23.5 at 256; k = 4096, so at other k the constant is the same share of a wave's copies, not of its start); few tiles (1
+// wave at any width) so take the narrowest.  The grouped launches keep 256.
+constexpr int kWaveConstant = 120;   // columns
+
+int64_t pair_cost(int m_tiles, int n_total, int pairs, int bn)
+{
+  const int64_t tiles = static_cast<int64_t>(m_tiles) * ((n_total + bn - 1) / bn);
+  return (tiles + pairs - 1) / pairs * (bn + kWaveConstant);
+}
+
 int choose_pair_width(int m_tiles, int n_total, int pairs)
 {
-  constexpr int kWaveConstant = 120;   // columns
   const int widest = n_total < 256 ? (n_total + 31) & ~31 : 256;
   int best = 0;
   int64_t best_cost = 0;
   for (int bn = widest; bn >= 64; bn -= 32)
   {
-    const int64_t tiles = static_cast<int64_t>(m_tiles) * ((n_total + bn - 1) / bn);
-    const int64_t cost = (tiles + pairs - 1) / pairs * (bn + kWaveConstant);
+    const int64_t cost = pair_cost(m_tiles, n_total, pairs, bn);
     if (best == 0 || cost < best_cost)
     {
       best = bn;
@@ -1411,6 +1418,32 @@ bool umma_supported(const LinearArgs &g)
     default:
       return false;
   }
+}
+
+// Whether a product of an int8 / int4 weight that may expand it first gains by that.  Both forms take time in proportion to
+// k, so k does not enter.  Converting in the kernel takes 9.2 ns a k and wave of 128-wide tiles (int8 8.0 to 9.5); the
+// expansion 0.43 ps a weight (int8 0.56) and the product on it 4.1 ns a k and wave of 128-wide tiles on pairs.  So it does
+// not pay where the tiles are one wave of the SMs and two of the pairs.  us, converting / expanded, int4 and int8:
+//   14336 columns, k 4096: 128 rows 39 / 61 and 34 / 60, 256 rows 41 / 60 and 35 / 60, 512 rows 74 / 74 and 65 / 74
+//   4096 columns, k 4096: 128 rows 37 / 27 and 32 / 26, 512 rows 38 / 27 and 34 / 27
+//   4096 columns, k 14336: 128 rows 117 / 85 and 95 / 84; with an adapter, 1024 rows, k 4096: 51 / 45 and 49 / 43
+// Where the converting form takes 256-wide tiles (more tokens) it never won by more than a few percent.
+bool umma_expansion_pays(const LinearArgs &g)
+{
+  const int pairs = pair_count_umma();
+  const int n_total = g.backward ? g.w.in_dim : g.w.out_dim;
+  const int m_tiles = static_cast<int>((g.m + BM - 1) / BM);
+  if (!pairs_enabled(W_BF16) ||
+      ((n_total % 256) == 0 && static_cast<int64_t>(m_tiles) * (n_total / 256) >= sm_count_umma()))
+  {
+    return true;
+  }
+  const bool i8 = g.w.storage == CAIFQ_I8;
+  const int64_t tiles = static_cast<int64_t>(m_tiles) * ((n_total + 127) / 128);
+  const double converting = 9.2 * static_cast<double>((tiles + sm_count_umma() - 1) / sm_count_umma());
+  const int bn = choose_pair_width(m_tiles, n_total, pairs);
+  const double product = 4.1 * static_cast<double>(pair_cost(m_tiles, n_total, pairs, bn)) / (128 + kWaveConstant);
+  return (i8 ? 0.56e-3 : 0.43e-3) * n_total + product < converting;
 }
 
 int launch_linear_umma(const LinearArgs &g, cudaStream_t s)

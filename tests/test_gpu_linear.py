@@ -843,3 +843,31 @@ def test_a_wide_layer_on_one_cta():
     finally:
         nv.lib().caifq_set_cta_limit(0)
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("storage", [orc.I8, orc.I4])
+def test_wide_outputs_of_few_hundred_rows_convert_in_the_kernel(storage):
+    """One wave of tiles converts in place; more rows expand.  With an adapter the workspace is that of the largest call."""
+    rng = np.random.default_rng(8)
+    compute = orc.BF16
+    weight, codes, scales = make_weight(rng, 256, 14336, storage)         # dX has 14336 columns
+    turned, tcodes, tscales = make_weight(rng, 14336, 256, storage)       # so has this forward product
+    dense = torch.from_numpy(_oracle_w(weight, codes, scales, compute)).double().cuda()
+    tdense = torch.from_numpy(_oracle_w(turned, tcodes, tscales, compute)).double().cuda()
+    need = nv.lib().caifq_linear_workspace_bytes
+    for m in (128, 256):
+        assert need(weight.ref(), 1, nv.BF16, m, compute) == 0
+    assert need(weight.ref(), 1, nv.BF16, 1024, compute) > 0
+    assert need(turned.ref(), 1, nv.BF16, 128, compute) > 0               # (256 columns)
+    lora = nv.Lora(torch.randn(16, 256, device="cuda").bfloat16() / 16, torch.randn(14336, 16, device="cuda").bfloat16() / 64, 16.0)
+    small = nv.lora_fwd_workspace_bytes(turned, lora, 128, compute, True)
+    assert small <= nv.lora_fwd_workspace_bytes(turned, lora, 256, compute, True) <= nv.lora_fwd_workspace_bytes(
+        turned, lora, 1024, compute, True)
+    for m in (128, 256, 257, 1024):
+        dy = torch.randn(m, 256, device="cuda").bfloat16()
+        want = dy.double() @ dense
+        dx = nv.linear_dx(weight, dy, torch.float32, compute)
+        assert (dx.double() - want).norm() <= 4e-3 * want.norm()
+        want = dy.double() @ tdense.T + (dy.double() @ lora.a.double().T) @ lora.b.double().T
+        y, _ = nv.lora_linear_fwd(turned, lora, dy, compute, expanded=True)
+        assert (y.double() - want).norm() <= 1e-2 * want.norm()
