@@ -649,7 +649,7 @@ def bench_c2(ctx):
     roofline = {"bound": "hbm", "achieved": achieved, "peak": ctx.peaks["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / ctx.peaks["hbm_gbs"],
                 "traffic": ctx.traffic.get("linear_decode_kernel_c2") if world == 1 else None,
-                "peak_source": ctx.peaks["source"], "kernel": "linear_decode_kernel<4,*,2>",
+                "peak_source": ctx.peaks["source"], "kernel": "linear_decode_kernel<16,4,*,2,2>",
                 "note": "algorithmic bytes per launch (mean of M=1,4,16) over the average launch duration in the "
                         "timed region (CUDA events around the step / 768 launches; includes inter-launch gaps)"}
 

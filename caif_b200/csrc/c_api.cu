@@ -1059,9 +1059,9 @@ int caifq_lora_linear_bwd_noalloc(const caifq_weight *w, const caifq_lora *lora,
     }
     scratch = g_noalloc_ptr[dev];
   }
-  // Nothing in the buffer is assumed: the token reductions clear their fp32
-  // accumulator with a memset on `stream` before every use, and dH is fully
-  // overwritten before it is read.
+  // Nothing in the buffer is assumed.  The fp32 sums of the token reductions are zeroed on `stream` before every use
+  // (fused path: dB's by the launch that prepares the factors, dA's, in the same place, by a memset after dB has been
+  // rounded; general path: a memset each), and dH is fully overwritten before it is read.
   return caifq_lora_linear_bwd(w, lora, dy, x, hidden, m, dx, d_a, d_b, scratch, compute_dtype, stream);
 }
 
@@ -1180,7 +1180,7 @@ int concat_run(const caifq_weight *ws, int32_t count, bool backward, const void 
   probe.compute_dtype = compute_dtype;
   if (!umma_supported(probe))
   {
-    set_error("%s: needs the tensor-core path (bf16 activations, at least 32 rows, aligned buffers); call the layers "
+    set_error("%s: needs the tensor-core path (bf16 activations, at least 17 rows, widths of 128, aligned buffers); call the layers "
               "one by one, or caifq_linear_fwd_multi for up to 16 rows",
               who);
     return CAIFQ_ERR_UNSUPPORTED;

@@ -10,8 +10,8 @@
 // Here the roles are swapped: 128 weight rows are the M of the MMA and the tokens its N, 16 to 256 in steps of 16.  The
 // converted weight goes to tensor memory as the A operand, which leaves shared memory's bandwidth to the codes and the
 // activations (256 tokens: 50 us with A in shared memory, 40 with it here).
-// 4096 -> 14336 int4, us a call, many-token kernel / this one: 17 tokens 42 / 20, 96 tokens 42 / 22, 256 tokens 44 / 30,
-// 512 tokens 79 / 55; 4096 -> 4096: 38 / 11, 38 / 13, 41 / 19, 41 / 27; 64 experts of 2048 x 1408, 16 tokens top-6, three
+// 4096 -> 14336 int4, us a call, many-token kernel (converting) / this one: 17 tokens 42 / 20, 96 tokens 42 / 21, 256 tokens
+// 44 / 29, 512 tokens 79 / 52; 4096 -> 4096: 38 / 11, 38 / 13, 41 / 19, 41 / 27; 64 experts of 2048 x 1408, 16 tokens top-6, three
 // products: 249 / 121.
 //
 // One persistent CTA per SM, 19 warps, over tiles of 128 weight rows x up to 256 tokens:
@@ -75,8 +75,10 @@ constexpr int DONE = 8;                     // ring of "stage multiplied" barrie
 constexpr int TMEM_COLUMNS = 512;
 constexpr uint32_t SMEM_LIMIT = 226u * 1024u;
 constexpr uint32_t SCALES_LIMIT = 40u * 1024u;   // more would cost the activations their places
-// Most tokens for which a tile's conversion, repeated for every 256 tokens, is not yet more than the many-token kernel's,
-// repeated for every 256 of its rows: 768 tokens of 4096 -> 14336 take 94 us against 119, 1024 take 124 against 120.
+// Three tiles of tokens.  Set when 768 tokens of 4096 -> 14336 took 94 us and 1024 took 124, the many-token kernel 119 and
+// 120; it is still ahead at the line for every layer measured.  us at 768 tokens here, at 769 expanded / converted there:
+// 4096 -> 14336 int4 78, 108 / 111; 14336 -> 4096 84, 107 / 118; 4096 -> 4096 29, 38 / 39; int8 79, 110 / 127; 85, 104 / 116;
+// 29, 37 / 38.
 constexpr int kStreamMostTokens = 768;
 
 struct StreamEntry

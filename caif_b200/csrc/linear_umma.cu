@@ -17,9 +17,13 @@
 //   warp 1      TMEM allocation, MMA issue (one elected lane)
 //   warps 2-5   epilogue: TMEM -> registers -> scale -> global
 //   warps 6-13  dequantization of the weight tile
-// Tile 256 (two 128-row MMAs that share one dequantized weight tile) x 128 x 64,
-// four pipeline stages, two accumulator sets in TMEM (4 x 128 columns) so the
-// epilogue of one tile overlaps the main loop of the next.
+// A bf16 weight has no dequantization: warp 10 copies its tiles and warps 6-9 join
+// the epilogue.
+// Tiles of 256 rows x 128 or 256 columns x 64 k (a single CTA: two 128-row MMAs that
+// share a weight tile), or 256 rows on a CTA pair (a bf16 weight: 64 to 256 columns in
+// steps of 32), three to six pipeline stages; two accumulator sets in TMEM, so that the
+// epilogue of one tile overlaps the main loop of the next, except for a single CTA's
+// 256-wide tile, which fills TMEM.
 //
 // Forward uses the weight tile K-major (k = in is contiguous in memory);
 // backward uses the SAME codes MN-major (n = in is contiguous), so dX needs no
@@ -28,8 +32,10 @@
 // Exactness: int8 codes are exact in bf16 and the per-tensor scale multiplies
 // the fp32 accumulator in the epilogue, so with bf16 activations the products
 // are exact and the result matches an fp32 GEMM up to summation order.  int4
-// weights are scale*code rounded to bf16, the operand the reference's bf16
-// compute cell builds (dequantize to fp32, then To(bf16)).
+// weights converted here are code * bf16(scale), rounded to bf16 (fp32 compute: two
+// bf16 terms of scale * code); one that was expanded before the launch is a bf16 weight
+// of bf16(scale * code), the operand the reference's bf16 compute cell builds
+// (dequantize to fp32, then To(bf16)).
 //
 // Every wait is bounded; a wait that runs out sets a flag that the host can
 // read and lets the kernel finish (with wrong numbers) instead of hanging.
@@ -324,7 +330,7 @@ linear_umma_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   // A bf16 weight needs no dequant warps: four of them join the epilogue, so every quarter of the accumulator's
   // lanes is drained by two warps that take alternate 32-column chunks.
   constexpr int EPI_GROUPS = (WMODE == W_BF16) ? 2 : 1;
-    constexpr int DEQ_TEAMS = deq_teams(PAIR);
+  constexpr int DEQ_TEAMS = deq_teams(PAIR);
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bars[MAX_STAGES * 3 + 4];
   __shared__ uint64_t drain_bar;   // give-up path only: the MMAs issued so far have completed
@@ -1234,10 +1240,10 @@ int pair_count_umma() { return sm_count_umma() / 2; }
 // smallest number of resident pairs any pair-mode kernel reported for a device so far (0 = none launched yet)
 std::atomic<int> g_pair_capacity[kMaxDevices];
 
-// Whether 256-wide tiles go to CTA pairs or to single CTAs.  Measured on 4096 x 4096, 8192 tokens: a bf16
-// weight (operand fed by copies alone) runs 9 % faster on pairs (1211-1327 against 1109-1219 TFLOP/s); a
-// quantized weight does not (int8 980-1150 on pairs, 1026-1140 on single CTAs; int4 950-1015 against
-// 1007-1190): there the dequant warps' work per flop is the same in both forms and it, not the operand traffic,
+// Whether 256-wide tiles go to CTA pairs or to single CTAs.  Measured on 4096 x 4096, 8192 tokens, TFLOP/s: a bf16
+// weight (operand fed by copies alone) 1433-1546 on pairs, 1262-1383 on single CTAs; a
+// quantized weight is no faster on pairs (int8 992-1152 against 1133-1296, int4 974-1068 against
+// 1069-1210): there the dequant warps' work per flop is the same in both forms and it, not the operand traffic,
 // is the limit.  So pairs are the default for bf16 weights only; CAIFQ_UMMA_PAIR=1 / 0 forces them on / off.
 bool pairs_enabled(int mode)
 {
@@ -1405,7 +1411,7 @@ bool umma_supported(const LinearArgs &g)
       }
       return g.compute_dtype == CAIFQ_BF16 || g.compute_dtype == CAIFQ_F32;
     case CAIFQ_I4:
-      // bf16 compute: scale*code rounded once to bf16, the reference's value; fp32 compute: scale*code
+      // bf16 compute: code * bf16(scale), 2^-9 from the reference's bf16(scale * code); fp32 compute: scale*code
       // as two bf16 terms (2^-17 relative), within the fp32 tolerance
       if ((g.compute_dtype != CAIFQ_BF16 && g.compute_dtype != CAIFQ_F32) || w.scales == nullptr)
       {

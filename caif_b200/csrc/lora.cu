@@ -334,12 +334,12 @@ __device__ __forceinline__ void ldmatrix_x2_trans(uint32_t addr, uint32_t &r0, u
 // C[big, R] (+)= sum over a slice of tokens of (prescale . U)[m, big]^T * V[m, R]   (fp32 atomics into acc).
 // Both operands have the reduction index (the token) as their slow axis, so tiles of U and V are
 // staged in shared memory as they lie and the tensor-core fragments are read transposed
-// (ldmatrix.trans).  A CTA owns 64 columns of U, its 4 warps 16 each; gridDim.y slices the tokens.
-// With `transpose_out` the accumulator is indexed [R, big] (dA).
+// (ldmatrix.trans).  A CTA owns 128 columns of U, its 8 warps 16 each; gridDim.y slices the tokens.
+// With `transpose_out` the accumulator is indexed [R, big] (dA).  `acc` is zero before the launch.
 constexpr int TN_COLS = 128;   // 256 bytes of every row per CTA; one warp per 16 columns
 constexpr int STN_THREADS = (TN_COLS / 16) * 32;
 constexpr int TN_ROWS = 64;
-constexpr int TN_UPITCH = TN_COLS + 8;  // bf16 elements: 144-byte rows keep ldmatrix conflict-free
+constexpr int TN_UPITCH = TN_COLS + 8;  // bf16 elements: 272-byte rows keep ldmatrix conflict-free
 
 // Both gradients of an adapter are one launch: column tiles [0, tiles0) are dB's, the others dA's.
 struct SkinnyTn
@@ -627,7 +627,7 @@ int launch_skinny_tn(const void *dy, const void *h, void *db, float prescale, in
   const int64_t n = n0 + static_cast<int64_t>(in) * rank;
   const int tiles0 = (out + TN_COLS - 1) / TN_COLS;
   const int tiles = tiles0 + (in + TN_COLS - 1) / TN_COLS;
-  int64_t slices = (148 * 8 + tiles - 1) / tiles;   // ~8 CTAs of 128 threads per SM
+  int64_t slices = (148 * 8 + tiles - 1) / tiles;   // ~8 CTAs of 256 threads per SM
   const int64_t max_slices = (m + TN_ROWS - 1) / TN_ROWS;
   slices = slices > max_slices ? max_slices : slices;
   const SkinnyTn job0{static_cast<const __nv_bfloat16 *>(dy), static_cast<const __nv_bfloat16 *>(h), sums, prescale, out, 0};

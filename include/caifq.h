@@ -182,8 +182,15 @@ CAIFQ_API int caifq_linear_dx(const caifq_weight *w, const void *dy, int32_t dy_
  * The same two calls with a scratch for many tokens: with a workspace of caifq_linear_workspace_bytes(...) bytes, 256-byte
  * aligned, the weight is expanded once per call into a bf16 [out, in] matrix there (int8 codes as exact integers whose
  * scale is applied to the sum, int4 codes times their group scale, rounded once) and the tensor core reads plain tiles,
- * instead of converting every tile again for every 256 tokens.  A size of 0 means that these calls do not expand; with a
- * null or smaller workspace they are the plain calls.  The workspace is scratch: nothing in it outlives the call.
+ * instead of converting every tile again for every 256 tokens.  A size of 0 means that a call of these sizes does not
+ * expand; with a null or smaller workspace they are the plain calls.  The workspace is scratch: nothing in it outlives the
+ * call.
+ *
+ * int8 results do not depend on the form beyond the order of additions.  An int4 weight under bf16 compute enters the
+ * product as the exact code with the group scale applied to partial sums (up to 16 tokens), as code * bf16(scale) (above,
+ * where the code is converted in the kernel) or as bf16(code * scale) (expanded); the last two differ by the rounding of
+ * the scale, 2^-9 relative a weight.  So results of one layer differ within the bf16 bound between, say, 768 tokens, which
+ * are never expanded forward, and 769, which may be; between 127 and 128 in dX; and with and without a workspace.
  */
 CAIFQ_API size_t caifq_linear_workspace_bytes(const caifq_weight *w, int32_t backward, int32_t a_dtype, int64_t m,
                                               int32_t compute_dtype);
@@ -273,14 +280,14 @@ CAIFQ_API int caifq_lora_linear_bwd(const caifq_weight *w, const caifq_lora *lor
 /*
  * The same two calls for hosts that can spare a larger workspace (no counterpart in the reference, whose
  * cache_fp32 keeps an fp32 copy of every weight for good).  From 128 tokens on (bf16
- * adapter on an int8 base, or on an int4 base under bf16 compute, in_dim and out_dim multiples of 128) the
- * weight is expanded ONCE per call into a bf16 [out, in] matrix behind the other scratch -- int8 codes as
+ * adapter on an int8 base, or on an int4 base under bf16 compute, in_dim and out_dim multiples of 128), where it
+ * pays (not for a few hundred tokens into a wide output), the weight is expanded ONCE per call into a bf16 [out, in] matrix behind the other scratch -- int8 codes as
  * exact integers with the per-tensor scale left to the epilogue, int4 as bf16(scale * code), the value the
  * reference's dequantize-then-cast gives -- and the tensor core is fed from it by plain tile copies on CTA
  * pairs, instead of every CTA converting every weight tile again for each 256 rows of tokens.  Results: int8
  * bit-equal to caifq_lora_linear_fwd / _bwd; int4 the reference's own operand (closer to it than the
- * unexpanded form).  The workspace must hold caifq_lora_*_workspace_bytes_expanded(...) bytes (equal to the
- * plain size for calls that are not expanded), 256-byte aligned.
+ * unexpanded form).  The workspace must hold caifq_lora_*_workspace_bytes_expanded(...) bytes, 256-byte aligned;
+ * the size never shrinks with more tokens, so one for the largest call serves all.
  */
 CAIFQ_API size_t caifq_lora_fwd_workspace_bytes_expanded(const caifq_weight *w, const caifq_lora *lora, int64_t m,
                                                          int32_t compute_dtype);
