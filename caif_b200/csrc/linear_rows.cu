@@ -5,7 +5,7 @@
 // The float-storage cell of CAIF_DeviceFrozenLinear (src/caif_device_frozen_linear.cpp:381-524) and the router's
 // product over the experts (src/caif_device_moe_router.cpp:233-260).  Bound by reading the weight once when it is
 // large, by latency when it is small: a router of 64 x 2048 on 16 tokens ran as ONE block of the fp32-FMA kernel that
-// walked all of k (191 us, 7.7 here), by L2 for many rows (16384 tokens: 48 us, the FMA kernel 270).  Here a CTA owns
+// walked all of k (191 us, 7.7 here; alone, launched ahead of the previous kernel it costs less), by L2 for many rows (16384 tokens: 48 us, the FMA kernel 270).  Here a CTA owns
 // NT * 8 output columns and 16 rows, its eight warps split k and stream both operands from global memory straight into
 // bf16 tensor-core fragments, sixteen bytes a lane and operand (the order of k inside a fragment is the same for both,
 // which is all a dot product needs); the eight partial tiles meet in shared memory.  Products are exact in fp32 and
@@ -22,7 +22,7 @@ namespace
 {
 
 constexpr int kRowsWarps = 8;
-constexpr int kRowsUnroll = 4;   // k-steps of 32 whose loads are in flight per warp
+constexpr int kRowsChain = 4;   // k-steps of 32 in one chain of MMAs
 constexpr int64_t kRowsMost = 16 * 65535;   // rows of a launch: the grid's second dimension
 
 __device__ __forceinline__ void mma_rows(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
@@ -33,11 +33,13 @@ __device__ __forceinline__ void mma_rows(float (&c)[4], uint32_t a0, uint32_t a1
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-template <int NT>
+// CHAINS: chains whose loads are in flight at a time per warp
+template <int NT, int CHAINS>
 __global__ void __launch_bounds__(kRowsWarps * 32)
-linear_rows_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__restrict__ w, void *y, int y_dtype,
-                   int accumulate, int64_t m, int in_dim, int out_dim)
+linear_rows_kernel(const __nv_bfloat16 *x, const __nv_bfloat16 *w, void *y, int y_dtype, int accumulate, int64_t m,
+                   int in_dim, int out_dim)
 {
+  constexpr int UNROLL = kRowsChain * CHAINS;
   __shared__ float part[kRowsWarps][16][NT * 8 + 1];
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -63,39 +65,46 @@ linear_rows_kernel(const __nv_bfloat16 *__restrict__ x, const __nv_bfloat16 *__r
     sum[nt][0] = sum[nt][1] = sum[nt][2] = sum[nt][3] = 0.0f;
   }
   const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
-  for (int st = begin; st < end; st += kRowsUnroll)
+  // (launched ahead of the previous kernel's end; the operands are not __restrict__, whose loads could move ahead of the wait)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  for (int st = begin; st < end; st += UNROLL)
   {
-    uint4 xa[kRowsUnroll], xb[kRowsUnroll], wv[kRowsUnroll][NT];
+    uint4 xa[UNROLL], xb[UNROLL], wv[UNROLL][NT];
 #pragma unroll
-    for (int u = 0; u < kRowsUnroll; ++u)
+    for (int u = 0; u < UNROLL; ++u)
     {
       const bool in = st + u < end;
-      xa[u] = (in && lo_ok) ? __ldg(x_lo + (st + u) * 4) : zero4;
-      xb[u] = (in && hi_ok) ? __ldg(x_hi + (st + u) * 4) : zero4;
+      xa[u] = (in && lo_ok) ? x_lo[(st + u) * 4] : zero4;
+      xb[u] = (in && hi_ok) ? x_hi[(st + u) * 4] : zero4;
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
       {
-        wv[u][nt] = in ? __ldg(w_ptr[nt] + (st + u) * 4) : zero4;
+        wv[u][nt] = in ? w_ptr[nt][(st + u) * 4] : zero4;
       }
     }
-    float c[NT][4] = {};
 #pragma unroll
-    for (int u = 0; u < kRowsUnroll; ++u)
+    for (int ch = 0; ch < CHAINS; ++ch)
     {
+      float c[NT][4] = {};
+#pragma unroll
+      for (int u = ch * kRowsChain; u < (ch + 1) * kRowsChain; ++u)
+      {
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+        {
+          mma_rows(c[nt], xa[u].x, xb[u].x, xa[u].y, xb[u].y, wv[u][nt].x, wv[u][nt].y);
+          mma_rows(c[nt], xa[u].z, xb[u].z, xa[u].w, xb[u].w, wv[u][nt].z, wv[u][nt].w);
+        }
+      }
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
       {
-        mma_rows(c[nt], xa[u].x, xb[u].x, xa[u].y, xb[u].y, wv[u][nt].x, wv[u][nt].y);
-        mma_rows(c[nt], xa[u].z, xb[u].z, xa[u].w, xb[u].w, wv[u][nt].z, wv[u][nt].w);
-      }
-    }
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-    {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-      {
-        sum[nt][i] += c[nt][i];
+        for (int i = 0; i < 4; ++i)
+        {
+          sum[nt][i] += c[nt][i];
+        }
       }
     }
   }
@@ -151,17 +160,10 @@ int launch_linear_rows(const LinearArgs &g, cudaStream_t s)
   const int acc = g.accumulate ? 1 : 0;
   // 32 columns a CTA share the activations' loads; narrow outputs take 8, for more CTAs
   const int wide = (g.w.out_dim + 31) / 32;
-  if (wide * row_tiles >= 148)
-  {
-    linear_rows_kernel<4><<<dim3(static_cast<unsigned>(wide), row_tiles), kRowsWarps * 32, 0, s>>>(
-        x, w, g.c, g.c_dtype, acc, g.m, g.w.in_dim, g.w.out_dim);
-  }
-  else
-  {
-    linear_rows_kernel<1><<<dim3(static_cast<unsigned>((g.w.out_dim + 7) / 8), row_tiles), kRowsWarps * 32, 0, s>>>(
-        x, w, g.c, g.c_dtype, acc, g.m, g.w.in_dim, g.w.out_dim);
-  }
-  CAIFQ_CHECK_LAUNCH();
+  const bool many = wide * row_tiles >= 148;
+  const dim3 grid(static_cast<unsigned>(many ? wide : (g.w.out_dim + 7) / 8), row_tiles);
+  CAIFQ_CHECK_CUDA(launch_dependent(many ? linear_rows_kernel<4, 1> : linear_rows_kernel<1, 2>, grid, dim3(kRowsWarps * 32),
+                                    0, s, x, w, g.c, g.c_dtype, acc, g.m, g.w.in_dim, g.w.out_dim));
   return CAIFQ_OK;
 }
 

@@ -34,15 +34,25 @@ __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half(
 template <>
 __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16(v); }
 
+// The small kernels of a step follow one another: each is launched ahead of the previous one's end (launch_dependent),
+// lets the next one do the same, and reads nothing before the previous one has ended.  (Their inputs are not declared
+// __restrict__: loads that the compiler may take for invariant could move ahead of the wait.)
+__device__ __forceinline__ void after_previous_kernel()
+{
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ------------------------------------------------------------------------ top-k
 // One warp per row.  The reference lets thread 0 scan the row k times with a
 // strict '>' from index 0 against a -1e30 sentinel: the winner of each round is
 // the largest value, lowest index among equals, and (-1e30, index 0) when
 // nothing exceeds the sentinel.  The warp version keeps exactly that order.
 template <typename T>
-__global__ void topk_kernel(const T *__restrict__ input, int *__restrict__ indices, T *__restrict__ values,
+__global__ void topk_kernel(const T *input, int *indices, T *values,
                             int batch, int dim, int k)
 {
+  after_previous_kernel();
   extern __shared__ float s_rows[];
   const int warps_per_block = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5;
@@ -248,8 +258,9 @@ __global__ void route_grouped_kernel(const T *__restrict__ input, const T *__res
 // ... and a shared-memory tree (stride 128..1) adds the 256 partials.  A warp
 // reproduces that order: lane l owns partials l, l+32, ..., l+224.
 template <typename T>
-__global__ void normalize_rows_kernel(const T *__restrict__ input, T *__restrict__ output, int batch, int dim)
+__global__ void normalize_rows_kernel(const T *input, T *output, int batch, int dim)
 {
+  after_previous_kernel();
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * warps_per_block + (threadIdx.x >> 5);
@@ -321,9 +332,9 @@ __device__ __forceinline__ void softmax_absorb(float &m, float &s, float m_other
 }
 
 template <typename T>
-__global__ void router_softmax_kernel(const T *__restrict__ logits, const T *__restrict__ bias,
-                                      T *__restrict__ probs, int rows, int cols)
+__global__ void router_softmax_kernel(const T *logits, const T *bias, T *probs, int rows, int cols)
 {
+  after_previous_kernel();
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * warps_per_block + (threadIdx.x >> 5);
@@ -729,9 +740,10 @@ constexpr int kMapThreads = 1024;
 constexpr int kMapWarps = kMapThreads / 32;
 
 __global__ void __launch_bounds__(kMapThreads)
-build_dispatch_kernel(const int *__restrict__ expert_indices, int64_t total, int64_t slice, int num_experts, int capacity,
-                      int *__restrict__ dispatch_map, int *__restrict__ expert_offsets)
+build_dispatch_kernel(const int *expert_indices, int64_t total, int64_t slice, int num_experts, int capacity,
+                      int *dispatch_map, int *expert_offsets)
 {
+  after_previous_kernel();
   extern __shared__ int s_map[];
   int *running = s_map;                      // [E]
   int *warp_hist = s_map + num_experts;      // [warps][E]
@@ -756,7 +768,7 @@ build_dispatch_kernel(const int *__restrict__ expert_indices, int64_t total, int
       const int64_t n4 = begin >> 2;
       for (int64_t j = tid; j < n4; j += kMapThreads)
       {
-        const int4 v = __ldg(v4 + j);
+        const int4 v = v4[j];
         const int e[4] = {expert_of(v.x), expert_of(v.y), expert_of(v.z), expert_of(v.w)};
 #pragma unroll
         for (int k = 0; k < 4; ++k)
@@ -771,7 +783,7 @@ build_dispatch_kernel(const int *__restrict__ expert_indices, int64_t total, int
     }
     for (int64_t j = done + tid; j < begin; j += kMapThreads)
     {
-      const int e = expert_of(__ldg(expert_indices + j));
+      const int e = expert_of(expert_indices[j]);
       if (e >= 0)
       {
         atomicAdd(hist + e, 1);
@@ -867,10 +879,10 @@ build_dispatch_kernel(const int *__restrict__ expert_indices, int64_t total, int
 
 // ------------------------------------------------------------- dispatch / combine
 template <typename T>
-__global__ void moe_dispatch_kernel(const T *__restrict__ input, const int *__restrict__ expert_indices,
-                                    const int *__restrict__ dispatch_map, const int *__restrict__ expert_offsets,
-                                    T *__restrict__ buffer, int64_t assignments, int dim, int top_k)
+__global__ void moe_dispatch_kernel(const T *input, const int *expert_indices, const int *dispatch_map,
+                                    const int *expert_offsets, T *buffer, int64_t assignments, int dim, int top_k)
 {
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int64_t a = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   if (a >= assignments)
@@ -890,9 +902,22 @@ __global__ void moe_dispatch_kernel(const T *__restrict__ input, const int *__re
   {
     const uint4 *s4 = reinterpret_cast<const uint4 *>(src);
     uint4 *d4 = reinterpret_cast<uint4 *>(dst);
-    for (int i = lane; i < dim / vec; i += 32)
+    for (int i = lane; i < dim / vec; i += 4 * 32)
     {
-      d4[i] = s4[i];
+      uint4 v[4];   // (loads of a round before its stores: the compiler cannot know that they do not overlap)
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+      {
+        v[j] = i + 32 * j < dim / vec ? s4[i + 32 * j] : make_uint4(0u, 0u, 0u, 0u);
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+      {
+        if (i + 32 * j < dim / vec)
+        {
+          d4[i + 32 * j] = v[j];
+        }
+      }
     }
   }
   else
@@ -905,11 +930,11 @@ __global__ void moe_dispatch_kernel(const T *__restrict__ input, const int *__re
 }
 
 template <typename T>
-__global__ void moe_combine_kernel(const T *__restrict__ buffer, const int *__restrict__ expert_indices,
-                                   const T *__restrict__ expert_weights, const int *__restrict__ dispatch_map,
-                                   const int *__restrict__ expert_offsets, T *__restrict__ output, int num_tokens,
+__global__ void moe_combine_kernel(const T *buffer, const int *expert_indices, const T *expert_weights,
+                                   const int *dispatch_map, const int *expert_offsets, T *output, int num_tokens,
                                    int dim, int top_k)
 {
+  after_previous_kernel();
   const int64_t total = static_cast<int64_t>(num_tokens) * dim;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < total; i += stride)
@@ -934,9 +959,10 @@ __global__ void moe_combine_kernel(const T *__restrict__ buffer, const int *__re
 
 // ------------------------------------------------------------------- SwiGLU
 template <typename T>
-__global__ void swiglu_fwd_kernel(const T *__restrict__ gate, const T *__restrict__ up, T *__restrict__ hidden,
+__global__ void swiglu_fwd_kernel(const T *gate, const T *up, T *hidden,
                                   int64_t n)
 {
+  after_previous_kernel();
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
   {
@@ -1009,7 +1035,7 @@ struct Vec16
 template <typename T>
 __device__ __forceinline__ void load_vec(const T *p, float (&v)[Vec16<T>::N])
 {
-  const uint4 raw = __ldg(reinterpret_cast<const uint4 *>(p));
+  const uint4 raw = *reinterpret_cast<const uint4 *>(p);
   const T *e = reinterpret_cast<const T *>(&raw);
 #pragma unroll
   for (int i = 0; i < Vec16<T>::N; ++i)
@@ -1032,9 +1058,9 @@ __device__ __forceinline__ void store_vec(T *p, const float (&v)[Vec16<T>::N])
 }
 
 template <typename T>
-__global__ void swiglu_fwd_vec_kernel(const T *__restrict__ gate, const T *__restrict__ up, T *__restrict__ hidden,
-                                      int64_t n_vec)
+__global__ void swiglu_fwd_vec_kernel(const T *gate, const T *up, T *hidden, int64_t n_vec)
 {
+  after_previous_kernel();
   constexpr int N = Vec16<T>::N;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n_vec; i += stride)
@@ -1080,11 +1106,11 @@ __global__ void swiglu_bwd_vec_kernel(const T *__restrict__ g_hidden, const T *_
 }
 
 template <typename T>
-__global__ void moe_combine_vec_kernel(const T *__restrict__ buffer, const int *__restrict__ expert_indices,
-                                       const T *__restrict__ expert_weights, const int *__restrict__ dispatch_map,
-                                       const int *__restrict__ expert_offsets, T *__restrict__ output,
-                                       int num_tokens, int dim, int top_k)
+__global__ void moe_combine_vec_kernel(const T *buffer, const int *expert_indices, const T *expert_weights,
+                                       const int *dispatch_map, const int *expert_offsets, T *output, int num_tokens,
+                                       int dim, int top_k)
 {
+  after_previous_kernel();
   constexpr int N = Vec16<T>::N;
   const int dim_vec = dim / N;
   const int64_t total = static_cast<int64_t>(num_tokens) * dim_vec;
@@ -1378,9 +1404,9 @@ int launch_moe_topk(const void *probs, int dtype, int *indices, void *values, in
     return CAIFQ_ERR_UNSUPPORTED;
   }
   const int grid = (batch + warps - 1) / warps;
-  CAIFQ_DISPATCH_FLOAT(dtype, (topk_kernel<T><<<grid, warps * 32, smem, s>>>(
-                                  static_cast<const T *>(probs), indices, static_cast<T *>(values), batch, dim, k)));
-  CAIFQ_CHECK_LAUNCH();
+  CAIFQ_DISPATCH_FLOAT(dtype, CAIFQ_CHECK_CUDA(launch_dependent(topk_kernel<T>, dim3(grid), dim3(warps * 32), smem, s,
+                                                                static_cast<const T *>(probs), indices,
+                                                                static_cast<T *>(values), batch, dim, k)));
   return CAIFQ_OK;
 }
 
@@ -1420,9 +1446,9 @@ int launch_moe_normalize_rows(const void *input, void *output, int dtype, int ba
   }
   const int warps = 8;
   const int grid = (batch + warps - 1) / warps;
-  CAIFQ_DISPATCH_FLOAT(dtype, (normalize_rows_kernel<T><<<grid, warps * 32, 0, s>>>(
-                                  static_cast<const T *>(input), static_cast<T *>(output), batch, dim)));
-  CAIFQ_CHECK_LAUNCH();
+  CAIFQ_DISPATCH_FLOAT(dtype, CAIFQ_CHECK_CUDA(launch_dependent(normalize_rows_kernel<T>, dim3(grid), dim3(warps * 32), 0, s,
+                                                                static_cast<const T *>(input),
+                                                                static_cast<T *>(output), batch, dim)));
   return CAIFQ_OK;
 }
 
@@ -1435,10 +1461,10 @@ int launch_moe_router_softmax(const void *logits, const void *bias, void *probs,
   }
   const int warps = 8;
   const int grid = (rows + warps - 1) / warps;
-  CAIFQ_DISPATCH_FLOAT(dtype, (router_softmax_kernel<T><<<grid, warps * 32, 0, s>>>(
-                                  static_cast<const T *>(logits), static_cast<const T *>(bias),
-                                  static_cast<T *>(probs), rows, cols)));
-  CAIFQ_CHECK_LAUNCH();
+  CAIFQ_DISPATCH_FLOAT(dtype, CAIFQ_CHECK_CUDA(launch_dependent(router_softmax_kernel<T>, dim3(grid), dim3(warps * 32), 0, s,
+                                                                static_cast<const T *>(logits),
+                                                                static_cast<const T *>(bias), static_cast<T *>(probs),
+                                                                rows, cols)));
   return CAIFQ_OK;
 }
 
@@ -1530,9 +1556,9 @@ int launch_moe_build_dispatch(const int *expert_indices, int num_tokens, int top
   const int64_t per = (chunks + 147) / 148;
   const int64_t slice = (per > 0 ? per : 1) * kMapThreads;
   const int64_t ctas = (total + slice - 1) / slice;
-  build_dispatch_kernel<<<static_cast<unsigned>(ctas > 0 ? ctas : 1), kMapThreads, smem, s>>>(
-      expert_indices, total, slice, num_experts, capacity, dispatch_map, expert_offsets);
-  CAIFQ_CHECK_LAUNCH();
+  CAIFQ_CHECK_CUDA(launch_dependent(build_dispatch_kernel, dim3(static_cast<unsigned>(ctas > 0 ? ctas : 1)),
+                                    dim3(kMapThreads), smem, s, expert_indices, total, slice, num_experts, capacity,
+                                    dispatch_map, expert_offsets));
   return CAIFQ_OK;
 }
 
@@ -1545,10 +1571,10 @@ int launch_moe_dispatch(const void *input, int dtype, const int *expert_indices,
     return CAIFQ_OK;
   }
   const int64_t grid = (assignments * 32 + 255) / 256;
-  CAIFQ_DISPATCH_FLOAT(dtype, (moe_dispatch_kernel<T><<<static_cast<unsigned>(grid), 256, 0, s>>>(
-                                  static_cast<const T *>(input), expert_indices, dispatch_map, expert_offsets,
-                                  static_cast<T *>(buffer), assignments, dim, top_k)));
-  CAIFQ_CHECK_LAUNCH();
+  CAIFQ_DISPATCH_FLOAT(dtype, CAIFQ_CHECK_CUDA(launch_dependent(moe_dispatch_kernel<T>, dim3(static_cast<unsigned>(grid)),
+                                                                dim3(256), 0, s, static_cast<const T *>(input),
+                                                                expert_indices, dispatch_map, expert_offsets,
+                                                                static_cast<T *>(buffer), assignments, dim, top_k)));
   return CAIFQ_OK;
 }
 
@@ -1563,13 +1589,12 @@ int launch_moe_combine(const void *buffer, int dtype, const int *expert_indices,
   }
   const bool vec = aligned16(buffer) && aligned16(output);
   CAIFQ_DISPATCH_FLOAT(
-      dtype, (vec && (dim % Vec16<T>::N) == 0
-                  ? moe_combine_vec_kernel<T><<<ew_grid(total / Vec16<T>::N), 256, 0, s>>>(
-                        static_cast<const T *>(buffer), expert_indices, static_cast<const T *>(expert_weights),
-                        dispatch_map, expert_offsets, static_cast<T *>(output), num_tokens, dim, top_k)
-                  : moe_combine_kernel<T><<<ew_grid(total), 256, 0, s>>>(
-                        static_cast<const T *>(buffer), expert_indices, static_cast<const T *>(expert_weights),
-                        dispatch_map, expert_offsets, static_cast<T *>(output), num_tokens, dim, top_k)));
+      dtype, const bool vec16 = vec && (dim % Vec16<T>::N) == 0;
+      CAIFQ_CHECK_CUDA(launch_dependent(vec16 ? moe_combine_vec_kernel<T> : moe_combine_kernel<T>,
+                                        dim3(static_cast<unsigned>(ew_grid(vec16 ? total / Vec16<T>::N : total))), dim3(256),
+                                        0, s, static_cast<const T *>(buffer), expert_indices,
+                                        static_cast<const T *>(expert_weights), dispatch_map, expert_offsets,
+                                        static_cast<T *>(output), num_tokens, dim, top_k)));
   CAIFQ_CHECK_LAUNCH();
   return CAIFQ_OK;
 }
@@ -1644,13 +1669,12 @@ int launch_swiglu_fwd(const void *gate, const void *up, void *hidden, int dtype,
   }
   const bool vec = aligned16(gate) && aligned16(up) && aligned16(hidden);
   CAIFQ_DISPATCH_FLOAT(
-      dtype, (vec && (n % Vec16<T>::N) == 0
-                  ? swiglu_fwd_vec_kernel<T><<<ew_grid(n / Vec16<T>::N), 256, 0, s>>>(
-                        static_cast<const T *>(gate), static_cast<const T *>(up), static_cast<T *>(hidden),
-                        n / Vec16<T>::N)
-                  : swiglu_fwd_kernel<T><<<ew_grid(n), 256, 0, s>>>(static_cast<const T *>(gate),
-                                                                    static_cast<const T *>(up),
-                                                                    static_cast<T *>(hidden), n)));
+      dtype, const bool vec16 = vec && (n % Vec16<T>::N) == 0;
+      const int64_t items = vec16 ? n / Vec16<T>::N : n;
+      CAIFQ_CHECK_CUDA(launch_dependent(vec16 ? swiglu_fwd_vec_kernel<T> : swiglu_fwd_kernel<T>,
+                                        dim3(static_cast<unsigned>(ew_grid(items))), dim3(256), 0, s,
+                                        static_cast<const T *>(gate), static_cast<const T *>(up),
+                                        static_cast<T *>(hidden), items)));
   CAIFQ_CHECK_LAUNCH();
   return CAIFQ_OK;
 }

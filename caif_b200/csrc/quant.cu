@@ -542,12 +542,28 @@ __device__ __forceinline__ float cast_one<int8_t, float>(int8_t v) { return stat
 
 // Any pair goes through fp32, which is how CAIF_DeviceTensor::To composes them.
 template <typename S, typename D>
-__global__ void cast_kernel(const S *__restrict__ src, D *__restrict__ dst, int64_t n)
+__global__ void cast_kernel(const S *src, D *dst, int64_t n)
 {
+  // (launched ahead of the previous kernel's end; not __restrict__, whose loads could move ahead of the wait)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += 4 * stride)
   {
-    dst[i] = cast_one<float, D>(cast_one<S, float>(src[i]));
+    S v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+    {
+      v[j] = src[i + j * stride < n ? i + j * stride : i];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+    {
+      if (i + j * stride < n)
+      {
+        dst[i + j * stride] = cast_one<float, D>(cast_one<S, float>(v[j]));
+      }
+    }
   }
 }
 
@@ -584,16 +600,16 @@ int cast_from(const S *src, void *dst, int dst_dtype, int64_t n, cudaStream_t s)
   switch (dst_dtype)
   {
     case CAIFQ_F32:
-      cast_kernel<S, float><<<g, kBlock, 0, s>>>(src, static_cast<float *>(dst), n);
+      CAIFQ_CHECK_CUDA(launch_dependent(cast_kernel<S, float>, dim3(g), dim3(kBlock), 0, s, src, static_cast<float *>(dst), n));
       break;
     case CAIFQ_F16:
-      cast_kernel<S, __half><<<g, kBlock, 0, s>>>(src, static_cast<__half *>(dst), n);
+      CAIFQ_CHECK_CUDA(launch_dependent(cast_kernel<S, __half>, dim3(g), dim3(kBlock), 0, s, src, static_cast<__half *>(dst), n));
       break;
     case CAIFQ_BF16:
-      cast_kernel<S, __nv_bfloat16><<<g, kBlock, 0, s>>>(src, static_cast<__nv_bfloat16 *>(dst), n);
+      CAIFQ_CHECK_CUDA(launch_dependent(cast_kernel<S, __nv_bfloat16>, dim3(g), dim3(kBlock), 0, s, src, static_cast<__nv_bfloat16 *>(dst), n));
       break;
     case CAIFQ_I8:
-      cast_kernel<S, int8_t><<<g, kBlock, 0, s>>>(src, static_cast<int8_t *>(dst), n);
+      CAIFQ_CHECK_CUDA(launch_dependent(cast_kernel<S, int8_t>, dim3(g), dim3(kBlock), 0, s, src, static_cast<int8_t *>(dst), n));
       break;
     default:
       set_error("caifq_cast: unsupported destination dtype %d", dst_dtype);
