@@ -1469,6 +1469,31 @@ static bool few_rows(int num_experts, const int32_t *offsets, int dtype)
          static_cast<int64_t>(offsets[num_experts]) <= static_cast<int64_t>(kFewRowsPerExpert) * num_experts;
 }
 
+// Whether the few-token kernel, 16 rows at a time, is the faster one for these entries.  Up to 8 rows it is, for all widths
+// measured (us for the three products of an expert layer, this kernel / the streaming one, 8 rows each: int4 2944 x 1280 74 /
+// 98, 4096 x 2048 63 / 106, 1536 squared 29 / 39, 1024 x 512 40 / 39; int8 93 / 93, 78 / 103, 36 / 38, 36 / 36).  From 9 rows
+// on a second tile of tokens doubles its MMAs: int4 4096 x 2048 89 / 106, 2048 x 1408 115 / 139, but 104 / 98 and 55 / 40 where
+// k is not a multiple of what its eight warps take at a time; int8 104 / 103 at best.
+static bool few_tokens_each(const GroupedStreamArgs &g)
+{
+  int64_t live = 0;
+  int64_t passes = 0;
+  int most = 0;
+  for (int e = 0; e < g.count; ++e)
+  {
+    const int rows = g.row_end[e] - g.row_begin[e];
+    live += rows > 0 ? 1 : 0;
+    passes += (rows + 15) / 16;
+    most = rows > most ? rows : most;
+  }
+  if (most <= 8 || g.weights[0].storage != CAIFQ_I4)
+  {
+    return most <= 8;
+  }
+  const int64_t pieces = (g.weights[0].in_dim + 127) / 128;
+  return 82 * passes * ((pieces + 15) / 16 * 16) <= 100 * live * pieces;
+}
+
 // One launch per run of `sets` weight lists over the experts' rows: list i writes to outs[i].  CAIFQ_ERR_UNSUPPORTED
 // (nothing launched, no message) when the kernel does not take them.
 static int stream_experts(const caifq_weight *const *lists, void *const *outs, int sets, int num_experts,
@@ -1486,9 +1511,9 @@ static int stream_experts(const caifq_weight *const *lists, void *const *outs, i
     {
       const int n = (num_experts - first < per_run) ? (num_experts - first) : per_run;
       GroupedStreamArgs g{};
-      for (int i = 0; i < sets; ++i)
+      for (int e = 0; e < n; ++e)
       {
-        for (int e = 0; e < n; ++e)
+        for (int i = 0; i < sets; ++i)   // side by side: the products of one expert share its rows
         {
           ws[g.count] = lists[i][first + e];
           row_begin[g.count] = offsets[first + e];
@@ -1514,7 +1539,8 @@ static int stream_experts(const caifq_weight *const *lists, void *const *outs, i
         }
         continue;
       }
-      const int rc = launch_linear_stream_grouped(g, s);
+      const int rc = few_tokens_each(g) && decode_grouped_supported(g) ? launch_linear_decode_grouped(g, s)
+                                                                       : launch_linear_stream_grouped(g, s);
       if (rc != CAIFQ_OK)
       {
         return rc;

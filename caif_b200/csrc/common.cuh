@@ -508,6 +508,8 @@ bool stream_supported(const LinearArgs &args);
 int launch_linear_stream(const LinearArgs &args, cudaStream_t s);
 bool stream_grouped_supported(const GroupedStreamArgs &args);
 int launch_linear_stream_grouped(const GroupedStreamArgs &args, cudaStream_t s);
+bool decode_grouped_supported(const GroupedStreamArgs &args);
+int launch_linear_decode_grouped(const GroupedStreamArgs &args, cudaStream_t s);
 bool take_umma_stall();   // self-test hook of the tensor-core kernels' waits
 
 // tcgen05 / TMEM tensor-core kernel for many tokens

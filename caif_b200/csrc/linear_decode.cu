@@ -25,6 +25,11 @@
 //   * each warp parks its partial sums of every tile (live tokens only) in shared
 //     memory, and one pass at the end adds the warps' partials of each output in a
 //     fixed order; consecutive lanes store consecutive rows of a token.
+// Experts that see up to 16 rows each are the same product over a table of code matrices (the expert loop,
+// src/caif_device_moe_layer.cpp:534-557): two CTAs of eight warps an SM, each with hundreds of weight rows; a round of
+// tiles ends with its expert, and the next one's activations are awaited while the other CTA works.  Bound by the
+// conversion and by the rounds' ends: 64 experts of 2048 x 1408 int4, 16 tokens top-6, three products 65 us (the
+// streaming kernel 113, HBM 34).
 // Codes and activations are exact in bf16 and products accumulate in fp32, so
 // the result matches an fp32 GEMM on the dequantized weight up to summation
 // order.  The summation order of an output does not depend on which CTA owns
@@ -142,6 +147,21 @@ __device__ __forceinline__ void cp_async_wait()
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// 32 bytes: a whole sector a lane (a lane's pieces of int4 codes have 64 bytes of x; every CTA reads all of x from L2, and
+// that phase is 2 of a launch's 11 us: 4096 -> 4096, 16 tokens 8.8 -> 8.1 us, 14336 -> 4096 23.6 -> 21.9)
+__device__ __forceinline__ void ldg256(const void *p, bool live, uint32_t *r)
+{
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.u32 q, %9, 0;\n\t"
+      "mov.b32 %0, 0;\n\tmov.b32 %1, 0;\n\tmov.b32 %2, 0;\n\tmov.b32 %3, 0;\n\t"
+      "mov.b32 %4, 0;\n\tmov.b32 %5, 0;\n\tmov.b32 %6, 0;\n\tmov.b32 %7, 0;\n\t"
+      "@q ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n\t}"
+      : "=&r"(r[0]), "=&r"(r[1]), "=&r"(r[2]), "=&r"(r[3]), "=&r"(r[4]), "=&r"(r[5]), "=&r"(r[6]), "=&r"(r[7])
+      : "l"(p), "r"(live ? 1u : 0u)
+      : "memory");
+}
+
 // activations are the previous kernel's output: never moved ahead of the wait on that kernel; zeros where not `live`
 __device__ __forceinline__ void ldg128(const void *p, bool live, uint32_t &a, uint32_t &b, uint32_t &c, uint32_t &d)
 {
@@ -236,8 +256,28 @@ struct DecodeParams
   uint32_t scale_bytes;   // int4: one buffer of them (round_tiles tiles); two buffers when there are several rounds
   uint32_t park_offset;   // byte offset of the parked partial sums
   uint32_t row_bytes;     // packed bytes per weight row
+  int entry_tiles;        // experts: tiles of one of them (out_dim: the rows of all of them)
   uint32_t spin_limit;    // polls of one wait before it gives up
   uint32_t stall_bytes;   // self-test only: bytes the first wait announces but never receives
+};
+
+// Experts: the same product for entries of one shape, each with its own codes and up to 16 rows of x.  Their weight rows
+// lie end to end; out_dim is a multiple of 16, so a tile has one entry.
+struct DecodeEntry
+{
+  const uint8_t *codes;
+  const void *scales;
+  void *c;               // [.., out_dim]; row 0 is packed row 0
+  int row0;              // first packed row
+  int rows;
+};
+
+constexpr int MAX_ENTRIES = 256;
+
+template <int N>
+struct DecodeTable
+{
+  DecodeEntry e[N];
 };
 
 // int4 codes are turned into the bf16 integers 24 + q (q in [-8,7]): the nibble, flipped to offset binary, is dropped
@@ -272,18 +312,12 @@ __device__ __forceinline__ uint32_t park_swizzle(int row, int tokp)
 // An output as a plain fp32 sum of products: for tokens with an infinity or NaN, and where sums overflow only before the
 // scale.  (Called without inlining it cost the 16-token forms 1.3 to 3 us a launch, registers being spilled around it.)
 template <int BITS>
-__device__ __forceinline__ float plain_sum(const DecodeParams &p, int row, int token)
+__device__ __forceinline__ float plain_sum(const DecodeParams &p, const uint8_t *codes, const void *scales, int row,
+                                           const __nv_bfloat16 *x)
 {
-  int sg = 0;
-  while (sg + 1 < p.num_seg && row >= p.seg_row0[sg + 1])
-  {
-    ++sg;
-  }
-  row -= p.seg_row0[sg];
-  const uint8_t *codes = p.codes[sg] + static_cast<size_t>(row) * p.row_bytes;
-  const __half *group_scales = static_cast<const __half *>(p.scales[sg]) + static_cast<size_t>(row) * p.groups_per_row;
-  const float tensor_scale = (BITS == 8 && p.scales[sg] != nullptr) ? *static_cast<const float *>(p.scales[sg]) : 1.0f;
-  const __nv_bfloat16 *x = p.x + static_cast<size_t>(token) * p.in_dim;
+  codes += static_cast<size_t>(row) * p.row_bytes;
+  const __half *group_scales = static_cast<const __half *>(scales) + static_cast<size_t>(row) * p.groups_per_row;
+  const float tensor_scale = (BITS == 8 && scales != nullptr) ? *static_cast<const float *>(scales) : 1.0f;
   float sum = 0.0f;
 #pragma unroll 1
   for (int k = 0; k < p.in_dim; ++k)
@@ -295,9 +329,13 @@ __device__ __forceinline__ float plain_sum(const DecodeParams &p, int row, int t
   return sum;
 }
 
-template <int WARPS, int BITS, int MT, int NCH, int PCH>
-__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_kernel(const __grid_constant__ DecodeParams p)
+// N: entries of the table (experts), or 1: layers that share their input, which the parameters describe
+template <int WARPS, int BITS, int MT, int NCH, int PCH, int N>
+__global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1)
+linear_decode_kernel(const __grid_constant__ DecodeParams p, const __grid_constant__ DecodeTable<N> table)
 {
+  constexpr bool EXPERTS = N > 1;
+  constexpr int QUANTUM = EXPERTS ? kTileRows : kRowQuantum;
   typedef DecodeCfg<WARPS, BITS, MT, NCH, PCH> Cfg;
   constexpr int ELEMS = 128 / BITS;      // codes per 16-byte load: 32 or 16
   constexpr int CHUNK_K = 4 * ELEMS;     // k covered by a quad of lanes: 128 or 64
@@ -317,16 +355,39 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
 
   const int q_begin = static_cast<int>((static_cast<int64_t>(blockIdx.x) * p.num_quanta) / gridDim.x);
   const int q_end = static_cast<int>((static_cast<int64_t>(blockIdx.x + 1) * p.num_quanta) / gridDim.x);
-  const int row_begin = q_begin * kRowQuantum;
-  const int row_end = min(q_end * kRowQuantum, p.out_dim);
+  const int row_begin = q_begin * QUANTUM;
+  const int row_end = min(q_end * QUANTUM, p.out_dim);
   const int my_tiles = (row_end - row_begin + kTileRows - 1) / kTileRows;
   const uint32_t smem_base = smem_u32(smem);
   const uint32_t ring = smem_base + static_cast<uint32_t>(warp) * Cfg::WARP_RING + static_cast<uint32_t>(lane) * 16u;
+
+  // A code matrix and its rows' place among the launch's: of the entry of a tile, or of the layer that a row belongs to
+  auto entry_of = [&](int tile) { return (q_begin + tile) / p.entry_tiles; };
+  auto layer_of = [&](int row)
+  {
+    int sg = 0;
+    while (sg + 1 < p.num_seg && row >= p.seg_row0[sg + 1])
+    {
+      ++sg;
+    }
+    return sg;
+  };
+  // The tiles are worked off in rounds, as many as the parking area takes; a round has one entry.
+  auto round_stop = [&](int first)
+  {
+    int stop = min(first + p.round_tiles, my_tiles);
+    if (EXPERTS)
+    {
+      stop = min(stop, (entry_of(first) + 1) * p.entry_tiles - q_begin);
+    }
+    return stop;
+  };
 
   // The copies run DEPTH slots ahead of the compute loop, in its order: rounds, passes over k, tiles, slots.  Rows past
   // the CTA's last one are read as that one (their sums are never stored), pieces past the row's end not at all
   // (their activations are zero).
   int f_round = 0;   // first tile of the round being fetched
+  int f_stop = round_stop(0);
   int f_tile = 0;
   int f_kseg = 0;
   const uint8_t *f_lo;   // this lane's first piece of row g, and of row g + 8, of the tile
@@ -335,13 +396,15 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
   {
     row = min(row, row_end - 1);
     const uint8_t *base = p.codes[0];
-    if (p.num_seg > 1)
+    if (EXPERTS)
     {
-      int sg = 0;
-      while (sg + 1 < p.num_seg && row >= p.seg_row0[sg + 1])
-      {
-        ++sg;
-      }
+      const int entry = row / (p.entry_tiles * kTileRows);
+      base = table.e[entry].codes;
+      row -= entry * p.entry_tiles * kTileRows;
+    }
+    else if (p.num_seg > 1)
+    {
+      const int sg = layer_of(row);
       base = p.codes[sg];
       row -= p.seg_row0[sg];
     }
@@ -351,7 +414,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
   {
     const int row = row_begin + f_tile * kTileRows + g;
     f_lo = row_ptr(row);
-    f_hi = row_ptr(row + 8);
+    f_hi = EXPERTS ? f_lo + 8u * p.row_bytes : row_ptr(row + 8);
   };
   auto fetch = [&](int slab, uint32_t dst)
   {
@@ -370,16 +433,25 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
       }
       if (slab == NSLAB - 1)
       {
-        if (++f_tile == min(f_round + p.round_tiles, my_tiles))
+        if (++f_tile == f_stop)
         {
           if (++f_kseg == p.num_ksegs)
           {
             f_kseg = 0;
             f_round = f_tile;
+            f_stop = f_round < my_tiles ? round_stop(f_round) : f_stop;
           }
           f_tile = f_round;
         }
-        fetch_rows();
+        if (EXPERTS && f_tile > f_round)
+        {
+          f_lo += static_cast<uint32_t>(kTileRows) * p.row_bytes;
+          f_hi += static_cast<uint32_t>(kTileRows) * p.row_bytes;
+        }
+        else
+        {
+          fetch_rows();
+        }
       }
     }
     cp_async_commit();
@@ -389,7 +461,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
   {
     uint64_t *bar = &scale_bar[round & 1];
     const int row0 = row_begin + first_tile * kTileRows;
-    const int row1 = min(row_end, row0 + p.round_tiles * kTileRows);
+    const int row1 = min(row_end, row_begin + round_stop(first_tile) * kTileRows);
     const uint32_t per_row = (BITS == 4) ? static_cast<uint32_t>(p.groups_per_row) * 2u : 0u;
     mbar_expect_tx(bar, static_cast<uint32_t>(row1 - row0) * per_row + (round == 0 ? p.stall_bytes : 0u));
     if (BITS == 4)
@@ -397,13 +469,11 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
       uint32_t dst = smem_base + p.scale_offset + static_cast<uint32_t>(round & 1) * p.scale_bytes;
       for (int row = row0; row < row1;)
       {
-        int sg = 0;
-        while (sg + 1 < p.num_seg && row >= p.seg_row0[sg + 1])
-        {
-          ++sg;
-        }
-        const int n = min(row1, p.seg_row0[sg + 1]) - row;
-        const uint8_t *src = static_cast<const uint8_t *>(p.scales[sg]) + static_cast<size_t>(row - p.seg_row0[sg]) * per_row;
+        const int sg = EXPERTS ? entry_of(first_tile) : layer_of(row);
+        const int sg_row0 = EXPERTS ? sg * p.entry_tiles * kTileRows : p.seg_row0[sg];
+        const int n = EXPERTS ? row1 - row : min(row1, p.seg_row0[sg + 1]) - row;
+        const uint8_t *src = static_cast<const uint8_t *>(EXPERTS ? table.e[sg].scales : p.scales[sg]) +
+                             static_cast<size_t>(row - sg_row0) * per_row;
         bulk_g2s(dst, src, static_cast<uint32_t>(n) * per_row, bar);
         dst += static_cast<uint32_t>(n) * per_row;
         row += n;
@@ -414,6 +484,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
   // The frozen codes and scales never depend on earlier work in the stream: their copies start before the wait on
   // the previous kernel.  The next kernel in the stream may place its CTAs as soon as this grid's CTAs have all
   // come this far (programmatic dependent launch).
+  const int f_stop_0 = f_stop;
   fetch_rows();
 #pragma unroll
   for (int i = 0; i < Cfg::DEPTH; ++i)
@@ -426,9 +497,9 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
     mbar_init(&scale_bar[1], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fetch_scales(0, 0);
-    if (p.round_tiles < my_tiles)
+    if (f_stop_0 < my_tiles)
     {
-      fetch_scales(1, p.round_tiles);
+      fetch_scales(1, f_stop_0);
     }
   }
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -442,9 +513,10 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
   uint32_t xf[NCH][MT][XR];
   float sx[NCH][MT][4];     // int4: -24 * (sum of x over the chunk's 128 elements) as an accumulator fragment
   uint32_t scale_off[NCH];  // byte offset of row g's scale for the chunk inside a tile's scales
-  auto load_x = [&](int kseg)
+  auto load_x = [&](int kseg, const __nv_bfloat16 *x, int m)
   {
     // all loads first: one round trip
+    const bool wide = (reinterpret_cast<uintptr_t>(x) & 31u) == 0;   // (rows are a multiple of 128 bytes)
 #pragma unroll
     for (int ch = 0; ch < NCH; ++ch)
     {
@@ -453,12 +525,23 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
       for (int mt = 0; mt < MT; ++mt)
       {
         const int token = g + 8 * mt;
-        const bool live = c < p.num_chunks && token < p.m;
-        const __nv_bfloat16 *src = p.x + static_cast<size_t>(token) * p.in_dim + c * CHUNK_K + t * ELEMS;
-#pragma unroll
-        for (int i = 0; i < XR / 4; ++i)
+        const bool live = c < p.num_chunks && token < m;
+        const __nv_bfloat16 *src = x + static_cast<size_t>(token) * p.in_dim + c * CHUNK_K + t * ELEMS;
+        if (wide)
         {
-          ldg128(src + 8 * i, live, xf[ch][mt][4 * i], xf[ch][mt][4 * i + 1], xf[ch][mt][4 * i + 2], xf[ch][mt][4 * i + 3]);
+#pragma unroll
+          for (int i = 0; i < XR / 8; ++i)
+          {
+            ldg256(src + 16 * i, live, &xf[ch][mt][8 * i]);
+          }
+        }
+        else
+        {
+#pragma unroll
+          for (int i = 0; i < XR / 4; ++i)
+          {
+            ldg128(src + 8 * i, live, xf[ch][mt][4 * i], xf[ch][mt][4 * i + 1], xf[ch][mt][4 * i + 2], xf[ch][mt][4 * i + 3]);
+          }
         }
       }
     }
@@ -532,29 +615,23 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
     park_off[mt] = static_cast<uint32_t>(warp) * park_warp_bytes +
                    (static_cast<uint32_t>(g * p.tokp) + 4u * quad + 2u * static_cast<uint32_t>(t & 1)) * 4u;
   }
-  // int8: an output row takes the per-tensor scale of its segment
-  auto tensor_scale_of = [&](int row)
-  {
-    int sg = 0;
-    while (sg + 1 < p.num_seg && row >= p.seg_row0[sg + 1])
-    {
-      ++sg;
-    }
-    return p.scales[sg] != nullptr ? __ldg(static_cast<const float *>(p.scales[sg])) : 1.0f;
-  };
-
   const float zero4[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   uint32_t slot = 0;   // byte offset in the ring
   int round = 0;
-  for (int round_begin = 0; round_begin < my_tiles; round_begin += p.round_tiles, ++round)
+  int entry = -1;
+  for (int round_begin = 0, round_end = 0; round_begin < my_tiles; round_begin = round_end, ++round)
   {
-    const int round_end = min(round_begin + p.round_tiles, my_tiles);
+    round_end = round_stop(round_begin);
+    const int entry_before = entry;
+    entry = EXPERTS ? entry_of(round_begin) : 0;
+    const int m = EXPERTS ? table.e[entry].rows : p.m;
+    const __nv_bfloat16 *x = p.x + (EXPERTS ? static_cast<size_t>(table.e[entry].row0) * p.in_dim : 0);
     const uint32_t scale_base = smem_base + p.scale_offset + static_cast<uint32_t>(round & 1) * p.scale_bytes;
     for (int kseg = 0; kseg < p.num_ksegs; ++kseg)
     {
-      if (round == 0 || p.num_ksegs > 1)
+      if (entry != entry_before || p.num_ksegs > 1)
       {
-        load_x(kseg);
+        load_x(kseg, x, m);
       }
       if (kseg == 0)
       {
@@ -724,9 +801,13 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
       }
     }
     __syncthreads();
-    if (tid == 0 && round_end + p.round_tiles < my_tiles)
+    if (tid == 0 && round_end < my_tiles)
     {
-      fetch_scales(round + 2, round_end + p.round_tiles);
+      const int next = round_stop(round_end);
+      if (next < my_tiles)
+      {
+        fetch_scales(round + 2, next);
+      }
     }
 
     // Cross-warp reduction: an output is the sum of its warps' partial sums in warp order.  A thread takes up to
@@ -734,7 +815,7 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
     // the warp.  With peers the plain stores travel over NVLink and are complete when the kernel is.
     const int rows = (round_end - round_begin) * kTileRows;
     const int live_rows = min(rows, row_end - row_begin - round_begin * kTileRows);
-    const int quads = (p.m + 3) >> 2;
+    const int quads = (m + 3) >> 2;
     for (int tq = tid >> 7; tq < quads; tq += (WARPS * 32) / 128)
     {
       for (int local = tid & 127; local < live_rows; local += 128)
@@ -769,14 +850,15 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
         const int row = row_begin + round_begin * kTileRows + local;
         if (BITS == 8)
         {
-          const float tensor_scale = tensor_scale_of(row);
+          const void *scale = EXPERTS ? table.e[entry].scales : p.scales[layer_of(row)];
+          const float tensor_scale = scale != nullptr ? __ldg(static_cast<const float *>(scale)) : 1.0f;
 #pragma unroll
           for (int i = 0; i < 4; ++i)
           {
             acc[i] *= tensor_scale;
           }
         }
-        const int live = min(4, p.m - 4 * tq);
+        const int live = min(4, m - 4 * tq);
         // (summed before the scale, and int4 with an offset that turns an infinity into infinity - infinity)
         if (__builtin_expect(!(fabsf(acc[0]) + fabsf(acc[1]) + fabsf(acc[2]) + fabsf(acc[3]) <= 3.402823466e38f), 0))
         {
@@ -788,7 +870,11 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
             {
               continue;
             }
-            const float v = plain_sum<BITS>(p, row, 4 * tq + i);
+            const int sg = EXPERTS ? entry : layer_of(row);
+            const int row0 = EXPERTS ? entry * p.entry_tiles * kTileRows : p.seg_row0[sg];
+            const float v = plain_sum<BITS>(p, EXPERTS ? table.e[sg].codes : p.codes[sg],
+                                            EXPERTS ? table.e[sg].scales : p.scales[sg], row - row0,
+                                            x + static_cast<size_t>(4 * tq + i) * p.in_dim);
             acc[0] = i == 0 ? v : acc[0];
             acc[1] = i == 1 ? v : acc[1];
             acc[2] = i == 2 ? v : acc[2];
@@ -796,7 +882,16 @@ __global__ void __launch_bounds__(WARPS * 32, WARPS == 8 ? 2 : 1) linear_decode_
           }
         }
         int64_t idx = static_cast<int64_t>(4 * tq) * p.y_ld + p.y_col0 + row;
-        if (p.y_dtype == CAIFQ_F32 && !p.accumulate && p.num_y == 1)
+        if (EXPERTS)
+        {
+          idx = (static_cast<int64_t>(table.e[entry].row0) + 4 * tq) * p.y_ld + row - entry * p.entry_tiles * kTileRows;
+#pragma unroll 1
+          for (int i = 0; i < live; ++i, idx += p.y_ld)
+          {
+            store_from_float(table.e[entry].c, idx, p.y_dtype, i == 0 ? acc[0] : (i == 1 ? acc[1] : (i == 2 ? acc[2] : acc[3])));
+          }
+        }
+        else if (p.y_dtype == CAIFQ_F32 && !p.accumulate && p.num_y == 1)
         {
           float *dst = static_cast<float *>(p.y[0]) + idx;
 #pragma unroll
@@ -881,10 +976,10 @@ void decode_stall_next_launch() { t_stall_next = true; }
 namespace
 {
 
-template <int WARPS, int BITS, int MT, int NCH, int PCH>
-int launch_decode_inst(const DecodeParams &p, uint32_t smem, cudaStream_t s)
+template <int WARPS, int BITS, int MT, int NCH, int PCH, int N>
+int launch_decode_inst(const DecodeParams &p, const DecodeTable<N> &table, uint32_t smem, cudaStream_t s)
 {
-  auto kernel = linear_decode_kernel<WARPS, BITS, MT, NCH, PCH>;
+  auto kernel = linear_decode_kernel<WARPS, BITS, MT, NCH, PCH, N>;
   static std::atomic<bool> configured[kMaxDevices];
   int dev = 0;
   CAIFQ_CHECK_CUDA(cudaGetDevice(&dev));
@@ -899,7 +994,7 @@ int launch_decode_inst(const DecodeParams &p, uint32_t smem, cudaStream_t s)
                                           static_cast<int>(kSmemFull)));
     configured[dev].store(true, std::memory_order_release);
   }
-  int grid = sm_count();
+  int grid = sm_count() * (N > 1 && WARPS == 8 ? 2 : 1);
   if (grid > p.num_quanta)
   {
     grid = p.num_quanta;
@@ -916,13 +1011,14 @@ int launch_decode_inst(const DecodeParams &p, uint32_t smem, cudaStream_t s)
   // codes written just ahead in this stream by one of the library's own calls: a plain launch
   // orders the early copies behind that kernel
   cfg.numAttrs = (dependent_launches() && !take_codes_written(s)) ? 1 : 0;
-  CAIFQ_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
+  CAIFQ_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, p, table));
   CAIFQ_CHECK_LAUNCH();
   return CAIFQ_OK;
 }
 
 int tokp_for(int64_t m) { return m <= 2 ? 2 : (m <= 4 ? 4 : (m <= 8 ? 8 : 16)); }
 
+// How a launch is cut, by the shape of its rows and the most tokens of an entry.
 struct Layout
 {
   int warps;
@@ -934,7 +1030,8 @@ struct Layout
   int round_tiles;
 };
 
-Layout layout_for(const caifq_weight &w, int64_t m)
+// (w.out_dim: all the rows of the launch)
+Layout layout_for(const caifq_weight &w, int64_t m, bool experts)
 {
   Layout l{};
   const bool i4 = (w.storage == CAIFQ_I4);
@@ -944,11 +1041,12 @@ Layout layout_for(const caifq_weight &w, int64_t m)
   // so that the next launch's CTA sits beside this one with its copies done (1024 -> 1024, m = 1: 2.4 us a launch
   // against 2.7).  Longer rows, and two token tiles, want the 16 warps: the launch is bound by the dequantization's
   // instructions and their latencies, not by its start (4096 -> 14336, m = 1: 10.4 us, 11.4 with eight, 11.6 with 32).
-  l.warps = (num_chunks <= 16 && mt == 1) ? 8 : 16;
+  // Experts: a CTA has hundreds of rows, and one of two on an SM works while the other waits for its next entry's activations.
+  l.warps = (experts || (num_chunks <= 16 && mt == 1)) ? 8 : 16;
   // Chunks a warp holds token fragments of at a time: as many as 64 registers take (a lane needs 16 of them per
   // int4 chunk and token tile, 8 per int8 chunk), no more than the row has.
   const int most = (i4 ? 4 : 8) / mt;
-  l.nch = 1;
+  l.nch = experts ? 2 : 1;
   while (l.nch < most && l.nch * l.warps < num_chunks)
   {
     l.nch *= 2;
@@ -957,14 +1055,15 @@ Layout layout_for(const caifq_weight &w, int64_t m)
   const uint32_t ring = static_cast<uint32_t>(l.warps) * (deep ? 8u : 6u) * 1024u;   // WARPS * DecodeCfg::WARP_RING
   const uint32_t scales = i4 ? static_cast<uint32_t>(kTileRows * (w.in_dim / w.group_size) * 2) : 0u;
   const uint32_t park = static_cast<uint32_t>(l.warps * kTileRows * tokp_for(m) * sizeof(float));
-  const int quanta = (w.out_dim + kRowQuantum - 1) / kRowQuantum;
-  int grid = sm_count();
+  const int quantum = experts ? kTileRows : kRowQuantum;
+  const int quanta = (w.out_dim + quantum - 1) / quantum;
+  int grid = sm_count() * (experts ? 2 : 1);
   if (grid > quanta)
   {
     grid = quanta;
   }
   const int max_quanta = (quanta + grid - 1) / grid;
-  const int max_tiles = (max_quanta * kRowQuantum + kTileRows - 1) / kTileRows;
+  const int max_tiles = (max_quanta * quantum + kTileRows - 1) / kTileRows;
   // all of a CTA's tiles in one round if they fit, else in several equal rounds
   const uint32_t budget = l.warps == 8 ? kSmemHalf : kSmemFull;
   auto align128 = [](uint32_t v) { return (v + 127u) & ~127u; };
@@ -973,12 +1072,12 @@ Layout layout_for(const caifq_weight &w, int64_t m)
            static_cast<uint32_t>(tiles) * park; };
   int rounds = 1;
   int tiles = max_tiles;
-  while (tiles > 1 && bytes(tiles, rounds > 1 ? 2 : 1) > budget)
+  while (tiles > 1 && bytes(tiles, rounds > 1 || experts ? 2 : 1) > budget)
   {
     ++rounds;
     tiles = (max_tiles + rounds - 1) / rounds;
   }
-  const int buffers = (tiles < max_tiles) ? 2 : 1;
+  const int buffers = (tiles < max_tiles || experts) ? 2 : 1;   // (experts: a round ends with its entry, too)
   if (bytes(tiles, buffers) > kSmemFull)
   {
     return l;
@@ -992,6 +1091,18 @@ Layout layout_for(const caifq_weight &w, int64_t m)
 }
 
 }  // namespace
+
+// int4 with groups of whole 128-element pieces, int8 with one scale or none.  bf16 compute in the reference rounds
+// scale*code to bf16 before the product; this kernel keeps the exact fp32 scale.  Both are inside the bf16 tolerance, and
+// fp32 compute is matched exactly.
+static bool decode_weight(const caifq_weight &w)
+{
+  if (w.storage == CAIFQ_I4)
+  {
+    return w.scales != nullptr && w.group_size >= 128 && (w.group_size % 128) == 0 && (w.in_dim % w.group_size) == 0;
+  }
+  return w.storage == CAIFQ_I8 && (w.scales == nullptr || w.scheme == CAIFQ_PER_TENSOR) && (w.in_dim % 64) == 0;
+}
 
 // The launch's rows: the layer's own, or those of all the layers that share the input laid end to end.
 static caifq_weight all_rows(const LinearArgs &args)
@@ -1043,38 +1154,13 @@ bool decode_supported(const LinearArgs &args)
   {
     return false;
   }
-  if (w.storage == CAIFQ_I4)
+  if (!decode_weight(w) || (w.storage == CAIFQ_I4 && (w.out_dim % kRowQuantum) != 0 && ((w.in_dim / w.group_size) % 8) != 0))
   {
-    if (w.scales == nullptr || w.group_size < 128 || (w.group_size % 128) != 0 || (w.in_dim % w.group_size) != 0)
-    {
-      return false;
-    }
-    // a ragged last item copies rows * groups_per_row fp16 scales: keep that a 16-byte multiple
-    if ((w.out_dim % kRowQuantum) != 0 && ((w.in_dim / w.group_size) % 8) != 0)
-    {
-      return false;
-    }
-    // bf16 compute in the reference rounds scale*code to bf16 before the
-    // product; this kernel keeps the exact fp32 scale.  Both are inside the
-    // bf16 tolerance, and fp32 compute is matched exactly.
-  }
-  else if (w.storage == CAIFQ_I8)
-  {
-    if (w.scales != nullptr && w.scheme != CAIFQ_PER_TENSOR)
-    {
-      return false;
-    }
-    if ((w.in_dim % 64) != 0)
-    {
-      return false;
-    }
-  }
-  else
-  {
+    // (a ragged last item copies rows * groups_per_row fp16 scales: that is kept a multiple of 16 bytes)
     return false;
   }
   // a tile's scales and parked sums must fit beside the rings
-  if (layout_for(w, m).smem_bytes == 0)
+  if (layout_for(w, m, false).smem_bytes == 0)
   {
     return false;
   }
@@ -1085,6 +1171,21 @@ bool decode_supported(const LinearArgs &args)
     return false;
   }
   return true;
+}
+
+static void shape_params(DecodeParams &p, const caifq_weight &w, const Layout &lay)
+{
+  const bool i4 = (w.storage == CAIFQ_I4);
+  p.in_dim = w.in_dim;
+  p.row_bytes = static_cast<uint32_t>(i4 ? w.in_dim / 2 : w.in_dim);
+  p.groups_per_row = i4 ? w.in_dim / w.group_size : 0;
+  p.chunks_per_group = i4 ? w.group_size / 128 : 1;
+  p.num_chunks = w.in_dim / (i4 ? 128 : 64);
+  p.num_ksegs = (p.num_chunks + lay.nch * lay.warps - 1) / (lay.nch * lay.warps);
+  p.round_tiles = lay.round_tiles;
+  p.scale_offset = lay.scale_offset;
+  p.scale_bytes = lay.scale_bytes;
+  p.park_offset = lay.park_offset;
 }
 
 int launch_linear_decode(const LinearArgs &args, cudaStream_t s)
@@ -1140,33 +1241,15 @@ int launch_linear_decode(const LinearArgs &args, cudaStream_t s)
   p.accumulate = args.accumulate ? 1 : 0;
   p.m = static_cast<int>(m);
   p.tokp = tokp_for(m);
-  p.in_dim = w.in_dim;
   p.out_dim = w.out_dim;
   p.num_quanta = (w.out_dim + kRowQuantum - 1) / kRowQuantum;
-  const bool i4 = (w.storage == CAIFQ_I4);
-  p.row_bytes = i4 ? static_cast<uint32_t>(w.in_dim / 2) : static_cast<uint32_t>(w.in_dim);
-  if (i4)
-  {
-    p.groups_per_row = w.in_dim / w.group_size;
-    p.chunks_per_group = w.group_size / 128;
-  }
-  else
-  {
-    p.groups_per_row = 0;
-    p.chunks_per_group = 1;
-  }
-  p.num_chunks = w.in_dim / (i4 ? 128 : 64);
-  const Layout lay = layout_for(w, m);
+  const Layout lay = layout_for(w, m, false);
   if (lay.smem_bytes == 0)
   {
     set_error("frozen linear (decode): row too long for the shared memory");
     return CAIFQ_ERR_UNSUPPORTED;
   }
-  p.num_ksegs = (p.num_chunks + lay.nch * lay.warps - 1) / (lay.nch * lay.warps);
-  p.round_tiles = lay.round_tiles;
-  p.scale_offset = lay.scale_offset;
-  p.scale_bytes = lay.scale_bytes;
-  p.park_offset = lay.park_offset;
+  shape_params(p, w, lay);
   p.spin_limit = kSpinLimit;
   p.stall_bytes = 0;
   if (t_stall_next)
@@ -1177,11 +1260,13 @@ int launch_linear_decode(const LinearArgs &args, cudaStream_t s)
     p.stall_bytes = 16;
   }
 
+  const bool i4 = w.storage == CAIFQ_I4;
   const int mt = (m > 8) ? 2 : 1;
+  const DecodeTable<1> none{};
 #define CAIFQ_DECODE_CASE(W, B, M, N)                                                      \
   if (lay.warps == W && lay.nch == N && mt == M)                                           \
   {                                                                                        \
-    return launch_decode_inst<W, B, M, N, (N > 1 ? 2 : 1)>(p, lay.smem_bytes, s);          \
+    return launch_decode_inst<W, B, M, N, (N > 1 ? 2 : 1), 1>(p, none, lay.smem_bytes, s); \
   }
   if (i4)
   {
@@ -1205,6 +1290,115 @@ int launch_linear_decode(const LinearArgs &args, cudaStream_t s)
   }
 #undef CAIFQ_DECODE_CASE
   set_error("frozen linear (decode): no kernel instance for in_dim=%d m=%lld", w.in_dim, static_cast<long long>(m));
+  return CAIFQ_ERR_UNSUPPORTED;
+}
+
+// Experts: entries of more than 16 rows are taken 16 at a time (their codes come from L2 again).
+static int decode_entries(const GroupedStreamArgs &g, DecodeTable<MAX_ENTRIES> *table, int &most)
+{
+  int count = 0;
+  most = 0;
+  for (int e = 0; e < g.count; ++e)
+  {
+    for (int row = g.row_begin[e]; row < g.row_end[e]; row += 16)
+    {
+      const int rows = g.row_end[e] - row < 16 ? g.row_end[e] - row : 16;
+      if (count == MAX_ENTRIES)
+      {
+        return -1;
+      }
+      if (table != nullptr)
+      {
+        table->e[count] = DecodeEntry{static_cast<const uint8_t *>(g.weights[e].codes), g.weights[e].scales, g.c[e], row, rows};
+      }
+      most = rows > most ? rows : most;
+      ++count;
+    }
+  }
+  return count;
+}
+
+bool decode_grouped_supported(const GroupedStreamArgs &g)
+{
+  int most = 0;
+  const int entries = g.count < 1 ? -1 : decode_entries(g, nullptr, most);
+  if (entries < 1 || g.accumulate || !is_float_dtype(g.c_dtype) || (reinterpret_cast<uintptr_t>(g.a) & 15u) != 0 ||
+      (g.compute_dtype != CAIFQ_F32 && g.compute_dtype != CAIFQ_BF16))
+  {
+    return false;
+  }
+  const caifq_weight &w0 = g.weights[0];
+  if ((w0.out_dim % kTileRows) != 0 || static_cast<int64_t>(entries) * w0.out_dim > 0x7FFFFFFF)
+  {
+    return false;
+  }
+  for (int e = 0; e < g.count; ++e)
+  {
+    const caifq_weight &w = g.weights[e];
+    if (!decode_weight(w) || w.storage != w0.storage || w.in_dim != w0.in_dim || w.out_dim != w0.out_dim ||
+        w.group_size != w0.group_size || (reinterpret_cast<uintptr_t>(w.codes) & 15u) != 0 ||
+        (w.storage == CAIFQ_I4 && (reinterpret_cast<uintptr_t>(w.scales) & 15u) != 0))
+    {
+      return false;
+    }
+  }
+  caifq_weight all = w0;
+  all.out_dim *= entries;
+  return layout_for(all, most, true).smem_bytes != 0;
+}
+
+int launch_linear_decode_grouped(const GroupedStreamArgs &g, cudaStream_t s)
+{
+  static thread_local DecodeTable<MAX_ENTRIES> table;
+  int most = 0;
+  const int entries = decode_entries(g, &table, most);
+  if (entries < 1)
+  {
+    return entries == 0 ? CAIFQ_OK : CAIFQ_ERR_UNSUPPORTED;
+  }
+  caifq_weight w = g.weights[0];
+  DecodeParams p{};
+  p.entry_tiles = w.out_dim / kTileRows;
+  p.y_ld = w.out_dim;
+  w.out_dim *= entries;
+  const Layout lay = layout_for(w, most, true);
+  if (lay.smem_bytes == 0)
+  {
+    set_error("frozen experts (decode): row too long for the shared memory");
+    return CAIFQ_ERR_UNSUPPORTED;
+  }
+  shape_params(p, w, lay);
+  p.num_seg = 1;
+  p.x = static_cast<const __nv_bfloat16 *>(g.a);
+  p.num_y = 1;
+  p.y_dtype = g.c_dtype;
+  p.m = most;
+  p.tokp = tokp_for(most);
+  p.out_dim = w.out_dim;
+  p.num_quanta = w.out_dim / kTileRows;
+  p.spin_limit = kSpinLimit;
+  const int mt = (most > 8) ? 2 : 1;
+#define CAIFQ_DECODE_CASE(B, M, N)                                                                         \
+  if (mt == M && lay.nch == N)                                                                             \
+  {                                                                                                        \
+    return launch_decode_inst<8, B, M, N, 2, MAX_ENTRIES>(p, table, lay.smem_bytes, s);                    \
+  }
+  if (w.storage == CAIFQ_I4)
+  {
+    CAIFQ_DECODE_CASE(4, 1, 2)
+    CAIFQ_DECODE_CASE(4, 1, 4)
+    CAIFQ_DECODE_CASE(4, 2, 2)
+  }
+  else
+  {
+    CAIFQ_DECODE_CASE(8, 1, 2)
+    CAIFQ_DECODE_CASE(8, 1, 4)
+    CAIFQ_DECODE_CASE(8, 1, 8)
+    CAIFQ_DECODE_CASE(8, 2, 2)
+    CAIFQ_DECODE_CASE(8, 2, 4)
+  }
+#undef CAIFQ_DECODE_CASE
+  set_error("frozen experts (decode): no kernel instance for in_dim=%d rows=%d", w.in_dim, most);
   return CAIFQ_ERR_UNSUPPORTED;
 }
 

@@ -866,6 +866,59 @@ def test_experts_of_few_rows(storage, compute, counts, gated):
         assert max_rel_err(up_out[lo:hi].float().cpu().numpy(), u) <= 2e-2
 
 
+@pytest.mark.parametrize("storage", [orc.I4, orc.I8])
+@pytest.mark.parametrize("counts,in_dim,hid", [
+    ([1] * 7, 2048, 1408),                  # one tile of tokens; 11 pieces of k for eight warps of two
+    ([8, 0, 3, 1], 1024, 384),
+    ([16, 9, 0, 0, 2], 2048, 2048),         # two tiles of tokens
+    ([17, 1, 1, 1, 1, 1, 1, 1], 2048, 2048),  # 16 rows and one more
+    ([2, 5, 8], 4608, 128),                 # rows too long for one pass over k
+    ([1, 2] * 60, 256, 128),                # a round of tiles ends with its expert, many times per CTA
+])
+def test_experts_on_the_few_token_kernel(storage, counts, in_dim, hid):
+    """Expert by expert against 64 bits of the dequantized weights.  What is stored in bf16 is off by half a bf16 ulp at most,
+    2^-8 of the value, and the kernel's own error is an fp32 GEMM's (1e-6 of the norm); the result of `down` is compared
+    for the hidden rows as they were rounded."""
+    rng = np.random.default_rng(sum(counts) + in_dim)
+    offsets = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32)
+    ws = [[make_weight(rng, o, i, storage, std=0.05) for _ in counts]
+          for (o, i) in ((hid, in_dim), (hid, in_dim), (in_dim, hid))]
+    deq = [[torch.from_numpy(orc.weight_to_compute(c, s, storage, w.in_dim, w.out_dim, orc.F32, w.scheme, w.group_size)).double().cuda()
+            for (w, c, s) in l] for l in ws]
+    gate, up, down = [[w for (w, _, _) in l] for l in ws]
+    _, x = act(rng, int(offsets[-1]), in_dim, orc.BF16)
+
+    def close(got, want):
+        exact = (got.double() - want).abs()
+        assert (exact <= want.abs() * 2.0 ** -8 + 1e-6 * want.norm()).all()
+
+    def run():
+        out, gate_out, up_out = nv.grouped_expert_fwd(gate, up, down, offsets.tolist(), x, orc.BF16)
+        assert nv.lib().caifq_device_status() == 0
+        return out, gate_out, up_out
+
+    out, gate_out, up_out = run()
+    g32 = gate_out.float()
+    hidden = ((g32 * torch.sigmoid(g32)).bfloat16().float() * up_out.float()).bfloat16()
+    for e in range(len(counts)):
+        lo, hi = int(offsets[e]), int(offsets[e + 1])
+        if lo == hi:
+            continue
+        rows = x[lo:hi].double()
+        close(gate_out[lo:hi], rows @ deq[0][e].T)
+        close(up_out[lo:hi], rows @ deq[1][e].T)
+        # (a hidden value may be the other neighbour where sigmoid rounds differently: 2^-8 of each of its products)
+        want = hidden[lo:hi].double() @ deq[2][e].T
+        slack = 2.0 ** -8 * (hidden[lo:hi].double() ** 2 @ (deq[2][e] ** 2).T).sqrt()
+        assert ((out[lo:hi].double() - want).abs() <= want.abs() * 2.0 ** -8 + 1e-6 * want.norm() + 6 * slack).all()
+    # an infinity stays in its row
+    bad = int(offsets[-1]) - 1
+    x[bad, 3] = float("inf")
+    out2, gate2, _ = run()
+    assert torch.equal(out2[:bad], out[:bad]) and torch.equal(gate2[:bad], gate_out[:bad])
+    assert not torch.isfinite(gate2[bad]).any()
+
+
 @pytest.mark.parametrize("rank", [8, 16, 64])
 @pytest.mark.parametrize("m,in_dim,out_dim", [(33, 14336, 128), (128, 2048, 1152), (1000, 640, 4096)])
 def test_lora_products_split_over_clusters(rank, m, in_dim, out_dim):
