@@ -183,3 +183,37 @@ def test_int8_slices_of_rows_bit_exact(shape):
     oq, os_ = orc.quantize_int8_per_tensor(x.numpy())
     assert np.array_equal(q.cpu().numpy(), oq)
     assert np.array_equal(_bits(s), os_.view(np.int32))
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 8192, 8193, 40961])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_int8_block_maxima_lie_where_the_codes_will(n, offset):
+    """Fewer codes than a block's maximum has bytes, one block and several, codes that start on any byte; and a value and a
+    weight quantized again into the same codes."""
+    g = torch.Generator().manual_seed(18)
+    codes = torch.zeros(n + offset + 4, dtype=torch.int8, device=dev())
+    scale = torch.zeros(1, device=dev())
+    for std in (0.02, 3.0):
+        x = torch.randn(n, generator=g) * std
+        xd = x.to(dev())
+        rc = nv.lib().caifq_quantize_int8_per_tensor(xd.data_ptr(), codes.data_ptr() + offset, scale.data_ptr(), n,
+                                                     torch.cuda.current_stream().cuda_stream)
+        assert rc == 0
+        oq, os_ = orc.quantize_int8_per_tensor(x.numpy())
+        assert np.array_equal(codes[offset:offset + n].cpu().numpy(), oq)
+        assert np.array_equal(_bits(scale), os_.view(np.int32))
+        assert not codes[:offset].any() and not codes[offset + n:].any()
+
+
+@pytest.mark.parametrize("rows,cols", [(1, 1), (7, 30), (9, 4096), (2049, 36), (1025, 31), (300, 9600), (65, 19000)])
+def test_int8_per_channel_clusters_bit_exact(rows, cols):
+    """Eight row slices a column block of 16 (512 threads), 32, 64 and 128; slices without rows; infinities and NaNs."""
+    g = torch.Generator().manual_seed(19)
+    x = torch.randn(rows, cols, generator=g) * 0.02
+    x[0, 0] = float("inf")
+    x[rows - 1, cols // 2] = float("nan")
+    q, s = nv.quantize_int8_per_channel(x.to(dev()))
+    oq, os_ = orc.quantize_int8_per_channel(x.numpy())
+    assert np.array_equal(_bits(s), os_.view(np.int32))
+    live = np.isfinite(x.numpy() / os_[None, :])   # (what a NaN or an infinity is cast to is not defined on the CPU)
+    assert np.array_equal(q.cpu().numpy()[live], oq[live])
