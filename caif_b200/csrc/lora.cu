@@ -689,6 +689,8 @@ __global__ void expand_prepare_kernel(const ExpandPrepare p)
 {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t first = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  // (the wait first: the thin product that follows starts on activations, which must then be complete)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (blockIdx.y == 0 && p.wb != nullptr)
   {
@@ -760,15 +762,8 @@ int launch_expand_prepare(const caifq_weight &w, void *wb, const void *a, const 
   p.r = rank;
   const bool factors = bp != nullptr || bt != nullptr;
   const dim3 grid(wb != nullptr ? 148 * 8 : 148 * 2, wb != nullptr && factors ? 2 : 1);
-  if (i8)
-  {
-    expand_prepare_kernel<EXPAND_I8><<<grid, 256, 0, s>>>(p);
-  }
-  else
-  {
-    expand_prepare_kernel<EXPAND_I4><<<grid, 256, 0, s>>>(p);
-  }
-  CAIFQ_CHECK_LAUNCH();
+  CAIFQ_CHECK_CUDA(launch_dependent(i8 ? expand_prepare_kernel<EXPAND_I8> : expand_prepare_kernel<EXPAND_I4>, grid, dim3(256), 0,
+                                    s, p));
   return CAIFQ_OK;
 }
 

@@ -313,8 +313,9 @@ rmsnorm_fwd_rows_kernel(const T *input, const float *__restrict__ gamma, T *outp
 {
   constexpr int WARPS = 8 / V;   // per row; V rows per CTA
   __shared__ float sums[V][8];
-  // (launched ahead of the previous kernel's end; the next kernel may follow once that one is complete)
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // (launched ahead of the previous kernel's end; the next kernel may follow once that one is complete.  gamma's address
+  // comes out of the wait, so that its invariant loads stay behind it)
+  asm volatile("griddepcontrol.wait;" : "+l"(gamma)::"memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int slot = (threadIdx.x >> 5) / WARPS;
   const int warp_in_row = (threadIdx.x >> 5) % WARPS;
@@ -493,10 +494,13 @@ rmsnorm_bwd_kernel(const T *__restrict__ grad_output, const T *__restrict__ inpu
 // now 31).
 template <typename T, int STRIPES>
 __global__ void __launch_bounds__(kNormThreads, 2)
-rmsnorm_bwd_rows_kernel(const T *__restrict__ grad_output, const T *__restrict__ input, const float *__restrict__ gamma,
-                        const float *__restrict__ rms_cache, T *__restrict__ grad_input, float *__restrict__ grad_gamma,
-                        int rows, int dim, int gamma_vec)
+rmsnorm_bwd_rows_kernel(const T *grad_output, const T *input, const float *gamma, const float *rms_cache,
+                        T *grad_input, float *grad_gamma, int rows, int dim, int gamma_vec)
 {
+  // (launched ahead of the previous kernel's end; the next kernel may follow once that one is complete.  gamma's address
+  // comes out of the wait, so that its invariant loads stay behind it)
+  asm volatile("griddepcontrol.wait;" : "+l"(gamma)::"memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   constexpr int V = 2;
   constexpr bool PREFETCH = STRIPES * sizeof(T) <= 32;
   __shared__ float sums[V][8];
@@ -542,7 +546,7 @@ rmsnorm_bwd_rows_kernel(const T *__restrict__ grad_output, const T *__restrict__
     {
       load(r, x, d);
     }
-    const float rstd = __fdiv_rn(1.0f, live ? __ldg(rms_cache + r) : 1.0f);
+    const float rstd = __fdiv_rn(1.0f, live ? rms_cache[r] : 1.0f);
     float part[V] = {0.0f, 0.0f};
 #pragma unroll
     for (int j = 0; j < STRIPES; ++j)
@@ -642,9 +646,9 @@ void rows_bwd_inst(const void *dy, const void *x, const float *gamma, const floa
 {
   const int pairs = (rows + 1) / 2;
   const int grid = pairs < 148 * 2 ? pairs : 148 * 2;
-  rmsnorm_bwd_rows_kernel<T, STRIPES><<<grid, kNormThreads, static_cast<size_t>(dim) * 4, s>>>(
-      static_cast<const T *>(dy), static_cast<const T *>(x), gamma, rms, static_cast<T *>(dx), grad_gamma, rows, dim,
-      (reinterpret_cast<uintptr_t>(grad_gamma) & 7u) == 0 ? 1 : 0);
+  launch_dependent(rmsnorm_bwd_rows_kernel<T, STRIPES>, dim3(static_cast<unsigned>(grid)), dim3(kNormThreads),
+                   static_cast<size_t>(dim) * 4, s, static_cast<const T *>(dy), static_cast<const T *>(x), gamma, rms,
+                   static_cast<T *>(dx), grad_gamma, rows, dim, (reinterpret_cast<uintptr_t>(grad_gamma) & 7u) == 0 ? 1 : 0);
 }
 
 template <typename T>

@@ -836,6 +836,9 @@ struct ExpandTable
 template <int MODE>
 __global__ void expand_kernel(const __grid_constant__ ExpandTable t, GroupOf group_of)
 {
+  // (the scratch may still be read by the kernel before this one; what follows may read the codes and scratch of others)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int e = blockIdx.y;
   expand_span<MODE>(t.codes[e], t.scales[e], t.dst[e], t.units[e], group_of);
 }
@@ -877,8 +880,8 @@ int launch_expand(const caifq_weight *ws, int count, uint8_t *dst, cudaStream_t 
       gx = cap;
     }
     const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(n));
-    expand_kernel<MODE><<<grid, kBlock, 0, s>>>(t, GroupOf::make(MODE == EXPAND_I4 ? ws[0].group_size : 1));
-    CAIFQ_CHECK_LAUNCH();
+    CAIFQ_CHECK_CUDA(launch_dependent(expand_kernel<MODE>, grid, dim3(kBlock), 0, s, t,
+                                      GroupOf::make(MODE == EXPAND_I4 ? ws[0].group_size : 1)));
   }
   return CAIFQ_OK;
 }
