@@ -656,6 +656,25 @@ def test_fp32_activations_on_the_tensor_core(storage, group, m, in_dim, out_dim)
     assert torch.equal(nv.linear_fwd_residual(weight, x, res.clone()), y + res)
 
 
+@pytest.mark.parametrize("storage,group", [(orc.I8, 128), (orc.I4, 128), (orc.I4, 64)])
+@pytest.mark.parametrize("m,in_dim,out_dim", [(1, 64, 64), (3, 192, 320), (16, 1152, 64), (16, 128, 1088), (17, 64, 128),
+                                              (2, 4096, 640)])
+def test_fp32_activations_of_few_rows(storage, group, m, in_dim, out_dim):
+    """The 16-row tile takes 128 of k at a time: k that ends half way through them (or never gets there), two scale groups
+    in one of them, k over clusters; 17 rows are the other tile's.  Bound: as above, an fp32 GEMM's own error."""
+    if storage == orc.I4 and in_dim % group:
+        pytest.skip("groups straddle rows: the generic kernel's")
+    rng = np.random.default_rng(7 * m + in_dim + out_dim + group)
+    weight, codes, scales = make_weight(rng, out_dim, in_dim, storage, group=group)
+    wc = _oracle_w(weight, codes, scales, orc.F32).astype(np.float64)
+    x_np, x = act(rng, m, in_dim, orc.F32)
+    dy_np, dy = act(rng, m, out_dim, orc.F32)
+    for got, want in ((nv.linear_fwd(weight, x), x_np.astype(np.float64) @ wc.T),
+                      (nv.linear_dx(weight, dy), dy_np.astype(np.float64) @ wc)):
+        assert nv.last_path() == "umma"
+        assert np.linalg.norm(got.cpu().numpy() - want) <= 1e-6 * np.linalg.norm(want)
+
+
 @pytest.mark.parametrize("bits", [0x7FC00000, 0x7F800001, 0xFF80FFFF, 0x7F800000, 0xFF800000])
 def test_fp32_activations_that_are_not_finite(bits, monkeypatch):
     """A NaN of any payload stays one; an infinity gives what the fp32-FMA kernel gives; other rows keep their bits."""
