@@ -317,19 +317,32 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b)
 // bf16, one rounding.  The reference's dequantize-then-cast forms scale * code in fp32 and rounds once;
 // the two differ by the bf16 rounding of the fp16 scale (2^-9 relative), far inside the bf16 bound, and
 // the conversion takes 17 instructions per eight weights instead of 31: the int4 launches are bound by
-// this conversion, not by the tensor core.
+// this conversion, not by the tensor core.  One asm block: apart, the compiler put three moves in between
+// (1.0 -> 0.87 of the time in a loop of conversions and tensor-memory stores; 4096 -> 14336, 96 tokens,
+// 20.9 -> 20.8 us; 4096 -> 4096, 48 tokens, 11.2 -> 11.1).
 __device__ __forceinline__ void int4x8_to_bf16(uint32_t w, uint32_t scale2, uint32_t (&out)[4])
 {
-  const uint32_t ev = (w & 0x0F0F0F0Fu) ^ 0x08080808u;         // u0 u2 u4 u6   (u = q + 8)
-  const uint32_t od = ((w >> 4) & 0x0F0F0F0Fu) ^ 0x08080808u;  // u1 u3 u5 u7
-  const uint32_t t0 = __byte_perm(ev, od, 0x5140);             // u0 u1 u2 u3
-  const uint32_t t1 = __byte_perm(ev, od, 0x7362);             // u4 u5 u6 u7
-  constexpr uint32_t kExp = 0x43434343u;                       // high byte of bf16 128.0 .. 143.0
-  constexpr uint32_t k136 = 0x43084308u;
-  out[0] = mul_bf16x2(sub_bf16x2(__byte_perm(t0, kExp, 0x4140), k136), scale2);
-  out[1] = mul_bf16x2(sub_bf16x2(__byte_perm(t0, kExp, 0x4342), k136), scale2);
-  out[2] = mul_bf16x2(sub_bf16x2(__byte_perm(t1, kExp, 0x4140), k136), scale2);
-  out[3] = mul_bf16x2(sub_bf16x2(__byte_perm(t1, kExp, 0x4342), k136), scale2);
+  // e: u0 u2 u4 u6 (u = q + 8), d: u1 u3 u5 u7; t, v: in element order; 0x43: the high byte of bf16 128.0 .. 143.0
+  asm("{\n\t.reg .b32 e, d, t, v;\n\t"
+      "lop3.b32 e, %4, 0x0F0F0F0F, 0x08080808, 0x6A;\n\t"
+      "shr.u32 d, %4, 4;\n\t"
+      "lop3.b32 d, d, 0x0F0F0F0F, 0x08080808, 0x6A;\n\t"
+      "prmt.b32 t, e, d, 0x5140;\n\t"
+      "prmt.b32 v, e, d, 0x7362;\n\t"
+      "prmt.b32 %0, t, 0x43434343, 0x4140;\n\t"
+      "prmt.b32 %1, t, 0x43434343, 0x4342;\n\t"
+      "prmt.b32 %2, v, 0x43434343, 0x4140;\n\t"
+      "prmt.b32 %3, v, 0x43434343, 0x4342;\n\t"
+      "sub.rn.bf16x2 %0, %0, %6;\n\t"
+      "sub.rn.bf16x2 %1, %1, %6;\n\t"
+      "sub.rn.bf16x2 %2, %2, %6;\n\t"
+      "sub.rn.bf16x2 %3, %3, %6;\n\t"
+      "mul.rn.bf16x2 %0, %0, %5;\n\t"
+      "mul.rn.bf16x2 %1, %1, %5;\n\t"
+      "mul.rn.bf16x2 %2, %2, %5;\n\t"
+      "mul.rn.bf16x2 %3, %3, %5;\n\t}"
+      : "=&r"(out[0]), "=&r"(out[1]), "=&r"(out[2]), "=&r"(out[3])
+      : "r"(w), "r"(scale2), "r"(0x43084308u));
 }
 
 // the same eight codes as two bf16 terms of scale * code: hi = bf16(w), lo = bf16(w - hi)
