@@ -982,3 +982,21 @@ def test_lora_operands_that_start_on_any_element():
     for x2, h2, l2 in ((shifted(x), h, lora), (x, shifted(h), lora), (x, h, odd)):
         for got, want in zip(nv.lora_linear_bwd(weight, l2, dy, x2, h2, orc.F32, expanded=True), grads):
             assert max_rel_err(got.float().cpu().numpy(), want.float().cpu().numpy()) <= 2e-2
+
+
+@pytest.mark.parametrize("dtype,dim", [(torch.bfloat16, 2048), (torch.float32, 1024)])
+def test_combine_of_many_and_of_few_tokens(dtype, dim):
+    """More pieces than one trip of the grid read the rows as constants; fewer are a dependent launch: the same bits.
+    Against x times its weights: one rounding of bf16 (2^-9), and of fp32 sums in another order."""
+    tokens, experts, top_k = 2369, 8, 2
+    g = torch.Generator().manual_seed(23)
+    idx = torch.stack([torch.randperm(experts, generator=g)[:top_k] for _ in range(tokens)]).int().contiguous().to(dev())
+    w = torch.rand(tokens, top_k, generator=g).to(dev()).to(dtype)
+    x = torch.randn(tokens, dim, generator=g).to(dev()).to(dtype)
+    dispatch_map, offsets = nv.moe_build_dispatch(idx, experts)[:2]
+    buf = nv.moe_dispatch(x, idx, dispatch_map, offsets, tokens * top_k)
+    many = nv.moe_combine(buf, idx, w, dispatch_map, offsets, tokens)
+    few = nv.moe_combine(buf, idx[:64].contiguous(), w[:64].contiguous(), dispatch_map[:64 * top_k].contiguous()
+                         if dispatch_map.dim() == 1 else dispatch_map[:64].contiguous(), offsets, 64)
+    assert torch.equal(many[:64], few)
+    assert torch.allclose(many.float(), x.float() * w.float().sum(1, keepdim=True), rtol=2**-8, atol=2**-8)
