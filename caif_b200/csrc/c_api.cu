@@ -559,9 +559,11 @@ int caifq_cast(const void *src, int32_t src_dtype, void *dst, int32_t dst_dtype,
 {
   CAIFQ_CHECK_ARG(n >= 0, "cast: negative n");
   CAIFQ_CHECK_ARG(n == 0 || (src && dst), "cast: null pointer");
-  if (dst_dtype == CAIFQ_I8)
+  if (dst_dtype == CAIFQ_I8 || dst_dtype == CAIFQ_F16 || dst_dtype == CAIFQ_F32)
   {
-    note_codes_written(static_cast<cudaStream_t>(stream));  // int8 codes without scales are a valid weight
+    // int8 codes without scales are a valid weight; fp16 and fp32 are what scales are held in.  (bf16 weights and adapters
+    // are read behind the wait by every kernel that takes them.)
+    note_codes_written(static_cast<cudaStream_t>(stream));
   }
   return launch_cast(src, src_dtype, dst, dst_dtype, n, static_cast<cudaStream_t>(stream));
 }

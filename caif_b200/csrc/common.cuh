@@ -468,10 +468,10 @@ bool umma_swiglu_supported(const GroupedSwigluArgs &args);
 int launch_linear_umma_swiglu(const GroupedSwigluArgs &args, cudaStream_t s);
 bool umma_grouped_supported(const GroupedLinearArgs &args);
 int launch_linear_umma_grouped(const GroupedLinearArgs &args, cudaStream_t s);
-// The few-token kernel reads codes and scales ahead of the previous kernel's completion (dependent
-// launch).  The library's own quantize and cast kernels produce codes: the first few-token launch
-// on the same device and stream after one of them is a plain launch, which orders it (and
-// everything after it) behind that kernel.
+// Codes and scales are read ahead of the previous kernel's completion (dependent launch) by the few-token kernel, the
+// streaming kernel and the fp32 kernels.  The library's own quantize and cast kernels write codes and scales, and let the
+// next kernel in before they have: the first launch of an early reader on the same device and stream after one of them is
+// a plain launch, which orders it (and everything after it) behind that kernel.
 void note_codes_written(cudaStream_t s);
 bool take_codes_written(cudaStream_t s);
 // self-test hook: the next few-token launch of this thread waits for bytes that never arrive

@@ -890,3 +890,66 @@ def test_wide_outputs_of_few_hundred_rows_convert_in_the_kernel(storage):
         want = dy.double() @ tdense.T + (dy.double() @ lora.a.double().T) @ lora.b.double().T
         y, _ = nv.lora_linear_fwd(turned, lora, dy, compute, expanded=True)
         assert (y.double() - want).norm() <= 1e-2 * want.norm()
+
+
+def _early_reader(name, weight):
+    """A product by one of the kernels that read codes and scales ahead of the previous kernel's end."""
+    g = torch.Generator(device="cuda").manual_seed(29)
+    m = {"decode": 4, "stream": 64, "fp32_rows": 8, "fp32": 64, "experts": 8, "experts_stream": 96}[name]
+    x = torch.randn(m, weight.in_dim, generator=g, device="cuda")
+    if name.startswith("fp32"):
+        return lambda: nv.linear_fwd(weight, x)
+    x = x.bfloat16()
+    if not name.startswith("experts"):
+        return lambda: nv.linear_fwd(weight, x, torch.float32, nv.BF16)
+    ws = [weight] * 4
+    offsets = [m // 4 * e for e in range(5)]
+    return lambda: nv.grouped_expert_fwd(ws, ws, ws, offsets, x, nv.BF16)[1]
+
+
+@pytest.mark.parametrize("reader", ["decode", "stream", "fp32_rows", "fp32", "experts", "experts_stream"])
+@pytest.mark.parametrize("writer", ["cast_scales", "cast_scale", "cast_codes", "int4", "int8"])
+def test_products_see_what_was_just_written(reader, writer):
+    """The library's own writers of codes and scales let the next kernel in at once, and the products read codes and scales
+    before their wait: what was written just ahead on the stream has to be what is multiplied, bit for bit.  The weight lies
+    at the end of a large buffer, so that its writer is under way for long after its successor could have started."""
+    lib, stream = nv.lib(), torch.cuda.current_stream().cuda_stream
+    dim, pad = 1024, 1 << 26
+    n = dim * dim
+    g = torch.Generator(device="cuda").manual_seed(31)
+    source = 40.0 * torch.randn(pad + n, generator=g, device="cuda").clamp_(-3.0, 3.0)
+    if writer in ("cast_scales", "int4"):
+        codes = torch.randint(0, 256, ((pad + n) // 2,), dtype=torch.uint8, generator=g, device="cuda")
+        scales = torch.rand(pad + n // 128, generator=g, device="cuda").half()
+        at = pad if writer == "cast_scales" else pad // 128
+        weight = nv.Weight(codes[pad // 2:], nv.I4, dim, dim, scales[at:at + n // 128], group_size=128)
+    else:
+        codes = torch.randint(-127, 128, (pad + n,), dtype=torch.int8, generator=g, device="cuda")
+        scales = torch.rand(pad + 1, generator=g, device="cuda")
+        at = pad if writer == "cast_scale" else 0
+        weight = nv.Weight(codes[pad:], nv.I8, dim, dim, None if writer == "cast_codes" else scales[at:at + 1])
+    half = source.half()
+
+    def write():
+        if writer == "cast_scales":
+            return lib.caifq_cast(source.data_ptr(), nv.F32, scales.data_ptr(), nv.F16, scales.numel(), stream)
+        if writer == "cast_scale":
+            return lib.caifq_cast(half.data_ptr(), nv.F16, scales.data_ptr(), nv.F32, scales.numel(), stream)
+        if writer == "cast_codes":
+            return lib.caifq_cast(source.data_ptr(), nv.F32, codes.data_ptr(), nv.I8, codes.numel(), stream)
+        if writer == "int4":
+            return lib.caifq_quantize_int4_per_group(source.data_ptr(), codes.data_ptr(), scales.data_ptr(), pad + n, 128, stream)
+        return lib.caifq_quantize_int8_per_tensor(source.data_ptr(), codes.data_ptr(), scales.data_ptr(), pad + n, stream)
+
+    product = _early_reader(reader, weight)
+    before = product()
+    filler = torch.empty(1 << 28, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(4):
+        filler.zero_()      # (the host is ahead of the device from here on)
+    assert write() == 0
+    got = product()
+    torch.cuda.synchronize()
+    want = product()
+    assert torch.equal(got, want)
+    assert not torch.equal(before, want)
