@@ -689,12 +689,15 @@ __global__ void expand_prepare_kernel(const ExpandPrepare p)
 {
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   const int64_t first = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  // (the wait first: the thin product that follows starts on activations, which must then be complete)
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const void *codes = p.codes;
+  const __half *scales = p.scales;
+  // (the wait first: the thin product that follows starts on activations, which must then be complete.  The codes' and
+  // scales' addresses come out of it, so that their invariant loads stay behind it: a quantizer may be the kernel before)
+  asm volatile("griddepcontrol.wait;" : "+l"(codes), "+l"(scales)::"memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   if (blockIdx.y == 0 && p.wb != nullptr)
   {
-    expand_span<MODE>(p.codes, p.scales, p.wb, p.units, p.group_of);
+    expand_span<MODE>(codes, scales, p.wb, p.units, p.group_of);
     return;
   }
   const __nv_bfloat16 zero = __float2bfloat16(0.0f);

@@ -836,11 +836,15 @@ struct ExpandTable
 template <int MODE>
 __global__ void expand_kernel(const __grid_constant__ ExpandTable t, GroupOf group_of)
 {
-  // (the scratch may still be read by the kernel before this one; what follows may read the codes and scratch of others)
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int e = blockIdx.y;
-  expand_span<MODE>(t.codes[e], t.scales[e], t.dst[e], t.units[e], group_of);
+  const void *codes = t.codes[e];
+  const void *scales = t.scales[e];
+  // (the scratch may still be read by the kernel before this one; what follows may read the codes and scratch of others.
+  // The codes' and scales' addresses come out of the wait, so that their invariant loads stay behind it: a quantizer may be
+  // the kernel before)
+  asm volatile("griddepcontrol.wait;" : "+l"(codes), "+l"(scales)::"memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  expand_span<MODE>(codes, scales, t.dst[e], t.units[e], group_of);
 }
 
 namespace

@@ -1000,3 +1000,57 @@ def test_combine_of_many_and_of_few_tokens(dtype, dim):
                          if dispatch_map.dim() == 1 else dispatch_map[:64].contiguous(), offsets, 64)
     assert torch.equal(many[:64], few)
     assert torch.allclose(many.float(), x.float() * w.float().sum(1, keepdim=True), rtol=2**-8, atol=2**-8)
+
+
+@pytest.mark.parametrize("reader", ["experts", "lora", "concat"])
+@pytest.mark.parametrize("writer", ["int4", "int8", "cast_scales"])
+def test_expansions_see_what_was_just_written(reader, writer):
+    """An expansion to bf16 is launched ahead of its predecessor's end, and its predecessor may be a quantizer or a cast of
+    scales, which let it in at once: the same bits as when the device was idle in between."""
+    lib, stream = nv.lib(), torch.cuda.current_stream().cuda_stream
+    dim, pad = 512, 1 << 25
+    n = dim * dim
+    g = torch.Generator(device="cuda").manual_seed(37)
+    source = torch.randn(pad + n, generator=g, device="cuda")
+    if writer == "int8":
+        codes = torch.randint(-127, 128, (pad + n,), dtype=torch.int8, generator=g, device="cuda")
+        scales = torch.rand(1, generator=g, device="cuda")
+        weight = nv.Weight(codes[pad:], nv.I8, dim, dim, scales)
+    else:
+        codes = torch.randint(0, 256, ((pad + n) // 2,), dtype=torch.uint8, generator=g, device="cuda")
+        scales = torch.rand(pad + n // 128, generator=g, device="cuda").half()
+        at = pad if writer == "cast_scales" else pad // 128
+        weight = nv.Weight(codes[pad // 2:], nv.I4, dim, dim, scales[at:at + n // 128], group_size=128)
+    x = torch.randn(2048, dim, generator=g, device="cuda").bfloat16()
+    lora = nv.Lora(torch.randn(16, dim, generator=g, device="cuda").bfloat16() / 16,
+                   torch.randn(dim, 16, generator=g, device="cuda").bfloat16() / 64, 16.0)
+    expanded = torch.empty(max(1, nv.grouped_expert_expanded_bytes([weight], [weight], [weight], nv.BF16, nv.BF16)),
+                           dtype=torch.uint8, device="cuda")
+
+    def write():
+        if writer == "cast_scales":
+            return lib.caifq_cast(source.data_ptr(), nv.F32, scales.data_ptr(), nv.F16, scales.numel(), stream)
+        if writer == "int4":
+            return lib.caifq_quantize_int4_per_group(source.data_ptr(), codes.data_ptr(), scales.data_ptr(), pad + n, 128, stream)
+        return lib.caifq_quantize_int8_per_tensor(source.data_ptr(), codes.data_ptr(), scales.data_ptr(), pad + n, stream)
+
+    def read():
+        if reader == "experts":
+            nv.grouped_expert_expand([weight], [weight], [weight], expanded, nv.BF16, nv.BF16)
+            return expanded.clone()
+        if reader == "lora":
+            return nv.lora_linear_fwd(weight, lora, x, nv.BF16, expanded=True)[0]
+        return nv.linear_concat([weight, weight], x)
+
+    before = read()
+    filler = torch.empty(1 << 28, dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(4):
+        filler.zero_()      # (the host is ahead of the device from here on)
+    assert write() == 0
+    got = read()
+    torch.cuda.synchronize()
+    want = read()
+    assert expanded.numel() > 1
+    assert torch.equal(got, want)
+    assert not torch.equal(before, want)
