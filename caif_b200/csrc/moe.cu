@@ -37,9 +37,18 @@ __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return
 // The small kernels of a step follow one another: each is launched ahead of the previous one's end (launch_dependent),
 // lets the next one do the same, and reads nothing before the previous one has ended.  (Their inputs are not declared
 // __restrict__: loads that the compiler may take for invariant could move ahead of the wait.)
-__device__ __forceinline__ void after_previous_kernel()
+// `most`: CTAs of a grid that lets the next one in at once.  CTAs that are placed beside those of a larger grid take what
+// room is left, two on one SM and none on another, and keep it for as long as they run; after such a grid the next one
+// follows as its CTAs end.  (us a launch, back to back, next one in at once / as the CTAs end: rows of 14 KB, 256 CTAs 17.4 /
+// 6.5, 450 CTAs 18.9 / 10.4; softmax of 256, 256 CTAs 12.4 / 5.8; the map, 1024 threads a CTA, 128 CTAs 18.6 / 13.5.  Up to a
+// CTA an SM there is room for all: rows of 14 KB, 128 CTAs 5.9, launched plainly 6.2.)
+constexpr unsigned kEarlyCtas = 148;
+__device__ __forceinline__ void after_previous_kernel(unsigned most = 0xFFFFFFFFu)
 {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (gridDim.x <= most)
+  {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
@@ -334,7 +343,7 @@ __device__ __forceinline__ void softmax_absorb(float &m, float &s, float m_other
 template <typename T>
 __global__ void router_softmax_kernel(const T *logits, const T *bias, T *probs, int rows, int cols)
 {
-  after_previous_kernel();
+  after_previous_kernel(kEarlyCtas);
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * warps_per_block + (threadIdx.x >> 5);
@@ -743,7 +752,7 @@ __global__ void __launch_bounds__(kMapThreads)
 build_dispatch_kernel(const int *expert_indices, int64_t total, int64_t slice, int num_experts, int capacity,
                       int *dispatch_map, int *expert_offsets)
 {
-  after_previous_kernel();
+  after_previous_kernel(kEarlyCtas / 2);
   extern __shared__ int s_map[];
   int *running = s_map;                      // [E]
   int *warp_hist = s_map + num_experts;      // [warps][E]
@@ -882,7 +891,7 @@ template <typename T>
 __global__ void moe_dispatch_kernel(const T *input, const int *expert_indices, const int *dispatch_map,
                                     const int *expert_offsets, T *buffer, int64_t assignments, int dim, int top_k)
 {
-  after_previous_kernel();
+  after_previous_kernel(kEarlyCtas);
   const int lane = threadIdx.x & 31;
   const int64_t a = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   if (a >= assignments)

@@ -74,3 +74,19 @@ def act(rng, m, k, dtype_code):
     """N(0,1) activations already rounded to the storage dtype; returns (fp32 numpy, device tensor)."""
     x = orc.round_through(rng.standard_normal((m, k)).astype(np.float32), dtype_code)
     return x, to_dev(x, TORCH_DTYPE[dtype_code])
+
+
+def best_time(fn, calls=20, rounds=7):
+    """Microseconds of a call among others of its kind: the least of several rounds, so that noise only adds."""
+    for _ in range(3):
+        fn()
+    begin, end = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    best = float("inf")
+    for _ in range(rounds):
+        begin.record()
+        for _ in range(calls):
+            fn()
+        end.record()
+        end.synchronize()
+        best = min(best, begin.elapsed_time(end) * 1e3 / calls)
+    return best

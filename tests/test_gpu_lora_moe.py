@@ -7,7 +7,7 @@ import torch
 import caif_oracle as orc
 import refkernels as ref
 from caif_b200 import native as nv
-from gpu_util import TORCH_DTYPE, act, dev, make_weight, max_rel_err, to_dev
+from gpu_util import TORCH_DTYPE, act, best_time, dev, make_weight, max_rel_err, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -1054,3 +1054,58 @@ def test_expansions_see_what_was_just_written(reader, writer):
     assert expanded.numel() > 1
     assert torch.equal(got, want)
     assert not torch.equal(before, want)
+
+
+def _route(tokens, experts, top_k, dim, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    logits = torch.randn(tokens, experts, generator=g, device="cuda")
+    return logits, torch.randn(tokens, dim, generator=g, device="cuda").bfloat16()
+
+
+@pytest.mark.parametrize("tokens,experts,top_k", [
+    (592, 8, 2), (593, 8, 2),            # 1184 rows are dispatched by 148 CTAs, 1186 by one more
+    (1184, 16, 1), (1185, 16, 1),        # the same for the softmax
+    (74 * 512, 8, 2), (74 * 512 + 1, 8, 2),   # the map's 74 CTAs of 1024 entries, and one more
+])
+def test_routing_steps_follow_one_another(tokens, experts, top_k):
+    """The steps of a routed layer back to back, twice, give the bits that they give one at a time: grids that let the next
+    step in at once and grids whose CTAs have to end first."""
+    logits, x = _route(tokens, experts, top_k, 64, 41)
+
+    def steps(after):
+        out = []
+        for _ in range(2):
+            probs = after(nv.moe_softmax(logits))
+            idx, val = after(nv.moe_topk(probs, top_k))
+            w = after(nv.cast(nv.moe_normalize_rows(val), torch.bfloat16))
+            dmap, offs = after(nv.moe_build_dispatch(idx, experts)[:2])
+            buf = after(nv.moe_dispatch(x, idx, dmap, offs, tokens * top_k))
+            out += [probs, idx, w, dmap, offs, buf, after(nv.moe_combine(buf, idx, w, dmap, offs, tokens))]
+        return out
+
+    def alone(v):
+        torch.cuda.synchronize()
+        return v
+
+    want = steps(alone)
+    filler = torch.empty(1 << 28, dtype=torch.uint8, device="cuda")
+    filler.zero_()
+    filler.zero_()
+    got = steps(lambda v: v)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    assert torch.allclose(want[0], torch.softmax(logits, -1), rtol=1e-5, atol=1e-7)
+
+
+def test_dispatch_of_a_few_ctas_per_sm_is_no_slower_than_combine():
+    """Copying rows costs no more than adding them up.  (With the next grid let in at once 2048 rows of 14 KB took 17 us and
+    their sums 10; as the CTAs end 6.5.)"""
+    tokens, experts, top_k, dim = 1024, 8, 2, 7168
+    logits, x = _route(tokens, experts, top_k, dim, 43)
+    idx, val = nv.moe_topk(nv.moe_softmax(logits), top_k)
+    w = val.bfloat16()
+    dmap, offs = nv.moe_build_dispatch(idx, experts)[:2]
+    buf = nv.moe_dispatch(x, idx, dmap, offs, tokens * top_k)
+    copy = best_time(lambda: nv.moe_dispatch(x, idx, dmap, offs, tokens * top_k))
+    add = best_time(lambda: nv.moe_combine(buf, idx, w, dmap, offs, tokens))
+    assert copy < 1.25 * add, (copy, add)
