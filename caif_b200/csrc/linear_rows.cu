@@ -5,8 +5,8 @@
 // The float-storage cell of CAIF_DeviceFrozenLinear (src/caif_device_frozen_linear.cpp:381-524) and the router's
 // product over the experts (src/caif_device_moe_router.cpp:233-260).  Bound by reading the weight once when it is
 // large, by latency when it is small: a router of 64 x 2048 on 16 tokens ran as ONE block of the fp32-FMA kernel that
-// walked all of k (191 us, 7.7 here; alone, launched ahead of the previous kernel it costs less), by L2 for many rows (16384 tokens: 48 us, the FMA kernel 270).  Here a CTA owns
-// NT * 8 output columns and 16 rows, its eight warps split k and stream both operands from global memory straight into
+// walked all of k (191 us; here 7.7 by itself, 4.0 among calls of its kind), by L2 for many rows (16384 tokens: 40 us, the FMA
+// kernel 270).  Here a CTA owns NT * 8 output columns and 16 rows, its eight warps split k and stream both operands straight into
 // bf16 tensor-core fragments, sixteen bytes a lane and operand (the order of k inside a fragment is the same for both,
 // which is all a dot product needs); the eight partial tiles meet in shared memory.  Products are exact in fp32 and
 // accumulate in fp32, so fp32 and bf16 compute are the same here.  The tensor core truncates where it adds, so a chain of
@@ -23,6 +23,7 @@ namespace
 
 constexpr int kRowsWarps = 8;
 constexpr int kRowsChain = 4;   // k-steps of 32 in one chain of MMAs
+constexpr unsigned kRowsEarly = 37;   // CTAs (of 256 threads) of a grid that leaves three quarters of the SMs free
 constexpr int64_t kRowsMost = 16 * 65535;   // rows of a launch: the grid's second dimension
 
 __device__ __forceinline__ void mma_rows(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
@@ -41,6 +42,16 @@ linear_rows_kernel(const __nv_bfloat16 *x, const __nv_bfloat16 *w, void *y, int 
 {
   constexpr int UNROLL = kRowsChain * CHAINS;
   __shared__ float part[kRowsWarps][16][NT * 8 + 1];
+  // Launched ahead of the previous kernel's end.  A few CTAs let the next kernel in at once (a router's softmax: 0.8 us of an
+  // expert layer); of more, it follows as they end: CTAs of the next kernel that are placed earlier share SMs with this one's
+  // while others have none (us back to back, let in at once / after the loads / at the end: 14336 -> 1024, 16 rows 19.2 / - /
+  // 11.7; -> 1184 11.9 / 13.2 / 11.8; -> 3072 24.5 / 24.1 / 21.2).
+  // (The operands' addresses come out of the wait, so that their read-only loads stay behind it.)
+  if (gridDim.x * gridDim.y <= kRowsEarly)
+  {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  }
+  asm volatile("griddepcontrol.wait;" : "+l"(x), "+l"(w)::"memory");
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2;
@@ -65,9 +76,6 @@ linear_rows_kernel(const __nv_bfloat16 *x, const __nv_bfloat16 *w, void *y, int 
     sum[nt][0] = sum[nt][1] = sum[nt][2] = sum[nt][3] = 0.0f;
   }
   const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
-  // (launched ahead of the previous kernel's end; the operands are not __restrict__, whose loads could move ahead of the wait)
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int st = begin; st < end; st += UNROLL)
   {
     uint4 xa[UNROLL], xb[UNROLL], wv[UNROLL][NT];
@@ -75,12 +83,12 @@ linear_rows_kernel(const __nv_bfloat16 *x, const __nv_bfloat16 *w, void *y, int 
     for (int u = 0; u < UNROLL; ++u)
     {
       const bool in = st + u < end;
-      xa[u] = (in && lo_ok) ? x_lo[(st + u) * 4] : zero4;
-      xb[u] = (in && hi_ok) ? x_hi[(st + u) * 4] : zero4;
+      xa[u] = (in && lo_ok) ? __ldg(x_lo + (st + u) * 4) : zero4;
+      xb[u] = (in && hi_ok) ? __ldg(x_hi + (st + u) * 4) : zero4;
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt)
       {
-        wv[u][nt] = in ? w_ptr[nt][(st + u) * 4] : zero4;
+        wv[u][nt] = in ? __ldg(w_ptr[nt] + (st + u) * 4) : zero4;
       }
     }
 #pragma unroll
@@ -158,12 +166,17 @@ int launch_linear_rows(const LinearArgs &g, cudaStream_t s)
   const __nv_bfloat16 *x = static_cast<const __nv_bfloat16 *>(g.a);
   const __nv_bfloat16 *w = static_cast<const __nv_bfloat16 *>(g.w.codes);
   const int acc = g.accumulate ? 1 : 0;
-  // 32 columns a CTA share the activations' loads; narrow outputs take 8, for more CTAs
+  // 32 columns a CTA share the activations' loads; narrow outputs take 8, for more CTAs, and two chains' loads at a time as
+  // long as all CTAs are resident: with 66 registers a thread three are on an SM, and a fourth would be a second wave (us, one
+  // row, two chains / one: 4096 -> 3072 4.9 / 6.9, 14336 -> 3552 25 / 31; beyond, 4096 -> 4096 7.7 / 6.9, 14336 -> 4096 49 / 32)
+  const int sms = device_sm_count();
   const int wide = (g.w.out_dim + 31) / 32;
-  const bool many = wide * row_tiles >= 148;
+  const bool many = wide * row_tiles >= sms;
   const dim3 grid(static_cast<unsigned>(many ? wide : (g.w.out_dim + 7) / 8), row_tiles);
-  CAIFQ_CHECK_CUDA(launch_dependent(many ? linear_rows_kernel<4, 1> : linear_rows_kernel<1, 2>, grid, dim3(kRowsWarps * 32),
-                                    0, s, x, w, g.c, g.c_dtype, acc, g.m, g.w.in_dim, g.w.out_dim));
+  const bool one_wave = grid.x * grid.y <= 3u * static_cast<unsigned>(sms);
+  auto kernel = many ? linear_rows_kernel<4, 1> : (one_wave ? linear_rows_kernel<1, 2> : linear_rows_kernel<1, 1>);
+  CAIFQ_CHECK_CUDA(launch_dependent(kernel, grid, dim3(kRowsWarps * 32), 0, s, x, w, g.c, g.c_dtype, acc, g.m, g.w.in_dim,
+                                    g.w.out_dim));
   return CAIFQ_OK;
 }
 

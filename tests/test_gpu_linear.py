@@ -13,7 +13,7 @@ import torch
 
 import caif_oracle as orc
 from caif_b200 import native as nv
-from gpu_util import TORCH_DTYPE, act, make_weight, max_rel_err, to_dev
+from gpu_util import TORCH_DTYPE, act, best_time, make_weight, max_rel_err, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -953,3 +953,31 @@ def test_products_see_what_was_just_written(reader, writer):
     want = product()
     assert torch.equal(got, want)
     assert not torch.equal(before, want)
+
+
+@pytest.mark.parametrize("m", [1, 16, 17])
+@pytest.mark.parametrize("out_dim", [1176, 3544, 3552, 3553, 3560, 4712, 4737])
+def test_bf16_weight_either_side_of_a_resident_wave(m, out_dim):
+    """147, 443 to 445 and 589 CTAs of 8 columns (two chains' loads at a time while three CTAs an SM take them all), and 32
+    columns a CTA beyond.  Bound: products are exact, an fp32 sum of chains of 128 is within 1e-6 of the norm."""
+    in_dim = 544       # 17 steps of 32: warps of two and of three
+    g = torch.Generator(device="cuda").manual_seed(out_dim + m)
+    w = torch.randn(out_dim, in_dim, generator=g, device="cuda").bfloat16()
+    x = torch.randn(m, in_dim, generator=g, device="cuda").bfloat16()
+    want = x.double() @ w.double().T
+    weight = nv.Weight(w, nv.BF16, in_dim, out_dim)
+    got = nv.linear_fwd(weight, x)
+    assert (got.double() - want).norm() <= 1e-6 * want.norm()
+    res = torch.randn(m, out_dim, generator=g, device="cuda")
+    assert torch.equal(nv.linear_fwd_residual(weight, x, res.clone()), got + res)
+
+
+def test_a_wider_bf16_weight_takes_no_second_wave():
+    """14336 -> 4096, one row, is 15 % more bytes than 14336 -> 3552.  (With two chains' loads a time its 512 CTAs were two
+    waves: 49 us against 25; 32 us with one.)"""
+    x = torch.randn(1, 14336, device="cuda").bfloat16()
+    t = {}
+    for out_dim in (3552, 4096):
+        weight = nv.Weight(torch.randn(out_dim, 14336, device="cuda").bfloat16(), nv.BF16, 14336, out_dim)
+        t[out_dim] = best_time(lambda: nv.linear_fwd(weight, x))
+    assert t[4096] < 1.6 * t[3552], t
