@@ -596,26 +596,30 @@ __device__ __forceinline__ float cast_one<int8_t, float>(int8_t v) { return stat
 template <typename S, typename D>
 __global__ void cast_kernel(const S *src, D *dst, int64_t n)
 {
-  // (launched ahead of the previous kernel's end; not __restrict__, whose loads could move ahead of the wait)
+  // Launched ahead of the previous kernel's end; the source's address comes out of the wait, so that its read-only loads stay
+  // behind it.  Four elements a trip whose loads nothing holds up: neither a bound of their own nor stores that they might
+  // overlap (us, bounded and plain / so: 10 M fp32 -> bf16 10.0 / 6.9, 100 M fp32 -> int8 109 / 80; one a trip 8.2 and 90).
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" : "+l"(src)::"memory");
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += 4 * stride)
+  int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  for (; i + 3 * stride < n; i += 4 * stride)
   {
     S v[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j)
     {
-      v[j] = src[i + j * stride < n ? i + j * stride : i];
+      v[j] = __ldg(src + i + j * stride);
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j)
     {
-      if (i + j * stride < n)
-      {
-        dst[i + j * stride] = cast_one<float, D>(cast_one<S, float>(v[j]));
-      }
+      dst[i + j * stride] = cast_one<float, D>(cast_one<S, float>(v[j]));
     }
+  }
+  for (; i < n; i += stride)
+  {
+    dst[i] = cast_one<float, D>(cast_one<S, float>(__ldg(src + i)));
   }
 }
 

@@ -7,7 +7,7 @@ import torch
 import caif_oracle as orc
 import refkernels as ref
 from caif_b200 import native as nv
-from gpu_util import dev, to_dev
+from gpu_util import best_time, dev, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -217,3 +217,29 @@ def test_int8_per_channel_clusters_bit_exact(rows, cols):
     assert np.array_equal(_bits(s), os_.view(np.int32))
     live = np.isfinite(x.numpy() / os_[None, :])   # (what a NaN or an infinity is cast to is not defined on the CPU)
     assert np.array_equal(q.cpu().numpy()[live], oq[live])
+
+
+@pytest.mark.parametrize("n", [1, 255, 257, 606207, 606209, 3 * 606208, 3 * 606208 + 1, 4 * 606208 - 1, 4 * 606208, 4 * 606208 + 1,
+                               7 * 606208 + 300])
+@pytest.mark.parametrize("src,dst", [(torch.float32, torch.bfloat16), (torch.float16, torch.float32),
+                                     (torch.bfloat16, torch.bfloat16)])
+def test_cast_trips_of_four(n, src, dst):
+    """A grid of 2368 blocks takes 606208 elements at a time, four times a trip: whole trips, trips that are cut, none; a
+    source that starts on any element; the same buffer as source and result."""
+    g = torch.Generator(device="cuda").manual_seed(n)
+    base = torch.randn(n + 1, generator=g, device="cuda").to(src)
+    for x in (base[:n], base[1:]):
+        assert torch.equal(nv.cast(x, dst), x.to(dst))
+    if src == dst:
+        want = base[:n].clone()
+        rc = nv.lib().caifq_cast(base.data_ptr(), nv.dtype_code(src), base.data_ptr(), nv.dtype_code(dst), n,
+                                 torch.cuda.current_stream().cuda_stream)
+        assert rc == 0 and torch.equal(base[:n], want)
+
+
+def test_cast_to_a_byte_moves_fewer_bytes_than_to_a_word():
+    """500 MB against 800.  (With a bound for each element of a trip 109 us against 128; 80 without.)"""
+    x = torch.randn(100_000_000, device="cuda")
+    byte = best_time(lambda: nv.cast(x, torch.int8), calls=5)
+    word = best_time(lambda: nv.cast(x, torch.float32), calls=5)
+    assert byte < 0.74 * word, (byte, word)
