@@ -1041,9 +1041,8 @@ struct Vec16
   static constexpr int N = 16 / static_cast<int>(sizeof(T));
 };
 
-// CONSTANT: through the read-only path, for what no kernel beside this one writes.  Sums of gathered rows need it (16384
-// tokens top-6, rows of 2048: combine 85 us against 103, dispatch backward 85 against 105), products of two rows do not
-// (gradients of the weights 87 against 78).
+// CONSTANT: through the read-only path.  Sums of many gathered rows need it (16384 tokens top-6, rows of 2048: combine 85 us
+// against 103, dispatch backward 85 against 105), products of two rows do not (gradients of the weights 87 against 78).
 template <typename T, bool CONSTANT = false>
 __device__ __forceinline__ void load_vec(const T *p, float (&v)[Vec16<T>::N])
 {
@@ -1117,16 +1116,15 @@ __global__ void swiglu_bwd_vec_kernel(const T *__restrict__ g_hidden, const T *_
   }
 }
 
-// DEPENDENT: launched ahead of the previous kernel's end, whose results it then must not read as constants
-template <typename T, bool DEPENDENT>
+// CONSTANT: as in load_vec.  Launched ahead of the end of the kernel that wrote the rows: their address comes out of the wait,
+// so that read-only loads stay behind it.
+template <typename T, bool CONSTANT>
 __global__ void moe_combine_vec_kernel(const T *buffer, const int *expert_indices, const T *expert_weights,
                                        const int *dispatch_map, const int *expert_offsets, T *output, int num_tokens,
                                        int dim, int top_k)
 {
-  if (DEPENDENT)
-  {
-    after_previous_kernel();
-  }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" : "+l"(buffer)::"memory");
   constexpr int N = Vec16<T>::N;
   const int dim_vec = dim / N;
   const int64_t total = static_cast<int64_t>(num_tokens) * dim_vec;
@@ -1149,7 +1147,7 @@ __global__ void moe_combine_vec_kernel(const T *buffer, const int *expert_indice
       {
         const float w = to_f<T>(expert_weights[token * top_k + k]);
         float v[N];
-        load_vec<T, !DEPENDENT>(buffer + (static_cast<int64_t>(expert_offsets[e]) + pos) * dim + d, v);
+        load_vec<T, CONSTANT>(buffer + (static_cast<int64_t>(expert_offsets[e]) + pos) * dim + d, v);
 #pragma unroll
         for (int j = 0; j < N; ++j)
         {
@@ -1601,15 +1599,13 @@ static cudaError_t launch_combine_inst(const T *buffer, const int *indices, cons
   const bool vec16 = vec && (dim % Vec16<T>::N) == 0;
   const int64_t items = static_cast<int64_t>(num_tokens) * (vec16 ? dim / Vec16<T>::N : dim);
   const dim3 grid(static_cast<unsigned>(ew_grid(items)));
-  // More pieces than one trip of the largest grid: the rate of the reads counts, not the gap before the launch
-  if (vec16 && items > 148 * 16 * 256)
-  {
-    moe_combine_vec_kernel<T, false>
-        <<<grid, 256, 0, s>>>(buffer, indices, weights, map, offsets, output, num_tokens, dim, top_k);
-    return cudaSuccess;
-  }
-  return launch_dependent(vec16 ? moe_combine_vec_kernel<T, true> : moe_combine_kernel<T>, grid, dim3(256), 0, s, buffer, indices,
-                          weights, map, offsets, output, num_tokens, dim, top_k);
+  // More pieces than six CTAs an SM take at a time: the rate of the reads counts, and the read-only path has the better one
+  // (us, bf16, plain / read-only: 1024 tokens top-8, rows of 2048, 262144 pieces 8.6 / 7.0, of 4096 13.8 / 12.0; below, 400
+  // tokens top-6, rows of 4096, 204800 pieces 4.9 / 6.2, 1500 of 1024, 192000 pieces 4.8 / 6.2)
+  const bool many = items > static_cast<int64_t>(device_sm_count()) * 6 * 256;
+  auto vectors = many ? moe_combine_vec_kernel<T, true> : moe_combine_vec_kernel<T, false>;
+  return launch_dependent(vec16 ? vectors : moe_combine_kernel<T>, grid, dim3(256), 0, s, buffer, indices, weights, map, offsets,
+                          output, num_tokens, dim, top_k);
 }
 
 int launch_moe_combine(const void *buffer, int dtype, const int *expert_indices, const void *expert_weights,

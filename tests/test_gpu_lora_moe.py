@@ -1109,3 +1109,29 @@ def test_dispatch_of_a_few_ctas_per_sm_is_no_slower_than_combine():
     copy = best_time(lambda: nv.moe_dispatch(x, idx, dmap, offs, tokens * top_k))
     add = best_time(lambda: nv.moe_combine(buf, idx, w, dmap, offs, tokens))
     assert copy < 1.25 * add, (copy, add)
+
+
+@pytest.mark.parametrize("tokens", [888, 889, 2368, 2369])
+def test_combine_reads_what_was_just_written(tokens):
+    """888 tokens of 256 pieces are what plain loads read, one more and the read-only path does; both directly behind the
+    kernel that writes the rows, in a buffer that held others and was read before.  The same bits as one token at a time."""
+    experts, top_k, dim = 16, 8, 2048
+    logits, x = _route(tokens, experts, top_k, dim, 47)
+    idx, val = nv.moe_topk(nv.moe_softmax(logits), top_k)
+    w = val.bfloat16()
+    dmap, offs = nv.moe_build_dispatch(idx, experts)[:2]
+    lib, stream, rows = nv.lib(), torch.cuda.current_stream().cuda_stream, tokens * top_k
+    buf = nv.moe_dispatch(x, idx, dmap, offs, rows)
+
+    def rewrite(src):
+        assert lib.caifq_cast(src.data_ptr(), nv.F32, buf.data_ptr(), nv.BF16, rows * dim, stream) == 0
+
+    sources = [torch.randn(rows, dim, device="cuda") for _ in range(2)]
+    for src in sources + sources:
+        rewrite(src)
+        got = nv.moe_combine(buf, idx, w, dmap, offs, tokens)
+        torch.cuda.synchronize()
+        halves = [nv.moe_combine(buf, idx[a:b].contiguous(), w[a:b].contiguous(), dmap.view(tokens, top_k)[a:b].contiguous(),
+                                 offs, b - a) for a, b in ((0, 400), (400, 800), (800, tokens))]
+        assert torch.equal(got[:800], torch.cat(halves[:2]))
+        assert torch.equal(got[800:], halves[2])
