@@ -39,10 +39,10 @@ __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return
 // __restrict__: loads that the compiler may take for invariant could move ahead of the wait.)
 // `most`: CTAs of a grid that lets the next one in at once.  CTAs that are placed beside those of a larger grid take what
 // room is left, two on one SM and none on another, and keep it for as long as they run; after such a grid the next one
-// follows as its CTAs end.  (us a launch, back to back, next one in at once / as the CTAs end: rows of 14 KB, 256 CTAs 17.4 /
-// 6.5, 450 CTAs 18.9 / 10.4; softmax of 256, 256 CTAs 12.4 / 5.8; the map, 1024 threads a CTA, 128 CTAs 18.6 / 13.5.  Up to a
-// CTA an SM there is room for all: rows of 14 KB, 128 CTAs 5.9, launched plainly 6.2.)
-constexpr unsigned kEarlyCtas = 148;
+// follows as its CTAs end.  Two grids of half the SMs have an SM for every CTA.  (us a launch, back to back, next one in at
+// once / as the CTAs end: rows of 14 KB, 96 CTAs 6.3 / 4.3, 256 CTAs 17.4 / 6.5, 450 CTAs 18.9 / 10.4; softmax of 256, 128 CTAs
+// 6.2 / 5.5, 256 CTAs 12.4 / 5.8; top-8 of 256, 256 CTAs 11.5 / 4.7; the map, 128 CTAs 18.6 / 13.5.)
+constexpr unsigned kEarlyCtas = 74;
 __device__ __forceinline__ void after_previous_kernel(unsigned most = 0xFFFFFFFFu)
 {
   if (gridDim.x <= most)
@@ -61,7 +61,7 @@ template <typename T>
 __global__ void topk_kernel(const T *input, int *indices, T *values,
                             int batch, int dim, int k)
 {
-  after_previous_kernel();
+  after_previous_kernel(kEarlyCtas);
   extern __shared__ float s_rows[];
   const int warps_per_block = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5;
@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(kMapThreads)
 build_dispatch_kernel(const int *expert_indices, int64_t total, int64_t slice, int num_experts, int capacity,
                       int *dispatch_map, int *expert_offsets)
 {
-  after_previous_kernel(kEarlyCtas / 2);
+  after_previous_kernel(kEarlyCtas);
   extern __shared__ int s_map[];
   int *running = s_map;                      // [E]
   int *warp_hist = s_map + num_experts;      // [warps][E]
