@@ -929,8 +929,17 @@ linear_decode_kernel(const __grid_constant__ DecodeParams p, const __grid_consta
   }  // rounds
 }
 
-// One CTA per SM, fewer when the host runs a collective beside this kernel and wants to leave it SMs.
+// One CTA per SM, fewer when the host runs a collective beside this kernel and wants to leave it SMs.  Experts take two, of
+// half an SM each, and are not taken under a limit of either persistent kernel: twice as many CTAs would not keep to it, and
+// with as many as it says half of each SM idles (three products of 64 experts of 2048 x 1408, 8 rows each, limit of 132:
+// int4 176 us, int8 231, the streaming kernel 154 and 147).
 int sm_count() { return persistent_ctas("CAIFQ_DECODE_CTAS"); }
+int expert_ctas() { return 2 * device_sm_count(); }
+bool limited()
+{
+  const int sms = device_sm_count();
+  return persistent_ctas("CAIFQ_DECODE_CTAS") < sms || persistent_ctas("CAIFQ_UMMA_CTAS") < sms;
+}
 
 // Streams (per device) on which one of this library's calls has just written codes or scales.
 std::mutex g_written_mutex;
@@ -995,7 +1004,7 @@ int launch_decode_inst(const DecodeParams &p, const DecodeTable<N> &table, uint3
                                           static_cast<int>(kSmemFull)));
     configured[dev].store(true, std::memory_order_release);
   }
-  int grid = sm_count() * (N > 1 && WARPS == 8 ? 2 : 1);
+  int grid = N > 1 ? expert_ctas() : sm_count();
   if (grid > p.num_quanta)
   {
     grid = p.num_quanta;
@@ -1058,7 +1067,7 @@ Layout layout_for(const caifq_weight &w, int64_t m, bool experts)
   const uint32_t park = static_cast<uint32_t>(l.warps * kTileRows * tokp_for(m) * sizeof(float));
   const int quantum = experts ? kTileRows : kRowQuantum;
   const int quanta = (w.out_dim + quantum - 1) / quantum;
-  int grid = sm_count() * (experts ? 2 : 1);
+  int grid = experts ? expert_ctas() : sm_count();
   if (grid > quanta)
   {
     grid = quanta;
@@ -1323,7 +1332,7 @@ bool decode_grouped_supported(const GroupedStreamArgs &g)
 {
   int most = 0;
   const int entries = g.count < 1 ? -1 : decode_entries(g, nullptr, most);
-  if (entries < 1 || g.accumulate || !is_float_dtype(g.c_dtype) || (reinterpret_cast<uintptr_t>(g.a) & 15u) != 0 ||
+  if (limited() || entries < 1 || g.accumulate || !is_float_dtype(g.c_dtype) || (reinterpret_cast<uintptr_t>(g.a) & 15u) != 0 ||
       (g.compute_dtype != CAIFQ_F32 && g.compute_dtype != CAIFQ_BF16))
   {
     return false;

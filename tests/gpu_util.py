@@ -1,4 +1,8 @@
 """Helpers shared by the GPU parity tests (test infrastructure)."""
+import json
+import os
+import tempfile
+
 import numpy as np
 import torch
 
@@ -90,3 +94,18 @@ def best_time(fn, calls=20, rounds=7):
         end.synchronize()
         best = min(best, begin.elapsed_time(end) * 1e3 / calls)
     return best
+
+
+def kernels_of(fn):
+    """[(name, number of CTAs)] of the kernels that fn launches, in their order."""
+    torch.cuda.synchronize()
+    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
+        fn()
+        torch.cuda.synchronize()
+    with tempfile.TemporaryDirectory() as folder:
+        path = os.path.join(folder, "trace.json")
+        prof.export_chrome_trace(path)
+        with open(path) as f:
+            events = json.load(f)["traceEvents"]
+    launched = sorted((e for e in events if e.get("cat") == "kernel"), key=lambda e: e["ts"])
+    return [(e["name"], int(np.prod(e["args"]["grid"]))) for e in launched]

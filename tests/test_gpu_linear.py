@@ -13,7 +13,7 @@ import torch
 
 import caif_oracle as orc
 from caif_b200 import native as nv
-from gpu_util import TORCH_DTYPE, act, best_time, make_weight, max_rel_err, to_dev
+from gpu_util import TORCH_DTYPE, act, best_time, kernels_of, make_weight, max_rel_err, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -981,3 +981,40 @@ def test_a_wider_bf16_weight_takes_no_second_wave():
         weight = nv.Weight(torch.randn(out_dim, 14336, device="cuda").bfloat16(), nv.BF16, 14336, out_dim)
         t[out_dim] = best_time(lambda: nv.linear_fwd(weight, x))
     assert t[4096] < 1.6 * t[3552], t
+
+
+@pytest.mark.parametrize("storage", [orc.I4, orc.I8])
+@pytest.mark.parametrize("limit,how", [(1, "call"), (37, "call"), (132, "call"), (90, "CAIFQ_DECODE_CTAS"),
+                                       (90, "CAIFQ_UMMA_CTAS")])
+def test_experts_of_few_rows_keep_to_a_limit_of_ctas(storage, limit, how, monkeypatch):
+    """A host's collective finds the SMs that the limit leaves it: no launch of the experts' products has more CTAs.  (Without
+    a limit the few-token kernel has two an SM; the streaming kernel, which rounds an int4 weight to bf16, keeps to one.)"""
+    rng = np.random.default_rng(59)
+    counts = [1, 5, 0, 8] * 8
+    gate, up, down = ([make_weight(rng, o, i, storage)[0] for _ in counts] for o, i in ((384, 512), (384, 512), (512, 384)))
+    offsets = np.concatenate([[0], np.cumsum(counts)]).astype(np.int32).tolist()
+    x = torch.randn(offsets[-1], 512, device="cuda").bfloat16()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+
+    def run():
+        return nv.grouped_expert_fwd(gate, up, down, offsets, x, nv.BF16)
+
+    def products():
+        return [(name.split("linear_")[1].split("_kernel")[0], ctas) for name, ctas in kernels_of(run) if "linear_" in name]
+
+    want = run()
+    assert products() == [("decode", 2 * sms), ("decode", 2 * sms)]
+    if how == "call":
+        nv.lib().caifq_set_cta_limit(limit)
+    else:
+        monkeypatch.setenv(how, str(limit))
+    try:
+        got = run()
+        ran = products()
+        most = sms if how == "CAIFQ_DECODE_CTAS" else limit     # (the other kernel's variable)
+        assert len(ran) == 2 and all(name == "stream" and ctas <= most for name, ctas in ran)
+        assert nv.lib().caifq_device_status() == 0
+    finally:
+        nv.lib().caifq_set_cta_limit(0)
+    for a, b in zip(got, want):
+        assert (a.float() - b.float()).norm() <= 1e-2 * b.float().norm()
