@@ -1488,9 +1488,9 @@ static bool few_tokens_each(const GroupedStreamArgs &g)
     passes += (rows + 15) / 16;
     most = rows > most ? rows : most;
   }
-  if (most <= 8 || g.weights[0].storage != CAIFQ_I4)
+  if (most <= 8)
   {
-    return most <= 8;
+    return true;
   }
   const int64_t pieces = (g.weights[0].in_dim + 127) / 128;
   return 82 * passes * ((pieces + 15) / 16 * 16) <= 100 * live * pieces;

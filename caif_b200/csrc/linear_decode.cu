@@ -1338,6 +1338,10 @@ bool decode_grouped_supported(const GroupedStreamArgs &g)
     return false;
   }
   const caifq_weight &w0 = g.weights[0];
+  if (w0.storage != CAIFQ_I4 && most > 8)   // (a second tile of tokens pays for int4 alone, see the caller)
+  {
+    return false;
+  }
   if ((w0.out_dim % kTileRows) != 0 || static_cast<int64_t>(entries) * w0.out_dim > 0x7FFFFFFF)
   {
     return false;
@@ -1404,8 +1408,6 @@ int launch_linear_decode_grouped(const GroupedStreamArgs &g, cudaStream_t s)
     CAIFQ_DECODE_CASE(8, 1, 2)
     CAIFQ_DECODE_CASE(8, 1, 4)
     CAIFQ_DECODE_CASE(8, 1, 8)
-    CAIFQ_DECODE_CASE(8, 2, 2)
-    CAIFQ_DECODE_CASE(8, 2, 4)
   }
 #undef CAIFQ_DECODE_CASE
   set_error("frozen experts (decode): no kernel instance for in_dim=%d rows=%d", w.in_dim, most);

@@ -7,7 +7,7 @@ import torch
 import caif_oracle as orc
 import refkernels as ref
 from caif_b200 import native as nv
-from gpu_util import TORCH_DTYPE, act, best_time, dev, make_weight, max_rel_err, to_dev
+from gpu_util import TORCH_DTYPE, act, best_time, dev, kernels_of, make_weight, max_rel_err, to_dev
 
 pytestmark = pytest.mark.gpu
 
@@ -870,8 +870,8 @@ def test_experts_of_few_rows(storage, compute, counts, gated):
 @pytest.mark.parametrize("counts,in_dim,hid", [
     ([1] * 7, 2048, 1408),                  # one tile of tokens; 11 pieces of k for eight warps of two
     ([8, 0, 3, 1], 1024, 384),
-    ([16, 9, 0, 0, 2], 2048, 2048),         # two tiles of tokens
-    ([17, 1, 1, 1, 1, 1, 1, 1], 2048, 2048),  # 16 rows and one more
+    ([16, 9, 0, 0, 2], 2048, 2048),         # int4: two tiles of tokens; int8: the streaming kernel
+    ([17, 1, 1, 1, 1, 1, 1, 1], 2048, 2048),  # int4: 16 rows and one more; int8: the streaming kernel
     ([2, 5, 8], 4608, 128),                 # rows too long for one pass over k
     ([1, 2] * 60, 256, 128),                # a round of tiles ends with its expert, many times per CTA
 ])
@@ -897,6 +897,8 @@ def test_experts_on_the_few_token_kernel(storage, counts, in_dim, hid):
         assert nv.lib().caifq_device_status() == 0
         return out, gate_out, up_out
 
+    ran = {name.split("linear_")[1].split("_kernel")[0] for name, _ in kernels_of(run) if "linear_" in name}
+    assert ran == {"decode" if storage == orc.I4 or max(counts) <= 8 else "stream"}
     out, gate_out, up_out = run()
     g32 = gate_out.float()
     hidden = ((g32 * torch.sigmoid(g32)).bfloat16().float() * up_out.float()).bfloat16()
