@@ -381,6 +381,149 @@ cudaError_t launch_int8_pc(const float *x, int8_t *q, float *scales, int rows, i
   return cudaLaunchKernelEx(&cfg, quantize_int8_pc_kernel<W, THREADS>, x, q, scales, rows, cols, vec);
 }
 
+// Tall tensors.  Eight slices of the rows leave SMs idle or unevenly loaded there, so the rows are cut as often as fills the
+// device.  Column maxima: a block takes 128 columns (a warp one row of them, 16 bytes a lane where rows are aligned) and a
+// slice of the rows; its eight warps' maxima meet in shared memory and go to scales[] as an integer atomicMax, which the caller
+// cleared.  Then a launch for the scales and one for the codes.  Bound by the launches up to 16384 rows or so (13 to 15 us),
+// by reading twice beyond (us, clusters / this: 65536 x 31 42.8 / 23.6, x 256 41 / 30, x 1024 121 / 105; 262144 x 31 160 / 52).
+constexpr int kPcCols = 128;
+
+__global__ void __launch_bounds__(kBlock)
+channel_absmax_kernel(const float *__restrict__ x, float *__restrict__ scales, int rows, int cols, int rows_per_block,
+                      int vec)
+{
+  __shared__ float part[kBlock / 32][kPcCols];
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int c0 = blockIdx.x * kPcCols;
+  const int r_end = min(rows, (static_cast<int>(blockIdx.y) + 1) * rows_per_block);
+  float m[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  constexpr int U = 8;
+  for (int r = static_cast<int>(blockIdx.y) * rows_per_block + warp; r < r_end; r += U * (kBlock / 32))
+  {
+    float4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+    {
+      const int rr = r + u * (kBlock / 32);
+      v[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      if (rr < r_end)
+      {
+        const float *row = x + static_cast<int64_t>(rr) * cols;
+        const int c = c0 + 4 * lane;
+        if (vec)
+        {
+          if (c < cols)
+          {
+            v[u] = *reinterpret_cast<const float4 *>(row + c);
+          }
+        }
+        else
+        {
+          v[u].x = (c + 0 < cols) ? row[c + 0] : 0.0f;
+          v[u].y = (c + 1 < cols) ? row[c + 1] : 0.0f;
+          v[u].z = (c + 2 < cols) ? row[c + 2] : 0.0f;
+          v[u].w = (c + 3 < cols) ? row[c + 3] : 0.0f;
+        }
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+    {
+      m[0] = absmax_step(m[0], v[u].x);
+      m[1] = absmax_step(m[1], v[u].y);
+      m[2] = absmax_step(m[2], v[u].z);
+      m[3] = absmax_step(m[3], v[u].w);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+  {
+    part[warp][4 * lane + i] = m[i];
+  }
+  __syncthreads();
+  if (threadIdx.x < kPcCols && c0 + static_cast<int>(threadIdx.x) < cols)
+  {
+    float best = 0.0f;
+#pragma unroll
+    for (int w = 0; w < kBlock / 32; ++w)
+    {
+      best = fmaxf(best, part[w][threadIdx.x]);
+    }
+    if (best > 0.0f)
+    {
+      atomicMax(reinterpret_cast<int *>(scales) + c0 + threadIdx.x, __float_as_int(best));
+    }
+  }
+}
+
+__global__ void finalize_channel_scales_kernel(float *scales, int cols)
+{
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c < cols)
+  {
+    const float m = scales[c];
+    scales[c] = (m > 0.0f) ? __fdiv_rn(m, 127.0f) : 1.0f;
+  }
+}
+
+// Same shape of work: a lane keeps its columns' reciprocals and takes the rows of its slice, last slices first (they
+// are the ones the maxima's pass left in L2).
+__global__ void __launch_bounds__(kBlock)
+channel_codes_kernel(const float *__restrict__ x, int8_t *__restrict__ q, const float *__restrict__ scales, int rows,
+                        int cols, int rows_per_block, int vec)
+{
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int slice = static_cast<int>(gridDim.y) - 1 - static_cast<int>(blockIdx.y);
+  const int c = blockIdx.x * kPcCols + 4 * lane;
+  const int r_end = min(rows, (slice + 1) * rows_per_block);
+  float inv[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+  {
+    const float s = (c + i < cols) ? scales[c + i] : 0.0f;
+    inv[i] = (s > 0.0f) ? __fdiv_rn(1.0f, s) : 0.0f;
+  }
+  constexpr int U = 4;
+  for (int r = slice * rows_per_block + warp; r < r_end; r += U * (kBlock / 32))
+  {
+    if (vec)
+    {
+      float4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+      {
+        const int rr = r + u * (kBlock / 32);
+        v[u] = (rr < r_end && c < cols) ? __ldcs(reinterpret_cast<const float4 *>(x + static_cast<int64_t>(rr) * cols + c))
+                                        : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+      {
+        const int rr = r + u * (kBlock / 32);
+        if (rr < r_end && c < cols)
+        {
+          *reinterpret_cast<uint32_t *>(q + static_cast<int64_t>(rr) * cols + c) =
+              quant_int8x4(v[u], make_float4(inv[0], inv[1], inv[2], inv[3]));
+        }
+      }
+    }
+    else
+    {
+      for (int u = 0; u < U; ++u)
+      {
+        const int rr = r + u * (kBlock / 32);
+        for (int i = 0; i < 4 && rr < r_end && c + i < cols; ++i)
+        {
+          const int64_t at = static_cast<int64_t>(rr) * cols + c + i;
+          q[at] = static_cast<int8_t>(quant_int8(x[at], inv[i]));
+        }
+      }
+    }
+  }
+}
+
 __global__ void dequantize_int8_pc_kernel(const int8_t *__restrict__ q, float *__restrict__ out,
                                           const float *__restrict__ scales, int64_t total, int cols)
 {
@@ -716,15 +859,47 @@ int launch_quantize_int8_per_channel(const float *x, int8_t *q, float *scales, i
     return CAIFQ_OK;
   }
   const int vec = (cols % 4) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (reinterpret_cast<uintptr_t>(q) & 3u) == 0;
-  // The widest columns that still give every SM two CTAs; where even 32 of them do not, and there are many rows, 16 and twice
-  // the threads (14336 x 512: 27.6 us without)
   auto ctas = [&](int width) { return (cols + width - 1) / width * kPcSlices; };
-  auto launch = launch_int8_pc<32, kBlock>;
-  if (ctas(64) >= 2 * 148)
+  const int sms = device_sm_count();
+  // A cluster's CTA walks an eighth of the rows, 2 to 2.5 ns a row (columns that 16-byte loads cannot read 2 to 5); the tall form
+  // has its launches, 13 to 17 us, and then the whole device's rate.  So the line lies at a number of rows, lower where rows take
+  // longer and where the columns make two to three CTAs of 256 threads an SM, too few loads in flight (us, clusters / tall):
+  //   16384 x 31 13.2 / 15.4, x 256 12.4 / 17.4, x 768 23.6 / 24.6, x 2048 50 / 57; 32768 x 128 18.7 / 17.4, x 1536 89 / 85
+  //   10240 x 1280 25.0 / 27.2, x 1536 26.5 / 29.8; 14336 x 1280 37.5 / 29.9, x 1536 39.6 / 36.6
+  //   off 16 bytes: 4096 x 101 10.7 / 14.4, x 255 11.0 / 17.4; 8192 x 101 17.6 / 14.4; 2048 x 767 14.3 / 16.4, x 1535 13.6 / 19.5;
+  //   4096 x 767 22.8 / 18.4, x 1279 24.3 / 21.7, but 8192 x 4095 76 / 90
+  const bool few_loads = ctas(32) >= 2 * sms - kPcSlices && ctas(32) < 3 * sms;
+  int cluster_rows = few_loads ? 10240 : 16384;
+  if (vec == 0 && cols < 3072)
   {
-    launch = ctas(128) >= 2 * 148 ? launch_int8_pc<128, kBlock> : launch_int8_pc<64, kBlock>;
+    cluster_rows = cols <= 256 ? 4096 : 2048;
   }
-  else if (ctas(32) < 2 * 148 && rows > 1024)
+  if (rows > cluster_rows)
+  {
+    CAIFQ_CHECK_CUDA(cudaMemsetAsync(scales, 0, static_cast<size_t>(cols) * sizeof(float), s));
+    const int col_blocks = (cols + kPcCols - 1) / kPcCols;
+    // about eight blocks per SM over all columns, at least one trip of eight rows a warp each
+    int slices = (sms * 8 + col_blocks - 1) / col_blocks;
+    const int most = static_cast<int>((static_cast<int64_t>(rows) + 63) / 64);
+    slices = slices < most ? slices : most;
+    const int per = static_cast<int>((static_cast<int64_t>(rows) + slices - 1) / slices);
+    const dim3 grid(static_cast<unsigned>(col_blocks), static_cast<unsigned>((static_cast<int64_t>(rows) + per - 1) / per));
+    channel_absmax_kernel<<<grid, kBlock, 0, s>>>(x, scales, rows, cols, per, vec);
+    CAIFQ_CHECK_LAUNCH();
+    finalize_channel_scales_kernel<<<(cols + kBlock - 1) / kBlock, kBlock, 0, s>>>(scales, cols);
+    CAIFQ_CHECK_LAUNCH();
+    channel_codes_kernel<<<grid, kBlock, 0, s>>>(x, q, scales, rows, cols, per, vec);
+    CAIFQ_CHECK_LAUNCH();
+    return CAIFQ_OK;
+  }
+  // The widest columns that still give every SM two CTAs; where even 32 of them do not, and there are many rows, 16 and twice
+  // the threads (14336 x 512: 27.6 us without), as long as all of its clusters run at a time
+  auto launch = launch_int8_pc<32, kBlock>;
+  if (ctas(64) >= 2 * sms)
+  {
+    launch = ctas(128) >= 2 * sms ? launch_int8_pc<128, kBlock> : launch_int8_pc<64, kBlock>;
+  }
+  else if (ctas(32) < 2 * sms - kPcSlices && rows > 1024)
   {
     launch = launch_int8_pc<16, 2 * kBlock>;
   }
