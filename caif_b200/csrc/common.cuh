@@ -33,6 +33,7 @@ void set_path(const char *name);
     cudaError_t err__ = (expr);                                                           \
     if (err__ != cudaSuccess)                                                             \
     {                                                                                     \
+      cudaGetLastError(); /* this call's error is not the next one's */                   \
       ::caifq::set_error("%s failed: %s (%s:%d)", #expr, cudaGetErrorString(err__), __FILE__, __LINE__); \
       return CAIFQ_ERR_CUDA;                                                              \
     }                                                                                     \

@@ -270,3 +270,30 @@ def test_int8_per_channel_of_a_tall_tensor_uses_the_whole_device():
     channel = best_time(lambda: nv.quantize_int8_per_channel(x))
     tensor = best_time(lambda: nv.quantize_int8_per_tensor(x))
     assert channel < 7.0 * tensor, (channel, tensor)
+
+
+def test_a_launch_that_was_refused_leaves_no_error_behind():
+    """A launch into a capture that something else has broken fails on the host; the next call is none the worse."""
+    import ctypes
+
+    rt = ctypes.CDLL("libcudart.so.12")
+    lib = nv.lib()
+    x = torch.randn(4096, device="cuda")
+    y = torch.empty(4096, dtype=torch.bfloat16, device="cuda")
+    packed = torch.empty(2048, dtype=torch.uint8, device="cuda")
+    scales = torch.empty(32, dtype=torch.float16, device="cuda")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    raw = ctypes.c_void_p(stream.cuda_stream)
+    assert rt.cudaStreamBeginCapture(raw, 0) == 0                       # the mode that forbids allocations meanwhile
+    p = ctypes.c_void_p()
+    assert rt.cudaMalloc(ctypes.byref(p), ctypes.c_size_t(256)) != 0    # and with one the capture is void
+    rc = lib.caifq_cast(x.data_ptr(), nv.F32, y.data_ptr(), nv.BF16, x.numel(), stream.cuda_stream)
+    graph = ctypes.c_void_p()
+    rt.cudaStreamEndCapture(raw, ctypes.byref(graph))
+    rt.cudaGetLastError()
+    assert rc != 0
+    here = torch.cuda.current_stream().cuda_stream
+    assert lib.caifq_quantize_int4_per_group(x.data_ptr(), packed.data_ptr(), scales.data_ptr(), x.numel(), 128, here) == 0
+    assert lib.caifq_cast(x.data_ptr(), nv.F32, y.data_ptr(), nv.BF16, x.numel(), here) == 0
+    assert torch.equal(y, x.bfloat16())
