@@ -93,3 +93,19 @@ def test_rmsnorm_rows_in_registers_match_the_element_kernels(dtype, rows, dim):
         dx2, dg2 = nv.rmsnorm_bwd(shifted(dy), shifted(x), gamma, rms)
         assert torch.equal(dx, dx2)
         assert float((dg - dg2).abs().max()) <= 1e-4 * float(dg2.abs().max())
+
+
+@pytest.mark.parametrize("dim", [6016, 6017, 6143, 6144, 6145])
+def test_rmsnorm_backward_of_rows_that_just_fill_the_shared_memory(dim):
+    """Two fp32 rows of 6144 are 48 KB, what a launch has without asking, beside the kernel's own few words: against the
+    oracle, bit for bit."""
+    rows, eps = 5, 1e-5
+    g = torch.Generator(device="cuda").manual_seed(dim)
+    x, dy = (torch.randn(rows, dim, generator=g, device="cuda") for _ in range(2))
+    gamma = 1.0 + 0.1 * torch.randn(dim, generator=g, device="cuda")
+    f = lambda t: t.cpu().numpy()
+    _, rms = nv.rmsnorm_fwd(x, gamma, eps)
+    dx, gg = nv.rmsnorm_bwd(dy, x, gamma, rms)
+    o_dx, o_gg = orc.rmsnorm_backward(f(dy), f(x), f(gamma), f(rms), orc.F32)
+    assert np.array_equal(f(dx), o_dx)
+    assert np.max(np.abs(f(gg) - o_gg)) <= 1e-4 * max(1.0, float(np.max(np.abs(o_gg))))
