@@ -1471,11 +1471,12 @@ static bool few_rows(int num_experts, const int32_t *offsets, int dtype)
          static_cast<int64_t>(offsets[num_experts]) <= static_cast<int64_t>(kFewRowsPerExpert) * num_experts;
 }
 
-// Whether the few-token kernel, 16 rows at a time, is the faster one for these entries.  Up to 8 rows it is, for all widths
-// measured (us for the three products of an expert layer, this kernel / the streaming one, 8 rows each: int4 2944 x 1280 74 /
-// 98, 4096 x 2048 63 / 106, 1536 squared 29 / 39, 1024 x 512 40 / 39; int8 93 / 93, 78 / 103, 36 / 38, 36 / 36).  From 9 rows
-// on a second tile of tokens doubles its MMAs: int4 4096 x 2048 89 / 106, 2048 x 1408 115 / 139, but 104 / 98 and 55 / 40 where
-// k is not a multiple of what its eight warps take at a time; int8 104 / 103 at best.
+// Whether the few-token kernel, 16 rows at a time, is the one for these entries (entries of more rows are taken 16 at a time, their
+// codes read again).  Up to 8 rows it is the faster one or as fast (us for the three products of an expert layer, this kernel /
+// the streaming one, 8 rows each: int4 2944 x 1280 74 / 98, 4096 x 2048 61 / 109, 1536 squared 29 / 39, 1024 x 512 25 / 29; int8
+// 93 / 93, 78 / 107, 36 / 38, 21 / 25).  From 9 rows on a second tile of tokens doubles its MMAs: int4 4096 x 2048 88 / 109,
+// 2048 x 1408 117 / 142, but 104 / 98 and 55 / 40 where k is not a multiple of what its eight warps take at a time; int8 104 /
+// 103 at best, which the kernel does not take.
 static bool few_tokens_each(const GroupedStreamArgs &g)
 {
   int64_t live = 0;

@@ -25,8 +25,8 @@
 //   * each warp parks its partial sums of every tile (live tokens only) in shared
 //     memory, and one pass at the end adds the warps' partials of each output in a
 //     fixed order; consecutive lanes store consecutive rows of a token.
-// Experts that see up to 16 rows each are the same product over a table of code matrices (the expert loop,
-// src/caif_device_moe_layer.cpp:534-557): two CTAs of eight warps an SM, each with hundreds of weight rows; a round of
+// Experts that see few rows each are the same product over a table of code matrices (the expert loop,
+// src/caif_device_moe_layer.cpp:534-557), up to 16 rows an entry (int8: 8), an expert of more being several entries: two CTAs of eight warps an SM, each with hundreds of weight rows; a round of
 // tiles ends with its expert, and the next one's activations are awaited while the other CTA works.  Bound by the
 // conversion and by the rounds' ends: 64 experts of 2048 x 1408 int4, 16 tokens top-6, three products 65 us (the
 // streaming kernel 113, HBM 34).

@@ -705,7 +705,8 @@ int launch_f32_inst(F32Params p, cudaStream_t s)
   const unsigned mt = static_cast<unsigned>((p.m + tile - 1) / tile);
   // k is split until the SMs hold two CTAs each, as long as a CTA keeps two blocks of 64 to overlap; the smaller tile's CTAs
   // are cheaper to have fewer of (4096 -> 4096, one row: 17.5 us with four a tile, 19.6 with eight)
-  const int64_t fill = few ? 148 : 2 * 148 - 1;
+  const int sms = device_sm_count();
+  const int64_t fill = few ? sms : 2 * sms - 1;
   p.splits = 1;
   while (p.splits < 8 && static_cast<int64_t>(nt) * mt * p.splits <= fill && p.k_total / 64 >= 4 * p.splits)
   {
@@ -727,7 +728,7 @@ int launch_f32_inst(F32Params p, cudaStream_t s)
   // codes written just ahead in this stream by one of the library's own calls: a plain launch orders the early loads
   // behind that kernel.  64-row tiles of more CTAs than SMs are launched plainly too: while the previous kernel still has
   // its SMs the others get two CTAs each (3712 <- 768, 64 rows, 232 CTAs: 11.1 us, plainly 9.8).
-  const bool dependent = dependent_launches() && !take_codes_written(s) && (few || static_cast<int64_t>(nt) * mt * p.splits <= 148);
+  const bool dependent = dependent_launches() && !take_codes_written(s) && (few || static_cast<int64_t>(nt) * mt * p.splits <= sms);
   cfg.numAttrs = dependent ? 2 : 1;
   CAIFQ_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, p));
   return CAIFQ_OK;

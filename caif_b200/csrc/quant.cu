@@ -52,7 +52,7 @@ __device__ __forceinline__ float clamp_sym(float v, float lim)
 // ---------------------------------------------------------------- int8 / tensor
 
 // Three launches, each placed while the one before it still runs: the blocks' maxima, the scale, the codes.  Small and
-// middling tensors are bound by the launches (us, a cleared scale, atomic maxima and plain launches / now: 309 x 768 12.1 / 8.5,
+// middling tensors are bound by the launches (us, a cleared scale, atomic maxima and plain launches / now: 309 x 768 12.1 / 7.3,
 // 2000 x 4096 18.5 / 12.5, 14336 x 4096 84 / 80).  The maxima lie where the codes will: the caller has no scratch.
 __device__ __forceinline__ void after_previous_kernel()
 {

@@ -317,9 +317,9 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b)
 // bf16, one rounding.  The reference's dequantize-then-cast forms scale * code in fp32 and rounds once;
 // the two differ by the bf16 rounding of the fp16 scale (2^-9 relative), far inside the bf16 bound, and
 // the conversion takes 17 instructions per eight weights instead of 31: the int4 launches are bound by
-// this conversion, not by the tensor core.  One asm block: apart, the compiler put three moves in between
-// (1.0 -> 0.87 of the time in a loop of conversions and tensor-memory stores; 4096 -> 14336, 96 tokens,
-// 20.9 -> 20.8 us; 4096 -> 4096, 48 tokens, 11.2 -> 11.1).
+// this conversion, not by the tensor core.  One asm block: a loop of conversions and tensor-memory stores takes
+// 53.2 us, with the same steps as C++ and single instructions 62.4 (4096 -> 14336, 96 tokens, 20.9 -> 20.8 us;
+// 4096 -> 4096, 48 tokens, 11.2 -> 11.1).
 __device__ __forceinline__ void int4x8_to_bf16(uint32_t w, uint32_t scale2, uint32_t (&out)[4])
 {
   // e: u0 u2 u4 u6 (u = q + 8), d: u1 u3 u5 u7; t, v: in element order; 0x43: the high byte of bf16 128.0 .. 143.0

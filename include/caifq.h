@@ -116,7 +116,9 @@ CAIFQ_API void caifq_selftest_stall_next_umma(void);
  * collectives (NCCL) beside them on another stream caps their grids with this call so that the
  * collective's CTAs find SMs of their own; a persistent CTA that finds its SM taken would wait for
  * the whole collective.  max_ctas <= 0 restores one CTA per SM.  Process-wide; applies to launches
- * made after the call.  (No counterpart in the reference, which is single-device.)
+ * made after the call.  Under a limit the products of experts that see few rows run on the streaming
+ * kernel, whose int4 weights are rounded to bf16 (the few-token kernel takes two CTAs per SM for them).
+ * (No counterpart in the reference, which is single-device.)
  */
 CAIFQ_API void caifq_set_cta_limit(int32_t max_ctas);
 /* The tensor-core kernel runs 256-wide tiles on pairs of CTAs (two SMs of one cluster).  Returns how many
@@ -241,7 +243,9 @@ CAIFQ_API int caifq_linear_fwd_multi(const caifq_weight *ws, int32_t num_weights
                                      int64_t m, void *y, int32_t y_dtype, int32_t compute_dtype, void *stream);
 
 /* Name of the kernel family the last caifq_linear_fwd / caifq_linear_dx call
- * on this thread chose ("decode", "umma", "generic"); for tests and reports. */
+ * on this thread chose ("decode", "umma", "generic"); for tests and reports.
+ * Calls for a run of experts report "umma-grouped" for launches over all of them,
+ * whichever kernel these were (experts of few rows: the few-token or the streaming one). */
 CAIFQ_API const char *caifq_last_path(void);
 
 /* ---- LoRA on a frozen linear --------------------------------------------- */

@@ -988,7 +988,7 @@ def test_lora_operands_that_start_on_any_element():
 
 @pytest.mark.parametrize("dtype,dim", [(torch.bfloat16, 2048), (torch.float32, 1024)])
 def test_combine_of_many_and_of_few_tokens(dtype, dim):
-    """More pieces than one trip of the grid read the rows as constants; fewer are a dependent launch: the same bits.
+    """Many pieces are read through the read-only path, few are not: the same bits.
     Against x times its weights: one rounding of bf16 (2^-9), and of fp32 sums in another order."""
     tokens, experts, top_k = 2369, 8, 2
     g = torch.Generator().manual_seed(23)
