@@ -34,22 +34,23 @@ __device__ __forceinline__ __half from_f<__half>(float v) { return __float2half(
 template <>
 __device__ __forceinline__ __nv_bfloat16 from_f<__nv_bfloat16>(float v) { return __float2bfloat16(v); }
 
-// The small kernels of a step follow one another: each is launched ahead of the previous one's end (launch_dependent),
-// lets the next one do the same, and reads nothing before the previous one has ended.  (Their inputs are not declared
-// __restrict__: loads that the compiler may take for invariant could move ahead of the wait.)
-// `most`: CTAs of a grid that lets the next one in at once.  CTAs that are placed beside those of a larger grid take what
-// room is left, two on one SM and none on another, and keep it for as long as they run; after such a grid the next one
-// follows as its CTAs end.  Two grids of half the SMs have an SM for every CTA.  (us a launch, back to back, next one in at
-// once / as the CTAs end: rows of 14 KB, 96 CTAs 6.3 / 4.3, 256 CTAs 17.4 / 6.5, 450 CTAs 18.9 / 10.4; softmax of 256, 128 CTAs
-// 6.2 / 5.5, 256 CTAs 12.4 / 5.8; top-8 of 256, 256 CTAs 11.5 / 4.7; the map, 128 CTAs 18.6 / 13.5.)
-constexpr unsigned kEarlyCtas = 74;
-__device__ __forceinline__ void after_previous_kernel(unsigned most = 0xFFFFFFFFu)
+// The small kernels of a step follow one another: each is launched ahead of the previous one's end (launch_dependent) and reads
+// nothing before that one has ended.  (Their inputs are not declared __restrict__: loads that the compiler may take for
+// invariant could move ahead of the wait.)
+// Letting the next one in early as well pays where it has something to do before its own wait: the experts' products, which
+// copy codes, after dispatch and SwiGLU.  Elsewhere it costs: CTAs that are placed beside those of a running grid take what room
+// is left, two on one SM and none on another, and keep it for as long as they run.  (us a launch, back to back, next one in at
+// once / as the CTAs end: rows of 14 KB, 96 CTAs 6.3 / 4.3, 256 CTAs 17.4 / 6.5; softmax of 256, 256 CTAs 12.4 / 5.8; top-8 of
+// 256, 256 CTAs 11.5 / 4.7; the map, 128 CTAs 18.6 / 13.5; all steps for 400 tokens top-8 of 256, rows of 2048, 32.3 / 25.9, for
+// 1024 43.8 / 31.7.  An expert layer of 16 tokens is 0.8 slower where dispatch does not let the products in.)
+constexpr unsigned kEarlyCtas = 37;   // CTAs of a dispatch that leave the products three SMs of four
+__device__ __forceinline__ void after_previous_kernel()
 {
-  if (gridDim.x <= most)
-  {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  }
   asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+__device__ __forceinline__ void let_next_kernel_in()
+{
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // ------------------------------------------------------------------------ top-k
@@ -61,7 +62,7 @@ template <typename T>
 __global__ void topk_kernel(const T *input, int *indices, T *values,
                             int batch, int dim, int k)
 {
-  after_previous_kernel(kEarlyCtas);
+  after_previous_kernel();
   extern __shared__ float s_rows[];
   const int warps_per_block = blockDim.x >> 5;
   const int warp = threadIdx.x >> 5;
@@ -343,7 +344,7 @@ __device__ __forceinline__ void softmax_absorb(float &m, float &s, float m_other
 template <typename T>
 __global__ void router_softmax_kernel(const T *logits, const T *bias, T *probs, int rows, int cols)
 {
-  after_previous_kernel(kEarlyCtas);
+  after_previous_kernel();
   const int warps_per_block = blockDim.x >> 5;
   const int lane = threadIdx.x & 31;
   const int row = blockIdx.x * warps_per_block + (threadIdx.x >> 5);
@@ -752,7 +753,7 @@ __global__ void __launch_bounds__(kMapThreads)
 build_dispatch_kernel(const int *expert_indices, int64_t total, int64_t slice, int num_experts, int capacity,
                       int *dispatch_map, int *expert_offsets)
 {
-  after_previous_kernel(kEarlyCtas);
+  after_previous_kernel();
   extern __shared__ int s_map[];
   int *running = s_map;                      // [E]
   int *warp_hist = s_map + num_experts;      // [warps][E]
@@ -891,7 +892,11 @@ template <typename T>
 __global__ void moe_dispatch_kernel(const T *input, const int *expert_indices, const int *dispatch_map,
                                     const int *expert_offsets, T *buffer, int64_t assignments, int dim, int top_k)
 {
-  after_previous_kernel(kEarlyCtas);
+  if (gridDim.x <= kEarlyCtas)
+  {
+    let_next_kernel_in();
+  }
+  after_previous_kernel();
   const int lane = threadIdx.x & 31;
   const int64_t a = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   if (a >= assignments)
@@ -943,6 +948,7 @@ __global__ void moe_combine_kernel(const T *buffer, const int *expert_indices, c
                                    const int *dispatch_map, const int *expert_offsets, T *output, int num_tokens,
                                    int dim, int top_k)
 {
+  let_next_kernel_in();
   after_previous_kernel();
   const int64_t total = static_cast<int64_t>(num_tokens) * dim;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -971,6 +977,7 @@ template <typename T>
 __global__ void swiglu_fwd_kernel(const T *gate, const T *up, T *hidden,
                                   int64_t n)
 {
+  let_next_kernel_in();
   after_previous_kernel();
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
   for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride)
@@ -1071,6 +1078,7 @@ __device__ __forceinline__ void store_vec(T *p, const float (&v)[Vec16<T>::N])
 template <typename T>
 __global__ void swiglu_fwd_vec_kernel(const T *gate, const T *up, T *hidden, int64_t n_vec)
 {
+  let_next_kernel_in();
   after_previous_kernel();
   constexpr int N = Vec16<T>::N;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
@@ -1123,7 +1131,7 @@ __global__ void moe_combine_vec_kernel(const T *buffer, const int *expert_indice
                                        const int *dispatch_map, const int *expert_offsets, T *output, int num_tokens,
                                        int dim, int top_k)
 {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  let_next_kernel_in();
   asm volatile("griddepcontrol.wait;" : "+l"(buffer)::"memory");
   constexpr int N = Vec16<T>::N;
   const int dim_vec = dim / N;

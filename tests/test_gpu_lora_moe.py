@@ -1065,10 +1065,8 @@ def _route(tokens, experts, top_k, dim, seed):
 
 
 @pytest.mark.parametrize("tokens,experts,top_k", [
-    (296, 8, 2), (297, 8, 2),            # 592 rows are dispatched by 74 CTAs, 594 by one more
-    (592, 16, 1), (593, 16, 1),          # the same for the softmax and top-k
-    (1184, 16, 1),
-    (74 * 512, 8, 2), (74 * 512 + 1, 8, 2),   # the map's 74 CTAs of 1024 entries, and one more
+    (148, 8, 2), (149, 8, 2),            # 296 rows are dispatched by 37 CTAs, which let the next kernel in at once, 298 by one more
+    (1, 8, 2), (593, 16, 1), (74 * 512 + 1, 8, 2),
 ])
 def test_routing_steps_follow_one_another(tokens, experts, top_k):
     """The steps of a routed layer back to back, twice, give the bits that they give one at a time: grids that let the next
