@@ -34,9 +34,9 @@ __device__ __forceinline__ void mma_rows(float (&c)[4], uint32_t a0, uint32_t a1
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// CHAINS: chains whose loads are in flight at a time per warp
-template <int NT, int CHAINS>
-__global__ void __launch_bounds__(kRowsWarps * 32)
+// CHAINS: chains whose loads are in flight at a time per warp; CTAS: that an SM must hold, which bounds the registers (0: any)
+template <int NT, int CHAINS, int CTAS>
+__global__ void __launch_bounds__(kRowsWarps * 32, CTAS)
 linear_rows_kernel(const __nv_bfloat16 *x, const __nv_bfloat16 *w, void *y, int y_dtype, int accumulate, int64_t m,
                    int in_dim, int out_dim)
 {
@@ -173,8 +173,15 @@ int launch_linear_rows(const LinearArgs &g, cudaStream_t s)
   const int wide = (g.w.out_dim + 31) / 32;
   const bool many = wide * row_tiles >= sms;
   const dim3 grid(static_cast<unsigned>(many ? wide : (g.w.out_dim + 7) / 8), row_tiles);
-  const bool one_wave = grid.x * grid.y <= 3u * static_cast<unsigned>(sms);
-  auto kernel = many ? linear_rows_kernel<4, 1> : (one_wave ? linear_rows_kernel<1, 2> : linear_rows_kernel<1, 1>);
+  const unsigned ctas = grid.x * grid.y;
+  const bool three = ctas <= 3u * static_cast<unsigned>(sms);
+  // 32 columns: 112 registers and two CTAs an SM, except where 80 and three make one wave of what two do not, of rows that share
+  // the weight, and where a warp has one trip (us, two / three: 4096 -> 4704, 48 rows 19.1 / 16.9; 14336 -> 3552, 64 rows 89 / 76; 512 ->
+  // 1192, 2048 rows 44 / 42; but 4096 -> 9504, 32 rows 30.5 / 35.8; 2048 -> 264, 2048 rows 22 / 26)
+  const bool dense = ctas > 2u * static_cast<unsigned>(sms) &&
+                     ((three && row_tiles > 2) || g.w.in_dim <= kRowsWarps * kRowsChain * 32);
+  auto wide_kernel = dense ? linear_rows_kernel<4, 1, 3> : linear_rows_kernel<4, 1, 0>;
+  auto kernel = many ? wide_kernel : (three ? linear_rows_kernel<1, 2, 0> : linear_rows_kernel<1, 1, 0>);
   CAIFQ_CHECK_CUDA(launch_dependent(kernel, grid, dim3(kRowsWarps * 32), 0, s, x, w, g.c, g.c_dtype, acc, g.m, g.w.in_dim,
                                     g.w.out_dim));
   return CAIFQ_OK;

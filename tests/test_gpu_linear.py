@@ -955,11 +955,11 @@ def test_products_see_what_was_just_written(reader, writer):
     assert not torch.equal(before, want)
 
 
-@pytest.mark.parametrize("m", [1, 16, 17])
-@pytest.mark.parametrize("out_dim", [1176, 3544, 3552, 3553, 3560, 4712, 4737])
+@pytest.mark.parametrize("m", [1, 16, 17, 33, 48, 65])
+@pytest.mark.parametrize("out_dim", [1176, 3144, 3176, 3544, 3552, 3553, 3560, 4712, 4737])
 def test_bf16_weight_either_side_of_a_resident_wave(m, out_dim):
     """147, 443 to 445 and 589 CTAs of 8 columns (two chains' loads at a time while three CTAs an SM take them all), and 32
-    columns a CTA beyond.  Bound: products are exact, an fp32 sum of chains of 128 is within 1e-6 of the norm."""
+    columns a CTA beyond, fewer registers from two CTAs an SM to three with three tiles of rows (3144 and 3176: 297 and 300).  Bound: products are exact, an fp32 sum of chains of 128 is within 1e-6 of the norm."""
     in_dim = 544       # 17 steps of 32: warps of two and of three
     g = torch.Generator(device="cuda").manual_seed(out_dim + m)
     w = torch.randn(out_dim, in_dim, generator=g, device="cuda").bfloat16()
